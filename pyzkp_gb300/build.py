@@ -59,7 +59,7 @@ def _compile(src: str, extra: List[str], obj_dir: str) -> str:
 
 
 def build(force: bool = False, verbose_ptxas: bool = False, defines: List[str] = (), lib_path: str = "") -> str:
-    """Compile and link; ``defines`` (e.g. ["ZK_MUL_STYLE=1"]) build a variant into ``lib_path``."""
+    """Compile and link; ``defines`` (e.g. ["ZK_MSM_SEGMENT=24"]) build a variant into ``lib_path``."""
     obj_dir, out_path = OBJ_DIR, LIB_PATH
     if defines or lib_path:
         tag = "_".join(d.replace("=", "") for d in defines) or "custom"

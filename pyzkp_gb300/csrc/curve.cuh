@@ -44,11 +44,9 @@ struct c_pair {
     T x, y;
 };
 
-// Two independent products; for Fq they go through fe_mul2 (one interleaved pair when
-// ZK_USE_MUL2 is set).
+// Two independent products.
 __device__ __forceinline__ c_pair<fe> c_mul2(const fe& a, const fe& b, const fe& c, const fe& d) {
-    const fe2 r = fe_mul2<FqP>(a, b, c, d);
-    return {r.x, r.y};
+    return {c_mul(a, b), c_mul(c, d)};
 }
 
 __device__ __forceinline__ fq2 c_add(const fq2& a, const fq2& b) { return {c_add(a.c0, b.c0), c_add(a.c1, b.c1)}; }
@@ -188,8 +186,7 @@ __device__ __forceinline__ XyzzT<T> xyzz_neg(const XyzzT<T>& p) {
     return r;
 }
 
-// The formulas below issue their multiplications in independent pairs (c_mul2), so the
-// two carry-chain sequences of a pair can overlap.
+// The formulas below list their independent multiplications in pairs (c_mul2).
 
 // 2 * (x, y) for an affine point that is not infinity (y != 0 on these curves).
 template <class T>

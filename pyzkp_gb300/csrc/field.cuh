@@ -5,14 +5,12 @@
 // runtime/metal/ecc_source.py:14-25 hold the same moduli), so the bytes of a device
 // element are the bytes of the reference's "fr_mont_u64x4" element.
 //
-// Multiplication is CIOS (coarsely integrated operand scanning): per limb b_i of
-// the multiplier, one carry chain adds the low halves a_j*b_i into t_j and one adds
-// the high halves into t_{j+1}; then m = t_0 * (-p^-1) and two chains add m*p and
-// shift one limb. Every carry chain is one inline-PTX block (mad.lo.cc / madc.hi.cc
-// map to IMAD with carry in/out), so carries stay in the condition-code register.
-// Both moduli are below 2^254, so the running value stays below 2^288 (9 limbs)
-// and below 2p after each row; one conditional subtraction yields the canonical
-// representative in [0, p).
+// Multiplication is CIOS (coarsely integrated operand scanning): per limb b_i of the
+// multiplier, T += a b_i, then T += m p with m = t_0 (-p^-1), and one limb is shifted out.
+// Both moduli are below 2^254, so the running value stays below 2^288 (9 limbs) and the
+// result below 2p for inputs below 2p; one conditional subtraction yields the canonical
+// representative in [0, p). How a row maps to wide multiply-adds, and what bounds it, is at
+// the products below.
 //
 // Fr values are always fully reduced (equal values have equal bits: NTT outputs are
 // stored and compared). Fq values inside the curve formulas are kept "lazy", in [0, 2p)
@@ -30,7 +28,7 @@ namespace zk {
 struct FrP {
     __host__ __device__ static constexpr uint32_t P(int i) { return i == 0 ? 0xf0000001u : i == 1 ? 0x43e1f593u : i == 2 ? 0x79b97091u : i == 3 ? 0x2833e848u : i == 4 ? 0x8181585du : i == 5 ? 0xb85045b6u : i == 6 ? 0xe131a029u : 0x30644e72u; }
     static constexpr uint32_t INV = 0xefffffffu  /* -r^-1 mod 2^32 */;
-    static constexpr int MUL_STYLE = 4;
+    static constexpr bool CALL_MUL = false;
     static constexpr bool LAZY = false;
     __host__ __device__ static constexpr uint32_t ONE(int i) { return i == 0 ? 0x4ffffffbu : i == 1 ? 0xac96341cu : i == 2 ? 0x9f60cd29u : i == 3 ? 0x36fc7695u : i == 4 ? 0x7879462eu : i == 5 ? 0x666ea36fu : i == 6 ? 0x9a07df2fu : 0x0e0a77c1u; }
     __host__ __device__ static constexpr uint32_t R2(int i) { return i == 0 ? 0xae216da7u : i == 1 ? 0x1bb8e645u : i == 2 ? 0xe35c59e3u : i == 3 ? 0x53fe3ab1u : i == 4 ? 0x53bb8085u : i == 5 ? 0x8c49833du : i == 6 ? 0x7f4e44a5u : 0x0216d0b1u; }
@@ -39,7 +37,7 @@ struct FrP {
 struct FqP {
     __host__ __device__ static constexpr uint32_t P(int i) { return i == 0 ? 0xd87cfd47u : i == 1 ? 0x3c208c16u : i == 2 ? 0x6871ca8du : i == 3 ? 0x97816a91u : i == 4 ? 0x8181585du : i == 5 ? 0xb85045b6u : i == 6 ? 0xe131a029u : 0x30644e72u; }
     static constexpr uint32_t INV = 0xe4866389u  /* -q^-1 mod 2^32 */;
-    static constexpr int MUL_STYLE = 3;
+    static constexpr bool CALL_MUL = true;
 #ifdef ZK_FQ_STRICT
     static constexpr bool LAZY = false;
 #else
@@ -70,7 +68,7 @@ struct FrLazyP : FrP {
 // Fr with one non-inlined copy of the product, for kernels whose loop bodies hold many
 // products (inlined, they overflow the instruction cache).
 struct FrCallP : FrP {
-    static constexpr int MUL_STYLE = 3;
+    static constexpr bool CALL_MUL = true;
 };
 
 // One field element: 8 little-endian 32-bit limbs (32 bytes, 32-byte aligned in memory).
@@ -285,456 +283,7 @@ __device__ __forceinline__ fe fe_dbl(const fe& a) {
     return fe_add<F>(a, a);
 }
 
-// One CIOS row: t += a * bi, then t += m * p with m = t0 * (-p^-1), then shift one limb.
-#define ZK_MUL_ROW(F, bi)                                                                                      \
-    do {                                                                                                       \
-        asm("mad.lo.cc.u32  %0, %9, %17, %0;\n\t"                                                              \
-            "madc.lo.cc.u32 %1, %10, %17, %1;\n\t"                                                             \
-            "madc.lo.cc.u32 %2, %11, %17, %2;\n\t"                                                             \
-            "madc.lo.cc.u32 %3, %12, %17, %3;\n\t"                                                             \
-            "madc.lo.cc.u32 %4, %13, %17, %4;\n\t"                                                             \
-            "madc.lo.cc.u32 %5, %14, %17, %5;\n\t"                                                             \
-            "madc.lo.cc.u32 %6, %15, %17, %6;\n\t"                                                             \
-            "madc.lo.cc.u32 %7, %16, %17, %7;\n\t"                                                             \
-            "addc.u32       %8, %8, 0;"                                                                        \
-            : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)        \
-            : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]),      \
-              "r"(a.v[7]), "r"(bi));                                                                           \
-        asm("mad.hi.cc.u32  %0, %8, %16, %0;\n\t"                                                              \
-            "madc.hi.cc.u32 %1, %9, %16, %1;\n\t"                                                              \
-            "madc.hi.cc.u32 %2, %10, %16, %2;\n\t"                                                             \
-            "madc.hi.cc.u32 %3, %11, %16, %3;\n\t"                                                             \
-            "madc.hi.cc.u32 %4, %12, %16, %4;\n\t"                                                             \
-            "madc.hi.cc.u32 %5, %13, %16, %5;\n\t"                                                             \
-            "madc.hi.cc.u32 %6, %14, %16, %6;\n\t"                                                             \
-            "madc.hi.u32    %7, %15, %16, %7;"                                                                 \
-            : "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)                   \
-            : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]),      \
-              "r"(a.v[7]), "r"(bi));                                                                           \
-        const uint32_t m_ = t0 * F::INV;                                                                       \
-        asm("mad.lo.cc.u32  %0, %9, %10, %0;\n\t"                                                              \
-            "madc.lo.cc.u32 %1, %9, %11, %1;\n\t"                                                              \
-            "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"                                                              \
-            "madc.lo.cc.u32 %3, %9, %13, %3;\n\t"                                                              \
-            "madc.lo.cc.u32 %4, %9, %14, %4;\n\t"                                                              \
-            "madc.lo.cc.u32 %5, %9, %15, %5;\n\t"                                                              \
-            "madc.lo.cc.u32 %6, %9, %16, %6;\n\t"                                                              \
-            "madc.lo.cc.u32 %7, %9, %17, %7;\n\t"                                                              \
-            "addc.u32       %8, %8, 0;"                                                                        \
-            : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)        \
-            : "r"(m_), "n"(F::P(0)), "n"(F::P(1)), "n"(F::P(2)), "n"(F::P(3)), "n"(F::P(4)), "n"(F::P(5)),   \
-              "n"(F::P(6)), "n"(F::P(7)));                                                                     \
-        asm("mad.hi.cc.u32  %0, %8, %9, %0;\n\t"                                                               \
-            "madc.hi.cc.u32 %1, %8, %10, %1;\n\t"                                                              \
-            "madc.hi.cc.u32 %2, %8, %11, %2;\n\t"                                                              \
-            "madc.hi.cc.u32 %3, %8, %12, %3;\n\t"                                                              \
-            "madc.hi.cc.u32 %4, %8, %13, %4;\n\t"                                                              \
-            "madc.hi.cc.u32 %5, %8, %14, %5;\n\t"                                                              \
-            "madc.hi.cc.u32 %6, %8, %15, %6;\n\t"                                                              \
-            "madc.hi.u32    %7, %8, %16, %7;"                                                                  \
-            : "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)                   \
-            : "r"(m_), "n"(F::P(0)), "n"(F::P(1)), "n"(F::P(2)), "n"(F::P(3)), "n"(F::P(4)), "n"(F::P(5)),   \
-              "n"(F::P(6)), "n"(F::P(7)));                                                                     \
-        t0 = t1;                                                                                               \
-        t1 = t2;                                                                                               \
-        t2 = t3;                                                                                               \
-        t3 = t4;                                                                                               \
-        t4 = t5;                                                                                               \
-        t5 = t6;                                                                                               \
-        t6 = t7;                                                                                               \
-        t7 = t8;                                                                                               \
-        t8 = 0;                                                                                                \
-    } while (0)
-
-// Code-size strategy of the multiplication, per field (F::MUL_STYLE; ZK_MUL_STYLE overrides
-// both at compile time for measurements):
-//   0: the 8 rows fully unrolled and inlined at every call site (largest code);
-//   1: one non-inlined copy of the unrolled body, called from every site;
-//   2: inlined, but the row loop kept rolled (b's limbs rotate through one register);
-//   3: like 1 on full-width products (fe_mul_wide_unrolled: mul.wide + add chains);
-//   4: like 0 on full-width products.
-// The curve formulas hold 10-14 multiplications per loop body, so inlining them all
-// overflows the instruction cache (the MSM accumulation stalled on "no instruction");
-// measured on GB300 at n = 2^20: MSM 125 / 160 / 147 / 179 / 143 Mpts/s and 2^22 NTT
-// 3013 / 2966 / 2643 / 3098 / 3136 Melem/s for styles 0 / 1 / 2 / 3 / 4.
-// Fq (curve) uses 3, Fr (NTT butterflies) uses 4.
-
-template <class F>
-__device__ __forceinline__ fe fe_mul_unrolled(const fe& a, const fe& b) {
-    uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0, t6 = 0, t7 = 0, t8 = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) ZK_MUL_ROW(F, b.v[i]);
-    fe t;
-    t.v[0] = t0;
-    t.v[1] = t1;
-    t.v[2] = t2;
-    t.v[3] = t3;
-    t.v[4] = t4;
-    t.v[5] = t5;
-    t.v[6] = t6;
-    t.v[7] = t7;
-    if constexpr (F::LAZY) return t;
-    else return fe_reduce_once<F>(t);
-}
-
-template <class F>
-__device__ __forceinline__ fe fe_mul_rolled(const fe& a, const fe& b) {
-    uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0, t6 = 0, t7 = 0, t8 = 0;
-    uint32_t b0 = b.v[0], b1 = b.v[1], b2 = b.v[2], b3 = b.v[3], b4 = b.v[4], b5 = b.v[5], b6 = b.v[6],
-             b7 = b.v[7];
-#pragma unroll 1
-    for (int i = 0; i < 8; i++) {
-        ZK_MUL_ROW(F, b0);
-        b0 = b1;
-        b1 = b2;
-        b2 = b3;
-        b3 = b4;
-        b4 = b5;
-        b5 = b6;
-        b6 = b7;
-    }
-    fe t;
-    t.v[0] = t0;
-    t.v[1] = t1;
-    t.v[2] = t2;
-    t.v[3] = t3;
-    t.v[4] = t4;
-    t.v[5] = t5;
-    t.v[6] = t6;
-    t.v[7] = t7;
-    if constexpr (F::LAZY) return t;
-    else return fe_reduce_once<F>(t);
-}
-
-// CIOS on full-width products: mul.wide.u32 (IMAD.WIDE) yields lo and hi of a_j * b_i
-// in one instruction -- measured on GB300 at twice the rate of a mad.lo + mad.hi pair,
-// whose hi half issues at half rate -- and two add-with-carry chains fold the halves
-// into t (lo(P_j) into t_j, hi(P_j) into t_{j+1}). Same bounds as ZK_MUL_ROW.
-#define ZK_ADD_LO_CHAIN(p0, p1, p2, p3, p4, p5, p6, p7)                                                         \
-    asm("add.cc.u32  %0, %0, %9;\n\t"                                                                          \
-        "addc.cc.u32 %1, %1, %10;\n\t"                                                                         \
-        "addc.cc.u32 %2, %2, %11;\n\t"                                                                         \
-        "addc.cc.u32 %3, %3, %12;\n\t"                                                                         \
-        "addc.cc.u32 %4, %4, %13;\n\t"                                                                         \
-        "addc.cc.u32 %5, %5, %14;\n\t"                                                                         \
-        "addc.cc.u32 %6, %6, %15;\n\t"                                                                         \
-        "addc.cc.u32 %7, %7, %16;\n\t"                                                                         \
-        "addc.u32    %8, %8, 0;"                                                                               \
-        : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)            \
-        : "r"((uint32_t)(p0)), "r"((uint32_t)(p1)), "r"((uint32_t)(p2)), "r"((uint32_t)(p3)),                 \
-          "r"((uint32_t)(p4)), "r"((uint32_t)(p5)), "r"((uint32_t)(p6)), "r"((uint32_t)(p7)))
-#define ZK_ADD_HI_CHAIN(p0, p1, p2, p3, p4, p5, p6, p7)                                                         \
-    asm("add.cc.u32  %0, %0, %8;\n\t"                                                                          \
-        "addc.cc.u32 %1, %1, %9;\n\t"                                                                          \
-        "addc.cc.u32 %2, %2, %10;\n\t"                                                                         \
-        "addc.cc.u32 %3, %3, %11;\n\t"                                                                         \
-        "addc.cc.u32 %4, %4, %12;\n\t"                                                                         \
-        "addc.cc.u32 %5, %5, %13;\n\t"                                                                         \
-        "addc.cc.u32 %6, %6, %14;\n\t"                                                                         \
-        "addc.u32    %7, %7, %15;"                                                                             \
-        : "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)                       \
-        : "r"((uint32_t)((p0) >> 32)), "r"((uint32_t)((p1) >> 32)), "r"((uint32_t)((p2) >> 32)),              \
-          "r"((uint32_t)((p3) >> 32)), "r"((uint32_t)((p4) >> 32)), "r"((uint32_t)((p5) >> 32)),              \
-          "r"((uint32_t)((p6) >> 32)), "r"((uint32_t)((p7) >> 32)))
-
-// Rows (bit i = row i) whose reduction half m * p uses mad.lo.cc / madc.hi.cc chains
-// (IMAD pipe) instead of mul.wide + add chains (IMAD.WIDE + ALU pipe).
-#ifndef ZK_MIX_ROWS
-#define ZK_MIX_ROWS 0
-#endif
-#define ZK_RED_MAD_ROW(F, m_)                                                                                  \
-    do {                                                                                                       \
-        asm("mad.lo.cc.u32  %0, %9, %10, %0;\n\t"                                                              \
-            "madc.lo.cc.u32 %1, %9, %11, %1;\n\t"                                                              \
-            "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"                                                              \
-            "madc.lo.cc.u32 %3, %9, %13, %3;\n\t"                                                              \
-            "madc.lo.cc.u32 %4, %9, %14, %4;\n\t"                                                              \
-            "madc.lo.cc.u32 %5, %9, %15, %5;\n\t"                                                              \
-            "madc.lo.cc.u32 %6, %9, %16, %6;\n\t"                                                              \
-            "madc.lo.cc.u32 %7, %9, %17, %7;\n\t"                                                              \
-            "addc.u32       %8, %8, 0;"                                                                        \
-            : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)        \
-            : "r"(m_), "n"(F::P(0)), "n"(F::P(1)), "n"(F::P(2)), "n"(F::P(3)), "n"(F::P(4)), "n"(F::P(5)),   \
-              "n"(F::P(6)), "n"(F::P(7)));                                                                     \
-        asm("mad.hi.cc.u32  %0, %8, %9, %0;\n\t"                                                               \
-            "madc.hi.cc.u32 %1, %8, %10, %1;\n\t"                                                              \
-            "madc.hi.cc.u32 %2, %8, %11, %2;\n\t"                                                              \
-            "madc.hi.cc.u32 %3, %8, %12, %3;\n\t"                                                              \
-            "madc.hi.cc.u32 %4, %8, %13, %4;\n\t"                                                              \
-            "madc.hi.cc.u32 %5, %8, %14, %5;\n\t"                                                              \
-            "madc.hi.cc.u32 %6, %8, %15, %6;\n\t"                                                              \
-            "madc.hi.u32    %7, %8, %16, %7;"                                                                  \
-            : "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)                   \
-            : "r"(m_), "n"(F::P(0)), "n"(F::P(1)), "n"(F::P(2)), "n"(F::P(3)), "n"(F::P(4)), "n"(F::P(5)),   \
-              "n"(F::P(6)), "n"(F::P(7)));                                                                     \
-    } while (0)
-
-// Row of the carry-save form: x_j = a_j * b + t_j as one 64-bit multiply-add each
-// (mul.wide with a 64-bit addend: (2^32 - 1)^2 + (2^32 - 1) < 2^64, no overflow), then a
-// single add-carry chain t_j = lo(x_j) + hi(x_{j-1}), t_8 += hi(x_7): one ALU addition per
-// partial product instead of two (the low halves ride in the multiply).
-#define ZK_ROW_ACC(a0, a1, a2, a3, a4, a5, a6, a7, bi)                                                          \
-    do {                                                                                                       \
-        const uint64_t x0 = (uint64_t)(a0) * (bi) + t0, x1 = (uint64_t)(a1) * (bi) + t1,                      \
-                       x2 = (uint64_t)(a2) * (bi) + t2, x3 = (uint64_t)(a3) * (bi) + t3,                      \
-                       x4 = (uint64_t)(a4) * (bi) + t4, x5 = (uint64_t)(a5) * (bi) + t5,                      \
-                       x6 = (uint64_t)(a6) * (bi) + t6, x7 = (uint64_t)(a7) * (bi) + t7;                      \
-        t0 = (uint32_t)x0;                                                                                     \
-        asm("add.cc.u32  %0, %8, %15;\n\t"                                                                      \
-            "addc.cc.u32 %1, %9, %16;\n\t"                                                                      \
-            "addc.cc.u32 %2, %10, %17;\n\t"                                                                     \
-            "addc.cc.u32 %3, %11, %18;\n\t"                                                                     \
-            "addc.cc.u32 %4, %12, %19;\n\t"                                                                     \
-            "addc.cc.u32 %5, %13, %20;\n\t"                                                                     \
-            "addc.cc.u32 %6, %14, %21;\n\t"                                                                     \
-            "addc.u32    %7, %7, %22;"                                                                         \
-            : "=r"(t1), "=r"(t2), "=r"(t3), "=r"(t4), "=r"(t5), "=r"(t6), "=r"(t7), "+r"(t8)                   \
-            : "r"((uint32_t)x1), "r"((uint32_t)x2), "r"((uint32_t)x3), "r"((uint32_t)x4), "r"((uint32_t)x5),   \
-              "r"((uint32_t)x6), "r"((uint32_t)x7), "r"((uint32_t)(x0 >> 32)), "r"((uint32_t)(x1 >> 32)),     \
-              "r"((uint32_t)(x2 >> 32)), "r"((uint32_t)(x3 >> 32)), "r"((uint32_t)(x4 >> 32)),                 \
-              "r"((uint32_t)(x5 >> 32)), "r"((uint32_t)(x6 >> 32)), "r"((uint32_t)(x7 >> 32)));                \
-    } while (0)
-
-// CIOS on the carry-save rows: per row 16 multiply-adds and two 8-long carry chains.
-template <class F>
-__device__ __forceinline__ fe fe_mul_acc_unrolled(const fe& a, const fe& b) {
-    uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0, t6 = 0, t7 = 0, t8 = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        ZK_ROW_ACC(a.v[0], a.v[1], a.v[2], a.v[3], a.v[4], a.v[5], a.v[6], a.v[7], b.v[i]);
-        const uint32_t m = t0 * F::INV;
-        ZK_ROW_ACC(F::P(0), F::P(1), F::P(2), F::P(3), F::P(4), F::P(5), F::P(6), F::P(7), m);
-        // t0 == 0 now (m was chosen so); shift one limb
-        t0 = t1;
-        t1 = t2;
-        t2 = t3;
-        t3 = t4;
-        t4 = t5;
-        t5 = t6;
-        t6 = t7;
-        t7 = t8;
-        t8 = 0;
-    }
-    fe t;
-    t.v[0] = t0;
-    t.v[1] = t1;
-    t.v[2] = t2;
-    t.v[3] = t3;
-    t.v[4] = t4;
-    t.v[5] = t5;
-    t.v[6] = t6;
-    t.v[7] = t7;
-    if constexpr (F::LAZY) return t;
-    else return fe_reduce_once<F>(t);
-}
-
-template <class F>
-__device__ __forceinline__ fe fe_mul_wide_unrolled(const fe& a, const fe& b) {
-    uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0, t6 = 0, t7 = 0, t8 = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const uint32_t bi = b.v[i];
-        const uint64_t p0 = (uint64_t)a.v[0] * bi, p1 = (uint64_t)a.v[1] * bi, p2 = (uint64_t)a.v[2] * bi,
-                       p3 = (uint64_t)a.v[3] * bi, p4 = (uint64_t)a.v[4] * bi, p5 = (uint64_t)a.v[5] * bi,
-                       p6 = (uint64_t)a.v[6] * bi, p7 = (uint64_t)a.v[7] * bi;
-        ZK_ADD_LO_CHAIN(p0, p1, p2, p3, p4, p5, p6, p7);
-        ZK_ADD_HI_CHAIN(p0, p1, p2, p3, p4, p5, p6, p7);
-        const uint32_t m = t0 * F::INV;
-        if ((ZK_MIX_ROWS >> i) & 1) {
-            // this row's m * p on the IMAD pipe (multiply-add with carry), balancing the ALU pipe
-            ZK_RED_MAD_ROW(F, m);
-        } else {
-            const uint64_t q0 = (uint64_t)m * F::P(0), q1 = (uint64_t)m * F::P(1), q2 = (uint64_t)m * F::P(2),
-                           q3 = (uint64_t)m * F::P(3), q4 = (uint64_t)m * F::P(4), q5 = (uint64_t)m * F::P(5),
-                           q6 = (uint64_t)m * F::P(6), q7 = (uint64_t)m * F::P(7);
-            ZK_ADD_LO_CHAIN(q0, q1, q2, q3, q4, q5, q6, q7);
-            ZK_ADD_HI_CHAIN(q0, q1, q2, q3, q4, q5, q6, q7);
-        }
-        t0 = t1;
-        t1 = t2;
-        t2 = t3;
-        t3 = t4;
-        t4 = t5;
-        t5 = t6;
-        t6 = t7;
-        t7 = t8;
-        t8 = 0;
-    }
-    fe t;
-    t.v[0] = t0;
-    t.v[1] = t1;
-    t.v[2] = t2;
-    t.v[3] = t3;
-    t.v[4] = t4;
-    t.v[5] = t5;
-    t.v[6] = t6;
-    t.v[7] = t7;
-    if constexpr (F::LAZY) return t;
-    else return fe_reduce_once<F>(t);
-}
-
-// Two independent products a*b and c*d with their rows interleaved: the carry chains of
-// one product fill the latency of the other's (a thread's carry flag serialises each chain).
-#define ZK_LO_CHAIN_R(r0, r1, r2, r3, r4, r5, r6, r7, r8, p0, p1, p2, p3, p4, p5, p6, p7)                     \
-    asm("add.cc.u32  %0, %0, %9;\n\t"                                                                          \
-        "addc.cc.u32 %1, %1, %10;\n\t"                                                                         \
-        "addc.cc.u32 %2, %2, %11;\n\t"                                                                         \
-        "addc.cc.u32 %3, %3, %12;\n\t"                                                                         \
-        "addc.cc.u32 %4, %4, %13;\n\t"                                                                         \
-        "addc.cc.u32 %5, %5, %14;\n\t"                                                                         \
-        "addc.cc.u32 %6, %6, %15;\n\t"                                                                         \
-        "addc.cc.u32 %7, %7, %16;\n\t"                                                                         \
-        "addc.u32    %8, %8, 0;"                                                                               \
-        : "+r"(r0), "+r"(r1), "+r"(r2), "+r"(r3), "+r"(r4), "+r"(r5), "+r"(r6), "+r"(r7), "+r"(r8)            \
-        : "r"((uint32_t)(p0)), "r"((uint32_t)(p1)), "r"((uint32_t)(p2)), "r"((uint32_t)(p3)),                 \
-          "r"((uint32_t)(p4)), "r"((uint32_t)(p5)), "r"((uint32_t)(p6)), "r"((uint32_t)(p7)))
-#define ZK_HI_CHAIN_R(r1, r2, r3, r4, r5, r6, r7, r8, p0, p1, p2, p3, p4, p5, p6, p7)                         \
-    asm("add.cc.u32  %0, %0, %8;\n\t"                                                                          \
-        "addc.cc.u32 %1, %1, %9;\n\t"                                                                          \
-        "addc.cc.u32 %2, %2, %10;\n\t"                                                                         \
-        "addc.cc.u32 %3, %3, %11;\n\t"                                                                         \
-        "addc.cc.u32 %4, %4, %12;\n\t"                                                                         \
-        "addc.cc.u32 %5, %5, %13;\n\t"                                                                         \
-        "addc.cc.u32 %6, %6, %14;\n\t"                                                                         \
-        "addc.u32    %7, %7, %15;"                                                                             \
-        : "+r"(r1), "+r"(r2), "+r"(r3), "+r"(r4), "+r"(r5), "+r"(r6), "+r"(r7), "+r"(r8)                       \
-        : "r"((uint32_t)((p0) >> 32)), "r"((uint32_t)((p1) >> 32)), "r"((uint32_t)((p2) >> 32)),              \
-          "r"((uint32_t)((p3) >> 32)), "r"((uint32_t)((p4) >> 32)), "r"((uint32_t)((p5) >> 32)),              \
-          "r"((uint32_t)((p6) >> 32)), "r"((uint32_t)((p7) >> 32)))
-
-struct fe2 {
-    fe x, y;
-};
-
-template <class F>
-__device__ __forceinline__ fe2 fe_mul2_wide_unrolled(const fe& a, const fe& b, const fe& c, const fe& d) {
-    uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0, t6 = 0, t7 = 0, t8 = 0;
-    uint32_t u0 = 0, u1 = 0, u2 = 0, u3 = 0, u4 = 0, u5 = 0, u6 = 0, u7 = 0, u8 = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const uint32_t bi = b.v[i], di = d.v[i];
-        const uint64_t p0 = (uint64_t)a.v[0] * bi, p1 = (uint64_t)a.v[1] * bi, p2 = (uint64_t)a.v[2] * bi,
-                       p3 = (uint64_t)a.v[3] * bi, p4 = (uint64_t)a.v[4] * bi, p5 = (uint64_t)a.v[5] * bi,
-                       p6 = (uint64_t)a.v[6] * bi, p7 = (uint64_t)a.v[7] * bi;
-        const uint64_t r0 = (uint64_t)c.v[0] * di, r1 = (uint64_t)c.v[1] * di, r2 = (uint64_t)c.v[2] * di,
-                       r3 = (uint64_t)c.v[3] * di, r4 = (uint64_t)c.v[4] * di, r5 = (uint64_t)c.v[5] * di,
-                       r6 = (uint64_t)c.v[6] * di, r7 = (uint64_t)c.v[7] * di;
-        ZK_LO_CHAIN_R(t0, t1, t2, t3, t4, t5, t6, t7, t8, p0, p1, p2, p3, p4, p5, p6, p7);
-        ZK_LO_CHAIN_R(u0, u1, u2, u3, u4, u5, u6, u7, u8, r0, r1, r2, r3, r4, r5, r6, r7);
-        ZK_HI_CHAIN_R(t1, t2, t3, t4, t5, t6, t7, t8, p0, p1, p2, p3, p4, p5, p6, p7);
-        ZK_HI_CHAIN_R(u1, u2, u3, u4, u5, u6, u7, u8, r0, r1, r2, r3, r4, r5, r6, r7);
-        const uint32_t m = t0 * F::INV, mu = u0 * F::INV;
-        const uint64_t q0 = (uint64_t)m * F::P(0), q1 = (uint64_t)m * F::P(1), q2 = (uint64_t)m * F::P(2),
-                       q3 = (uint64_t)m * F::P(3), q4 = (uint64_t)m * F::P(4), q5 = (uint64_t)m * F::P(5),
-                       q6 = (uint64_t)m * F::P(6), q7 = (uint64_t)m * F::P(7);
-        const uint64_t s0 = (uint64_t)mu * F::P(0), s1 = (uint64_t)mu * F::P(1), s2 = (uint64_t)mu * F::P(2),
-                       s3 = (uint64_t)mu * F::P(3), s4 = (uint64_t)mu * F::P(4), s5 = (uint64_t)mu * F::P(5),
-                       s6 = (uint64_t)mu * F::P(6), s7 = (uint64_t)mu * F::P(7);
-        ZK_LO_CHAIN_R(t0, t1, t2, t3, t4, t5, t6, t7, t8, q0, q1, q2, q3, q4, q5, q6, q7);
-        ZK_LO_CHAIN_R(u0, u1, u2, u3, u4, u5, u6, u7, u8, s0, s1, s2, s3, s4, s5, s6, s7);
-        ZK_HI_CHAIN_R(t1, t2, t3, t4, t5, t6, t7, t8, q0, q1, q2, q3, q4, q5, q6, q7);
-        ZK_HI_CHAIN_R(u1, u2, u3, u4, u5, u6, u7, u8, s0, s1, s2, s3, s4, s5, s6, s7);
-        t0 = t1, t1 = t2, t2 = t3, t3 = t4, t4 = t5, t5 = t6, t6 = t7, t7 = t8, t8 = 0;
-        u0 = u1, u1 = u2, u2 = u3, u3 = u4, u4 = u5, u5 = u6, u6 = u7, u7 = u8, u8 = 0;
-    }
-    fe x, y;
-    x.v[0] = t0, x.v[1] = t1, x.v[2] = t2, x.v[3] = t3, x.v[4] = t4, x.v[5] = t5, x.v[6] = t6, x.v[7] = t7;
-    y.v[0] = u0, y.v[1] = u1, y.v[2] = u2, y.v[3] = u3, y.v[4] = u4, y.v[5] = u5, y.v[6] = u6, y.v[7] = u7;
-    fe2 r;
-    if constexpr (F::LAZY) {
-        r.x = x;
-        r.y = y;
-    } else {
-        r.x = fe_reduce_once<F>(x);
-        r.y = fe_reduce_once<F>(y);
-    }
-    return r;
-}
-
-template <class F>
-__device__ __noinline__ fe2 fe_mul2_call(const fe a, const fe b, const fe c, const fe d) {
-    return fe_mul2_wide_unrolled<F>(a, b, c, d);
-}
-
-// (a*b, c*d): two calls of fe_mul, or (with ZK_USE_MUL2 and style 3) one call of the
-// interleaved product.
-template <class F>
-__device__ __forceinline__ fe2 fe_mul2(const fe& a, const fe& b, const fe& c, const fe& d);
-
-template <class F>
-__device__ __noinline__ fe fe_mul_call(const fe a, const fe b) {
-    return fe_mul_unrolled<F>(a, b);
-}
-
-template <class F>
-__host__ __device__ __forceinline__ fe fe_mul_sos(const fe& a, const fe& b);
-
-template <class F>
-__device__ __noinline__ fe fe_mul_wide_call(const fe a, const fe b) {
-#ifdef ZK_WIDE_ACC
-    return fe_mul_acc_unrolled<F>(a, b);
-#elif defined(ZK_SOS_MUL)
-    if constexpr (F::LAZY) return fe_mul_sos<F>(a, b);
-    else return fe_mul_wide_unrolled<F>(a, b);
-#else
-    return fe_mul_wide_unrolled<F>(a, b);
-#endif
-}
-
-// r = a * b * 2^-256 mod p (CIOS, see the file header).
-template <class F>
-__device__ __forceinline__ fe fe_mul(const fe& a, const fe& b) {
-#ifdef ZK_MUL_STYLE
-    constexpr int style = ZK_MUL_STYLE;
-#else
-    constexpr int style = F::MUL_STYLE;
-#endif
-    if constexpr (style == 0) {
-        return fe_mul_unrolled<F>(a, b);
-    } else if constexpr (style == 1) {
-        return fe_mul_call<F>(a, b);
-    } else if constexpr (style == 3) {
-        return fe_mul_wide_call<F>(a, b);
-    } else if constexpr (style == 4) {
-#ifdef ZK_WIDE_ACC
-        return fe_mul_acc_unrolled<F>(a, b);
-#else
-        return fe_mul_wide_unrolled<F>(a, b);
-#endif
-    } else {
-        return fe_mul_rolled<F>(a, b);
-    }
-}
-
-template <class F>
-__device__ __forceinline__ fe2 fe_mul2(const fe& a, const fe& b, const fe& c, const fe& d) {
-#ifdef ZK_USE_MUL2
-#ifdef ZK_MUL_STYLE
-    constexpr int style = ZK_MUL_STYLE;
-#else
-    constexpr int style = F::MUL_STYLE;
-#endif
-    // measured on GB300 (MSM 2^20): 179 Mpts/s with the interleaved pair, 180 without
-    if constexpr (style == 3) return fe_mul2_call<F>(a, b, c, d);
-#endif
-    fe2 r;
-    r.x = fe_mul<F>(a, b);
-    r.y = fe_mul<F>(c, d);
-    return r;
-}
-
-// ---- separated forms: a 512-bit product, then one Montgomery reduction -------------------
-//
-// Splitting the product from the reduction lets a square skip the 28 repeated cross
-// products (36 instead of 64 partial products) and lets a difference of two products
-// a b - c d share one reduction. They serve the lazy Fq of the curve formulas only.
-//
-// Reduction: for T = T_lo + 2^256 T_hi, the m_i of the Montgomery rows depend on T_lo alone,
-// so (T + M p) / 2^256 = T_hi + (T_lo + M p) / 2^256; the second term is a CIOS reduction of
-// the low 8 limbs (a 9-limb window, no carry beyond it) and is at most p. With T < 4p^2
-// (a product of two values below 2p) T_hi < 0.76 p, so the result stays below 2p; with
-// T < 8p^2 (a sum of two such products) it is below 2.52 p and one conditional subtraction
-// of 2p brings it below 2p (both moduli are below 0.19 * 2^256).
+// ---- products -------------------------------------------------------------------------------
 //
 // The carry flag primitives are one PTX instruction each on the device (asm volatile keeps
 // their order, so the flag flows from one to the next as in a single asm block); on the
@@ -813,6 +362,194 @@ __host__ __device__ __forceinline__ uint32_t u_subc(uint32_t a, uint32_t b) {
 #endif
 }
 
+// The 64-bit pair (lo, hi) += a * b, in two instructions that share a carry: lo and hi are
+// the limbs of an even-aligned register pair, so one wide multiply-add does both. _cc
+// leaves the carry out in the flag; kIn takes the flag's carry in.
+template <bool kIn>
+__host__ __device__ __forceinline__ void u_mad2_cc(uint32_t& lo, uint32_t& hi, uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+    if constexpr (kIn)
+        asm volatile("madc.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.cc.u32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
+    else
+        asm volatile("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.cc.u32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
+#else
+    const unsigned __int128 s = (unsigned __int128)((uint64_t)a * b) + (((uint64_t)hi << 32) | lo) + (kIn ? host_carry_flag() : 0u);
+    lo = (uint32_t)s;
+    hi = (uint32_t)(s >> 32);
+    host_carry_flag() = (uint32_t)(s >> 64);
+#endif
+}
+
+// ... and without a carry out (the caller's bound excludes one)
+template <bool kIn>
+__host__ __device__ __forceinline__ void u_mad2(uint32_t& lo, uint32_t& hi, uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+    if constexpr (kIn)
+        asm volatile("madc.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
+    else
+        asm volatile("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
+#else
+    const uint64_t s = (uint64_t)a * b + (((uint64_t)hi << 32) | lo) + (kIn ? host_carry_flag() : 0u);
+    lo = (uint32_t)s;
+    hi = (uint32_t)(s >> 32);
+#endif
+}
+
+// The product rows keep a running value T (9 limbs) as two accumulators of four 64-bit
+// columns each: e[0..7] at limbs 0..7 and o[0..7] at limbs 1..8, T = e + 2^32 o. A product
+// a_j b_i belongs to the accumulator that its limb position is aligned with, so each of the
+// 8 products of a row is ONE wide multiply-add with carry in and out (mad.lo.cc / madc.hi.cc
+// on an aligned pair) and a row has two chains of four.
+//
+// What bounds it on GB300: the wide multiply-add. One takes 4 issue cycles of a scheduler's
+// multiply pipe whether or not it adds and carries (measured: 10.1 T/s for the chip at
+// 2070 MHz, 16 lanes a cycle a scheduler at two passes), and an add with carry 2 cycles of
+// the other integer pipe. A product needs 128 of the former = 512 cycles a warp; this form
+// adds 8 low multiplies and ~40 adds. Measured (independent chains, 64 warps per SM): 70.1 G
+// products/s = 92% of the multiply pipe, against 47.8 G/s for full-width products folded in
+// by separate add-with-carry chains (290 adds: the two pipes then take turns); 64-bit adds
+// of full-width products 56.8 G/s.
+//
+// row_odd: o += {a_1, a_3, a_5, a_7} y, with the flag's carry into limb 1 when kIn. T stays
+// below 2^288, so o (at most T / 2^32) never carries out.
+template <bool kIn>
+__host__ __device__ __forceinline__ void row_odd(uint32_t* o, const uint32_t* a, uint32_t y) {
+    u_mad2_cc<kIn>(o[0], o[1], a[1], y);
+    u_mad2_cc<true>(o[2], o[3], a[3], y);
+    u_mad2_cc<true>(o[4], o[5], a[5], y);
+    u_mad2<true>(o[6], o[7], a[7], y);
+}
+
+// row_even: e += {a_0, a_2, a_4, a_6} y, the carry out of limb 7 into o's top limb.
+__host__ __device__ __forceinline__ void row_even(uint32_t* e, uint32_t* o, const uint32_t* a, uint32_t y) {
+    u_mad2_cc<false>(e[0], e[1], a[0], y);
+    u_mad2_cc<true>(e[2], e[3], a[2], y);
+    u_mad2_cc<true>(e[4], e[5], a[4], y);
+    u_mad2_cc<true>(e[6], e[7], a[6], y);
+    o[7] = u_addc(o[7], 0u);
+}
+
+// The first row: e, o = a * y, nothing to add to.
+__host__ __device__ __forceinline__ void row_first(uint32_t* e, uint32_t* o, const uint32_t* a, uint32_t y) {
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+        const uint64_t p = (uint64_t)a[j] * y, q = (uint64_t)a[j + 1] * y;
+        e[j] = (uint32_t)p;
+        e[j + 1] = (uint32_t)(p >> 32);
+        o[j] = (uint32_t)q;
+        o[j + 1] = (uint32_t)(q >> 32);
+    }
+}
+
+template <class F>
+__host__ __device__ __forceinline__ void modulus_limbs(uint32_t* p) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) p[j] = F::P(j);
+}
+
+// T += m p with m = T_0 (-p^-1): limb 0 becomes 0.
+template <class F>
+__host__ __device__ __forceinline__ void row_reduce(uint32_t* e, uint32_t* o) {
+    uint32_t p[8];
+    modulus_limbs<F>(p);
+    const uint32_t m = e[0] * F::INV;
+    row_odd<false>(o, p, m);
+    row_even(e, o, p, m);
+}
+
+// T / 2^32 once limb 0 is 0: o becomes the even accumulator, e without its limbs 0 and 1 the
+// odd one; limb 1 (returned) is left for the caller to add to the new even accumulator.
+__host__ __device__ __forceinline__ uint32_t row_shift(uint32_t* e, uint32_t* o) {
+    const uint32_t c = e[1];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const uint32_t x = j < 6 ? e[j + 2] : 0u;
+        e[j] = o[j];
+        o[j] = x;
+    }
+    return c;
+}
+
+// (e + 2^32 o) / 2^32 as 8 limbs, limb 0 being 0 and the value below 2^288.
+__host__ __device__ __forceinline__ fe row_result(const uint32_t* e, const uint32_t* o) {
+    fe r;
+    r.v[0] = u_add_cc(o[0], e[1]);
+#pragma unroll
+    for (int j = 1; j < 7; j++) r.v[j] = u_addc_cc(o[j], e[j + 1]);
+    r.v[7] = u_addc(o[7], 0u);
+    return r;
+}
+
+// a b 2^-256 mod p, below ab / 2^256 + p (CIOS rows): below 2p for a, b below 2p. T stays
+// below 2^32 (a + p) < 2^288 for a below 4p.
+template <class F>
+__host__ __device__ __forceinline__ fe mul_rows(const fe& a, const fe& b) {
+    uint32_t e[8], o[8];
+    row_first(e, o, a.v, b.v[0]);
+    row_reduce<F>(e, o);
+#pragma unroll
+    for (int i = 1; i < 8; i++) {
+        const uint32_t c = row_shift(e, o);
+        e[0] = u_add_cc(e[0], c);
+        row_odd<true>(o, a.v, b.v[i]);
+        row_even(e, o, a.v, b.v[i]);
+        row_reduce<F>(e, o);
+    }
+    return row_result(e, o);
+}
+
+// (a b + c d) 2^-256 mod p with one reduction, below (ab + cd) / 2^256 + p: below 2.52p for
+// inputs up to 2p. T stays below 2^32 (a + c + p) <= 5p 2^32 < 2^288.
+template <class F>
+__host__ __device__ __forceinline__ fe mul_add_rows(const fe& a, const fe& b, const fe& c, const fe& d) {
+    uint32_t e[8], o[8];
+    row_first(e, o, a.v, b.v[0]);
+    row_odd<false>(o, c.v, d.v[0]);
+    row_even(e, o, c.v, d.v[0]);
+    row_reduce<F>(e, o);
+#pragma unroll
+    for (int i = 1; i < 8; i++) {
+        const uint32_t t = row_shift(e, o);
+        e[0] = u_add_cc(e[0], t);
+        row_odd<true>(o, a.v, b.v[i]);
+        row_even(e, o, a.v, b.v[i]);
+        row_odd<false>(o, c.v, d.v[i]);
+        row_even(e, o, c.v, d.v[i]);
+        row_reduce<F>(e, o);
+    }
+    return row_result(e, o);
+}
+
+template <class F>
+__device__ __noinline__ fe fe_mul_call(const fe a, const fe b) {
+    return mul_rows<F>(a, b);
+}
+
+// r = a * b * 2^-256 mod p. F::CALL_MUL: one non-inlined copy of the product, called from
+// every site. The curve formulas hold 10-14 products per loop body, so inlining them all
+// overflows the instruction cache; the NTT butterflies hold one to four.
+template <class F>
+__device__ __forceinline__ fe fe_mul(const fe& a, const fe& b) {
+    fe r;
+    if constexpr (F::CALL_MUL) r = fe_mul_call<F>(a, b);
+    else r = mul_rows<F>(a, b);
+    if constexpr (F::LAZY) return r;
+    else return fe_reduce_once<F>(r);
+}
+
+// ---- separated forms: a 512-bit product, then one Montgomery reduction -------------------
+//
+// Splitting the product from the reduction lets a square skip the 28 repeated cross
+// products (36 instead of 64 partial products) and lets a difference of two products
+// a b - c d share one reduction. They serve the lazy Fq of the curve formulas only.
+//
+// Reduction: for T = T_lo + 2^256 T_hi, the m_i of the Montgomery rows depend on T_lo alone,
+// so (T + M p) / 2^256 = T_hi + (T_lo + M p) / 2^256; the second term is a CIOS reduction of
+// the low 8 limbs (a 9-limb window, no carry beyond it) and is at most p. With T < 4p^2
+// (a product of two values below 2p) T_hi < 0.76 p, so the result stays below 2p; with
+// T < 8p^2 (a sum of two such products) it is below 2.52 p and one conditional subtraction
+// of 2p brings it below 2p (both moduli are below 0.19 * 2^256).
+//
 __host__ __device__ __forceinline__ uint32_t lo32(uint64_t x) { return (uint32_t)x; }
 __host__ __device__ __forceinline__ uint32_t hi32(uint64_t x) { return (uint32_t)(x >> 32); }
 
@@ -1109,20 +846,11 @@ __device__ __noinline__ fe fe_mul_sub_sos_call(const fe a, const fe b, const fe 
     return fe_mul_sub_sos<F>(a, b, c, d);
 }
 
-// The separated forms are used for the lazy fields with the called multiplication (style
-// 3: the curve formulas over Fq); ZK_NO_SOS keeps every product on fe_mul for comparison.
+// The separated forms serve the lazy fields with the called multiplication: the curve
+// formulas over Fq.
 template <class F>
 __device__ __forceinline__ constexpr bool use_sos() {
-#if defined(ZK_NO_SOS)
-    return false;
-#else
-#ifdef ZK_MUL_STYLE
-    constexpr int style = ZK_MUL_STYLE;
-#else
-    constexpr int style = F::MUL_STYLE;
-#endif
-    return F::LAZY && style == 3;
-#endif
+    return F::LAZY && F::CALL_MUL;
 }
 
 template <class F>
