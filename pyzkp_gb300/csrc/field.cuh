@@ -540,137 +540,121 @@ __device__ __forceinline__ fe fe_mul(const fe& a, const fe& b) {
 // ---- separated forms: a 512-bit product, then one Montgomery reduction -------------------
 //
 // Splitting the product from the reduction lets a square skip the 28 repeated cross
-// products (36 instead of 64 partial products) and lets a difference of two products
-// a b - c d share one reduction. They serve the lazy Fq of the curve formulas only.
+// products (100 wide multiply-adds instead of 128), and lets the Fq2 product reduce sums of
+// products. They serve the lazy Fq of the curve formulas only.
 //
-// Reduction: for T = T_lo + 2^256 T_hi, the m_i of the Montgomery rows depend on T_lo alone,
-// so (T + M p) / 2^256 = T_hi + (T_lo + M p) / 2^256; the second term is a CIOS reduction of
-// the low 8 limbs (a 9-limb window, no carry beyond it) and is at most p. With T < 4p^2
-// (a product of two values below 2p) T_hi < 0.76 p, so the result stays below 2p; with
-// T < 8p^2 (a sum of two such products) it is below 2.52 p and one conditional subtraction
-// of 2p brings it below 2p (both moduli are below 0.19 * 2^256).
-//
-__host__ __device__ __forceinline__ uint32_t lo32(uint64_t x) { return (uint32_t)x; }
-__host__ __device__ __forceinline__ uint32_t hi32(uint64_t x) { return (uint32_t)(x >> 32); }
+// Reduction: (T + M p) / 2^256 row by row over a window of 9 limbs; T's limb 8 + i enters the
+// window at its limb 7 after row i, so the window stays below 2^256 + 2^32 p before a shift
+// and nothing carries out of it. The result is below T / 2^256 + p: below 2p for T < 4p^2 (a
+// product of two values below 2p: T / 2^256 < 0.76 p), below 2.52 p for T < 8p^2, which one
+// conditional subtraction of 2p brings below 2p (both moduli are below 0.19 * 2^256).
 
-// Row I of t += a * b_I with a below 2^255: the low halves of a_j b_I into t_{I+j} (carry
-// into t_{I+8}), the high halves into t_{I+j+1}. FIRST: t_{I..I+8} are not yet written
-// (the first product's rows). Two products accumulated row by row stay below
-// 2 * 2^255 * 2^(32(I+1)) = 2^(32(I+9)), so nothing carries out of t_{I+8}.
-template <int I, bool FIRST>
-__host__ __device__ __forceinline__ void sos_row(uint32_t* t, const uint32_t* a, uint32_t bi) {
-    uint64_t p[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) p[j] = (uint64_t)a[j] * bi;
-    if constexpr (FIRST && I == 0) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) t[j] = lo32(p[j]);
-        t[1] = u_add_cc(t[1], hi32(p[0]));
-#pragma unroll
-        for (int j = 1; j < 7; j++) t[j + 1] = u_addc_cc(t[j + 1], hi32(p[j]));
-        t[8] = u_addc(0u, hi32(p[7]));
-        return;
-    }
-    t[I] = u_add_cc(t[I], lo32(p[0]));
-#pragma unroll
-    for (int j = 1; j < 8; j++) t[I + j] = u_addc_cc(t[I + j], lo32(p[j]));
-    if constexpr (FIRST) t[I + 8] = u_addc(0u, 0u);
-    else t[I + 8] = u_addc(t[I + 8], 0u);
-    t[I + 1] = u_add_cc(t[I + 1], hi32(p[0]));
-#pragma unroll
-    for (int j = 1; j < 7; j++) t[I + j + 1] = u_addc_cc(t[I + j + 1], hi32(p[j]));
-    t[I + 8] = u_addc(t[I + 8], hi32(p[7]));
-}
-
-// Row I of the cross products a_I a_j (j > I) into t_{I+j}: 7 - I products.
-template <int I>
-__host__ __device__ __forceinline__ void sqr_cross_row(uint32_t* t, const uint32_t* a) {
-    constexpr int L = 7 - I;
-    uint64_t p[8];
-#pragma unroll
-    for (int j = I + 1; j < 8; j++) p[j] = (uint64_t)a[I] * a[j];
-    if constexpr (I == 0) {
-#pragma unroll
-        for (int j = 1; j < 8; j++) t[j] = lo32(p[j]);
-        t[2] = u_add_cc(t[2], hi32(p[1]));
-#pragma unroll
-        for (int j = 2; j < 7; j++) t[j + 1] = u_addc_cc(t[j + 1], hi32(p[j]));
-        t[8] = u_addc(0u, hi32(p[7]));
-        return;
-    }
-    // low halves: t_{2I+1} .. t_{I+7}, carry into t_{I+8} (not yet written)
-    t[2 * I + 1] = u_add_cc(t[2 * I + 1], lo32(p[I + 1]));
-#pragma unroll
-    for (int j = I + 2; j < 8; j++) t[I + j] = u_addc_cc(t[I + j], lo32(p[j]));
-    t[I + 8] = u_addc(0u, 0u);
-    // high halves: t_{2I+2} .. t_{I+8}
-    if constexpr (L == 1) {
-        t[I + 8] = t[I + 8] + hi32(p[7]);
+// c[0..2N-1] += {x_0, x_2, ..} y for N partial products (x strided by 2); kOut: the carry out
+// becomes c[2N] (not yet written), else the caller knows there is none (the top pair held at
+// most a carry before: (2^32 - 1)^2 + 2 < 2^64).
+template <int N, bool kOut>
+__host__ __device__ __forceinline__ void sos_chain(uint32_t* c, const uint32_t* x, uint32_t y) {
+    if constexpr (N == 1) {
+        if constexpr (kOut) u_mad2_cc<false>(c[0], c[1], x[0], y);
+        else u_mad2<false>(c[0], c[1], x[0], y);
     } else {
-        t[2 * I + 2] = u_add_cc(t[2 * I + 2], hi32(p[I + 1]));
+        u_mad2_cc<false>(c[0], c[1], x[0], y);
 #pragma unroll
-        for (int j = I + 2; j < 7; j++) t[I + j + 1] = u_addc_cc(t[I + j + 1], hi32(p[j]));
-        t[I + 8] = u_addc(t[I + 8], hi32(p[7]));
+        for (int k = 1; k + 1 < N; k++) u_mad2_cc<true>(c[2 * k], c[2 * k + 1], x[2 * k], y);
+        if constexpr (kOut) u_mad2_cc<true>(c[2 * N - 2], c[2 * N - 1], x[2 * N - 2], y);
+        else u_mad2<true>(c[2 * N - 2], c[2 * N - 1], x[2 * N - 2], y);
     }
+    if constexpr (kOut) c[2 * N] = u_addc(0u, 0u);
 }
 
-// t[0..15] = a * a: the cross products once, doubled, plus the squares a_i^2 at limb 2i.
+// t[0..15] = a * b for any 256-bit a, b, in even and odd columns (o[k] at limb k + 1). Rows 2k - 1
+// and 2k end at the same even column and rows 2k and 2k + 1 at the same odd one, so only the
+// second of each two can carry out.
+__host__ __device__ __forceinline__ void sos_mul_wide(uint32_t* t, const uint32_t* a, const uint32_t* b) {
+    uint32_t e[16], o[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) e[j] = o[j] = 0u;
+    row_first(e, o, a, b[0]);
+#pragma unroll
+    for (int i = 1; i < 8; i += 2) {
+        sos_chain<4, true>(o + i - 1, a, b[i]);       // limbs i .. i + 7
+        sos_chain<4, false>(e + i + 1, a + 1, b[i]);  // limbs i + 1 .. i + 8
+        if (i + 1 < 8) {
+            sos_chain<4, true>(e + i + 1, a, b[i + 1]);
+            sos_chain<4, false>(o + i + 1, a + 1, b[i + 1]);
+        }
+    }
+    t[0] = e[0];
+    t[1] = u_add_cc(e[1], o[0]);
+#pragma unroll
+    for (int j = 2; j < 15; j++) t[j] = u_addc_cc(e[j], o[j - 1]);
+    t[15] = u_addc(e[15], o[14]);
+}
+
+// t[0..15] = a * a: the cross products a_i a_j (i < j) once, doubled, plus the squares a_i^2
+// at limb 2i. Carries as in sos_mul_wide: of two rows that end at the same column the second.
 __host__ __device__ __forceinline__ void sos_sqr_wide(uint32_t* t, const uint32_t* a) {
-    sqr_cross_row<0>(t, a);
-    sqr_cross_row<1>(t, a);
-    sqr_cross_row<2>(t, a);
-    sqr_cross_row<3>(t, a);
-    sqr_cross_row<4>(t, a);
-    sqr_cross_row<5>(t, a);
-    sqr_cross_row<6>(t, a);
-    // t_1 .. t_14 hold the cross sum (below a^2 / 2 < 2^511); double it into t_1 .. t_15
-    t[1] = u_add_cc(t[1], t[1]);
+    uint32_t e[16], o[16];
 #pragma unroll
-    for (int j = 2; j < 15; j++) t[j] = u_addc_cc(t[j], t[j]);
-    t[15] = u_addc(0u, 0u);
-    uint64_t d[8];
+    for (int j = 0; j < 16; j++) e[j] = o[j] = 0u;
+    sos_chain<4, false>(o, a + 1, a[0]);      // a_0 a_{1,3,5,7}: limbs 1 .. 8
+    sos_chain<3, false>(e + 2, a + 2, a[0]);  // a_0 a_{2,4,6}
+    sos_chain<3, true>(o + 2, a + 2, a[1]);
+    sos_chain<3, false>(e + 4, a + 3, a[1]);
+    sos_chain<3, false>(o + 4, a + 3, a[2]);
+    sos_chain<2, true>(e + 6, a + 4, a[2]);
+    sos_chain<2, true>(o + 6, a + 4, a[3]);
+    sos_chain<2, false>(e + 8, a + 5, a[3]);
+    sos_chain<2, false>(o + 8, a + 5, a[4]);
+    sos_chain<1, true>(e + 10, a + 6, a[4]);
+    sos_chain<1, true>(o + 10, a + 6, a[5]);
+    sos_chain<1, false>(e + 12, a + 7, a[5]);
+    sos_chain<1, false>(o + 12, a + 7, a[6]);
+    // the cross sum x in limbs 1 .. 14 (below a^2 / 2 < 2^511)
+    uint32_t x[15];
+    x[1] = o[0];
+    x[2] = u_add_cc(e[2], o[1]);
 #pragma unroll
-    for (int i = 0; i < 8; i++) d[i] = (uint64_t)a[i] * a[i];
-    t[0] = lo32(d[0]);
-    t[1] = u_add_cc(t[1], hi32(d[0]));
+    for (int j = 3; j < 14; j++) x[j] = u_addc_cc(e[j], o[j - 1]);
+    x[14] = u_addc(0u, o[13]);
+    // doubled by shifting (no carry chain), then the squares
+    t[0] = 0u;
+    t[1] = x[1] << 1;
 #pragma unroll
-    for (int i = 1; i < 7; i++) {
-        t[2 * i] = u_addc_cc(t[2 * i], lo32(d[i]));
-        t[2 * i + 1] = u_addc_cc(t[2 * i + 1], hi32(d[i]));
-    }
-    t[14] = u_addc_cc(t[14], lo32(d[7]));
-    t[15] = u_addc(t[15], hi32(d[7]));
+    for (int j = 2; j < 15; j++) t[j] = (x[j] << 1) | (x[j - 1] >> 31);
+    t[15] = x[14] >> 31;
+    u_mad2_cc<false>(t[0], t[1], a[0], a[0]);
+#pragma unroll
+    for (int i = 1; i < 7; i++) u_mad2_cc<true>(t[2 * i], t[2 * i + 1], a[i], a[i]);
+    u_mad2<true>(t[14], t[15], a[7], a[7]);
 }
 
-// r = T_hi + (T_lo + M p) / 2^256 for t = T (16 limbs): T * 2^-256 mod p, below T_hi + p + 1.
+// (T + M p) / 2^256 for t = T (16 limbs): T * 2^-256 mod p, below T / 2^256 + p.
 template <class F>
 __host__ __device__ __forceinline__ fe sos_redc(const uint32_t* t) {
-    uint32_t w[9];
+    uint32_t e[8], o[8];
 #pragma unroll
-    for (int j = 0; j < 8; j++) w[j] = t[j];
+    for (int j = 0; j < 8; j++) {
+        e[j] = t[j];
+        o[j] = 0u;
+    }
+    row_reduce<F>(e, o);
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const uint32_t m = w[0] * F::INV;
-        uint64_t q[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) q[j] = (uint64_t)m * F::P(j);
-        w[0] = u_add_cc(w[0], lo32(q[0]));
-#pragma unroll
-        for (int j = 1; j < 8; j++) w[j] = u_addc_cc(w[j], lo32(q[j]));
-        w[8] = u_addc(0u, 0u);
-        w[1] = u_add_cc(w[1], hi32(q[0]));
-#pragma unroll
-        for (int j = 1; j < 7; j++) w[j + 1] = u_addc_cc(w[j + 1], hi32(q[j]));
-        w[8] = u_addc(w[8], hi32(q[7]));
-        // w_0 == 0 now (m was chosen so); shift one limb
-#pragma unroll
-        for (int j = 0; j < 8; j++) w[j] = w[j + 1];
+    for (int i = 1; i < 8; i++) {
+        const uint32_t c = row_shift(e, o);
+        o[6] = t[7 + i];
+        uint32_t p[8];
+        modulus_limbs<F>(p);
+        e[0] = u_add_cc(e[0], c);
+        const uint32_t m = e[0] * F::INV;
+        row_odd<true>(o, p, m);
+        row_even(e, o, p, m);
     }
     fe r;
-    r.v[0] = u_add_cc(w[0], t[8]);
+    r.v[0] = u_add_cc(o[0], e[1]);
 #pragma unroll
-    for (int j = 1; j < 7; j++) r.v[j] = u_addc_cc(w[j], t[j + 8]);
-    r.v[7] = u_addc(w[7], t[15]);
+    for (int j = 1; j < 7; j++) r.v[j] = u_addc_cc(o[j], e[j + 1]);
+    r.v[7] = u_addc(o[7], t[15]);
     return r;
 }
 
@@ -708,44 +692,21 @@ __host__ __device__ __forceinline__ fe fe_sqr_sos(const fe& a) {
     return sos_redc<F>(t);
 }
 
-// a b * 2^-256 mod p in [0, 2p) for a, b in [0, 2p): product rows, then the reduction
+// a b * 2^-256 mod p in [0, 2p) for a, b in [0, 2p): product, then the reduction
 template <class F>
 __host__ __device__ __forceinline__ fe fe_mul_sos(const fe& a, const fe& b) {
     static_assert(F::LAZY, "the separated forms keep lazy values");
     uint32_t t[16];
-    sos_row<0, true>(t, a.v, b.v[0]);
-    sos_row<1, true>(t, a.v, b.v[1]);
-    sos_row<2, true>(t, a.v, b.v[2]);
-    sos_row<3, true>(t, a.v, b.v[3]);
-    sos_row<4, true>(t, a.v, b.v[4]);
-    sos_row<5, true>(t, a.v, b.v[5]);
-    sos_row<6, true>(t, a.v, b.v[6]);
-    sos_row<7, true>(t, a.v, b.v[7]);
+    sos_mul_wide(t, a.v, b.v);
     return sos_redc<F>(t);
 }
 
-// (a b + c d) * 2^-256 mod p in [0, 2p) for inputs in [0, 2p] (one reduction)
+// (a b + c d) * 2^-256 mod p in [0, 2p) for inputs in [0, 2p] (one reduction, 192 wide
+// multiply-adds instead of 256)
 template <class F>
 __host__ __device__ __forceinline__ fe fe_mul_add_sos(const fe& a, const fe& b, const fe& c, const fe& d) {
     static_assert(F::LAZY, "the separated forms keep lazy values");
-    uint32_t t[16];
-    sos_row<0, true>(t, a.v, b.v[0]);
-    sos_row<0, false>(t, c.v, d.v[0]);
-    sos_row<1, true>(t, a.v, b.v[1]);
-    sos_row<1, false>(t, c.v, d.v[1]);
-    sos_row<2, true>(t, a.v, b.v[2]);
-    sos_row<2, false>(t, c.v, d.v[2]);
-    sos_row<3, true>(t, a.v, b.v[3]);
-    sos_row<3, false>(t, c.v, d.v[3]);
-    sos_row<4, true>(t, a.v, b.v[4]);
-    sos_row<4, false>(t, c.v, d.v[4]);
-    sos_row<5, true>(t, a.v, b.v[5]);
-    sos_row<5, false>(t, c.v, d.v[5]);
-    sos_row<6, true>(t, a.v, b.v[6]);
-    sos_row<6, false>(t, c.v, d.v[6]);
-    sos_row<7, true>(t, a.v, b.v[7]);
-    sos_row<7, false>(t, c.v, d.v[7]);
-    return sos_reduce_2p<F>(sos_redc<F>(t));
+    return sos_reduce_2p<F>(mul_add_rows<F>(a, b, c, d));
 }
 
 // (a b - c d) * 2^-256 mod p in [0, 2p) for inputs in [0, 2p): a b + (2p - c) d
@@ -757,8 +718,7 @@ __host__ __device__ __forceinline__ fe fe_mul_sub_sos(const fe& a, const fe& b, 
 // Fq2 product with lazy reduction (Karatsuba): T0 = a0 b0, T1 = a1 b1, T2 = (a0 + a1)(b0 + b1)
 // as 512-bit products, c0 = redc(T0 + (4q^2 - T1)), c1 = redc(T2 - T0 - T1) = redc(a0 b1 + a1 b0):
 // 3 products and 2 reductions instead of 3 full products. Inputs in [0, 2q): the sums a0 + a1
-// stay below 4q < 2^256 unreduced (one product row stays inside its 9 limbs for any 256-bit
-// operand), both arguments of the reductions are below 8q^2, results in [0, 2q).
+// stay below 4q < 2^256 unreduced, both arguments of the reductions are below 8q^2, results in [0, 2q).
 struct fe_pair {
     fe c0, c1;
 };
@@ -767,22 +727,8 @@ template <class F>
 __host__ __device__ __forceinline__ fe_pair fe2_mul_lazy(const fe& a0, const fe& a1, const fe& b0, const fe& b1) {
     static_assert(F::LAZY, "the separated forms keep lazy values");
     uint32_t t0[16], t1[16];
-    sos_row<0, true>(t0, a0.v, b0.v[0]);
-    sos_row<1, true>(t0, a0.v, b0.v[1]);
-    sos_row<2, true>(t0, a0.v, b0.v[2]);
-    sos_row<3, true>(t0, a0.v, b0.v[3]);
-    sos_row<4, true>(t0, a0.v, b0.v[4]);
-    sos_row<5, true>(t0, a0.v, b0.v[5]);
-    sos_row<6, true>(t0, a0.v, b0.v[6]);
-    sos_row<7, true>(t0, a0.v, b0.v[7]);
-    sos_row<0, true>(t1, a1.v, b1.v[0]);
-    sos_row<1, true>(t1, a1.v, b1.v[1]);
-    sos_row<2, true>(t1, a1.v, b1.v[2]);
-    sos_row<3, true>(t1, a1.v, b1.v[3]);
-    sos_row<4, true>(t1, a1.v, b1.v[4]);
-    sos_row<5, true>(t1, a1.v, b1.v[5]);
-    sos_row<6, true>(t1, a1.v, b1.v[6]);
-    sos_row<7, true>(t1, a1.v, b1.v[7]);
+    sos_mul_wide(t0, a0.v, b0.v);
+    sos_mul_wide(t1, a1.v, b1.v);
     // u = T0 + (4q^2 - T1) in (0, 8q^2); s = T0 + T1 (below 8q^2)
     uint32_t u[16], s[16];
     u[0] = u_sub_cc(F::FOUR_P_SQ(0), t1[0]);
@@ -810,14 +756,7 @@ __host__ __device__ __forceinline__ fe_pair fe2_mul_lazy(const fe& a0, const fe&
     for (int j = 1; j < 7; j++) sb.v[j] = u_addc_cc(b0.v[j], b1.v[j]);
     sb.v[7] = u_addc(b0.v[7], b1.v[7]);
     uint32_t t2[16];
-    sos_row<0, true>(t2, sa.v, sb.v[0]);
-    sos_row<1, true>(t2, sa.v, sb.v[1]);
-    sos_row<2, true>(t2, sa.v, sb.v[2]);
-    sos_row<3, true>(t2, sa.v, sb.v[3]);
-    sos_row<4, true>(t2, sa.v, sb.v[4]);
-    sos_row<5, true>(t2, sa.v, sb.v[5]);
-    sos_row<6, true>(t2, sa.v, sb.v[6]);
-    sos_row<7, true>(t2, sa.v, sb.v[7]);
+    sos_mul_wide(t2, sa.v, sb.v);
     t2[0] = u_sub_cc(t2[0], s[0]);
 #pragma unroll
     for (int j = 1; j < 15; j++) t2[j] = u_subc_cc(t2[j], s[j]);
