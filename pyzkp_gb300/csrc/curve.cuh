@@ -220,8 +220,45 @@ __device__ __forceinline__ XyzzT<T> xyzz_dbl(const XyzzT<T>& p) {
     return r;
 }
 
-// acc + (x, y), (x, y) affine and not infinity.
+// The products of a formula: through the one non-inlined copy, or (Inline) inlined at every
+// site, for a loop that holds one formula and runs it often enough to keep it in the
+// instruction cache.
 template <class T>
+struct CallOps {
+    static __device__ __forceinline__ T mul(const T& a, const T& b) { return c_mul(a, b); }
+    static __device__ __forceinline__ T sqr(const T& a) { return c_sqr(a); }
+    static __device__ __forceinline__ T mul_sub(const T& a, const T& b, const T& c, const T& d) {
+        return c_mul_sub(a, b, c, d);
+    }
+};
+
+template <class T>
+struct InlineOps;
+template <>
+struct InlineOps<fe> {
+    static __device__ __forceinline__ fe mul(const fe& a, const fe& b) { return mul_rows<FqP>(a, b); }
+    static __device__ __forceinline__ fe sqr(const fe& a) { return fe_sqr_sos<FqP>(a); }
+    static __device__ __forceinline__ fe mul_sub(const fe& a, const fe& b, const fe& c, const fe& d) {
+        return fe_mul_sub_sos<FqP>(a, b, c, d);
+    }
+};
+template <>
+struct InlineOps<fq2> {
+    static __device__ __forceinline__ fq2 mul(const fq2& a, const fq2& b) {
+        const fe_pair r = fe2_mul_lazy<FqP>(a.c0, a.c1, b.c0, b.c1);
+        return {r.c0, r.c1};
+    }
+    static __device__ __forceinline__ fq2 sqr(const fq2& a) {
+        const fe t0 = mul_rows<FqP>(c_add(a.c0, a.c1), c_sub(a.c0, a.c1));
+        return {t0, c_dbl(mul_rows<FqP>(a.c0, a.c1))};
+    }
+    static __device__ __forceinline__ fq2 mul_sub(const fq2& a, const fq2& b, const fq2& c, const fq2& d) {
+        return c_sub(mul(a, b), mul(c, d));
+    }
+};
+
+// acc + (x, y), (x, y) affine and not infinity.
+template <class T, class Ops = CallOps<T>>
 __device__ __forceinline__ XyzzT<T> xyzz_madd(const XyzzT<T>& acc, const T& x, const T& y) {
     if (xyzz_is_inf(acc)) {
         XyzzT<T> r;
@@ -231,21 +268,20 @@ __device__ __forceinline__ XyzzT<T> xyzz_madd(const XyzzT<T>& acc, const T& x, c
         c_set_one(r.ZZZ);
         return r;
     }
-    const c_pair<T> us = c_mul2(x, acc.ZZ, y, acc.ZZZ);  // U2, S2
-    const T P = c_sub(us.x, acc.X);
-    const T R = c_sub(us.y, acc.Y);
+    const T P = c_sub(Ops::mul(x, acc.ZZ), acc.X);   // U2 - X
+    const T R = c_sub(Ops::mul(y, acc.ZZZ), acc.Y);  // S2 - Y
     if (c_is_zero(P)) {
         if (c_is_zero(R)) return xyzz_dbl_affine(x, y);
         return xyzz_inf<T>();
     }
-    const c_pair<T> pr = c_sqr2(P, R);                  // PP, R^2
-    const c_pair<T> pq = c_mul2(P, pr.x, acc.X, pr.x);  // PPP, Q
+    const T PP = Ops::sqr(P);
     XyzzT<T> r;
-    r.X = c_sub(c_sub(pr.y, pq.x), c_dbl(pq.y));
-    const c_pair<T> zz = c_mul2(acc.ZZ, pr.x, acc.ZZZ, pq.x);
-    r.Y = c_mul_sub(R, c_sub(pq.y, r.X), acc.Y, pq.x);
-    r.ZZ = zz.x;
-    r.ZZZ = zz.y;
+    r.ZZ = Ops::mul(acc.ZZ, PP);
+    const T PPP = Ops::mul(P, PP);
+    const T Q = Ops::mul(acc.X, PP);
+    r.ZZZ = Ops::mul(acc.ZZZ, PPP);
+    r.X = c_sub(c_sub(Ops::sqr(R), PPP), c_dbl(Q));
+    r.Y = Ops::mul_sub(R, c_sub(Q, r.X), acc.Y, PPP);
     return r;
 }
 
@@ -322,8 +358,8 @@ __device__ __forceinline__ void xyzz_store(XyzzT<T>* p, const XyzzT<T>& a) {
 
 // The two groups as template arguments of the MSM kernels.
 // Minimum resident 128-thread CTAs per SM asked of the G1 accumulation: 4 caps it at 128
-// registers (no spills), 16 warps per SM; measured on GB300 against no cap (130 registers,
-// 12 warps): 3.26 / 3.29 ms at 2^20, 12.80 / 12.92 ms at 2^22.
+// registers (no spills), 16 warps per SM; measured on GB300 at 2^20 with 3 / 4 / 5: 2.26 / 2.18 /
+// 2.17 ms.
 #ifndef ZK_ACC_MINB
 #define ZK_ACC_MINB 4
 #endif

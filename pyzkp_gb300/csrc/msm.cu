@@ -791,7 +791,13 @@ __device__ __forceinline__ uint32_t bucket_of(const uint32_t* __restrict__ row_p
 }
 
 // Unit u: the CSR entries [u seg, (u + 1) seg) (M = total entries), bucket by bucket.
-template <class C, bool kSkipInf>
+//
+// What bounds the accumulation: the wide multiply-adds of the mixed addition, 1160 a G1 entry
+// (7 products, a product pair with one reduction, two squares) = 1.93 ms at 2^20 (16.8 M entries).
+// Measured there: 2.18 ms with the formula's products inlined in this one loop (2.37 ms
+// through the called product), the entry read one ahead 2.17 ms; prefetching its point too
+// measured the same, 3 or 5 CTAs per SM instead of 4: 2.26 / 2.17 ms. G2 2^16: 0.685 -> 0.672 ms.
+template <class C, bool kSkipInf, class Ops = CallOps<typename C::T>>
 __device__ __forceinline__ void acc_unit(const uint32_t* __restrict__ entries, uint32_t M,
                                          const uint32_t* __restrict__ row_ptr, const MsmInst* __restrict__ insts,
                                          const MsmShape& sh, uint32_t u, typename C::P* buckets, uint32_t* slot_keys,
@@ -807,6 +813,7 @@ __device__ __forceinline__ void acc_unit(const uint32_t* __restrict__ entries, u
     uint32_t end = row_ptr[cur + 1];  // > e0
     const A* bases = key_bases<C>(insts, sh, cur);
     P acc = xyzz_inf<typename C::T>();
+    uint32_t next = entries[e0];
     for (uint32_t e = e0; e < e1; e++) {
         if (e == end) {  // bucket cur ends here: emit it, move to the next non-empty bucket
             emit_piece(cur, acc, e0, e1, row_ptr, buckets, slot_keys, slot_pts, u);
@@ -817,12 +824,13 @@ __device__ __forceinline__ void acc_unit(const uint32_t* __restrict__ entries, u
             bases = key_bases<C>(insts, sh, cur);
             acc = xyzz_inf<typename C::T>();
         }
-        const uint32_t ent = entries[e];
+        const uint32_t ent = next;
+        if (e + 1 < e1) next = entries[e + 1];  // its latency passes behind this addition
         A p = affine_load(bases + (ent & 0x7fffffffu));
         if constexpr (kSkipInf)
             if (test_inf && affine_is_zero_bits(p)) continue;  // an infinity base adds nothing
         if (ent >> 31) p.y = c_neg(p.y);
-        acc = xyzz_madd(acc, p.x, p.y);
+        acc = xyzz_madd<typename C::T, Ops>(acc, p.x, p.y);
     }
     emit_piece(cur, acc, e0, e1, row_ptr, buckets, slot_keys, slot_pts, u);
 }
@@ -840,7 +848,8 @@ __global__ void __launch_bounds__(128, C::kAccMinBlocks) msm_accumulate_kernel(c
     if (u >= units) return;
     // kSkipInf: the points may hold infinity; a flag (when given) says whether they do
     const bool test_inf = kSkipInf && (inf_flag == nullptr || *inf_flag != 0);
-    acc_unit<C, kSkipInf>(entries, *d_total, row_ptr, insts, sh, u, buckets, slot_keys, slot_pts, test_inf);
+    acc_unit<C, kSkipInf, InlineOps<typename C::T>>(entries, *d_total, row_ptr, insts, sh, u, buckets, slot_keys,
+                                                    slot_pts, test_inf);
 }
 
 // Round r >= 2: unit u merges the slots of units [u*group, (u+1)*group) of the previous
