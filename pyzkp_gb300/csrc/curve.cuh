@@ -356,6 +356,140 @@ __device__ __forceinline__ void xyzz_store(XyzzT<T>* p, const XyzzT<T>& a) {
     c_store(&p->ZZZ, a.ZZZ);
 }
 
+// ---- points held by four lanes -------------------------------------------------------------
+// A quad (lanes 4k .. 4k + 3 of a warp) holds one point, lane l its l-th coordinate (X, Y, ZZ,
+// ZZZ), and adds two points with the four independent products of each step side by side: 4
+// product times instead of 13, at 16 product slots instead of 13 products. For the trees and
+// chains of the window reduction and the fixup, whose threads are too few to fill the chip:
+// one addition takes a warp ~4.6 us alone with a point per thread, ~2 us with a point per
+// quad. Every lane of the warp calls; quads without work pass infinity (all zero).
+template <class T>
+struct QuadOps {
+    using Ops = InlineOps<T>;
+};
+template <>
+struct QuadOps<fq2> {
+    using Ops = CallOps<fq2>;  // four inlined Fq2 products would fill the instruction cache
+};
+
+__device__ __forceinline__ fe c_shfl(const fe& a, int src) {  // src: lane of the quad
+    fe r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = __shfl_sync(0xffffffffu, a.v[i], src, 4);
+    return r;
+}
+__device__ __forceinline__ fe c_shfl_xor(const fe& a, int mask) {
+    fe r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = __shfl_xor_sync(0xffffffffu, a.v[i], mask);
+    return r;
+}
+__device__ __forceinline__ fq2 c_shfl(const fq2& a, int src) { return {c_shfl(a.c0, src), c_shfl(a.c1, src)}; }
+__device__ __forceinline__ fq2 c_shfl_xor(const fq2& a, int mask) {
+    return {c_shfl_xor(a.c0, mask), c_shfl_xor(a.c1, mask)};
+}
+__device__ __forceinline__ fe c_sel(bool c, const fe& a, const fe& b) {  // c ? a : b
+    fe r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = c ? a.v[i] : b.v[i];
+    return r;
+}
+__device__ __forceinline__ fq2 c_sel(bool c, const fq2& a, const fq2& b) {
+    return {c_sel(c, a.c0, b.c0), c_sel(c, a.c1, b.c1)};
+}
+
+// The lane's coordinate of 2 P (rare: a quad whose two points are equal): gathered, doubled by
+// every lane, its own coordinate taken.
+template <class T>
+__device__ __noinline__ T quad_dbl(const T p) {
+    const int l = threadIdx.x & 3;
+    const XyzzT<T> d = xyzz_dbl(XyzzT<T>{c_shfl(p, 0), c_shfl(p, 1), c_shfl(p, 2), c_shfl(p, 3)});
+    return c_sel(l < 2, c_sel(l == 0, d.X, d.Y), c_sel(l == 2, d.ZZ, d.ZZZ));
+}
+
+// The lane's coordinate of P + Q (the formula and cases of xyzz_add).
+template <class T>
+__device__ __forceinline__ T quad_add(const T& p, const T& q) {
+    using Ops = typename QuadOps<T>::Ops;
+    const int l = threadIdx.x & 3;
+    const uint32_t inf = __shfl_sync(0xffffffffu, (c_is_zero(p) ? 1u : 0u) | (c_is_zero(q) ? 2u : 0u), 2, 4);
+    const T m1 = Ops::mul(p, c_shfl_xor(q, 2));  // U1 = X1 ZZ2, S1 = Y1 ZZZ2, U2 = ZZ1 X2, S2 = ZZZ1 Y2
+    const T o1 = c_shfl_xor(m1, 2);              // U2, S2, U1, S1
+    const T d = c_sub(c_sel(l < 2, o1, m1), c_sel(l < 2, m1, o1));        // P, R, P, R
+    const uint32_t dz = c_is_zero(d) ? 1u : 0u;
+    const T m2 = Ops::mul(c_sel(l < 2, d, p), c_sel(l < 2, d, q));        // P^2, R^2, ZZ1 ZZ2, ZZZ1 ZZZ2
+    const T PP = c_shfl(m2, 0);
+    const T U1 = c_shfl(m1, 0);
+    const T m3 = Ops::mul(c_sel(l == 0, d, c_sel(l == 1, U1, m2)), PP);   // PPP, Q, ZZ3, -
+    const T PPP = c_shfl(m3, 0);
+    const T S1 = c_shfl(m1, 1);
+    const T X3 = c_sub(c_sub(m2, PPP), c_dbl(m3));                        // lane 1: R^2 - PPP - 2 Q
+    const T m4 = Ops::mul(c_sel(l == 1, d, c_sel(l == 3, m2, S1)),        // S1 PPP, R (Q - X3), -, ZZZ3
+                          c_sel(l == 1, c_sub(m3, X3), PPP));
+    const T o4 = c_shfl_xor(c_sel(l == 1, X3, m4), 1);                    // lane 0: X3, lane 1: S1 PPP
+    T r = c_sel(l < 2, c_sel(l == 0, o4, c_sub(m4, o4)), c_sel(l == 2, m3, m4));
+    const uint32_t pz = __shfl_sync(0xffffffffu, dz, 0, 4), rz = __shfl_sync(0xffffffffu, dz, 1, 4);
+    if (__any_sync(0xffffffffu, pz != 0 && inf == 0)) {  // the same x: twice the point, or infinity
+        const T dbl = quad_dbl(p);
+        T zero;
+        c_set_zero(zero);
+        r = c_sel(pz != 0, c_sel(rz != 0, dbl, zero), r);
+    }
+    r = c_sel((inf & 2u) != 0, p, r);
+    return c_sel((inf & 1u) != 0, q, r);
+}
+
+// The lane's coordinate of a stored point.
+template <bool kL2, class T>
+__device__ __forceinline__ T quad_get(const XyzzT<T>* p) {
+    const T* c = reinterpret_cast<const T*>(p) + (threadIdx.x & 3);
+    if constexpr (kL2) return c_ldcg(c);
+    else return c_load(c);
+}
+
+template <class T>
+__device__ __forceinline__ void quad_put(XyzzT<T>* p, const T& v) {
+    c_store(reinterpret_cast<T*>(p) + (threadIdx.x & 3), v);
+}
+
+// Sum of `terms` points by the warp: get(t) yields the lane's coordinate of term t; quad k
+// takes the terms first + k, first + k + stride, ..., then the quads add up in a butterfly.
+// Quad 0 ends with the sum. `first` and `stride` are multiples of 8.
+template <class T, class Get>
+__device__ __forceinline__ T warp_quad_sum(uint32_t terms, uint32_t first, uint32_t stride, Get&& get) {
+    const uint32_t k = (threadIdx.x & 31) >> 2;
+    T acc;
+    c_set_zero(acc);
+    if (first + k < terms) acc = get(first + k);
+    for (uint32_t base = first + stride; base < terms; base += stride) {
+        T v;
+        c_set_zero(v);
+        if (base + k < terms) v = get(base + k);
+        acc = quad_add(acc, v);
+    }
+    const uint32_t width = first < terms ? terms - first : 0;  // quads that hold a term
+    for (uint32_t off = 1; off < 8 && off < width; off <<= 1) acc = quad_add(acc, c_shfl_xor(acc, 4 * off));
+    return acc;
+}
+
+// ... by the whole CTA (every thread calls): warps first, their sums through `red` (a point per
+// warp). The sum is valid in quad 0.
+template <class T, class Get>
+__device__ __forceinline__ T cta_quad_sum(uint32_t terms, Get&& get, XyzzT<T>* red) {
+    const uint32_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const uint32_t used = min(nwarps, (terms + 7) / 8);  // warps with terms
+    T acc;
+    c_set_zero(acc);
+    if (warp < used) acc = warp_quad_sum<T>(terms, 8 * warp, 8 * nwarps, get);
+    if (used > 1) {
+        if (warp < used && (threadIdx.x & 31) < 4) quad_put(red + warp, acc);
+        __syncthreads();
+        if (warp == 0) acc = warp_quad_sum<T>(used, 0, 8, [&](uint32_t t) { return quad_get<false>(red + t); });
+        __syncthreads();  // red free again
+    }
+    return acc;
+}
+
 // The two groups as template arguments of the MSM kernels.
 // Minimum resident 128-thread CTAs per SM asked of the G1 accumulation: 4 caps it at 128
 // registers (no spills), 16 warps per SM; measured on GB300 at 2^20 with 3 / 4 / 5: 2.26 / 2.18 /

@@ -909,29 +909,39 @@ __global__ void __launch_bounds__(128, C::kRedMinBlocks) msm_merge_kernel(const 
 #endif
 static constexpr uint64_t kFixupDensity = ZK_FIXUP_DENSITY;  // CSR entries per bucket up to which the fixup is used
 
-// Buckets of at least kHugePieces pieces (a hot digit: 10% of the scalars equal to 1 put
-// ~3300 pieces into one bucket at 2^20) are summed in chunks of about kChunkPieces pieces by
-// many CTAs, at most kMaxChunks per bucket, the last CTA to finish one adding its chunk sums
-// (one CTA for the whole bucket took 0.5 ms). Their list, count and per-bucket chunk
-// counters share the long list's count block: counts[0] long buckets, counts[1] huge
-// buckets, counts[2 .. 2 + hcap) chunks done per huge bucket, counts[2 + hcap ..] the huge
-// buckets' keys; hcap bounds the huge buckets (units / kHugePieces + 2).
+// A straddling bucket over more than fixmax + 1 units is listed for msm_fixup_long_kernel, by
+// its pieces: up to kWarpPieces for one warp (its quads), more for a CTA, and of kHugePieces
+// or more (a hot digit: 10% of the scalars equal to 1 put ~3300 pieces into one bucket at
+// 2^20) in chunks of about kChunkPieces pieces by many CTAs, at most kMaxChunks per bucket,
+// the last CTA to finish one adding its chunk sums. The warp list fills the back of
+// long_list (cap entries; the two kinds together are at most that many), the CTA list its
+// front. The count block: counts[0] CTA buckets, counts[1] huge buckets, counts[2] warp
+// buckets, counts[kCountHead .. + hcap) chunks done per huge bucket, then the huge buckets'
+// keys; hcap bounds the huge buckets (units / kHugePieces + 2).
+static constexpr uint32_t kWarpPieces = 32;
 static constexpr uint32_t kHugePieces = 2048;
 static constexpr uint32_t kChunkPieces = 256;
 static constexpr uint32_t kMaxChunks = 64;
+static constexpr uint32_t kCountHead = 3;
 
 __host__ __device__ inline uint32_t huge_cap(uint32_t units) { return units / kHugePieces + 2; }
+__host__ __device__ inline uint32_t long_cap(uint32_t units, uint32_t fixmax) { return units / fixmax + 2; }
 
 template <class C, bool kL2>
 __device__ __forceinline__ void fixup_bucket(const uint32_t* __restrict__ row_ptr, uint32_t seg, uint32_t fixmax,
                                              const typename C::P* slot_pts, typename C::P* buckets,
-                                             uint32_t* long_list, uint32_t* long_count, uint32_t hcap, uint32_t k) {
+                                             uint32_t* long_list, uint32_t lcap, uint32_t* long_count, uint32_t hcap,
+                                             uint32_t k) {
     const uint32_t b0 = row_ptr[k], b1 = row_ptr[k + 1];
     if (b1 == b0) return;
     const uint32_t u0 = b0 / seg, u1 = (b1 - 1) / seg;
     if (u0 == u1) return;  // final already (written by the accumulation)
     if (u1 - u0 >= kHugePieces) {
-        long_count[2 + hcap + atomicAdd(long_count + 1, 1u)] = k;
+        long_count[kCountHead + hcap + atomicAdd(long_count + 1, 1u)] = k;
+        return;
+    }
+    if (u1 - u0 > fixmax && u1 - u0 < kWarpPieces) {
+        long_list[lcap - 1 - atomicAdd(long_count + 2, 1u)] = k;
         return;
     }
     if (u1 - u0 > fixmax) {
@@ -948,92 +958,74 @@ __global__ void __launch_bounds__(128, C::kRedMinBlocks) msm_fixup_kernel(const 
                                                         uint32_t seg, uint32_t fixmax,
                                                         const typename C::P* __restrict__ slot_pts,
                                                         typename C::P* __restrict__ buckets,
-                                                        uint32_t* __restrict__ long_list,
+                                                        uint32_t* __restrict__ long_list, uint32_t lcap,
                                                         uint32_t* __restrict__ long_count, uint32_t hcap) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nbuckets) return;
-    fixup_bucket<C, false>(row_ptr, seg, fixmax, slot_pts, buckets, long_list, long_count, hcap, k);
+    fixup_bucket<C, false>(row_ptr, seg, fixmax, slot_pts, buckets, long_list, lcap, long_count, hcap, k);
 }
 
-// The sum of the pieces of units [ua, ub] of a bucket whose first unit is u0 (its piece is
-// slot 1, the others' slot 0), or of `n` consecutive points at `pts` when pts is given, by
-// the CTA: strided partial sums, then a shared-memory tree over `red` (blockDim points)
-// spanning the next power of two of the terms. The result is valid in thread 0.
-template <class C, bool kL2>
-__device__ __forceinline__ typename C::P cta_sum(const typename C::P* slot_pts, uint32_t u0, uint32_t ua, uint32_t ub,
-                                                 const typename C::P* pts, uint32_t n, typename C::P* red) {
-    using P = typename C::P;
-    const uint32_t terms = pts != nullptr ? n : ub - ua + 1;
-    uint32_t width = 1;
-    while (width < terms && width < blockDim.x) width <<= 1;
-    P acc = xyzz_inf<typename C::T>();
-    if (threadIdx.x < width)
-        for (uint32_t t = threadIdx.x; t < terms; t += width) {
-            const P* src = pts != nullptr ? pts + t : slot_pts + 2 * (size_t)(ua + t) + (ua + t == u0 ? 1 : 0);
-            acc = xyzz_add(acc, pts != nullptr ? xyzz_ldcg(src) : xyzz_get<kL2>(src));
-        }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (uint32_t off = width / 2; off > 0; off >>= 1) {
-        if (threadIdx.x < off) red[threadIdx.x] = xyzz_add(red[threadIdx.x], red[threadIdx.x + off]);
-        __syncthreads();
-    }
-    acc = red[0];
-    __syncthreads();  // red free again
-    return acc;
+// Piece t of a bucket whose first unit is u0: slot 1 of unit u0, slot 0 of the later ones.
+template <class P>
+__device__ __forceinline__ const P* piece_at(const P* slot_pts, uint32_t u0, uint32_t t) {
+    return slot_pts + 2 * (size_t)(u0 + t) + (t == 0 ? 1 : 0);
 }
 
 // The chunks of the huge buckets (units item0, item0 + stride, ... of the CTAs: unit
 // h kMaxChunks + ch is chunk ch of huge bucket h). A chunk sum goes to chunk_pts
 // (h kMaxChunks + ch); the CTA whose chunk completes a bucket (counted after a fence) adds
-// the bucket's chunk sums, read through L2. Nothing waits on another CTA. Not inlined: the
-// long buckets' code around its call stays as it was without it (inlined, the long-bucket
-// kernel ran 2^12 single MSMs 8 us slower).
+// the bucket's chunk sums, read through L2. Nothing waits on another CTA. Not inlined: huge
+// buckets are rare.
 template <class C, bool kL2>
 __device__ __noinline__ void fixup_huge_units(const uint32_t* __restrict__ row_ptr, uint32_t seg,
                                               const typename C::P* slot_pts, typename C::P* buckets,
                                               uint32_t* long_count, uint32_t hcap, uint32_t huge,
                                               typename C::P* chunk_pts, typename C::P* red, uint32_t* s_last,
                                               uint32_t item0, uint32_t stride) {
-    using P = typename C::P;
+    using T = typename C::T;
     for (uint32_t unit = item0; unit < huge * kMaxChunks; unit += stride) {
         const uint32_t h = unit / kMaxChunks, ch = unit % kMaxChunks;
-        const uint32_t k = kL2 ? __ldcg(long_count + 2 + hcap + h) : long_count[2 + hcap + h];
+        const uint32_t key_at = kCountHead + hcap + h;
+        const uint32_t k = kL2 ? __ldcg(long_count + key_at) : long_count[key_at];
         const uint32_t u0 = row_ptr[k] / seg, u1 = (row_ptr[k + 1] - 1) / seg;
         const uint32_t pieces = u1 - u0 + 1;
         const uint32_t nch = min(kMaxChunks, (pieces + kChunkPieces - 1) / kChunkPieces);
         if (ch >= nch) continue;  // the same for the whole CTA
         const uint32_t per = (pieces + nch - 1) / nch;
-        const uint32_t ua = u0 + ch * per, ub = min(u1, ua + per - 1);
-        P r = cta_sum<C, kL2>(slot_pts, u0, ua, ub, nullptr, 0, red);
-        if (threadIdx.x == 0) {
-            xyzz_store(chunk_pts + (size_t)h * kMaxChunks + ch, r);
+        const uint32_t t0 = ch * per, t1 = min(pieces, t0 + per);
+        T r = cta_quad_sum<T>(t1 - t0, [&](uint32_t t) { return quad_get<kL2>(piece_at(slot_pts, u0, t0 + t)); }, red);
+        if (threadIdx.x < 4) {
+            quad_put(chunk_pts + (size_t)h * kMaxChunks + ch, r);
             __threadfence();  // the chunk sum is visible before it is counted
-            *s_last = atomicAdd(long_count + 2 + h, 1u) == nch - 1 ? 1u : 0u;
         }
+        __syncthreads();
+        if (threadIdx.x == 0) *s_last = atomicAdd(long_count + kCountHead + h, 1u) == nch - 1 ? 1u : 0u;
         __syncthreads();
         if (*s_last) {  // every chunk of bucket k is done: add their sums
             __threadfence();
-            r = cta_sum<C, kL2>(nullptr, 0, 0, 0, chunk_pts + (size_t)h * kMaxChunks, nch, red);
-            if (threadIdx.x == 0) xyzz_store(buckets + k, r);
+            r = cta_quad_sum<T>(
+                nch, [&](uint32_t t) { return quad_get<true>(chunk_pts + (size_t)h * kMaxChunks + t); }, red);
+            if (threadIdx.x < 4) quad_put(buckets + k, r);
         }
         __syncthreads();  // s_last read by every thread before it is written again
     }
 }
 
-// The huge buckets' chunks, then one CTA per listed long bucket: strided partial sums, then a
-// shared-memory tree over `red` (blockDim points). Long bucket i goes to CTA
-// (i + huge kMaxChunks) mod stride, past the CTAs of the chunk units, so that the two kinds
-// of work run side by side. (One warp per long bucket with a shuffle tree measured slower:
-// 2^14 single MSM 0.127 against 0.059 ms in this kernel; the chunks in a kernel of their own
-// before this one serialised the two, witness-like 2^20 0.25 against 0.14 ms.)
+// The huge buckets' chunks, then the listed buckets of more than kWarpPieces pieces, one CTA
+// each, and those of fewer, one warp each. The latter two kinds start past the CTAs of the
+// chunk units, so that the kinds of work run side by side.
+//
+// What bounds it: chains of dependent additions, so a point is held by four lanes (quad_add)
+// and a bucket of 16 pieces takes one serial addition and three butterfly levels. Measured
+// (events, against a point per thread and a CTA tree per bucket): 2^12 39 -> 19 us, 100003
+// witness-like 61 -> 29 us, G2 2^16 191 -> 51 us.
 template <class C, bool kL2>
 __device__ __forceinline__ void fixup_long_cta(const uint32_t* __restrict__ row_ptr, uint32_t seg,
                                                const typename C::P* slot_pts, typename C::P* buckets,
-                                               const uint32_t* long_list, uint32_t* long_count, uint32_t hcap,
-                                               typename C::P* chunk_pts, typename C::P* red, uint32_t item0,
-                                               uint32_t stride) {
-    using P = typename C::P;
+                                               const uint32_t* long_list, uint32_t lcap, uint32_t* long_count,
+                                               uint32_t hcap, typename C::P* chunk_pts, typename C::P* red,
+                                               uint32_t item0, uint32_t stride) {
+    using T = typename C::T;
     __shared__ uint32_t s_last;
     const uint32_t huge = kL2 ? __ldcg(long_count + 1) : long_count[1];
     if (huge != 0)
@@ -1041,25 +1033,24 @@ __device__ __forceinline__ void fixup_long_cta(const uint32_t* __restrict__ row_
                                  item0, stride);
     const uint32_t count = kL2 ? __ldcg(long_count) : *long_count;
     const uint32_t shift = (uint32_t)(((uint64_t)huge * kMaxChunks) % stride);
-    for (uint32_t item = (item0 + stride - shift) % stride; item < count; item += stride) {
+    const uint32_t cta = (item0 + stride - shift) % stride;
+    for (uint32_t item = cta; item < count; item += stride) {
         const uint32_t k = kL2 ? __ldcg(long_list + item) : long_list[item];
         const uint32_t u0 = row_ptr[k] / seg, u1 = (row_ptr[k + 1] - 1) / seg;
-        // the tree spans the next power of two of the pieces (at most the CTA): a bucket of 16
-        // segments takes 4 levels of serial additions, not log2(blockDim)
-        uint32_t width = 1;
-        while (width < u1 - u0 + 1 && width < blockDim.x) width <<= 1;
-        P acc = xyzz_inf<typename C::T>();
-        if (threadIdx.x < width)
-            for (uint32_t u = u0 + threadIdx.x; u <= u1; u += width)
-                acc = xyzz_add(acc, xyzz_get<kL2>(slot_pts + 2 * (size_t)u + (u == u0 ? 1 : 0)));
-        red[threadIdx.x] = acc;
-        __syncthreads();
-        for (uint32_t off = width / 2; off > 0; off >>= 1) {
-            if (threadIdx.x < off) red[threadIdx.x] = xyzz_add(red[threadIdx.x], red[threadIdx.x + off]);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) xyzz_store(buckets + k, red[0]);
-        __syncthreads();
+        const T r = cta_quad_sum<T>(
+            u1 - u0 + 1, [&](uint32_t t) { return quad_get<kL2>(piece_at(slot_pts, u0, t)); }, red);
+        if (threadIdx.x < 4) quad_put(buckets + k, r);
+    }
+    // past the CTAs that just had a bucket of their own; one bucket per CTA before a second
+    const uint32_t small = kL2 ? __ldcg(long_count + 2) : long_count[2];
+    const uint32_t base = (cta + stride - count % stride) % stride;
+    for (uint32_t item = base + stride * (threadIdx.x >> 5); item < small; item += stride * (blockDim.x >> 5)) {
+        const uint32_t* at = long_list + (lcap - 1 - item);
+        const uint32_t k = kL2 ? __ldcg(at) : *at;
+        const uint32_t u0 = row_ptr[k] / seg, u1 = (row_ptr[k + 1] - 1) / seg;
+        const T r = warp_quad_sum<T>(u1 - u0 + 1, 0, 8,
+                                     [&](uint32_t t) { return quad_get<kL2>(piece_at(slot_pts, u0, t)); });
+        if ((threadIdx.x & 31) < 4) quad_put(buckets + k, r);
     }
 }
 
@@ -1069,12 +1060,13 @@ __global__ void __launch_bounds__(C::kFixupLongThreads, C::kFixupLongMinBlocks) 
                                                                            const typename C::P* __restrict__ slot_pts,
                                                                            typename C::P* __restrict__ buckets,
                                                                            const uint32_t* __restrict__ long_list,
+                                                                           uint32_t lcap,
                                                                            uint32_t* __restrict__ long_count,
                                                                            uint32_t hcap,
                                                                            typename C::P* __restrict__ chunk_pts) {
-    __shared__ typename C::P red[C::kFixupLongThreads];
-    fixup_long_cta<C, false>(row_ptr, seg, slot_pts, buckets, long_list, long_count, hcap, chunk_pts, red, blockIdx.x,
-                             gridDim.x);
+    __shared__ typename C::P red[C::kFixupLongThreads / 32];
+    fixup_long_cta<C, false>(row_ptr, seg, slot_pts, buckets, long_list, lcap, long_count, hcap, chunk_pts, red,
+                             blockIdx.x, gridDim.x);
 }
 
 // ---- 5. window reduction ----------------------------------------------------------------
@@ -1160,24 +1152,14 @@ __device__ __forceinline__ void targets_cta(const typename C::P* P0, const typen
     const uint32_t per = (count + parts - 1) / parts;
     const uint32_t t0 = part * per, t1 = min(count, t0 + per);
     const uint32_t k = bits ? tg - sh.plain : 0;
-    // the tree spans the next power of two of this slice's terms (at most the CTA)
-    const uint32_t terms = t1 > t0 ? t1 - t0 : 0;
-    uint32_t width = 1;
-    while (width < terms && width < blockDim.x) width <<= 1;
-    P acc = xyzz_inf<typename C::T>();
-    if (threadIdx.x < width)
-        for (uint32_t t = t0 + threadIdx.x; t < t1; t += width) {
-            uint32_t j = t;
-            if (bits) j = ((t >> k) << (k + 1)) | (1u << k) | (t & ((1u << k) - 1));
-            acc = xyzz_add(acc, xyzz_get<kL2>(src + j));
-        }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (uint32_t off = width / 2; off > 0; off >>= 1) {
-        if (threadIdx.x < off) red[threadIdx.x] = xyzz_add(red[threadIdx.x], red[threadIdx.x + off]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[blk] = red[0];
+    const typename C::T r = cta_quad_sum<typename C::T>(
+        t1 > t0 ? t1 - t0 : 0,
+        [&](uint32_t i) {
+            const uint32_t t = t0 + i;
+            return quad_get<kL2>(src + (bits ? ((t >> k) << (k + 1)) | (1u << k) | (t & ((1u << k) - 1)) : t));
+        },
+        red);
+    if (threadIdx.x < 4) quad_put(out + blk, r);
 }
 
 template <class C>
@@ -1187,38 +1169,27 @@ __global__ void __launch_bounds__(C::kTargetThreads) msm_targets_kernel(const ty
                                                                         const typename C::P* __restrict__ Ylast,
                                                                         MsmShape sh, uint32_t parts,
                                                                         typename C::P* __restrict__ out) {
-    __shared__ typename C::P red[C::kTargetThreads];
+    __shared__ typename C::P red[C::kTargetThreads / 32];
     targets_cta<C, false>(P0, P1, P2, Ylast, sh, parts, out, red, blockIdx.x);
 }
 
-// The parts of each target summed: one CTA of kMergeThreads per (window, target).
+// The parts of each target summed: one warp per (window, target).
 static constexpr uint32_t kMergeThreads = 32;
 
 template <class C, bool kL2>
-__device__ __forceinline__ void targets_merge_cta(const typename C::P* in, uint32_t parts, typename C::P* out,
-                                                  typename C::P* red, uint32_t blk) {
-    using P = typename C::P;
-    const P* src = in + (size_t)blk * parts;
-    uint32_t width = 1;
-    while (width < parts && width < blockDim.x) width <<= 1;
-    P acc = xyzz_inf<typename C::T>();
-    if (threadIdx.x < width)
-        for (uint32_t t = threadIdx.x; t < parts; t += width) acc = xyzz_add(acc, xyzz_get<kL2>(src + t));
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (uint32_t off = width / 2; off > 0; off >>= 1) {
-        if (threadIdx.x < off) red[threadIdx.x] = xyzz_add(red[threadIdx.x], red[threadIdx.x + off]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[blk] = red[0];
+__device__ __forceinline__ void targets_merge_warp(const typename C::P* in, uint32_t parts, typename C::P* out,
+                                                   uint32_t blk) {
+    const typename C::P* src = in + (size_t)blk * parts;
+    const typename C::T r =
+        warp_quad_sum<typename C::T>(parts, 0, 8, [&](uint32_t t) { return quad_get<kL2>(src + t); });
+    if (threadIdx.x < 4) quad_put(out + blk, r);
 }
 
 template <class C>
 __global__ void __launch_bounds__(kMergeThreads) msm_targets_merge_kernel(const typename C::P* __restrict__ in,
                                                                           uint32_t parts,
                                                                           typename C::P* __restrict__ out) {
-    __shared__ typename C::P red[kMergeThreads];
-    targets_merge_cta<C, false>(in, parts, out, red, blockIdx.x);
+    targets_merge_warp<C, false>(in, parts, out, blockIdx.x);
 }
 
 // ---- persistent form of the post-sort stages (work queue) ----------------------------------
@@ -1247,7 +1218,7 @@ struct MsmQPipe {
     uint32_t* long_count;  // the count block (see fixup_bucket), hcap huge buckets at most
     P *Yb, *Eb, *Y2, *E2, *F2, *tgt_out, *tgt;
     MsmShape sh;
-    uint32_t units, nbuckets, parts, skip_inf, hcap;
+    uint32_t units, nbuckets, parts, skip_inf, hcap, lcap;
 };
 
 struct MsmQEntry {
@@ -1268,7 +1239,7 @@ __global__ void __launch_bounds__(kMsmQThreads, 2) msm_queue_kernel(const MsmQPi
                                                                    const uint64_t* __restrict__ limit,
                                                                    uint32_t* sticky) {
     using P = typename C::P;
-    __shared__ P red[kMsmQThreads];
+    __shared__ P red[kMsmQThreads / 32];
     __shared__ MsmQEntry sE;
     __shared__ MsmQPipe<C> sQ;
     __shared__ uint32_t s_next, s_item, s_entry, s_tile, s_stop;
@@ -1355,11 +1326,11 @@ __global__ void __launch_bounds__(kMsmQThreads, 2) msm_queue_kernel(const MsmQPi
             case kQFix:
                 if (i < q.nbuckets)
                     fixup_bucket<C, true>(q.row_ptr, q.sh.seg, q.sh.fixmax, q.slot_pts[0], q.buckets, q.long_list,
-                                          q.long_count, q.hcap, i);
+                                          q.lcap, q.long_count, q.hcap, i);
                 break;
             case kQFixLong:
-                fixup_long_cta<C, true>(q.row_ptr, q.sh.seg, q.slot_pts[0], q.buckets, q.long_list, q.long_count,
-                                        q.hcap, q.slot_pts[1], red, b, sE.items);
+                fixup_long_cta<C, true>(q.row_ptr, q.sh.seg, q.slot_pts[0], q.buckets, q.long_list, q.lcap,
+                                        q.long_count, q.hcap, q.slot_pts[1], red, b, sE.items);
                 break;
             case kQBlk1:
                 if (i < q.sh.sets * q.sh.G) blocks_thread<C, true>(q.buckets, q.sh, q.Yb, q.Eb, i);
@@ -1372,7 +1343,7 @@ __global__ void __launch_bounds__(kMsmQThreads, 2) msm_queue_kernel(const MsmQPi
                 else targets_cta<C, true>(q.Eb, q.Yb, q.Yb, q.Yb, q.sh, q.parts, q.tgt_out, red, b);
                 break;
             case kQTMerge:
-                targets_merge_cta<C, true>(q.tgt_out, q.parts, q.tgt, red, b);
+                if (threadIdx.x < 32) targets_merge_warp<C, true>(q.tgt_out, q.parts, q.tgt, b);
                 break;
         }
         __syncthreads();  // every store of the item issued; sE, sQ and red free again
@@ -1669,9 +1640,9 @@ static size_t pipe_layout(MsmPipeT<C>& p, char* base) {
     p.slot_pts_a = reinterpret_cast<P*>(take((size_t)2 * p.units * sizeof(P)));
     p.slot_keys_b = reinterpret_cast<uint32_t*>(take(2 * first_out * 4));
     p.slot_pts_b = reinterpret_cast<P*>(take(2 * first_out * sizeof(P)));
-    p.long_list = reinterpret_cast<uint32_t*>(take(((size_t)p.units / sh.fixmax + 2) * 4));
+    p.long_list = reinterpret_cast<uint32_t*>(take((size_t)long_cap(p.units, sh.fixmax) * 4));
     // the count block: long and huge counts, the huge buckets' chunk counters and keys
-    p.long_count = reinterpret_cast<uint32_t*>(take((2 + 2 * (size_t)huge_cap(p.units)) * 4));
+    p.long_count = reinterpret_cast<uint32_t*>(take((kCountHead + 2 * (size_t)huge_cap(p.units)) * 4));
     p.buckets = reinterpret_cast<P*>(take(p.nbuckets * sizeof(P)));
     p.Yb = reinterpret_cast<P*>(take((size_t)sh.sets * sh.G * sizeof(P)));
     p.Eb = reinterpret_cast<P*>(take((size_t)sh.sets * sh.G * sizeof(P)));
@@ -1850,15 +1821,16 @@ static int pipe_enqueue_reduce(Ctx* c, MsmPipeT<C>& p) {
     if (p.max_entries <= (uint64_t)p.nbuckets * kFixupDensity) {
         const uint32_t hcap = huge_cap(p.units);
         // counts and chunk counters to zero (the keys are written before they are read)
-        ZK_TRY_CUDA(cudaMemsetAsync(p.long_count, 0, (2 + (size_t)hcap) * 4, st));
+        const uint32_t lcap = long_cap(p.units, sh.fixmax);
+        ZK_TRY_CUDA(cudaMemsetAsync(p.long_count, 0, (kCountHead + (size_t)hcap) * 4, st));
         ZK_LAUNCH(c, "msm_fixup", msm_fixup_kernel<C>, (unsigned)((p.nbuckets + 127) / 128), 128, 0, p.row_ptr,
-                  (uint32_t)p.nbuckets, sh.seg, sh.fixmax, p.slot_pts_a, p.buckets, p.long_list, p.long_count, hcap);
+                  (uint32_t)p.nbuckets, sh.seg, sh.fixmax, p.slot_pts_a, p.buckets, p.long_list, lcap, p.long_count, hcap);
         ZK_TRY_CUDA(cudaGetLastError());
         // the chunk sums of huge buckets go to slot_pts_b (merge-round space, unused in fixup mode)
         // as many CTAs as fit at once (at least 2 per SM)
         ZK_LAUNCH(c, "msm_fixup_long", msm_fixup_long_kernel<C>,
                   (unsigned)(c->num_sms * std::max(2, C::kFixupLongMinBlocks)), C::kFixupLongThreads, 0,
-                  p.row_ptr, sh.seg, p.slot_pts_a, p.buckets, p.long_list, p.long_count, hcap, p.slot_pts_b);
+                  p.row_ptr, sh.seg, p.slot_pts_a, p.buckets, p.long_list, lcap, p.long_count, hcap, p.slot_pts_b);
         ZK_TRY_CUDA(cudaGetLastError());
     } else {
         uint64_t span = sh.seg;
@@ -2407,6 +2379,7 @@ static int queue_fill(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, MsmQueueT<C
         d.long_list = p.long_list;
         d.long_count = p.long_count;
         d.hcap = huge_cap(p.units);
+        d.lcap = long_cap(p.units, p.sh.fixmax);
         d.Yb = p.Yb;
         d.Eb = p.Eb;
         d.Y2 = p.Y2;
@@ -2436,7 +2409,7 @@ static int queue_launch(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, MsmQueueT
     ZK_TRY_CUDA(cudaMemsetAsync(state, 0, (kQueueDone + q.qe.size()) * 4, c->stream));
     for (size_t k = 0; k < pipes.size(); k++)
         if (q.fixup_mode[k])
-            ZK_TRY_CUDA(cudaMemsetAsync(pipes[k].long_count, 0, (2 + (size_t)huge_cap(pipes[k].units)) * 4, c->stream));
+            ZK_TRY_CUDA(cudaMemsetAsync(pipes[k].long_count, 0, (kCountHead + (size_t)huge_cap(pipes[k].units)) * 4, c->stream));
     if (c->bases_wait != nullptr) ZK_TRY_CUDA(cudaStreamWaitEvent(c->stream, c->bases_wait, 0));
     if constexpr (kQueueForm<C>) {
         ZK_LAUNCH(c, "msm_queue", msm_queue_kernel<C>, q.grid, kMsmQThreads, 0,
