@@ -524,7 +524,6 @@ struct CurveG1 {
     using T = fe;
     using A = affine_t;
     using P = xyzz_t;
-    static constexpr int kTargetThreads = 256;
     static constexpr int kAccMinBlocks = ZK_ACC_MINB;
     static constexpr int kFixupLongThreads = ZK_FIXUP_LONG_G1;
     static constexpr int kFixupLongMinBlocks = ZK_FIXUP_LONG_MINB_G1;
@@ -535,7 +534,6 @@ struct CurveG2 {
     using T = fq2;
     using A = affine2_t;
     using P = xyzz2_t;
-    static constexpr int kTargetThreads = 128;  // 128 x 256-byte points of shared memory
     static constexpr int kAccMinBlocks = ZK_ACC_MINB_G2;
     static constexpr int kFixupLongThreads = 128;
     static constexpr int kFixupLongMinBlocks = 1;

@@ -26,10 +26,12 @@
 //                         thread per bucket adds (short buckets), or tree rounds (pairs,
 //                         then groups of 4 units) merge, deciding "straddles" from the row
 //                         pointers.
-//  5. msm_bucket_blocks   per window, blocks of g buckets: sum_b b*B_b = sum_j E_j + g*WS(Y)
-//                         with Y_j the block sums and E_j = -(sum of the g-1 prefix sums).
-//  6. msm_targets_kernel  WS(Y) = sum_j Y_j + sum_k 2^k M_k with M_k the sum of the Y_j
-//                         whose index has bit k set: plain sums, reduced by CTA trees.
+//  5. msm_bucket_blocks   per window, blocks of g buckets (large pipelines): sum_b b*B_b =
+//                         sum_j E_j + g*WS(Y) with Y_j the block sums and E_j = -(sum of the
+//                         g-1 prefix sums).
+//  6. msm_lines, msm_targets  WS(Y) = sum_j Y_j + sum_k 2^k M_k with M_k the sum of the Y_j whose
+//                         index has bit k set: row and column sums of the index laid out as a
+//                         square, then the targets from those.
 //  7. host: per window S_w = T_E + g (T_Y + sum_k 2^k M_k), then Horner over windows.
 #include <algorithm>
 #include <atomic>
@@ -66,13 +68,13 @@ static constexpr uint32_t kSegment = ZK_MSM_SEGMENT;  // entries per thread in t
 static constexpr uint32_t kMinSegment = 8;            // ... at least, in small pipelines
 static constexpr uint32_t kFirstGroup = 2;            // units merged per thread in the first merge round
 static constexpr uint32_t kGroup = ZK_MSM_GROUP;      // units merged per thread in later rounds
-static constexpr uint32_t kBlockG = ZK_MSM_BLOCKG;    // buckets per block in the window reduction
-#ifndef ZK_MSM_BLOCKG2
-// measured at 2^20 (GLV, 8 windows): level-2 pass 0.154 ms with 8, 0.068 ms with 4 (its
-// threads are few and each runs a chain of g2 additions); the targets grow 0.078 -> 0.102 ms
-#define ZK_MSM_BLOCKG2 4
-#endif
-static constexpr uint32_t kBlockG2 = ZK_MSM_BLOCKG2;  // level-1 blocks per level-2 block
+// Buckets per block in the window reduction; small pipelines take the buckets themselves (blocks
+// of 1): blocks cost a launch and a chain of 2g - 1 additions a thread, lines read every block
+// twice. Measured on GB300 (blocks + lines + targets, us) with 1 / 2 / 4 / 8 / 16 buckets: 2^12
+// 41 / 45 / 68 / - / -, 2^16 fixed-base 80 / 74 / 92 / - / -, 2^20 265 / - / 227 / 196 / 262, 64
+// instances of 2^10..2^20 3.72 / - / 3.27 / 3.12 / 3.27 ms.
+static constexpr uint32_t kBlockG = ZK_MSM_BLOCKG;
+static constexpr uint32_t kLineWarps = 8;  // lines get a second and fourth warp while below this per SM
 // Straddling buckets over more than kFixupMax + 1 segments go to the long-bucket fixup (a
 // CTA tree per bucket); small pipelines, latency-bound, send them there from kFixupMaxSmall
 // + 2 segments on (a tree of log2(pieces) additions instead of a chain). Measured on GB300
@@ -90,12 +92,11 @@ struct MsmShape {
     uint32_t c;        // window bits
     uint32_t W;        // windows
     uint32_t B;        // buckets per window (|digit| in 1..B)
-    uint32_t g;        // level-1 block size of the window reduction (<= B)
-    uint32_t G;        // level-1 blocks per window
-    uint32_t g2;       // level-2 block size (1: no second level)
-    uint32_t G2;       // level-2 blocks per window (G / g2)
-    uint32_t K;        // log2(G2)
-    uint32_t plain;    // plain-sum targets: 2 (one level) or 3 (two levels)
+    uint32_t g;        // block size of the window reduction (1: the buckets themselves)
+    uint32_t G;        // blocks per window
+    uint32_t K;        // log2(G)
+    uint32_t m;        // the G blocks as 2^(K - m) rows of 2^m (see lines_cta)
+    uint32_t plain;    // plain-sum targets: 1 (g = 1) or 2
     uint32_t targets;  // plain + K
     uint32_t shared;   // 1: fixed-base mode, all windows share one bucket set (window-shifted bases)
     uint32_t Wr;       // bucket sets per instance: W, or 1 in fixed-base mode
@@ -117,17 +118,20 @@ struct MsmInst {
     uint32_t stride;
 };
 
-// Block structure of the window reduction for level-1 blocks of g buckets and level-2
-// blocks of g2 level-1 blocks.
-static void shape_blocks(MsmShape& s, uint32_t g, uint32_t g2 = kBlockG2) {
+// Block structure of the window reduction for blocks of g buckets.
+static void shape_blocks(MsmShape& s, uint32_t g) {
     s.g = std::min<uint32_t>(g, s.B);
     s.G = s.B / s.g;
-    s.g2 = s.G >= 2 * g2 ? g2 : 1;
-    s.G2 = s.G / s.g2;
     s.K = 0;
-    while ((1u << s.K) < s.G2) s.K++;
-    s.plain = s.g2 > 1 ? 3 : 2;
+    while ((1u << s.K) < s.G) s.K++;
+    s.m = s.K / 2;
+    s.plain = s.g > 1 ? 2 : 1;
     s.targets = s.plain + s.K;
+}
+
+// Lines summed per bucket set: the rows and columns of the block sums, and the rows of E.
+__host__ __device__ inline uint32_t lines_per_set(const MsmShape& s) {
+    return s.plain * (1u << (s.K - s.m)) + (1u << s.m);
 }
 
 static MsmShape make_shape(uint32_t c, bool glv = false) {
@@ -1072,10 +1076,10 @@ __global__ void __launch_bounds__(C::kFixupLongThreads, C::kFixupLongMinBlocks) 
 // ---- 5. window reduction ----------------------------------------------------------------
 // For points X_1..X_N with weights, WS(X) = sum_b b X_b. Blocks of g: X_{(j-1)g+u}, u = 1..g:
 // WS(X) = sum_j E_j + g WS(Y), Y_j = block sum, E_j = -(s_1 + ... + s_{g-1}) with s_u the
-// prefix sums inside the block (because sum_u u X_u = g Y_j - sum_{u<g} s_u). Applied
-// twice (buckets -> Y1, E1 -> Y2, E2, F2 = block sums of E1), then WS(Y2) by plain sums:
-// WS(Y2) = sum_j Y2_j + sum_k 2^k M_k, M_k = sum of Y2_j with bit k of (j - 1) set.
-// Level 1: block j of window w holds buckets b = j*g + 1 .. j*g + g (stored at index b - 1).
+// prefix sums inside the block (because sum_u u X_u = g Y_j - sum_{u<g} s_u). With g = 1 there
+// are no blocks: Y = X and no E. Then WS(Y) by plain sums over the block index j = 0 .. G - 1:
+// WS(Y) = sum_j Y_j + sum_k 2^k M_k, M_k = sum of Y_j with bit k of j set.
+// Block j of window w holds buckets b = j*g + 1 .. j*g + g (stored at index b - 1).
 template <class C, bool kL2>
 __device__ __forceinline__ void blocks_thread(const typename C::P* buckets, const MsmShape& sh, typename C::P* Y,
                                               typename C::P* E, uint32_t t) {
@@ -1100,96 +1104,71 @@ __global__ void __launch_bounds__(128) msm_bucket_blocks_kernel(const typename C
     blocks_thread<C, false>(buckets, sh, Y, E, t);
 }
 
-// Level 2 over (Y1, E1): Y2, E2 as above on Y1, and F2 = plain block sums of E1.
+// ---- 6. plain sums per (window, target) ---------------------------------------------
+// The K sums M_k and the total share their terms: with the G = 2^K blocks laid out as rows of
+// 2^m (j = hi 2^m + lo), M_k for k < m is a sum of the column sums with bit k of lo set, for
+// k >= m of the row sums with bit k - m of hi set. So each block is read twice (its row and its
+// column) instead of 1 + K/2 times, and the targets are sums of at most max(2^m, 2^(K-m)) lines.
+//
+// Line i of set w: rows of Y, columns of Y, then (g > 1) rows of E; idx = w lines_per_set + i.
+// One CTA a line; `red` holds a point per warp. Measured (lines and targets against level-2
+// blocks and one tree per target over all blocks, us): 100003 witness-like 65 against 65 + 39 of
+// blocks, 2^16 fixed-base 80 / 137, 2^20 67 / 126, G2 2^16 190 / 332.
 template <class C, bool kL2>
-__device__ __forceinline__ void blocks2_thread(const typename C::P* Y1, const typename C::P* E1, const MsmShape& sh,
-                                               typename C::P* Y2, typename C::P* E2, typename C::P* F2, uint32_t t) {
-    using P = typename C::P;
-    const size_t base = (size_t)t * sh.g2;
-    P s = xyzz_inf<typename C::T>();
-    P e = xyzz_inf<typename C::T>();
-    P f = xyzz_inf<typename C::T>();
-    for (uint32_t u = 0; u < sh.g2; u++) {
-        s = xyzz_add(s, xyzz_get<kL2>(Y1 + base + u));
-        if (u + 1 < sh.g2) e = xyzz_add(e, s);
-        f = xyzz_add(f, xyzz_get<kL2>(E1 + base + u));
-    }
-    xyzz_store(Y2 + t, s);
-    xyzz_store(E2 + t, xyzz_neg(e));
-    xyzz_store(F2 + t, f);
+__device__ __forceinline__ void lines_cta(const typename C::P* Y, const typename C::P* E, const MsmShape& sh,
+                                          typename C::P* lines, typename C::P* red, uint32_t idx) {
+    const uint32_t per = lines_per_set(sh), rows = 1u << (sh.K - sh.m), cols = 1u << sh.m;
+    const uint32_t w = idx / per, i = idx % per;
+    const bool col = i >= rows && i < rows + cols;
+    const typename C::P* src = (i < rows + cols ? Y : E) + (size_t)w * sh.G;
+    src += col ? i - rows : (size_t)(i < rows ? i : i - rows - cols) << sh.m;
+    const uint32_t step = col ? cols : 1u;
+    const typename C::T r = cta_quad_sum<typename C::T>(
+        col ? rows : cols, [&](uint32_t t) { return quad_get<kL2>(src + (size_t)t * step); }, red);
+    if (threadIdx.x < 4) quad_put(lines + idx, r);
 }
 
 template <class C>
-__global__ void __launch_bounds__(128) msm_bucket_blocks2_kernel(const typename C::P* __restrict__ Y1,
-                                                                 const typename C::P* __restrict__ E1, MsmShape sh,
-                                                                 typename C::P* __restrict__ Y2,
-                                                                 typename C::P* __restrict__ E2,
-                                                                 typename C::P* __restrict__ F2) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= sh.sets * sh.G2) return;
-    blocks2_thread<C, false>(Y1, E1, sh, Y2, E2, F2, t);
+__global__ void __launch_bounds__(128) msm_lines_kernel(const typename C::P* __restrict__ Y,
+                                                        const typename C::P* __restrict__ E, MsmShape sh,
+                                                        typename C::P* __restrict__ lines) {
+    __shared__ typename C::P red[4];
+    lines_cta<C, false>(Y, E, sh, lines, red, blockIdx.x);
 }
 
-// ---- 6. plain sums per (window, target) ---------------------------------------------
-// targets 0 .. plain-1: full sums of P0, P1 (, P2) over G2 entries per window;
-// target plain + k: sum of Ylast_j over j with bit k set.
-// Each target is split over `parts` CTAs (a slice of its terms each; large single bucket
-// sets of the fixed-base mode have G2 up to 2^14); out[(w * targets + tg) * parts + part].
-// `blk` is the CTA's index in that order; `red` holds blockDim points.
+// Target tg of set w (idx = w targets + tg): 0 (g > 1): the E lines; plain - 1: the rows of Y;
+// plain + k: M_k.
 template <class C, bool kL2>
-__device__ __forceinline__ void targets_cta(const typename C::P* P0, const typename C::P* P1, const typename C::P* P2,
-                                            const typename C::P* Ylast, const MsmShape& sh, uint32_t parts,
-                                            typename C::P* out, typename C::P* red, uint32_t blk) {
-    using P = typename C::P;
-    const uint32_t part = blk % parts;
-    const uint32_t wt = blk / parts;
-    const uint32_t w = wt / sh.targets;
-    const uint32_t tg = wt % sh.targets;
+__device__ __forceinline__ void targets_cta(const typename C::P* lines, const MsmShape& sh, typename C::P* out,
+                                            typename C::P* red, uint32_t idx) {
+    const uint32_t rows = 1u << (sh.K - sh.m), cols = 1u << sh.m;
+    const uint32_t w = idx / sh.targets, tg = idx % sh.targets;
+    const typename C::P* src = lines + (size_t)w * lines_per_set(sh);
     const bool bits = tg >= sh.plain;
-    const P* src = bits ? Ylast : (tg == 0 ? P0 : (tg == 1 ? P1 : P2));
-    src += (size_t)w * sh.G2;
-    const uint32_t count = bits ? sh.G2 / 2 : sh.G2;
-    const uint32_t per = (count + parts - 1) / parts;
-    const uint32_t t0 = part * per, t1 = min(count, t0 + per);
-    const uint32_t k = bits ? tg - sh.plain : 0;
+    uint32_t k = tg - sh.plain, terms = rows;
+    if (bits && k < sh.m) {
+        src += rows;
+        terms = cols / 2;
+    } else if (bits) {
+        k -= sh.m;
+        terms = rows / 2;
+    } else if (tg + 1 < sh.plain) {
+        src += rows + cols;
+    }
     const typename C::T r = cta_quad_sum<typename C::T>(
-        t1 > t0 ? t1 - t0 : 0,
-        [&](uint32_t i) {
-            const uint32_t t = t0 + i;
+        terms,
+        [&](uint32_t t) {
             return quad_get<kL2>(src + (bits ? ((t >> k) << (k + 1)) | (1u << k) | (t & ((1u << k) - 1)) : t));
         },
         red);
-    if (threadIdx.x < 4) quad_put(out + blk, r);
+    if (threadIdx.x < 4) quad_put(out + idx, r);
 }
 
 template <class C>
-__global__ void __launch_bounds__(C::kTargetThreads) msm_targets_kernel(const typename C::P* __restrict__ P0,
-                                                                        const typename C::P* __restrict__ P1,
-                                                                        const typename C::P* __restrict__ P2,
-                                                                        const typename C::P* __restrict__ Ylast,
-                                                                        MsmShape sh, uint32_t parts,
-                                                                        typename C::P* __restrict__ out) {
-    __shared__ typename C::P red[C::kTargetThreads / 32];
-    targets_cta<C, false>(P0, P1, P2, Ylast, sh, parts, out, red, blockIdx.x);
-}
-
-// The parts of each target summed: one warp per (window, target).
-static constexpr uint32_t kMergeThreads = 32;
-
-template <class C, bool kL2>
-__device__ __forceinline__ void targets_merge_warp(const typename C::P* in, uint32_t parts, typename C::P* out,
-                                                   uint32_t blk) {
-    const typename C::P* src = in + (size_t)blk * parts;
-    const typename C::T r =
-        warp_quad_sum<typename C::T>(parts, 0, 8, [&](uint32_t t) { return quad_get<kL2>(src + t); });
-    if (threadIdx.x < 4) quad_put(out + blk, r);
-}
-
-template <class C>
-__global__ void __launch_bounds__(kMergeThreads) msm_targets_merge_kernel(const typename C::P* __restrict__ in,
-                                                                          uint32_t parts,
-                                                                          typename C::P* __restrict__ out) {
-    targets_merge_warp<C, false>(in, parts, out, blockIdx.x);
+__global__ void __launch_bounds__(128) msm_targets_kernel(const typename C::P* __restrict__ lines, MsmShape sh,
+                                                          typename C::P* __restrict__ out) {
+    __shared__ typename C::P red[4];
+    targets_cta<C, false>(lines, sh, out, red, blockIdx.x);
 }
 
 // ---- persistent form of the post-sort stages (work queue) ----------------------------------
@@ -1201,7 +1180,7 @@ __global__ void __launch_bounds__(kMergeThreads) msm_targets_merge_kernel(const 
 // a stage); an item waits until its pipeline's previous stage has published all its items.
 // The same ticket discipline as the NTT queue keeps it deadlock-free for any number of
 // resident CTAs (the earliest unfinished item never waits), and every wait is bounded.
-enum : uint32_t { kQAcc = 0, kQMerge, kQFix, kQFixLong, kQBlk1, kQBlk2, kQTgt, kQTMerge };
+enum : uint32_t { kQAcc = 0, kQMerge, kQFix, kQFixLong, kQBlk, kQLines, kQTgt };
 
 template <class C>
 struct MsmQPipe {
@@ -1216,9 +1195,9 @@ struct MsmQPipe {
     P* slot_pts[2];
     uint32_t* long_list;
     uint32_t* long_count;  // the count block (see fixup_bucket), hcap huge buckets at most
-    P *Yb, *Eb, *Y2, *E2, *F2, *tgt_out, *tgt;
+    P *Yb, *Eb, *lines, *tgt;
     MsmShape sh;
-    uint32_t units, nbuckets, parts, skip_inf, hcap, lcap;
+    uint32_t units, nbuckets, skip_inf, hcap, lcap;
 };
 
 struct MsmQEntry {
@@ -1332,34 +1311,19 @@ __global__ void __launch_bounds__(kMsmQThreads, 2) msm_queue_kernel(const MsmQPi
                 fixup_long_cta<C, true>(q.row_ptr, q.sh.seg, q.slot_pts[0], q.buckets, q.long_list, q.lcap,
                                         q.long_count, q.hcap, q.slot_pts[1], red, b, sE.items);
                 break;
-            case kQBlk1:
+            case kQBlk:
                 if (i < q.sh.sets * q.sh.G) blocks_thread<C, true>(q.buckets, q.sh, q.Yb, q.Eb, i);
                 break;
-            case kQBlk2:
-                if (i < q.sh.sets * q.sh.G2) blocks2_thread<C, true>(q.Yb, q.Eb, q.sh, q.Y2, q.E2, q.F2, i);
+            case kQLines:
+                lines_cta<C, true>(q.Yb, q.Eb, q.sh, q.lines, red, b);
                 break;
             case kQTgt:
-                if (q.sh.g2 > 1) targets_cta<C, true>(q.F2, q.E2, q.Y2, q.Y2, q.sh, q.parts, q.tgt_out, red, b);
-                else targets_cta<C, true>(q.Eb, q.Yb, q.Yb, q.Yb, q.sh, q.parts, q.tgt_out, red, b);
-                break;
-            case kQTMerge:
-                if (threadIdx.x < 32) targets_merge_warp<C, true>(q.tgt_out, q.parts, q.tgt, b);
+                targets_cta<C, true>(q.lines, q.sh, q.tgt, red, b);
                 break;
         }
         __syncthreads();  // every store of the item issued; sE, sQ and red free again
         if (threadIdx.x == 0) s_next = nxt;
     }
-}
-
-// CTAs per target: one up to 8 terms per thread; the large single bucket sets of the
-// fixed-base mode (G2 up to 2^14) in slices of about 8 terms per thread, at most 64.
-#ifndef ZK_TARGET_SLICE
-#define ZK_TARGET_SLICE 8
-#endif
-template <class C>
-static uint32_t target_parts(const MsmShape& sh) {
-    const uint32_t slice = (uint32_t)ZK_TARGET_SLICE * (uint32_t)C::kTargetThreads;
-    return std::max<uint32_t>(1, std::min<uint32_t>(64, (sh.G2 + slice - 1) / slice));
 }
 
 // ---- fixed-base precomputation ----------------------------------------------------------
@@ -1520,8 +1484,8 @@ struct MsmPipeT {
     uint32_t *slot_keys_a = nullptr, *slot_keys_b = nullptr;
     P *slot_pts_a = nullptr, *slot_pts_b = nullptr;
     uint32_t *long_list = nullptr, *long_count = nullptr;  // fixup mode
-    P *buckets = nullptr, *Yb = nullptr, *Eb = nullptr, *Y2 = nullptr, *E2 = nullptr, *F2 = nullptr, *tgt = nullptr;
-    P* tgt_parts = nullptr;  // per-part target sums before the merge (null with one part)
+    P *buckets = nullptr, *Yb = nullptr, *Eb = nullptr;  // Yb: the buckets themselves when g = 1
+    P *lines = nullptr, *tgt = nullptr;
     // tiled CSR sort (B <= kTiledMaxB): set positions, tiles and per-tile bucket counts
     bool tiled = false;
     uint32_t te = 0, tiles = 0;
@@ -1562,27 +1526,16 @@ static int pipe_init(MsmPipeT<C>& p, uint32_t c, bool fixed, bool glv, const std
     ZK_CHECK_ARG(p.max_entries < (1ull << 32) - kSegment, "MSM too large for 32-bit CSR offsets");
     p.nbuckets = (uint64_t)p.sh.sets * p.sh.B;
     ZK_CHECK_ARG(p.nbuckets < (1ull << 32) - 1, "MSM batch has too many buckets for 32-bit keys");
-    // Small pipelines are latency-bound (each accumulation thread is a chain of seg additions,
-    // each reduction thread one of g or g2): shorter segments while there are fewer than about
-    // four waves of accumulation threads and buckets still span at most ~2 segments on average
-    // (more pieces cost more in the fixup than the shorter chains save), smaller blocks while
-    // there are fewer than two (level 1) or one (level 2) warps of block threads per SM.
-    // Measured on GB300 (single MSMs): 2^12 0.67 -> 0.48 ms, 2^14 0.69 -> 0.55 ms, 2^16
-    // 1.03 -> 0.88 ms, 2^18 1.89 -> 1.86 ms; 2^20 and larger unchanged.
+    // Small pipelines are latency-bound (each accumulation thread is a chain of seg additions):
+    // shorter segments while there are fewer than about four waves of accumulation threads and
+    // buckets still span at most ~2 segments on average (more pieces cost more in the fixup
+    // than the shorter chains save).
     const uint64_t acc_threads = (uint64_t)num_sms * 2048;
     const uint64_t density = p.max_entries / std::max<uint64_t>(1, p.nbuckets);
     while (p.sh.seg > kMinSegment && p.max_entries / p.sh.seg < acc_threads && p.sh.seg / 2 >= density / 2)
         p.sh.seg /= 2;
-    const uint64_t min_threads = (uint64_t)num_sms * 64;
-    uint32_t g = kBlockG, g2 = kBlockG2;
-    while (g > 2 && p.nbuckets / g < min_threads) g /= 2;
-    while (g2 > 2 && p.nbuckets / g / g2 < min_threads / 2) g2 /= 2;
-    // A small single MSM skips the level-2 blocks: the targets' trees get one level deeper,
-    // but a launch and its chain of 2 g2 additions go (measured on GB300: 2^10 / 2^12 /
-    // 2^14 0.327 / 0.365 / 0.490 -> 0.303 / 0.347 / 0.469 ms, 2^16 and larger the same);
-    // batches keep them (64 instances of 2^10..2^14: 1.6% slower without).
     const bool small = p.nbuckets < (uint64_t)num_sms * kSmallBucketsPerSm;
-    shape_blocks(p.sh, g, small && jobs.size() == 1 ? 1u : g2);
+    shape_blocks(p.sh, small ? 1u : kBlockG);
     if (small) p.sh.fixmax = kFixupMaxSmall;
     p.units = (uint32_t)((p.max_entries + p.sh.seg - 1) / p.sh.seg);
     // tiled sort when a set's counters fit shared memory: set s = k Wr + w holds n_k halves
@@ -1644,14 +1597,10 @@ static size_t pipe_layout(MsmPipeT<C>& p, char* base) {
     // the count block: long and huge counts, the huge buckets' chunk counters and keys
     p.long_count = reinterpret_cast<uint32_t*>(take((kCountHead + 2 * (size_t)huge_cap(p.units)) * 4));
     p.buckets = reinterpret_cast<P*>(take(p.nbuckets * sizeof(P)));
-    p.Yb = reinterpret_cast<P*>(take((size_t)sh.sets * sh.G * sizeof(P)));
-    p.Eb = reinterpret_cast<P*>(take((size_t)sh.sets * sh.G * sizeof(P)));
-    p.Y2 = reinterpret_cast<P*>(take((size_t)sh.sets * sh.G2 * sizeof(P)));
-    p.E2 = reinterpret_cast<P*>(take((size_t)sh.sets * sh.G2 * sizeof(P)));
-    p.F2 = reinterpret_cast<P*>(take((size_t)sh.sets * sh.G2 * sizeof(P)));
+    p.Yb = sh.g > 1 ? reinterpret_cast<P*>(take((size_t)sh.sets * sh.G * sizeof(P))) : p.buckets;
+    p.Eb = sh.g > 1 ? reinterpret_cast<P*>(take((size_t)sh.sets * sh.G * sizeof(P))) : nullptr;
+    p.lines = reinterpret_cast<P*>(take((size_t)sh.sets * lines_per_set(sh) * sizeof(P)));
     p.tgt = reinterpret_cast<P*>(take(p.host_elems() * sizeof(P)));
-    const uint32_t parts = target_parts<C>(sh);
-    p.tgt_parts = parts > 1 ? reinterpret_cast<P*>(take(p.host_elems() * parts * sizeof(P))) : nullptr;
     if (p.tiled) {
         p.set_base = reinterpret_cast<uint32_t*>(take(p.set_base_h.size() * 4));
         p.set_tile0 = reinterpret_cast<uint32_t*>(take(p.set_tile0_h.size() * 4));
@@ -1852,33 +1801,22 @@ static int pipe_enqueue_reduce(Ctx* c, MsmPipeT<C>& p) {
     }
 
     // window reduction
-    // the targets' CTAs sum G2 points each: no more threads than the power of two covering G2
-    uint32_t target_threads = 32;
-    while (target_threads < sh.G2 && target_threads < (uint32_t)C::kTargetThreads) target_threads <<= 1;
-    const uint32_t nb1 = sh.sets * sh.G;
-    ZK_LAUNCH(c, "msm_bucket_blocks", msm_bucket_blocks_kernel<C>, (nb1 + 127) / 128, 128, 0, p.buckets, sh, p.Yb, p.Eb);
-    ZK_TRY_CUDA(cudaGetLastError());
-    if (sh.g2 > 1) {
-        const uint32_t nb2 = sh.sets * sh.G2;
-        ZK_LAUNCH(c, "msm_bucket_blocks2", msm_bucket_blocks2_kernel<C>, (nb2 + 127) / 128, 128, 0, p.Yb, p.Eb, sh, p.Y2,
-                  p.E2, p.F2);
+    if (sh.g > 1) {
+        const uint32_t nb = sh.sets * sh.G;
+        ZK_LAUNCH(c, "msm_bucket_blocks", msm_bucket_blocks_kernel<C>, (nb + 127) / 128, 128, 0, p.buckets, sh, p.Yb,
+                  p.Eb);
         ZK_TRY_CUDA(cudaGetLastError());
     }
-    const uint32_t parts = target_parts<C>(sh);
-    P* tout = parts > 1 ? p.tgt_parts : p.tgt;
-    if (sh.g2 > 1) {
-        ZK_LAUNCH(c, "msm_targets", msm_targets_kernel<C>, sh.sets * sh.targets * parts, target_threads, 0, p.F2,
-                  p.E2, p.Y2, p.Y2, sh, parts, tout);
-    } else {
-        ZK_LAUNCH(c, "msm_targets", msm_targets_kernel<C>, sh.sets * sh.targets * parts, target_threads, 0, p.Eb,
-                  p.Yb, p.Yb, p.Yb, sh, parts, tout);
-    }
+    // warps a line: more while the lines are few and a warp's quads have two terms or more
+    const uint32_t nl = sh.sets * lines_per_set(sh), len = 1u << (sh.K - sh.m);
+    uint32_t lw = 1;
+    while (lw < 4 && nl * lw < (uint32_t)c->num_sms * kLineWarps && 16 * lw < len) lw *= 2;
+    ZK_LAUNCH(c, "msm_lines", msm_lines_kernel<C>, nl, 32 * lw, 0, p.Yb, p.Eb, sh, p.lines);
     ZK_TRY_CUDA(cudaGetLastError());
-    if (parts > 1) {
-        ZK_LAUNCH(c, "msm_targets_merge", msm_targets_merge_kernel<C>, sh.sets * sh.targets, kMergeThreads, 0,
-                  p.tgt_parts, parts, p.tgt);
-        ZK_TRY_CUDA(cudaGetLastError());
-    }
+    uint32_t tw = 1;
+    while (tw < 4 && 16 * tw < len) tw *= 2;
+    ZK_LAUNCH(c, "msm_targets", msm_targets_kernel<C>, sh.sets * sh.targets, 32 * tw, 0, p.lines, sh, p.tgt);
+    ZK_TRY_CUDA(cudaGetLastError());
     return ZK_OK;
 }
 
@@ -2014,17 +1952,14 @@ class HostPool {
     uint64_t gen_ = 0;   // under run_mu_
 };
 
-// Host: the sum S_w of window (or set) w of instance k from its targets:
-//   one level   S_w = T0 + g (T1 + H)            (T0 = sum E1, T1 = sum Y1)
-//   two levels  S_w = T0 + g (T1 + g2 (T2 + H))  (T0 = sum F2 = sum E1, T1 = sum E2, T2 = sum Y2)
-// with H = sum_k 2^k M_k (Horner).
+// Host: the sum S_w of window (or set) w of instance k from its targets: S_w = g (T_Y + H) + T_E
+// with T_Y = sum Y, H = sum_k 2^k M_k (Horner) and, for g > 1, T_E = sum E (target 0).
 template <class C>
 static zkh::XyzzT<typename HostOf<C>::T> window_sum(const MsmPipeT<C>& p, uint32_t k, uint32_t w) {
     using H = typename HostOf<C>::T;
     const MsmShape& sh = p.sh;
-    uint32_t log_g = 0, log_g2 = 0;
+    uint32_t log_g = 0;
     while ((1u << log_g) < sh.g) log_g++;
-    while ((1u << log_g2) < sh.g2) log_g2++;
     const typename C::P* T = p.h_tgt + ((size_t)k * sh.Wr + (size_t)w) * sh.targets;
     zkh::XyzzT<H> h = zkh::xyzz_inf<H>();
     for (int b = (int)sh.K - 1; b >= 0; b--) {
@@ -2032,10 +1967,7 @@ static zkh::XyzzT<typename HostOf<C>::T> window_sum(const MsmPipeT<C>& p, uint32
         h = zkh::xyzz_add(h, to_host<C>(T[sh.plain + b]));
     }
     zkh::XyzzT<H> sw = zkh::xyzz_add(h, to_host<C>(T[sh.plain - 1]));
-    if (sh.plain == 3) {
-        sw = host_dbl_n(sw, log_g2);
-        sw = zkh::xyzz_add(sw, to_host<C>(T[1]));
-    }
+    if (sh.g == 1) return sw;
     sw = host_dbl_n(sw, log_g);
     return zkh::xyzz_add(sw, to_host<C>(T[0]));
 }
@@ -2254,7 +2186,7 @@ static int queue_plan(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, MsmQueueT<C
     std::stable_sort(order.begin(), order.end(),
                      [&](size_t a, size_t b) { return pipes[a].max_entries > pipes[b].max_entries; });
     // each pipeline's stages as (slot, entry); slots: 0 accumulation, 1..R merge rounds, then
-    // fixup, long fixup, level 1, level 2, targets, target merge
+    // fixup, long fixup, blocks, lines, targets
     std::vector<std::vector<std::pair<uint32_t, MsmQEntry>>> st(np);
     uint32_t rmax = 0;
     q.fixup_mode.assign(np, 0);
@@ -2300,11 +2232,10 @@ static int queue_plan(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, MsmQueueT<C
             add(st[k], base, kQFix, (p.nbuckets + kMsmQThreads - 1) / kMsmQThreads);
             add(st[k], base + 1, kQFixLong, long_items);
         }
-        add(st[k], base + 2, kQBlk1, ((uint64_t)sh.sets * sh.G + kMsmQThreads - 1) / kMsmQThreads);
-        if (sh.g2 > 1) add(st[k], base + 3, kQBlk2, ((uint64_t)sh.sets * sh.G2 + kMsmQThreads - 1) / kMsmQThreads);
-        const uint32_t parts = target_parts<C>(sh);
-        add(st[k], base + 4, kQTgt, (uint64_t)sh.sets * sh.targets * parts);
-        if (parts > 1) add(st[k], base + 5, kQTMerge, (uint64_t)sh.sets * sh.targets);
+        if (sh.g > 1)
+            add(st[k], base + 2, kQBlk, ((uint64_t)sh.sets * sh.G + kMsmQThreads - 1) / kMsmQThreads);
+        add(st[k], base + 3, kQLines, (uint64_t)sh.sets * lines_per_set(sh));
+        add(st[k], base + 4, kQTgt, (uint64_t)sh.sets * sh.targets);
     }
     q.qe.clear();
     q.nitems = 0;
@@ -2382,11 +2313,7 @@ static int queue_fill(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, MsmQueueT<C
         d.lcap = long_cap(p.units, p.sh.fixmax);
         d.Yb = p.Yb;
         d.Eb = p.Eb;
-        d.Y2 = p.Y2;
-        d.E2 = p.E2;
-        d.F2 = p.F2;
-        d.parts = target_parts<C>(p.sh);
-        d.tgt_out = d.parts > 1 ? p.tgt_parts : p.tgt;
+        d.lines = p.lines;
         d.tgt = p.tgt;
         d.sh = p.sh;
         d.units = p.units;
