@@ -28,6 +28,8 @@ namespace zk {
 struct FrP {
     __host__ __device__ static constexpr uint32_t P(int i) { return i == 0 ? 0xf0000001u : i == 1 ? 0x43e1f593u : i == 2 ? 0x79b97091u : i == 3 ? 0x2833e848u : i == 4 ? 0x8181585du : i == 5 ? 0xb85045b6u : i == 6 ? 0xe131a029u : 0x30644e72u; }
     static constexpr uint32_t INV = 0xefffffffu  /* -r^-1 mod 2^32 */;
+    // (INV p + 1) / 2^32 (see the products below)
+    __host__ __device__ static constexpr uint32_t NP(int i) { return i == 0 ? 0x6d1e0a6du : i == 1 ? 0xb5ea65a9u : i == 2 ? 0xc9e9f13fu : i == 3 ? 0xd42f5166u : i == 4 ? 0x6118fd20u : i == 5 ? 0x3b99a131u : i == 6 ? 0x82ba37b4u : 0x2d5e098bu; }
     static constexpr bool CALL_MUL = false;
     static constexpr bool LAZY = false;
     __host__ __device__ static constexpr uint32_t ONE(int i) { return i == 0 ? 0x4ffffffbu : i == 1 ? 0xac96341cu : i == 2 ? 0x9f60cd29u : i == 3 ? 0x36fc7695u : i == 4 ? 0x7879462eu : i == 5 ? 0x666ea36fu : i == 6 ? 0x9a07df2fu : 0x0e0a77c1u; }
@@ -37,6 +39,8 @@ struct FrP {
 struct FqP {
     __host__ __device__ static constexpr uint32_t P(int i) { return i == 0 ? 0xd87cfd47u : i == 1 ? 0x3c208c16u : i == 2 ? 0x6871ca8du : i == 3 ? 0x97816a91u : i == 4 ? 0x8181585du : i == 5 ? 0xb85045b6u : i == 6 ? 0xe131a029u : 0x30644e72u; }
     static constexpr uint32_t INV = 0xe4866389u  /* -q^-1 mod 2^32 */;
+    // (INV p + 1) / 2^32 (see the products below)
+    __host__ __device__ static constexpr uint32_t NP(int i) { return i == 0 ? 0x705c70f2u : i == 1 ? 0xb5b479a3u : i == 2 ? 0x699a472au : i == 3 ? 0xef510c54u : i == 4 ? 0xb6c9df27u : i == 5 ? 0xb27cd0b5u : i == 6 ? 0x10b67b2fu : 0x2b32bd30u; }
     static constexpr bool CALL_MUL = true;
 #ifdef ZK_FQ_STRICT
     static constexpr bool LAZY = false;
@@ -143,7 +147,7 @@ template <class F>
 __device__ __forceinline__ fe fe_reduce_2p(const fe& t) {
     fe s;
     uint32_t borrow;
-    asm("sub.cc.u32  %0, %9, %17;\n\t"
+    asm volatile("sub.cc.u32  %0, %9, %17;\n\t"
         "subc.cc.u32 %1, %10, %18;\n\t"
         "subc.cc.u32 %2, %11, %19;\n\t"
         "subc.cc.u32 %3, %12, %20;\n\t"
@@ -175,7 +179,7 @@ template <class F>
 __device__ __forceinline__ fe fe_reduce_4p(const fe& t) {
     fe s;
     uint32_t borrow;
-    asm("sub.cc.u32  %0, %9, %17;\n\t"
+    asm volatile("sub.cc.u32  %0, %9, %17;\n\t"
         "subc.cc.u32 %1, %10, %18;\n\t"
         "subc.cc.u32 %2, %11, %19;\n\t"
         "subc.cc.u32 %3, %12, %20;\n\t"
@@ -200,7 +204,7 @@ template <class F>
 __device__ __forceinline__ fe fe_reduce_once(const fe& t) {
     fe s;
     uint32_t borrow;
-    asm("sub.cc.u32  %0, %9, %17;\n\t"
+    asm volatile("sub.cc.u32  %0, %9, %17;\n\t"
         "subc.cc.u32 %1, %10, %18;\n\t"
         "subc.cc.u32 %2, %11, %19;\n\t"
         "subc.cc.u32 %3, %12, %20;\n\t"
@@ -223,7 +227,7 @@ __device__ __forceinline__ fe fe_reduce_once(const fe& t) {
 template <class F>
 __device__ __forceinline__ fe fe_add(const fe& a, const fe& b) {
     fe t;
-    asm("add.cc.u32  %0, %8, %16;\n\t"
+    asm volatile("add.cc.u32  %0, %8, %16;\n\t"
         "addc.cc.u32 %1, %9, %17;\n\t"
         "addc.cc.u32 %2, %10, %18;\n\t"
         "addc.cc.u32 %3, %11, %19;\n\t"
@@ -243,7 +247,7 @@ template <class F>
 __device__ __forceinline__ fe fe_sub(const fe& a, const fe& b) {
     fe t;
     uint32_t m;
-    asm("sub.cc.u32  %0, %9, %17;\n\t"
+    asm volatile("sub.cc.u32  %0, %9, %17;\n\t"
         "subc.cc.u32 %1, %10, %18;\n\t"
         "subc.cc.u32 %2, %11, %19;\n\t"
         "subc.cc.u32 %3, %12, %20;\n\t"
@@ -257,7 +261,7 @@ __device__ __forceinline__ fe fe_sub(const fe& a, const fe& b) {
         : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
           "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
     fe r;
-    asm("add.cc.u32  %0, %8, %16;\n\t"
+    asm volatile("add.cc.u32  %0, %8, %16;\n\t"
         "addc.cc.u32 %1, %9, %17;\n\t"
         "addc.cc.u32 %2, %10, %18;\n\t"
         "addc.cc.u32 %3, %11, %19;\n\t"
@@ -286,7 +290,8 @@ __device__ __forceinline__ fe fe_dbl(const fe& a) {
 // ---- products -------------------------------------------------------------------------------
 //
 // The carry flag primitives are one PTX instruction each on the device (asm volatile keeps
-// their order, so the flag flows from one to the next as in a single asm block); on the
+// their order, so the flag flows from one to the next as in a single asm block; every other
+// asm block that writes the flag is volatile too, or it could be moved in between); on the
 // host they emulate the flag, so the same code runs in a host-side check of the arithmetic.
 #ifndef __CUDA_ARCH__
 inline uint32_t& host_carry_flag() {
@@ -405,8 +410,8 @@ __host__ __device__ __forceinline__ void u_mad2(uint32_t& lo, uint32_t& hi, uint
 // multiply pipe whether or not it adds and carries (measured: 10.1 T/s for the chip at
 // 2070 MHz, 16 lanes a cycle a scheduler at two passes), and an add with carry 2 cycles of
 // the other integer pipe. A product needs 128 of the former = 512 cycles a warp; this form
-// adds 8 low multiplies and ~40 adds. Measured (independent chains, 64 warps per SM): 70.1 G
-// products/s = 92% of the multiply pipe, against 47.8 G/s for full-width products folded in
+// adds 2 low multiplies and ~40 adds. Measured (independent chains, 64 warps per SM): 71.6 G
+// products/s = 91% of the multiply pipe, against 47.8 G/s for full-width products folded in
 // by separate add-with-carry chains (290 adds: the two pipes then take turns); 64-bit adds
 // of full-width products 56.8 G/s.
 //
@@ -447,6 +452,15 @@ __host__ __device__ __forceinline__ void modulus_limbs(uint32_t* p) {
     for (int j = 0; j < 8; j++) p[j] = F::P(j);
 }
 
+// The modulus multiple N = (-p^-1 mod 2^32) p has N_0 = 2^32 - 1, so T + T_0 N is divisible by 2^32
+// with the quotient floor(T / 2^32) + T_0 N', N' = (N + 1) / 2^32 < p: the row's multiplier is T's
+// own low limb, without the multiplication by -p^-1 (and the wait for it). N has 286 bits, so
+// a row leaves T up to 2^32 p larger than a row with p would; the last two rows use p (their
+// multipliers computed), which brings the result to its bound: the rows before add at most
+// 2^-32 p to it. Measured against 8 rows with p: 69.5 -> 71.6 G products/s, a lone product
+// 878 -> 843 cycles.
+static constexpr int kShortRows = 6;  // rows of a product that use N'
+
 // T += m p with m = T_0 (-p^-1): limb 0 becomes 0.
 template <class F>
 __host__ __device__ __forceinline__ void row_reduce(uint32_t* e, uint32_t* o) {
@@ -457,49 +471,80 @@ __host__ __device__ __forceinline__ void row_reduce(uint32_t* e, uint32_t* o) {
     row_even(e, o, p, m);
 }
 
-// T / 2^32 once limb 0 is 0: o becomes the even accumulator, e without its limbs 0 and 1 the
-// odd one; limb 1 (returned) is left for the caller to add to the new even accumulator.
-__host__ __device__ __forceinline__ uint32_t row_shift(uint32_t* e, uint32_t* o) {
+// T / 2^32 once limb 0 is 0: o becomes the even accumulator, e without its limbs 0 and 1 the odd
+// one with `top` at limb 7; limb 1 is added to the new even accumulator, its carry left in the
+// flag for the odd row that follows.
+__host__ __device__ __forceinline__ void row_shift(uint32_t* e, uint32_t* o, uint32_t top) {
     const uint32_t c = e[1];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-        const uint32_t x = j < 6 ? e[j + 2] : 0u;
+        const uint32_t x = j < 6 ? e[j + 2] : j == 6 ? top : 0u;
         e[j] = o[j];
         o[j] = x;
     }
-    return c;
+    e[0] = u_add_cc(e[0], c);
 }
 
-// (e + 2^32 o) / 2^32 as 8 limbs, limb 0 being 0 and the value below 2^288.
-__host__ __device__ __forceinline__ fe row_result(const uint32_t* e, const uint32_t* o) {
+// T = floor(T / 2^32) + m N' for m = T_0.
+template <class F>
+__host__ __device__ __forceinline__ void row_step(uint32_t* e, uint32_t* o, uint32_t top = 0u) {
+    uint32_t n[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) n[j] = F::NP(j);
+    const uint32_t m = e[0];
+    row_shift(e, o, top);
+    row_odd<true>(o, n, m);
+    row_even(e, o, n, m);
+}
+
+// T / 2^32 (limb 0 being 0), then T += m p as in row_reduce.
+template <class F>
+__host__ __device__ __forceinline__ void row_shift_reduce(uint32_t* e, uint32_t* o, uint32_t top) {
+    uint32_t p[8];
+    modulus_limbs<F>(p);
+    row_shift(e, o, top);
+    const uint32_t m = e[0] * F::INV;
+    row_odd<true>(o, p, m);
+    row_even(e, o, p, m);
+}
+
+// (e + 2^32 o) / 2^32 as 8 limbs, limb 0 being 0 and the value below 2^288; `top` is added to
+// limb 7 of the result.
+__host__ __device__ __forceinline__ fe row_result(const uint32_t* e, const uint32_t* o, uint32_t top = 0u) {
     fe r;
     r.v[0] = u_add_cc(o[0], e[1]);
 #pragma unroll
     for (int j = 1; j < 7; j++) r.v[j] = u_addc_cc(o[j], e[j + 1]);
-    r.v[7] = u_addc(o[7], 0u);
+    r.v[7] = u_addc(o[7], top);
     return r;
 }
 
-// a b 2^-256 mod p, below ab / 2^256 + p (CIOS rows): below 2p for a, b below 2p. T stays
-// below 2^32 (a + p) < 2^288 for a below 4p.
+// a b 2^-256 mod p, below ab / 2^256 + (1 + 2^-31) p (CIOS rows): below 2p for a, b below 2p. T
+// is largest in the first row with p, below 2^32 (a + N' + p) (1 + 2^-31) < 4p 2^32 < 2^288.
 template <class F>
 __host__ __device__ __forceinline__ fe mul_rows(const fe& a, const fe& b) {
     uint32_t e[8], o[8];
     row_first(e, o, a.v, b.v[0]);
-    row_reduce<F>(e, o);
 #pragma unroll
-    for (int i = 1; i < 8; i++) {
-        const uint32_t c = row_shift(e, o);
-        e[0] = u_add_cc(e[0], c);
+    for (int i = 1; i <= kShortRows; i++) {
+        row_step<F>(e, o);
+        row_odd<false>(o, a.v, b.v[i]);
+        row_even(e, o, a.v, b.v[i]);
+    }
+#pragma unroll
+    for (int i = kShortRows + 1; i < 8; i++) {
+        row_reduce<F>(e, o);
+        row_shift(e, o, 0u);
         row_odd<true>(o, a.v, b.v[i]);
         row_even(e, o, a.v, b.v[i]);
-        row_reduce<F>(e, o);
     }
+    row_reduce<F>(e, o);
     return row_result(e, o);
 }
 
 // (a b + c d) 2^-256 mod p with one reduction, below (ab + cd) / 2^256 + p: below 2.52p for
-// inputs up to 2p. T stays below 2^32 (a + c + p) <= 5p 2^32 < 2^288.
+// inputs up to 2p. T stays below 2^32 (a + c + p) <= 5p 2^32 < 2^288; rows with N' would leave no
+// room for the last rows' m p beside both products, so every row uses p.
 template <class F>
 __host__ __device__ __forceinline__ fe mul_add_rows(const fe& a, const fe& b, const fe& c, const fe& d) {
     uint32_t e[8], o[8];
@@ -509,8 +554,7 @@ __host__ __device__ __forceinline__ fe mul_add_rows(const fe& a, const fe& b, co
     row_reduce<F>(e, o);
 #pragma unroll
     for (int i = 1; i < 8; i++) {
-        const uint32_t t = row_shift(e, o);
-        e[0] = u_add_cc(e[0], t);
+        row_shift(e, o, 0u);
         row_odd<true>(o, a.v, b.v[i]);
         row_even(e, o, a.v, b.v[i]);
         row_odd<false>(o, c.v, d.v[i]);
@@ -629,7 +673,7 @@ __host__ __device__ __forceinline__ void sos_sqr_wide(uint32_t* t, const uint32_
     u_mad2<true>(t[14], t[15], a[7], a[7]);
 }
 
-// (T + M p) / 2^256 for t = T (16 limbs): T * 2^-256 mod p, below T / 2^256 + p.
+// (T + M p) / 2^256 for t = T (16 limbs): T * 2^-256 mod p, below T / 2^256 + (1 + 2^-31) p.
 template <class F>
 __host__ __device__ __forceinline__ fe sos_redc(const uint32_t* t) {
     uint32_t e[8], o[8];
@@ -638,24 +682,11 @@ __host__ __device__ __forceinline__ fe sos_redc(const uint32_t* t) {
         e[j] = t[j];
         o[j] = 0u;
     }
+#pragma unroll
+    for (int i = 0; i < kShortRows; i++) row_step<F>(e, o, t[8 + i]);
     row_reduce<F>(e, o);
-#pragma unroll
-    for (int i = 1; i < 8; i++) {
-        const uint32_t c = row_shift(e, o);
-        o[6] = t[7 + i];
-        uint32_t p[8];
-        modulus_limbs<F>(p);
-        e[0] = u_add_cc(e[0], c);
-        const uint32_t m = e[0] * F::INV;
-        row_odd<true>(o, p, m);
-        row_even(e, o, p, m);
-    }
-    fe r;
-    r.v[0] = u_add_cc(o[0], e[1]);
-#pragma unroll
-    for (int j = 1; j < 7; j++) r.v[j] = u_addc_cc(o[j], e[j + 1]);
-    r.v[7] = u_addc(o[7], t[15]);
-    return r;
+    row_shift_reduce<F>(e, o, t[14]);
+    return row_result(e, o, t[15]);
 }
 
 // 2p - c for c in [0, 2p): in (0, 2p], congruent to -c
@@ -819,7 +850,7 @@ __device__ __forceinline__ fe fe_to_mont(fe a) {
     for (int k = 0; k < 5; k++) {
         fe s;
         uint32_t br;
-        asm("sub.cc.u32  %0, %9, %17;\n\t"
+        asm volatile("sub.cc.u32  %0, %9, %17;\n\t"
             "subc.cc.u32 %1, %10, %18;\n\t"
             "subc.cc.u32 %2, %11, %19;\n\t"
             "subc.cc.u32 %3, %12, %20;\n\t"
