@@ -564,6 +564,146 @@ __host__ __device__ __forceinline__ fe mul_add_rows(const fe& a, const fe& b, co
     return row_result(e, o);
 }
 
+// ---- products with a constant known beforehand ------------------------------------------------
+//
+// x w mod p for a constant w (a twiddle factor) held with w' = floor(w 2^256 / p) (Shoup): the
+// quotient q = floor(x w' / 2^256) is at most 1 below floor(x w / p), so x w - q p, taken modulo
+// 2^256, lies in [0, 2p). Only the upper columns of x w' and the lower halves of the other two
+// products are needed: 99 wide and 16 low multiply-adds instead of 128 and 2, and half the
+// carry additions. w is canonical, x any value below 4p.
+//
+// Bound: x w / p - x w' / 2^256 < x / 2^256 < 4p / 2^256 < 0.757, and leaving out the columns below
+// limb 6 lowers the sum by less than 6 * 2^(64 + 160) = 6 * 2^-32 of q's unit, so the floor is
+// lowered by at most 1.
+struct fe_const {
+    fe w, ws;  // w, floor(w 2^256 / p)
+};
+
+__host__ __device__ __forceinline__ uint32_t u_madc_lo(uint32_t a, uint32_t b, uint32_t c) {  // a b + c + carry in
+#ifdef __CUDA_ARCH__
+    uint32_t r;
+    asm volatile("madc.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+#else
+    return a * b + c + host_carry_flag();
+#endif
+}
+
+// c[0..2N-1] += {x_0, x_2, ..} y for N partial products (x strided by 2); kOut: the carry out
+// becomes c[2N] (not yet written), else it is dropped or known to be none (a top pair that
+// held at most a carry before: (2^32 - 1)^2 + 2 < 2^64).
+template <int N, bool kOut>
+__host__ __device__ __forceinline__ void col_chain(uint32_t* c, const uint32_t* x, uint32_t y) {
+    if constexpr (N == 1) {
+        if constexpr (kOut) u_mad2_cc<false>(c[0], c[1], x[0], y);
+        else u_mad2<false>(c[0], c[1], x[0], y);
+    } else {
+        u_mad2_cc<false>(c[0], c[1], x[0], y);
+#pragma unroll
+        for (int k = 1; k + 1 < N; k++) u_mad2_cc<true>(c[2 * k], c[2 * k + 1], x[2 * k], y);
+        if constexpr (kOut) u_mad2_cc<true>(c[2 * N - 2], c[2 * N - 1], x[2 * N - 2], y);
+        else u_mad2<true>(c[2 * N - 2], c[2 * N - 1], x[2 * N - 2], y);
+    }
+    if constexpr (kOut) c[2 * N] = u_addc(0u, 0u);
+}
+
+// ... for N - 1 pairs and the low half of a last product at c[2N - 2] (modulo 2^32 there)
+template <int N>
+__host__ __device__ __forceinline__ void col_chain_low(uint32_t* c, const uint32_t* x, uint32_t y) {
+    if constexpr (N == 1) {
+        c[0] += x[0] * y;
+    } else {
+        u_mad2_cc<false>(c[0], c[1], x[0], y);
+#pragma unroll
+        for (int k = 1; k + 1 < N; k++) u_mad2_cc<true>(c[2 * k], c[2 * k + 1], x[2 * k], y);
+        c[2 * N - 2] = u_madc_lo(x[2 * N - 2], y, c[2 * N - 2]);
+    }
+}
+
+// (e + 2^32 o) += a x modulo 2^256, e at limbs 0..7, o at limbs 1..7
+__host__ __device__ __forceinline__ void mul_low(uint32_t* e, uint32_t* o, const uint32_t* a, const uint32_t* x) {
+    col_chain<4, false>(e, a, x[0]);
+    col_chain_low<4>(o, a + 1, x[0]);
+    col_chain<3, false>(e + 2, a + 1, x[1]);
+    col_chain_low<4>(o, a, x[1]);
+    col_chain<3, false>(e + 2, a, x[2]);
+    col_chain_low<3>(o + 2, a + 1, x[2]);
+    col_chain<2, false>(e + 4, a + 1, x[3]);
+    col_chain_low<3>(o + 2, a, x[3]);
+    col_chain<2, false>(e + 4, a, x[4]);
+    col_chain_low<2>(o + 4, a + 1, x[4]);
+    col_chain<1, false>(e + 6, a + 1, x[5]);
+    col_chain_low<2>(o + 4, a, x[5]);
+    col_chain<1, false>(e + 6, a, x[6]);
+    col_chain_low<1>(o + 6, a + 1, x[6]);
+    col_chain_low<1>(o + 6, a, x[7]);
+}
+
+// x w mod p in [0, 2p) for x below 4p
+template <class F>
+__host__ __device__ __forceinline__ fe fe_mul_const(const fe& x, const fe_const& c) {
+    const uint32_t *a = c.ws.v, *y = x.v;
+    // q: columns 6 .. 14 of x w', e at limbs 6 .. 15, o at limbs 7 .. 15
+    uint32_t e[10], o[9], q[8];
+#pragma unroll
+    for (int j = 0; j < 10; j++) e[j] = 0u;
+#pragma unroll
+    for (int j = 0; j < 9; j++) o[j] = 0u;
+    col_chain<1, false>(e, a + 6, y[0]);
+    col_chain<1, false>(o, a + 7, y[0]);
+    col_chain<2, false>(e, a + 5, y[1]);
+    col_chain<1, true>(o, a + 6, y[1]);
+    col_chain<2, true>(e, a + 4, y[2]);
+    col_chain<2, false>(o, a + 5, y[2]);
+    col_chain<3, false>(e, a + 3, y[3]);
+    col_chain<2, true>(o, a + 4, y[3]);
+    col_chain<3, true>(e, a + 2, y[4]);
+    col_chain<3, false>(o, a + 3, y[4]);
+    col_chain<4, false>(e, a + 1, y[5]);
+    col_chain<3, true>(o, a + 2, y[5]);
+    col_chain<4, true>(e, a, y[6]);
+    col_chain<4, false>(o, a + 1, y[6]);
+    col_chain<4, false>(e + 2, a + 1, y[7]);
+    col_chain<4, true>(o, a, y[7]);
+    (void)u_add_cc(e[1], o[0]);
+#pragma unroll
+    for (int j = 0; j < 7; j++) q[j] = u_addc_cc(e[j + 2], o[j + 1]);
+    q[7] = u_addc(e[9], o[8]);
+    // x w + q (2^256 - p) modulo 2^256
+    uint32_t n[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) n[j] = j == 0 ? 0u - F::P(0) : ~F::P(j);
+    uint32_t re[8], ro[7];
+#pragma unroll
+    for (int j = 0; j < 8; j++) re[j] = 0u;
+#pragma unroll
+    for (int j = 0; j < 7; j++) ro[j] = 0u;
+    mul_low(re, ro, c.w.v, y);
+    mul_low(re, ro, n, q);
+    fe r;
+    r.v[0] = re[0];
+    r.v[1] = u_add_cc(re[1], ro[0]);
+#pragma unroll
+    for (int j = 2; j < 7; j++) r.v[j] = u_addc_cc(re[j], ro[j - 1]);
+    r.v[7] = u_addc(re[7], ro[6]);
+    return r;
+}
+
+// a - b + 2p for a, b below 2p: in (0, 4p), an operand of fe_mul_const
+template <class F>
+__host__ __device__ __forceinline__ fe fe_sub_4p(const fe& a, const fe& b) {
+    fe t, r;
+    t.v[0] = u_sub_cc(a.v[0], b.v[0]);
+#pragma unroll
+    for (int j = 1; j < 7; j++) t.v[j] = u_subc_cc(a.v[j], b.v[j]);
+    t.v[7] = u_subc(a.v[7], b.v[7]);
+    r.v[0] = u_add_cc(t.v[0], p2_limb<F>(0));
+#pragma unroll
+    for (int j = 1; j < 7; j++) r.v[j] = u_addc_cc(t.v[j], p2_limb<F>(j));
+    r.v[7] = u_addc(t.v[7], p2_limb<F>(7));
+    return r;
+}
+
 template <class F>
 __device__ __noinline__ fe fe_mul_call(const fe a, const fe b) {
     return mul_rows<F>(a, b);
@@ -593,24 +733,6 @@ __device__ __forceinline__ fe fe_mul(const fe& a, const fe& b) {
 // product of two values below 2p: T / 2^256 < 0.76 p), below 2.52 p for T < 8p^2, which one
 // conditional subtraction of 2p brings below 2p (both moduli are below 0.19 * 2^256).
 
-// c[0..2N-1] += {x_0, x_2, ..} y for N partial products (x strided by 2); kOut: the carry out
-// becomes c[2N] (not yet written), else the caller knows there is none (the top pair held at
-// most a carry before: (2^32 - 1)^2 + 2 < 2^64).
-template <int N, bool kOut>
-__host__ __device__ __forceinline__ void sos_chain(uint32_t* c, const uint32_t* x, uint32_t y) {
-    if constexpr (N == 1) {
-        if constexpr (kOut) u_mad2_cc<false>(c[0], c[1], x[0], y);
-        else u_mad2<false>(c[0], c[1], x[0], y);
-    } else {
-        u_mad2_cc<false>(c[0], c[1], x[0], y);
-#pragma unroll
-        for (int k = 1; k + 1 < N; k++) u_mad2_cc<true>(c[2 * k], c[2 * k + 1], x[2 * k], y);
-        if constexpr (kOut) u_mad2_cc<true>(c[2 * N - 2], c[2 * N - 1], x[2 * N - 2], y);
-        else u_mad2<true>(c[2 * N - 2], c[2 * N - 1], x[2 * N - 2], y);
-    }
-    if constexpr (kOut) c[2 * N] = u_addc(0u, 0u);
-}
-
 // t[0..15] = a * b for any 256-bit a, b, in even and odd columns (o[k] at limb k + 1). Rows 2k - 1
 // and 2k end at the same even column and rows 2k and 2k + 1 at the same odd one, so only the
 // second of each two can carry out.
@@ -621,11 +743,11 @@ __host__ __device__ __forceinline__ void sos_mul_wide(uint32_t* t, const uint32_
     row_first(e, o, a, b[0]);
 #pragma unroll
     for (int i = 1; i < 8; i += 2) {
-        sos_chain<4, true>(o + i - 1, a, b[i]);       // limbs i .. i + 7
-        sos_chain<4, false>(e + i + 1, a + 1, b[i]);  // limbs i + 1 .. i + 8
+        col_chain<4, true>(o + i - 1, a, b[i]);       // limbs i .. i + 7
+        col_chain<4, false>(e + i + 1, a + 1, b[i]);  // limbs i + 1 .. i + 8
         if (i + 1 < 8) {
-            sos_chain<4, true>(e + i + 1, a, b[i + 1]);
-            sos_chain<4, false>(o + i + 1, a + 1, b[i + 1]);
+            col_chain<4, true>(e + i + 1, a, b[i + 1]);
+            col_chain<4, false>(o + i + 1, a + 1, b[i + 1]);
         }
     }
     t[0] = e[0];
@@ -641,19 +763,19 @@ __host__ __device__ __forceinline__ void sos_sqr_wide(uint32_t* t, const uint32_
     uint32_t e[16], o[16];
 #pragma unroll
     for (int j = 0; j < 16; j++) e[j] = o[j] = 0u;
-    sos_chain<4, false>(o, a + 1, a[0]);      // a_0 a_{1,3,5,7}: limbs 1 .. 8
-    sos_chain<3, false>(e + 2, a + 2, a[0]);  // a_0 a_{2,4,6}
-    sos_chain<3, true>(o + 2, a + 2, a[1]);
-    sos_chain<3, false>(e + 4, a + 3, a[1]);
-    sos_chain<3, false>(o + 4, a + 3, a[2]);
-    sos_chain<2, true>(e + 6, a + 4, a[2]);
-    sos_chain<2, true>(o + 6, a + 4, a[3]);
-    sos_chain<2, false>(e + 8, a + 5, a[3]);
-    sos_chain<2, false>(o + 8, a + 5, a[4]);
-    sos_chain<1, true>(e + 10, a + 6, a[4]);
-    sos_chain<1, true>(o + 10, a + 6, a[5]);
-    sos_chain<1, false>(e + 12, a + 7, a[5]);
-    sos_chain<1, false>(o + 12, a + 7, a[6]);
+    col_chain<4, false>(o, a + 1, a[0]);      // a_0 a_{1,3,5,7}: limbs 1 .. 8
+    col_chain<3, false>(e + 2, a + 2, a[0]);  // a_0 a_{2,4,6}
+    col_chain<3, true>(o + 2, a + 2, a[1]);
+    col_chain<3, false>(e + 4, a + 3, a[1]);
+    col_chain<3, false>(o + 4, a + 3, a[2]);
+    col_chain<2, true>(e + 6, a + 4, a[2]);
+    col_chain<2, true>(o + 6, a + 4, a[3]);
+    col_chain<2, false>(e + 8, a + 5, a[3]);
+    col_chain<2, false>(o + 8, a + 5, a[4]);
+    col_chain<1, true>(e + 10, a + 6, a[4]);
+    col_chain<1, true>(o + 10, a + 6, a[5]);
+    col_chain<1, false>(e + 12, a + 7, a[5]);
+    col_chain<1, false>(o + 12, a + 7, a[6]);
     // the cross sum x in limbs 1 .. 14 (below a^2 / 2 < 2^511)
     uint32_t x[15];
     x[1] = o[0];
@@ -914,6 +1036,8 @@ __device__ __forceinline__ fe fe_ldg(const fe* p) {
     r.v[7] = hi.w;
     return r;
 }
+
+__device__ __forceinline__ fe_const fe_ldg(const fe_const* p) { return {fe_ldg(&p->w), fe_ldg(&p->ws)}; }
 
 // A 32-byte element through L2 only (ld.global.cg): for data that other CTAs wrote earlier
 // in the same launch, which the non-coherent read-only path is not guaranteed to see.

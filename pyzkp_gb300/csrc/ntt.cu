@@ -49,10 +49,14 @@ static constexpr int kTileLogElems = 11;  // largest tile: R * T = 2048 elements
 // against 2^11-element tiles; tiles of 2^6..2^8 are within 5% of one another at every size.
 static constexpr int kDefaultTileLog = 8;
 
+// Elements a thread loads before it multiplies the first: 1 / 2 / 4 / 8 at 2^22 (narrow form) 893 / 879
+// / 886 / 924 us.
+static constexpr uint32_t kLoadBatch = 2;
+
 struct NttPassParams {
     const fe* in;
     fe* out;
-    const fe* radix_tw;  // w_R^i, i < R/2
+    const fe_const* radix_tw;  // narrow form: w_R^i, i < R/2; wide form: see wide_table
     const fe* tw_lo;
     const fe* tw_hi;
     const fe* pre_lo;
@@ -82,8 +86,11 @@ __device__ __forceinline__ fe lookup2(const fe* lo, const fe* hi, uint32_t e, ui
     return fe_mul<FrN>(a, fe_ldg(hi + h));
 }
 
-__device__ __forceinline__ uint32_t swz(uint32_t pos, uint32_t log_r) {
-    return log_r >= 6 ? (pos ^ ((pos >> (log_r - 3)) & 7u)) : pos;
+// Position of element pos of a column: its low three bits XORed with its higher base-8 digits, so
+// that eight lanes reading at any stride of 8^k (the steps' butterflies, the bit-reversed
+// read-back) fall into eight different 16-byte bank groups.
+__device__ __forceinline__ uint32_t swz(uint32_t pos) {
+    return pos ^ (((pos >> 3) ^ (pos >> 6) ^ (pos >> 9)) & 7u);
 }
 
 __device__ __forceinline__ fe smem_get(const uint4* s_lo, const uint4* s_hi, uint32_t i) {
@@ -105,37 +112,17 @@ __device__ __forceinline__ void smem_put(uint4* s_lo, uint4* s_hi, uint32_t i, c
     s_hi[i] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
 }
 
-// One CTA's tile `tile` of one pass (shared by the single-transform, the batch and the
-// queue kernel). l2_in: the pass input was written earlier in the same launch (a runtime
-// flag rather than a template argument: one copy of the body in the queue kernel).
-__device__ __forceinline__ void ntt_pass_body(const NttPassParams& P, uint32_t tile, uint4* smem,
-                                              bool l2_in = false) {
+// x w^i in [0, 2r) for a butterfly difference x in (0, 4r), w^i from the radix table
+__device__ __forceinline__ fe twiddle(const fe& x, const fe_const* radix_tw, uint32_t i) {
+    return i == 0 ? fe_reduce_2p<FrN>(x) : fe_mul_const<FrN>(x, fe_ldg(radix_tw + i));
+}
+
+// The narrow form of the DFTs: radix-2 stages, pairs of them as radix-4 steps where every thread
+// has one. For launches of few elements, where a thread's chain of products counts and not
+// the traffic.
+__device__ __forceinline__ void dft_narrow(const NttPassParams& P, uint4* s_lo, uint4* s_hi) {
     const uint32_t log_r = P.log_r, log_t = P.log_t;
-    const uint32_t R = 1u << log_r, T = 1u << log_t, E = R << log_t;
-    uint4* s_lo = smem;
-    uint4* s_hi = smem + E;
-    const uint32_t c0 = tile << log_t;
-    const uint32_t stride_log = P.log_n - log_r;
-    const uint32_t l_mask = (1u << P.log_l) - 1;
-    const uint32_t tw_shift = P.log_n - log_r - P.log_l;
-
-    // ---- load (+ coset scale on the first pass, + inter-pass twiddle) ----
-    for (uint32_t idx = threadIdx.x; idx < E; idx += blockDim.x) {
-        const uint32_t m = idx >> log_t, t = idx & (T - 1);
-        const uint32_t col = c0 + t;
-        const uint32_t g = col + (m << stride_log);
-        fe v = g < P.in_len ? (l2_in ? fe_ldcg(P.in + g) : fe_ldg(P.in + g)) : fe_zero();
-        if (P.reduce_in) v = fe_reduce_2p<FrN>(fe_reduce_4p<FrN>(v));
-        if (P.pre_lo != nullptr && g < P.in_len) v = fe_mul<FrN>(v, lookup2(P.pre_lo, P.pre_hi, g, P.s_bits));
-        if (P.log_l != 0) {
-            const uint32_t e = (m * (col & l_mask)) << tw_shift;
-            if (e != 0) v = fe_mul<FrN>(v, lookup2(P.tw_lo, P.tw_hi, e, P.s_bits));
-        }
-        smem_put(s_lo, s_hi, (swz(m, log_r) << log_t) + t, v);
-    }
-    __syncthreads();
-
-    // ---- R-point DFT per column: DIF stages in shared memory ----
+    const uint32_t T = 1u << log_t, E = 1u << (log_r + log_t);
     // Pairs of radix-2 stages (st, st + 1) run as one radix-4 step: for j < h/2 (h = the
     // half-size of stage st) the elements i0, i0 + h/2, i0 + h, i0 + 3h/2 of a block of 2h
     // are closed under both stages, so one thread loads four, applies the four butterflies
@@ -153,25 +140,20 @@ __device__ __forceinline__ void ntt_pass_body(const NttPassParams& P, uint32_t t
             const uint32_t t = qi & (T - 1), b = qi >> log_t;
             const uint32_t j = b & (hq - 1);
             const uint32_t i0 = ((b >> (log_h - 1)) << (log_h + 1)) + j;
-            const uint32_t a0 = (swz(i0, log_r) << log_t) + t;
-            const uint32_t a1 = (swz(i0 + hq, log_r) << log_t) + t;
-            const uint32_t a2 = (swz(i0 + h, log_r) << log_t) + t;
-            const uint32_t a3 = (swz(i0 + h + hq, log_r) << log_t) + t;
+            const uint32_t a0 = (swz(i0) << log_t) + t;
+            const uint32_t a1 = (swz(i0 + hq) << log_t) + t;
+            const uint32_t a2 = (swz(i0 + h) << log_t) + t;
+            const uint32_t a3 = (swz(i0 + h + hq) << log_t) + t;
             const fe x0 = smem_get(s_lo, s_hi, a0), x1 = smem_get(s_lo, s_hi, a1);
             const fe x2 = smem_get(s_lo, s_hi, a2), x3 = smem_get(s_lo, s_hi, a3);
             // stage st0: (x0, x2) with twiddle index j, (x1, x3) with j + h/2
             const fe p0 = fe_add<FrN>(x0, x2);
-            fe p2 = fe_sub<FrN>(x0, x2);
-            if (j != 0) p2 = fe_mul<FrN>(p2, fe_ldg(P.radix_tw + (j << st0)));
+            const fe p2 = twiddle(fe_sub_4p<FrN>(x0, x2), P.radix_tw, j << st0);
             const fe p1 = fe_add<FrN>(x1, x3);
-            const fe p3 = fe_mul<FrN>(fe_sub<FrN>(x1, x3), fe_ldg(P.radix_tw + ((j + hq) << st0)));
+            const fe p3 = fe_mul_const<FrN>(fe_sub_4p<FrN>(x1, x3), fe_ldg(P.radix_tw + ((j + hq) << st0)));
             // stage st0 + 1: (p0, p1) and (p2, p3), twiddle index j
-            fe q1 = fe_sub<FrN>(p0, p1), q3 = fe_sub<FrN>(p2, p3);
-            if (j != 0) {
-                const fe w = fe_ldg(P.radix_tw + (j << (st0 + 1)));
-                q1 = fe_mul<FrN>(q1, w);
-                q3 = fe_mul<FrN>(q3, w);
-            }
+            const fe q1 = twiddle(fe_sub_4p<FrN>(p0, p1), P.radix_tw, j << (st0 + 1));
+            const fe q3 = twiddle(fe_sub_4p<FrN>(p2, p3), P.radix_tw, j << (st0 + 1));
             smem_put(s_lo, s_hi, a0, fe_add<FrN>(p0, p1));
             smem_put(s_lo, s_hi, a1, q1);
             smem_put(s_lo, s_hi, a2, fe_add<FrN>(p2, p3));
@@ -187,18 +169,170 @@ __device__ __forceinline__ void ntt_pass_body(const NttPassParams& P, uint32_t t
             const uint32_t t = bi & (T - 1), b = bi >> log_t;
             const uint32_t j = b & (h - 1);
             const uint32_t i0 = ((b >> log_h) << (log_h + 1)) + j;
-            const uint32_t a0 = (swz(i0, log_r) << log_t) + t;
-            const uint32_t a1 = (swz(i0 + h, log_r) << log_t) + t;
+            const uint32_t a0 = (swz(i0) << log_t) + t;
+            const uint32_t a1 = (swz(i0 + h) << log_t) + t;
             fe u = smem_get(s_lo, s_hi, a0);
             fe v = smem_get(s_lo, s_hi, a1);
-            fe sum = fe_add<FrN>(u, v);
-            fe diff = fe_sub<FrN>(u, v);
-            if (j != 0) diff = fe_mul<FrN>(diff, fe_ldg(P.radix_tw + (j << st)));
-            smem_put(s_lo, s_hi, a0, sum);
-            smem_put(s_lo, s_hi, a1, diff);
+            smem_put(s_lo, s_hi, a0, fe_add<FrN>(u, v));
+            smem_put(s_lo, s_hi, a1, twiddle(fe_sub_4p<FrN>(u, v), P.radix_tw, j << st));
         }
         __syncthreads();
     }
+}
+
+__device__ __forceinline__ fe fe_add_4p(const fe& a, const fe& b) {  // a + b, not reduced
+    fe r;
+    r.v[0] = u_add_cc(a.v[0], b.v[0]);
+#pragma unroll
+    for (int j = 1; j < 7; j++) r.v[j] = u_addc_cc(a.v[j], b.v[j]);
+    r.v[7] = u_addc(a.v[7], b.v[7]);
+    return r;
+}
+
+// (a, b) = (a + b, (a - b) w) with values in [0, 2r); w: an entry of the table, null for 1
+__device__ __forceinline__ void butterfly(fe& a, fe& b, const fe_const* w) {
+    const fe d = fe_sub_4p<FrN>(a, b);
+    a = fe_add<FrN>(a, b);
+    b = w == nullptr ? fe_reduce_2p<FrN>(d) : fe_mul_const<FrN>(d, fe_ldg(w));
+}
+
+// The wide form: steps of radix 8, a thread's eight elements in registers through three DIF
+// stages, then radix 4 or 2 for what is left (no twiddles there). A step's stages multiply by
+// powers of w_8 alone (5 products, the same for every thread) and its outputs by one factor each
+// (7): output k of the 8-point DFT at offset j of a block of 8h gets w_{8h}^(j k), read
+// coalesced. Products as in radix-2 stages, but a third of the shared-memory traffic and
+// barriers and 7 instead of 12 table reads per eight elements.
+//
+// Table: [1], [2], [3]: w_8, w_4 = w_8^2, w_8^3; then per step 7 h entries, that of output k (1..7)
+// and offset j at (k - 1) h + j (see wide_table).
+//
+// What bounds it: the multiply pipe (99 + 16 multiply-adds a product with a known constant).
+// Measured (forward, us) against radix-4 steps with Montgomery products: 2^18 72 -> 58, 2^20 215 ->
+// 184, 2^22 886 -> 724; PLONK quotient step of 2^17 2118 -> 1745. Radix-4 steps with these products
+// alone gained nothing (895 at 2^22): their strided 64-byte table reads took what the
+// multiplies gave.
+__device__ __forceinline__ void dft_wide(const NttPassParams& P, uint4* s_lo, uint4* s_hi) {
+    const uint32_t log_t = P.log_t;
+    const uint32_t T = 1u << log_t, E = 1u << (P.log_r + log_t);
+    uint32_t log_b = P.log_r;  // blocks of 2^log_b elements left to transform
+    const fe_const* tw = P.radix_tw + 4;
+    for (; log_b >= 3; log_b -= 3) {
+        const uint32_t log_h = log_b - 3, h = 1u << log_h;
+        for (uint32_t bi = threadIdx.x; bi < (E >> 3); bi += blockDim.x) {
+            const uint32_t t = bi & (T - 1), b = bi >> log_t;
+            const uint32_t j = b & (h - 1);
+            const uint32_t i0 = ((b >> log_h) << log_b) + j;
+            fe x[8];
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++) x[k] = smem_get(s_lo, s_hi, (swz(i0 + (k << log_h)) << log_t) + t);
+            butterfly(x[0], x[4], nullptr);
+#pragma unroll
+            for (int i = 1; i < 4; i++) butterfly(x[i], x[i + 4], P.radix_tw + i);
+#pragma unroll
+            for (int i = 0; i < 8; i += 4) {
+                butterfly(x[i], x[i + 2], nullptr);
+                butterfly(x[i + 1], x[i + 3], P.radix_tw + 2);
+            }
+            if (h > 1) {
+                const fe_const* f = tw + j;
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    // outputs i and i + 1 are the frequencies rev(i) and rev(i) + 4
+                    const uint32_t k = ((i >> 2) & 1) | (i & 2);
+                    const fe d = fe_sub_4p<FrN>(x[i], x[i + 1]);
+                    x[i] = i == 0 ? fe_add<FrN>(x[0], x[1])
+                                  : fe_mul_const<FrN>(fe_add_4p(x[i], x[i + 1]), fe_ldg(f + ((k - 1) << log_h)));
+                    x[i + 1] = fe_mul_const<FrN>(d, fe_ldg(f + ((k + 3) << log_h)));
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) butterfly(x[i], x[i + 1], nullptr);
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++) smem_put(s_lo, s_hi, (swz(i0 + (k << log_h)) << log_t) + t, x[k]);
+        }
+        tw += 7u << log_h;
+        __syncthreads();
+    }
+    if (log_b == 2) {
+        for (uint32_t bi = threadIdx.x; bi < (E >> 2); bi += blockDim.x) {
+            const uint32_t t = bi & (T - 1), i0 = (bi >> log_t) << 2;
+            fe x[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) x[k] = smem_get(s_lo, s_hi, (swz(i0 + k) << log_t) + t);
+            butterfly(x[0], x[2], nullptr);
+            butterfly(x[1], x[3], P.radix_tw + 2);
+            butterfly(x[0], x[1], nullptr);
+            butterfly(x[2], x[3], nullptr);
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) smem_put(s_lo, s_hi, (swz(i0 + k) << log_t) + t, x[k]);
+        }
+        __syncthreads();
+    } else if (log_b == 1) {
+        for (uint32_t bi = threadIdx.x; bi < (E >> 1); bi += blockDim.x) {
+            const uint32_t t = bi & (T - 1), i0 = (bi >> log_t) << 1;
+            fe a = smem_get(s_lo, s_hi, (swz(i0) << log_t) + t), b = smem_get(s_lo, s_hi, (swz(i0 + 1) << log_t) + t);
+            butterfly(a, b, nullptr);
+            smem_put(s_lo, s_hi, (swz(i0) << log_t) + t, a);
+            smem_put(s_lo, s_hi, (swz(i0 + 1) << log_t) + t, b);
+        }
+        __syncthreads();
+    }
+}
+
+// One CTA's tile `tile` of one pass (shared by the single-transform, the batch and the
+// queue kernel). l2_in: the pass input was written earlier in the same launch (a runtime
+// flag rather than a template argument: one copy of the body in the queue kernel).
+template <bool kWide>
+__device__ __forceinline__ void ntt_pass_body(const NttPassParams& P, uint32_t tile, uint4* smem,
+                                              bool l2_in = false) {
+    const uint32_t log_r = P.log_r, log_t = P.log_t;
+    const uint32_t R = 1u << log_r, T = 1u << log_t, E = R << log_t;
+    uint4* s_lo = smem;
+    uint4* s_hi = smem + E;
+    const uint32_t c0 = tile << log_t;
+    const uint32_t stride_log = P.log_n - log_r;
+    const uint32_t l_mask = (1u << P.log_l) - 1;
+    const uint32_t tw_shift = P.log_n - log_r - P.log_l;
+
+    // ---- load (+ coset scale on the first pass, + inter-pass twiddle) ----
+    // kLoadBatch elements and their factors in flight per thread before the first product
+    for (uint32_t base = threadIdx.x; base < E; base += blockDim.x * kLoadBatch) {
+        fe v[kLoadBatch], f[kLoadBatch];
+#pragma unroll
+        for (uint32_t q = 0; q < kLoadBatch; q++) {
+            const uint32_t idx = base + q * blockDim.x;
+            if (idx >= E) break;
+            const uint32_t m = idx >> log_t, col = c0 + (idx & (T - 1));
+            const uint32_t g = col + (m << stride_log);
+            v[q] = g < P.in_len ? (l2_in ? fe_ldcg(P.in + g) : fe_ldg(P.in + g)) : fe_zero();
+            if (P.log_l != 0) {
+                const uint32_t e = (m * (col & l_mask)) << tw_shift;
+                f[q] = lookup2(P.tw_lo, P.tw_hi, e, P.s_bits);
+            } else if (P.pre_lo != nullptr && g < P.in_len) {
+                f[q] = lookup2(P.pre_lo, P.pre_hi, g, P.s_bits);
+            }
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kLoadBatch; q++) {
+            const uint32_t idx = base + q * blockDim.x;
+            if (idx >= E) break;
+            const uint32_t m = idx >> log_t, t = idx & (T - 1);
+            fe x = v[q];
+            if (P.reduce_in) x = fe_reduce_2p<FrN>(fe_reduce_4p<FrN>(x));
+            if (P.log_l != 0) {
+                if (m != 0 && ((c0 + t) & l_mask) != 0) x = fe_mul<FrN>(x, f[q]);
+            } else if (P.pre_lo != nullptr && c0 + t + (m << stride_log) < P.in_len) {
+                x = fe_mul<FrN>(x, f[q]);
+            }
+            smem_put(s_lo, s_hi, (swz(m) << log_t) + t, x);
+        }
+    }
+    __syncthreads();
+
+    // ---- R-point DFT per column, in place, outputs at bit-reversed positions ----
+    if constexpr (kWide) dft_wide(P, s_lo, s_hi);
+    else dft_narrow(P, s_lo, s_hi);
 
     // ---- store z_q (at bit-reversed position), + final scale on the last pass ----
     for (uint32_t idx = threadIdx.x; idx < E; idx += blockDim.x) {
@@ -212,7 +346,7 @@ __device__ __forceinline__ void ntt_pass_body(const NttPassParams& P, uint32_t t
         }
         const uint32_t col = c0 + t;
         const uint32_t pos = log_r ? (__brev(q) >> (32 - log_r)) : 0;
-        fe val = smem_get(s_lo, s_hi, (swz(pos, log_r) << log_t) + t);
+        fe val = smem_get(s_lo, s_hi, (swz(pos) << log_t) + t);
         const uint32_t o = ((col >> P.log_l) << (log_r + P.log_l)) + (col & l_mask) + (q << P.log_l);
         if (P.post_lo != nullptr) {
             fe s = P.post_hi != nullptr ? lookup2(P.post_lo, P.post_hi, o, P.s_bits) : fe_ldg(P.post_lo);
@@ -223,15 +357,17 @@ __device__ __forceinline__ void ntt_pass_body(const NttPassParams& P, uint32_t t
     }
 }
 
+template <bool kWide>
 __global__ void __launch_bounds__(kNttThreads, ZK_NTT_MINB) ntt_pass_kernel(NttPassParams P) {
     extern __shared__ uint4 smem[];
-    ntt_pass_body(P, blockIdx.x, smem);
+    ntt_pass_body<kWide>(P, blockIdx.x, smem);
 }
 
 // Batch: one launch runs the same pass level of many transforms. CTA b runs tile
 // b - first_tile[i] of item i, the largest i with first_tile[i] <= b; the item's
 // parameters are staged in shared memory once per CTA.
-__global__ void __launch_bounds__(kNttThreads, ZK_NTT_BATCH_MINB) ntt_pass_batch_kernel(const NttPassParams* __restrict__ items,
+template <bool kWide>
+__global__ void __launch_bounds__(kNttThreads, kWide ? ZK_NTT_MINB : ZK_NTT_BATCH_MINB) ntt_pass_batch_kernel(const NttPassParams* __restrict__ items,
                                                                        const uint32_t* __restrict__ first_tile,
                                                                        uint32_t nitems) {
     extern __shared__ uint4 smem[];
@@ -248,7 +384,7 @@ __global__ void __launch_bounds__(kNttThreads, ZK_NTT_BATCH_MINB) ntt_pass_batch
         s_tile = blockIdx.x - first_tile[lo];
     }
     __syncthreads();
-    ntt_pass_body(sP, s_tile, smem);
+    ntt_pass_body<kWide>(sP, s_tile, smem);
 }
 
 // ---- persistent launch from a device work queue --------------------------------------------
@@ -349,7 +485,7 @@ __global__ void __launch_bounds__(kNttThreads, ZK_NTT_BATCH_MINB) ntt_queue_kern
         // always runnable.
         uint32_t nxt = 0;
         if (threadIdx.x == 0) nxt = queue_ticket(state, nitems);
-        ntt_pass_body(sE.P, s_tile, smem, sE.dep >= 0);
+        ntt_pass_body<false>(sE.P, s_tile, smem, sE.dep >= 0);
         __syncthreads();  // every store of the tile issued; sE and s_tile free again
         if (threadIdx.x == 0) s_next = nxt;
     }
@@ -390,6 +526,26 @@ static int upload_table(Ctx* c, NttPlan* plan, const std::vector<zkh::F4>& v, fe
     return ZK_OK;
 }
 
+// -r^-1 mod 2^256: for t = w 2^256 mod r (the Montgomery form of w), floor(w 2^256 / r) =
+// (w 2^256 - t) / r = t (-r^-1) mod 2^256.
+__host__ __device__ constexpr uint64_t neg_inv_r(int i) {
+    return i == 0 ? 0xc2e1f593efffffffull : i == 1 ? 0x6586864b4c6911b3ull : i == 2 ? 0xe39a982899062391ull : 0x73f82f1d0d8341b2ull;
+}
+
+// floor(w 2^256 / r) from the Montgomery form of w (fe_mul_const)
+static zkh::F4 shoup_quotient(const zkh::F4& t) {
+    zkh::F4 q = {{0, 0, 0, 0}};
+    for (int i = 0; i < 4; i++) {
+        uint64_t carry = 0;
+        for (int j = 0; i + j < 4; j++) {
+            const unsigned __int128 x = (unsigned __int128)t.v[i] * neg_inv_r(j) + q.v[i + j] + carry;
+            q.v[i + j] = (uint64_t)x;
+            carry = (uint64_t)(x >> 64);
+        }
+    }
+    return q;
+}
+
 // powers base^i for i < count (Montgomery)
 static std::vector<zkh::F4> powers(const zkh::F4& base, size_t count) {
     const zkh::Field& F = zkh::fr();
@@ -398,6 +554,38 @@ static std::vector<zkh::F4> powers(const zkh::F4& base, size_t count) {
     for (size_t i = 0; i < count; i++) {
         v[i] = cur;
         cur = zkh::mul(F, cur, base);
+    }
+    return v;
+}
+
+// A constant and its quotient as fe_const stores them.
+struct ConstPair {
+    zkh::F4 w, ws;
+};
+
+static int upload_pairs(Ctx* c, NttPlan* plan, const std::vector<ConstPair>& v, fe_const** out) {
+    static_assert(sizeof(ConstPair) == sizeof(fe_const), "fe_const layout");
+    std::vector<zkh::F4> flat(2 * v.size());
+    std::memcpy(flat.data(), v.data(), v.size() * sizeof(ConstPair));
+    fe* table = nullptr;
+    const int rc = upload_table(c, plan, flat, &table);
+    *out = reinterpret_cast<fe_const*>(table);
+    return rc;
+}
+
+// The wide form's table of a radix-2^lr pass from t[i] = w_R^i, i < R = 2^lr (see dft_wide).
+static std::vector<ConstPair> wide_table(const std::vector<ConstPair>& t, uint32_t lr) {
+    const size_t R = t.size();
+    std::vector<ConstPair> v(4, t[0]);
+    if (lr >= 2) v[2] = t[R / 4];
+    if (lr >= 3) {
+        v[1] = t[R / 8];
+        v[3] = t[3 * (R / 8)];
+    }
+    for (uint32_t log_b = lr; log_b > 3; log_b -= 3) {
+        const size_t h = (size_t)1 << (log_b - 3), step = R >> log_b;  // w_{8h} = w_R^step
+        for (size_t k = 1; k < 8; k++)
+            for (size_t j = 0; j < h; j++) v.push_back(t[j * k * step]);
     }
     return v;
 }
@@ -446,8 +634,12 @@ static int build_plan(Ctx* c, int mode, uint32_t log_n, const zkh::F4& omega_m, 
     for (int p = 0; p < plan->npass; p++) {
         const uint32_t lr = plan->pass_log_r[p];
         const zkh::F4 wr = zkh::pow_u64(F, w, n >> lr);
-        std::vector<zkh::F4> t = powers(wr, std::max<uint64_t>(1, (1ull << lr) / 2));
-        if ((rc = upload_table(c, plan, t, &plan->radix_tw[p])) != ZK_OK) return rc;
+        std::vector<ConstPair> t;
+        for (const zkh::F4& x : powers(wr, 1ull << lr)) t.push_back({zkh::from_mont(F, x), shoup_quotient(x)});
+        const std::vector<ConstPair> wide = wide_table(t, lr);
+        t.resize(std::max<size_t>(1, t.size() / 2));
+        if ((rc = upload_pairs(c, plan, t, &plan->radix_tw[p])) != ZK_OK) return rc;
+        if ((rc = upload_pairs(c, plan, wide, &plan->wide_tw[p])) != ZK_OK) return rc;
     }
     if (mode == ZK_NTT_COSET_EVALS_FROM_COEFFS) {
         std::vector<zkh::F4> lo = powers(shift_m, lo_count);
@@ -536,10 +728,9 @@ static int set_smem_attr(int device) {
     ZK_CHECK_ARG(device >= 0 && device < 64, "device index out of range");
     std::lock_guard<std::mutex> g(mu);
     if (!done[device]) {
-        ZK_TRY_CUDA(cudaFuncSetAttribute(ntt_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (2 << kTileLogElems) * 16));
-        ZK_TRY_CUDA(cudaFuncSetAttribute(ntt_pass_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (2 << kTileLogElems) * 16));
+        for (const void* k : {(const void*)ntt_pass_kernel<false>, (const void*)ntt_pass_kernel<true>,
+                              (const void*)ntt_pass_batch_kernel<false>, (const void*)ntt_pass_batch_kernel<true>})
+            ZK_TRY_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (2 << kTileLogElems) * 16));
         ZK_TRY_CUDA(cudaFuncSetAttribute(ntt_queue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (2 << kTileLogElems) * 16));
         done[device] = true;
@@ -547,15 +738,24 @@ static int set_smem_attr(int device) {
     return ZK_OK;
 }
 
+// Launches of at least this many elements take the wide form of the pass kernels (an eighth as
+// many threads). Measured on GB300, narrow / wide (us): 2^16 26.5 / 41.3, 2^17 37.5 / 43.2, 2^18
+// 72.0 / 57.5.
+static constexpr uint64_t kWideElems = 1ull << 18;
+// Its tiles: 2^8 .. 2^10 elements are within 2% of one another, 2^11 12% slower at 2^20 (fewer,
+// longer CTAs: an emptier last wave).
+static constexpr int kWideTileLog = 10;
+
 // Columns per CTA of a radix-2^lr pass of a 2^log_n transform: fill a tile of up to
 // 2^tile_log elements, but not beyond the number of columns. ZK_NTT_TILE_LOG (5..11)
-// overrides kDefaultTileLog (read once per process).
-static uint32_t pass_log_t(uint32_t log_n, uint32_t lr) {
-    static const int tile_log = [] {
+// overrides the default tiles (read once per process).
+static uint32_t pass_log_t(uint32_t log_n, uint32_t lr, bool wide) {
+    static const int env_log = [] {
         const char* e = std::getenv("ZK_NTT_TILE_LOG");
         const int v = e ? std::atoi(e) : 0;
-        return (v >= 5 && v <= kTileLogElems) ? v : kDefaultTileLog;
+        return (v >= 5 && v <= kTileLogElems) ? v : 0;
     }();
+    const int tile_log = env_log ? env_log : wide ? kWideTileLog : kDefaultTileLog;
     uint32_t lt = tile_log > (int)lr ? tile_log - lr : 0;
     if (lt > log_n - lr) lt = log_n - lr;
     return lt;
@@ -579,7 +779,7 @@ static size_t pass_scratch_elems(const NttPlan* plan, const fe* out, const fe* i
 // passes go to scratch (and, out of place with 3+ passes, alternate with `out` so that
 // one scratch buffer suffices); the last pass writes `out`.
 static void make_passes(const NttPlan* plan, fe* out, const fe* in, uint32_t valid, fe* scratch,
-                        std::vector<PassLaunch>* launches, bool canon_io = false) {
+                        std::vector<PassLaunch>* launches, bool wide, bool canon_io = false) {
     const uint32_t log_n = plan->log_n;
     const uint64_t n = 1ull << log_n;
     launches->clear();
@@ -590,7 +790,7 @@ static void make_passes(const NttPlan* plan, fe* out, const fe* in, uint32_t val
     if (log_n == 0) {  // n == 1: the transform is the identity up to the scale factors
         P.in = in;
         P.out = out;
-        P.radix_tw = plan->tw_lo;
+        P.radix_tw = nullptr;  // no butterflies
         P.pre_lo = plan->pre_lo;
         P.pre_hi = plan->pre_hi;
         P.post_lo = plan->post_lo;
@@ -606,7 +806,7 @@ static void make_passes(const NttPlan* plan, fe* out, const fe* in, uint32_t val
     const fe* src = in;
     for (int p = 0; p < plan->npass; p++) {
         const uint32_t lr = plan->pass_log_r[p];
-        const uint32_t lt = pass_log_t(log_n, lr);
+        const uint32_t lt = pass_log_t(log_n, lr, wide);
         const int remaining = plan->npass - 1 - p;
         fe* dst;
         if (remaining == 0) dst = out;
@@ -614,7 +814,7 @@ static void make_passes(const NttPlan* plan, fe* out, const fe* in, uint32_t val
         else dst = (remaining % 2 == 0) ? out : scratch;
         P.in = src;
         P.out = dst;
-        P.radix_tw = plan->radix_tw[p];
+        P.radix_tw = wide ? plan->wide_tw[p] : plan->radix_tw[p];
         P.pre_lo = p == 0 ? plan->pre_lo : nullptr;
         P.pre_hi = p == 0 ? plan->pre_hi : nullptr;
         P.post_lo = remaining == 0 ? plan->post_lo : nullptr;
@@ -627,7 +827,9 @@ static void make_passes(const NttPlan* plan, fe* out, const fe* in, uint32_t val
         P.last = remaining == 0 ? 1u : 0u;
         P.reduce_in = canon_io && p == 0 ? 1u : 0u;
         const uint32_t elems = 1u << (lr + lt);
-        const uint32_t threads = elems / 2 < (uint32_t)kNttThreads ? (elems / 2 < 32 ? 32 : elems / 2) : kNttThreads;
+        // a butterfly a thread: of two elements, or (wide) of eight
+        const uint32_t work = wide ? elems / 8 : elems / 2;
+        const uint32_t threads = std::min<uint32_t>(kNttThreads, std::max<uint32_t>(32, work));
         launches->push_back({P, (uint32_t)(n >> (lr + lt)), threads, elems * 32});
         src = dst;
         log_l += lr;
@@ -664,9 +866,12 @@ int ntt_run(Ctx* c, int mode, fe* out, const fe* in, size_t in_len, uint32_t log
     const size_t se = pass_scratch_elems(plan, out, in);
     if (se && (rc = scratch_alloc(c, se * 32, reinterpret_cast<void**>(&scratch))) != ZK_OK) return rc;
     std::vector<PassLaunch> launches;
-    make_passes(plan, out, in, valid, scratch, &launches, canon_io);
+    const bool wide = n >= kWideElems;
+    make_passes(plan, out, in, valid, scratch, &launches, wide, canon_io);
+    auto* kernel = wide ? &ntt_pass_kernel<true> : &ntt_pass_kernel<false>;
     for (const PassLaunch& L : launches) {
-        ZK_LAUNCH(c, "ntt_pass", ntt_pass_kernel, L.blocks, L.threads, L.smem, L.P);
+        ZK_LAUNCH(c, "ntt_pass", kernel, L.blocks, L.threads, L.smem,
+                  L.P);
         ZK_TRY_CUDA(cudaGetLastError());
     }
     if (scratch) scratch_free(c, scratch);
@@ -689,6 +894,7 @@ struct NttBatch {
     // queue form (one persistent launch): entries in queue order, then the wait limit (ns)
     // and the state words (ticket, status, finished items per entry), all inside desc
     bool queue = false;
+    bool wide = false;  // the wide form of the pass kernel (never in the queue form)
     std::vector<NttQueueEntry> qentries;
     uint32_t qitems = 0, qsmem = 32, qgrid = 0;
     size_t queue_at = 0, limit_at = 0, state_at = 0;
@@ -710,6 +916,9 @@ static int batch_prepare(Ctx* c, const NttJob* jobs, size_t count, NttBatch* b) 
         b->scratch_at[j] = b->scratch_elems;
         b->scratch_elems += pass_scratch_elems(plans[j], J.out, J.in);
     }
+    uint64_t elems = 0;
+    for (size_t j = 0; j < count; j++) elems += 1ull << jobs[j].log_n;
+    b->wide = !b->queue && elems >= kWideElems;
     size_t levels = 0;
     for (size_t j = 0; j < count; j++) levels = std::max<size_t>(levels, std::max(plans[j]->npass, 1));
     b->items.assign(levels, {});
@@ -737,7 +946,8 @@ static int batch_layout(const NttJob* jobs, size_t count, NttBatch* b, Ctx* c) {
         }
         const uint64_t n = 1ull << J.log_n;
         const uint32_t valid = (uint32_t)(J.in_len < n ? J.in_len : n);
-        make_passes(plan, J.out, J.in, valid, b->scratch ? b->scratch + b->scratch_at[j] : nullptr, &b->jobs[j]);
+        make_passes(plan, J.out, J.in, valid, b->scratch ? b->scratch + b->scratch_at[j] : nullptr, &b->jobs[j],
+                    b->wide);
         for (size_t L = 0; L < b->jobs[j].size(); L++) {
             const PassLaunch& pl = b->jobs[j][L];
             b->first[L].push_back(b->blocks[L]);
@@ -837,9 +1047,10 @@ static int batch_enqueue(Ctx* c, const NttBatch* b) {
         ZK_TRY_CUDA(cudaGetLastError());
         return ZK_OK;
     }
+    auto* kernel = b->wide ? &ntt_pass_batch_kernel<true> : &ntt_pass_batch_kernel<false>;
     for (size_t L = 0; L < b->items.size(); L++) {
         if (b->blocks[L] == 0) continue;
-        ZK_LAUNCH(c, "ntt_pass_batch", ntt_pass_batch_kernel, b->blocks[L], b->threads[L], b->smem[L],
+        ZK_LAUNCH(c, "ntt_pass_batch", kernel, b->blocks[L], b->threads[L], b->smem[L],
                   reinterpret_cast<const NttPassParams*>(b->desc + b->items_at[L]),
                   reinterpret_cast<const uint32_t*>(b->desc + b->first_at[L]), (uint32_t)b->items[L].size());
         ZK_TRY_CUDA(cudaGetLastError());
@@ -1072,8 +1283,8 @@ namespace zk {
 
 static constexpr uint32_t kNoAllocMaxLogN = 16;
 static constexpr size_t kNoAllocDataElems = (size_t)1 << kNoAllocMaxLogN;
-// tables for log_n <= 16: two-level twiddles (<= 256 + 257), radix tables (<= 1024),
-// first-pass scale (<= 513), last-pass scale (<= 513): at most 2563 elements
+// tables for log_n <= 16: two-level twiddles (<= 256 + 257), radix tables (<= 1024 pairs),
+// first-pass scale (<= 513), last-pass scale (<= 513): at most 3587 elements
 static constexpr size_t kNoAllocTableElems = 4096;
 
 static __device__ __align__(256) fe g_ntt_noalloc_scratch[kNoAllocDataElems + kNoAllocTableElems];
@@ -1101,13 +1312,15 @@ static int noalloc_setup(int device, fe** out) {
     return ZK_OK;
 }
 
-// The tables as segments: table[off + i] = start * base^i for i < count (Montgomery),
-// built on the device from these values, which the launch carries by value.
+// The tables as segments: table[off + i] = start * base^i for i < count (Montgomery), or (pairs)
+// the fe_const of that power at table[off + 2 i], built on the device from these values, which
+// the launch carries by value.
 static constexpr int kNoAllocMaxSegs = 10;
 struct NoAllocTableSpec {
     uint32_t nseg;
     uint32_t off[kNoAllocMaxSegs];
     uint32_t count[kNoAllocMaxSegs];
+    uint32_t pairs[kNoAllocMaxSegs];
     fe start[kNoAllocMaxSegs];
     fe base[kNoAllocMaxSegs];
 };
@@ -1122,7 +1335,26 @@ __global__ void ntt_noalloc_tables_kernel(fe* __restrict__ tables, NoAllocTableS
                 if (e & 1) acc = fe_mul<FrP>(acc, b);
                 if (e > 1) b = fe_mul<FrP>(b, b);
             }
-            fe_store(tables + S.off[s] + i, acc);
+            if (S.pairs[s]) {
+                uint32_t n[8], e[8], o[7];  // t (-r^-1) mod 2^256
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    n[j] = (uint32_t)(neg_inv_r(j / 2) >> (32 * (j & 1)));
+                    e[j] = 0u;
+                    if (j < 7) o[j] = 0u;
+                }
+                mul_low(e, o, n, acc.v);
+                fe_store(tables + S.off[s] + 2 * i, fe_from_mont<FrP>(acc));
+                fe q;
+                q.v[0] = e[0];
+                q.v[1] = u_add_cc(e[1], o[0]);
+#pragma unroll
+                for (int j = 2; j < 7; j++) q.v[j] = u_addc_cc(e[j], o[j - 1]);
+                q.v[7] = u_addc(e[7], o[6]);
+                fe_store(tables + S.off[s] + 2 * i + 1, q);
+            } else {
+                fe_store(tables + S.off[s] + i, acc);
+            }
         }
     }
 }
@@ -1135,14 +1367,15 @@ static fe to_fe(const zkh::F4& x) {
 
 // Appends the segment start * base^i, i < count, at *pos; false when the spec is full.
 static bool add_segment(NoAllocTableSpec* S, size_t* pos, const zkh::F4& base, size_t count,
-                        const zkh::F4* start = nullptr) {
+                        const zkh::F4* start = nullptr, bool pairs = false) {
     if (S->nseg >= (uint32_t)kNoAllocMaxSegs) return false;
     const uint32_t k = S->nseg++;
     S->off[k] = (uint32_t)*pos;
     S->count[k] = (uint32_t)count;
+    S->pairs[k] = pairs ? 1u : 0u;
     S->start[k] = to_fe(start ? *start : zkh::one(zkh::fr()));
     S->base[k] = to_fe(base);
-    *pos += count;
+    *pos += pairs ? 2 * count : count;
     return true;
 }
 
@@ -1189,7 +1422,8 @@ static int ntt_run_noalloc(Ctx* c, int mode, fe* out, const fe* in, size_t in_le
     for (int p = 0; p < plan.npass; p++) {
         off_radix[p] = pos;
         const uint32_t lr = plan.pass_log_r[p];
-        ok = ok && add_segment(&spec, &pos, zkh::pow_u64(F, w, n >> lr), std::max<uint64_t>(1, (1ull << lr) / 2));
+        ok = ok && add_segment(&spec, &pos, zkh::pow_u64(F, w, n >> lr), std::max<uint64_t>(1, (1ull << lr) / 2),
+                               nullptr, true);
     }
     size_t off_pre_lo = 0, off_pre_hi = 0, off_post_lo = 0, off_post_hi = 0;
     bool has_pre = false, has_post = false, post_const = false;
@@ -1230,14 +1464,14 @@ static int ntt_run_noalloc(Ctx* c, int mode, fe* out, const fe* in, size_t in_le
     if (log_n == 0) {
         P.in = in;
         P.out = out;
-        P.radix_tw = tables + off_lo;
+        P.radix_tw = nullptr;  // no butterflies
         P.pre_lo = has_pre ? tables + off_pre_lo : nullptr;
         P.pre_hi = has_pre ? tables + off_pre_hi : nullptr;
         P.post_lo = has_post ? tables + off_post_lo : nullptr;
         P.post_hi = (has_post && !post_const) ? tables + off_post_hi : nullptr;
         P.in_len = valid;
         P.last = 1;
-        ZK_LAUNCH(c, "ntt_pass", ntt_pass_kernel, 1, 32, 2 * 16, P);
+        ZK_LAUNCH(c, "ntt_pass", ntt_pass_kernel<false>, 1, 32, 2 * 16, P);
         ZK_TRY_CUDA(cudaGetLastError());
         return ZK_OK;
     }
@@ -1245,12 +1479,12 @@ static int ntt_run_noalloc(Ctx* c, int mode, fe* out, const fe* in, size_t in_le
     const fe* src = in;
     for (int p = 0; p < plan.npass; p++) {
         const uint32_t lr = plan.pass_log_r[p];
-        const uint32_t lt = pass_log_t(log_n, lr);
+        const uint32_t lt = pass_log_t(log_n, lr, false);
         const int remaining = plan.npass - 1 - p;
         fe* dst = (remaining % 2 == 0) ? out : data;
         P.in = src;
         P.out = dst;
-        P.radix_tw = tables + off_radix[p];
+        P.radix_tw = reinterpret_cast<const fe_const*>(tables + off_radix[p]);
         P.pre_lo = (p == 0 && has_pre) ? tables + off_pre_lo : nullptr;
         P.pre_hi = (p == 0 && has_pre) ? tables + off_pre_hi : nullptr;
         const bool last = p == plan.npass - 1;
@@ -1265,7 +1499,7 @@ static int ntt_run_noalloc(Ctx* c, int mode, fe* out, const fe* in, size_t in_le
         const uint32_t elems = 1u << (lr + lt);
         const uint32_t threads = elems / 2 < (uint32_t)kNttThreads ? (elems / 2 < 32 ? 32 : elems / 2) : kNttThreads;
         const uint32_t blocks = (uint32_t)(n >> (lr + lt));
-        ZK_LAUNCH(c, "ntt_pass", ntt_pass_kernel, blocks, threads, (size_t)elems * 32, P);
+        ZK_LAUNCH(c, "ntt_pass", ntt_pass_kernel<false>, blocks, threads, (size_t)elems * 32, P);
         ZK_TRY_CUDA(cudaGetLastError());
         src = dst;
         log_l += lr;

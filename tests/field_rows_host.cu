@@ -54,6 +54,21 @@ struct Gen {
     }
 };
 
+// floor(w 2^256 / p) by long division, bit by bit
+static zkh::F4 quotient(const zkh::F4& w, const zkh::Field& F) {
+    zkh::F4 rem = w, q = {{0, 0, 0, 0}};
+    for (int i = 0; i < 256; i++) {
+        zkh::add4(rem.v, rem.v, rem.v);  // rem < p < 2^254: no carry
+        for (int j = 3; j > 0; j--) q.v[j] = (q.v[j] << 1) | (q.v[j - 1] >> 63);
+        q.v[0] <<= 1;
+        if (zkh::geq(rem.v, F.p)) {
+            zkh::sub4(rem.v, rem.v, F.p);
+            q.v[0] |= 1;
+        }
+    }
+    return q;
+}
+
 static long bad = 0;
 
 static void check(const char* what, const fe& got, const zkh::F4& want, const zkh::Field& F) {
@@ -82,6 +97,21 @@ int main(int argc, char** argv) {
         check("Fq2 product, 1", f.c0, zkh::sub(Q, zkh::mul(Q, A, C), zkh::mul(Q, B, D)), Q);
         check("Fq2 product, u", f.c1, zkh::add(Q, zkh::mul(Q, A, D), zkh::mul(Q, B, C)), Q);
         const fe x = gen.lazy(R), y = gen.lazy(R);
+        // x w for a constant w with floor(w 2^256 / r), x below 4r (a sum of two lazy values)
+        zk::fe_const k;
+        const zkh::F4 W = canon(words(gen.lazy(R)), R), ws = quotient(W, R);
+        std::memcpy(k.w.v, W.v, 32);
+        std::memcpy(k.ws.v, ws.v, 32);
+        const fe u = gen.lazy(R), v = gen.lazy(R);
+        zkh::F4 x4;
+        zkh::add4(x4.v, words(u).v, words(v).v);
+        fe xs;
+        std::memcpy(xs.v, x4.v, 32);
+        const zkh::F4 xw = zkh::mul(R, zkh::to_mont(R, canon(x4, R)), W);
+        check("Fr product with a constant", zk::fe_mul_const<zk::FrLazyP>(xs, k), xw, R);
+        const fe du = zk::fe_sub_4p<zk::FrLazyP>(u, v);
+        const zkh::F4 duv = zkh::sub(R, canon(words(u), R), canon(words(v), R));
+        check("Fr (u - v) w", zk::fe_mul_const<zk::FrLazyP>(du, k), zkh::mul(R, zkh::to_mont(R, duv), W), R);
         check("Fr product", zk::mul_rows<zk::FrLazyP>(x, y), zkh::mul(R, canon(words(x), R), canon(words(y), R)), R);
     }
     std::printf("%ld differ\n", bad);

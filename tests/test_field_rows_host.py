@@ -19,5 +19,5 @@ def test_product_rows_match_host_arithmetic(tmp_path):
                           os.path.join(REPO, "tests", "field_rows_host.cu"), "-o", str(exe)],
                          capture_output=True, text=True)
     assert res.returncode == 0, res.stderr
-    res = subprocess.run([str(exe), "1000000"], capture_output=True, text=True)
+    res = subprocess.run([str(exe), "300000"], capture_output=True, text=True)
     assert res.returncode == 0, res.stdout
