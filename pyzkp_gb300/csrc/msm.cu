@@ -65,7 +65,7 @@ static constexpr uint32_t kNone = 0xffffffffu;
 #define ZK_MSM_GROUP 4  // measured at 2^20 / 2^22: merge 0.73 / 1.36 ms with 16, 0.48 / 1.02 ms with 4
 #endif
 static constexpr uint32_t kSegment = ZK_MSM_SEGMENT;  // entries per thread in the first accumulation round
-static constexpr uint32_t kMinSegment = 8;            // ... at least, in small pipelines
+static constexpr uint32_t kMinSegment = 4;            // ... at least, in small pipelines
 static constexpr uint32_t kFirstGroup = 2;            // units merged per thread in the first merge round
 static constexpr uint32_t kGroup = ZK_MSM_GROUP;      // units merged per thread in later rounds
 // Buckets per block in the window reduction; small pipelines take the buckets themselves (blocks
@@ -655,14 +655,13 @@ __global__ void msm_hist_offsets_kernel(uint32_t* __restrict__ M, const uint32_t
     }
 }
 
-// Small pipelines: the bucket totals, their exclusive scan (row_ptr, the total at
+// Few buckets in several tiles (small fixed-base pipelines: one set of n W entries): the bucket
+// totals, their exclusive scan (row_ptr, the total at
 // row_ptr[sets B]) and the per-tile cursors in one CTA, instead of four or five launches of
 // a few microseconds each (the totals and cursors walk buckets strided by the CTA size, so
-// the count table is read and written coalesced; the scan takes contiguous runs).
+// the count table is read and written coalesced; the scan takes contiguous runs). Measured on GB300: fixed-base 2000 points
+// 225 -> 215 us.
 static constexpr uint32_t kMetaThreads = 1024;
-// Limits of the one-CTA form (measured on GB300: 2^12 single MSM 0.374 -> 0.360 ms with it;
-// at 2^14, 48 k counts, and in batches of 64 instances the one CTA ran as long as the
-// launches it replaces or longer)
 static constexpr uint64_t kMetaMaxBuckets = 1u << 13;  // row_ptr slots the one CTA handles
 static constexpr uint64_t kMetaMaxCounts = 1u << 14;   // per-tile counts (tiles x B) it walks
 
@@ -714,6 +713,118 @@ __global__ void __launch_bounds__(kMetaThreads) msm_sort_meta_kernel(uint32_t* _
     }
 }
 
+// Pipelines whose sets have one tile each (at most kOneTileMax entries): a CTA per set counts its
+// buckets and scans the counts where they are, then a CTA per set adds the totals of the sets
+// before its own and places the entries: two launches instead of five to six (or, for few
+// buckets, of three with a one-CTA scan of all of them). Measured on GB300 (whole MSM, us): 2^12
+// 262 -> 249, 10000 points 309 -> 294 (311 with the limit at 16384), witness-like 2^14 312 ->
+// 296; a limit of 65536 the same.
+static constexpr uint64_t kOneTileMax = 32768;
+
+// row_ptr[s B + b] := the entries of set s in buckets before b; set_total[s] := its entries.
+__global__ void __launch_bounds__(kTiledThreads) msm_set_hist_kernel(const uint32_t* __restrict__ codes,
+                                                                     const uint32_t* __restrict__ set_base, uint32_t B,
+                                                                     uint32_t* __restrict__ row_ptr,
+                                                                     uint32_t* __restrict__ set_total) {
+    extern __shared__ uint32_t hist[];
+    __shared__ uint32_t warp_sum[kTiledThreads / 32];
+    const uint32_t s = blockIdx.x;
+    const uint32_t e0 = set_base[s], e1 = set_base[s + 1];
+    for (uint32_t b = threadIdx.x; b < B; b += blockDim.x) hist[b] = 0;
+    __syncthreads();
+    for (uint32_t base = e0 + threadIdx.x; base < e1; base += blockDim.x * kSortBatch) {
+        uint32_t code[kSortBatch];
+#pragma unroll
+        for (uint32_t q = 0; q < kSortBatch; q++) {
+            const uint32_t e = base + q * blockDim.x;
+            code[q] = e < e1 ? __ldg(codes + e) : kNoCode;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kSortBatch; q++)
+            if (code[q] != kNoCode) atomicAdd(hist + (code[q] & 0x7fffffffu), 1u);
+    }
+    __syncthreads();
+    // exclusive scan: each thread's run of counters, the runs' sums over the warp, then the warps'
+    const uint32_t per = (B + blockDim.x - 1) / blockDim.x;
+    const uint32_t b0 = min(B, threadIdx.x * per), b1 = min(B, b0 + per);
+    uint32_t sum = 0;
+    for (uint32_t b = b0; b < b1; b++) sum += hist[b];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = sum;
+#pragma unroll
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += v;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t w = warp_sum[lane];
+#pragma unroll
+        for (uint32_t off = 1; off < 32; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, w, off);
+            if (lane >= off) w += v;
+        }
+        warp_sum[lane] = w;
+    }
+    __syncthreads();
+    uint32_t at = incl - sum + (warp ? warp_sum[warp - 1] : 0u);
+    for (uint32_t b = b0; b < b1; b++) {
+        row_ptr[(size_t)s * B + b] = at;
+        at += hist[b];
+    }
+    if (threadIdx.x == 0) set_total[s] = warp_sum[kTiledThreads / 32 - 1];
+}
+
+// The entry of position idx of a set: fixed-base: row w of the shifted bases; GLV: the phi(P) half
+// for h = 1.
+__device__ __forceinline__ uint32_t entry_of(const MsmShape& sh, uint32_t idx, uint32_t nk, uint32_t stride,
+                                             uint32_t code) {
+    const uint32_t point = sh.shared ? (idx / nk) * stride + idx % nk
+                                     : (sh.glv ? (idx >> 1) + (idx & 1) * stride : idx);
+    return point | (code & 0x80000000u);
+}
+
+__global__ void __launch_bounds__(kTiledThreads) msm_set_scatter_kernel(const uint32_t* __restrict__ codes,
+                                                                        const uint32_t* __restrict__ set_base,
+                                                                        MsmShape sh, const MsmInst* __restrict__ insts,
+                                                                        const uint32_t* __restrict__ set_total,
+                                                                        uint32_t* __restrict__ row_ptr,
+                                                                        uint32_t* __restrict__ entries) {
+    extern __shared__ uint32_t cursor[];
+    __shared__ uint32_t warp_sum[kTiledThreads / 32];
+    const uint32_t s = blockIdx.x;
+    const uint32_t sb = set_base[s], e1 = set_base[s + 1];
+    uint32_t before = 0;  // entries of the sets before s
+    for (uint32_t t = threadIdx.x; t < s; t += blockDim.x) before += set_total[t];
+    before = __reduce_add_sync(0xffffffffu, before);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = before;
+    __syncthreads();
+    before = __reduce_add_sync(0xffffffffu, warp_sum[threadIdx.x & 31]);
+    for (uint32_t b = threadIdx.x; b < sh.B; b += blockDim.x) {
+        const uint32_t at = row_ptr[(size_t)s * sh.B + b] + before;
+        cursor[b] = at;
+        row_ptr[(size_t)s * sh.B + b] = at;
+    }
+    if (s == sh.sets - 1 && threadIdx.x == 0) row_ptr[(size_t)sh.sets * sh.B] = before + set_total[s];
+    const uint32_t k = s / sh.Wr;
+    const uint32_t nk = insts[k].n, stride = insts[k].stride;
+    __syncthreads();
+    for (uint32_t base = sb + threadIdx.x; base < e1; base += blockDim.x * kSortBatch) {
+        uint32_t code[kSortBatch];
+#pragma unroll
+        for (uint32_t q = 0; q < kSortBatch; q++) {
+            const uint32_t e = base + q * blockDim.x;
+            code[q] = e < e1 ? __ldcs(codes + e) : kNoCode;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kSortBatch; q++)
+            if (code[q] != kNoCode)
+                entries[atomicAdd(cursor + (code[q] & 0x7fffffffu), 1u)] =
+                    entry_of(sh, base + q * blockDim.x - sb, nk, stride, code[q]);
+    }
+}
+
 __global__ void __launch_bounds__(kTiledThreads) msm_scatter_tiles_kernel(const uint32_t* __restrict__ codes,
                                                                           const uint32_t* __restrict__ set_base,
                                                                           const uint32_t* __restrict__ set_tile0,
@@ -742,12 +853,8 @@ __global__ void __launch_bounds__(kTiledThreads) msm_scatter_tiles_kernel(const 
 #pragma unroll
         for (uint32_t q = 0; q < kSortBatch; q++) {
             if (code[q] == kNoCode) continue;
-            const uint32_t idx = base + q * blockDim.x - sb;
-            // fixed-base: row w of the shifted bases; GLV: the phi(P) half for h = 1
-            const uint32_t point = sh.shared ? (idx / nk) * stride + idx % nk
-                                             : (sh.glv ? (idx >> 1) + (idx & 1) * stride : idx);
             const uint32_t pos = atomicAdd(cursor + (code[q] & 0x7fffffffu), 1u);
-            entries[pos] = point | (code[q] & 0x80000000u);
+            entries[pos] = entry_of(sh, base + q * blockDim.x - sb, nk, stride, code[q]);
         }
     }
 }
@@ -931,6 +1038,14 @@ static constexpr uint32_t kCountHead = 3;
 __host__ __device__ inline uint32_t huge_cap(uint32_t units) { return units / kHugePieces + 2; }
 __host__ __device__ inline uint32_t long_cap(uint32_t units, uint32_t fixmax) { return units / fixmax + 2; }
 
+// Lists bucket k, whose pieces are in span + 1 units, by its pieces.
+__device__ __forceinline__ void list_long(uint32_t* long_list, uint32_t lcap, uint32_t* long_count, uint32_t hcap,
+                                          uint32_t span, uint32_t k) {
+    if (span >= kHugePieces) long_count[kCountHead + hcap + atomicAdd(long_count + 1, 1u)] = k;
+    else if (span < kWarpPieces) long_list[lcap - 1 - atomicAdd(long_count + 2, 1u)] = k;
+    else long_list[atomicAdd(long_count, 1u)] = k;
+}
+
 template <class C, bool kL2>
 __device__ __forceinline__ void fixup_bucket(const uint32_t* __restrict__ row_ptr, uint32_t seg, uint32_t fixmax,
                                              const typename C::P* slot_pts, typename C::P* buckets,
@@ -940,16 +1055,8 @@ __device__ __forceinline__ void fixup_bucket(const uint32_t* __restrict__ row_pt
     if (b1 == b0) return;
     const uint32_t u0 = b0 / seg, u1 = (b1 - 1) / seg;
     if (u0 == u1) return;  // final already (written by the accumulation)
-    if (u1 - u0 >= kHugePieces) {
-        long_count[kCountHead + hcap + atomicAdd(long_count + 1, 1u)] = k;
-        return;
-    }
-    if (u1 - u0 > fixmax && u1 - u0 < kWarpPieces) {
-        long_list[lcap - 1 - atomicAdd(long_count + 2, 1u)] = k;
-        return;
-    }
     if (u1 - u0 > fixmax) {
-        long_list[atomicAdd(long_count, 1u)] = k;
+        list_long(long_list, lcap, long_count, hcap, u1 - u0, k);
         return;
     }
     typename C::P acc = xyzz_get<kL2>(slot_pts + 2 * (size_t)u0 + 1);
@@ -957,22 +1064,58 @@ __device__ __forceinline__ void fixup_bucket(const uint32_t* __restrict__ row_pt
     xyzz_store(buckets + k, acc);
 }
 
+// Piece t of a bucket whose first unit is u0: slot 1 of unit u0, slot 0 of the later ones.
+template <class P>
+__device__ __forceinline__ const P* piece_at(const P* slot_pts, uint32_t u0, uint32_t t) {
+    return slot_pts + 2 * (size_t)(u0 + t) + (t == 0 ? 1 : 0);
+}
+
+// The same with a bucket per quad (every lane of the warp calls; k >= nbuckets: no bucket).
 template <class C>
+__device__ __forceinline__ void fixup_quad(const uint32_t* __restrict__ row_ptr, uint32_t nbuckets, uint32_t seg,
+                                           uint32_t fixmax, const typename C::P* slot_pts, typename C::P* buckets,
+                                           uint32_t* long_list, uint32_t lcap, uint32_t* long_count, uint32_t hcap,
+                                           uint32_t k) {
+    using T = typename C::T;
+    uint32_t u0 = 0, pieces = 0;
+    if (k < nbuckets) {
+        const uint32_t b0 = row_ptr[k], b1 = row_ptr[k + 1];
+        u0 = b0 / seg;
+        const uint32_t span = b1 > b0 ? (b1 - 1) / seg - u0 : 0u;
+        if (span > fixmax) {
+            if ((threadIdx.x & 3) == 0) list_long(long_list, lcap, long_count, hcap, span, k);
+        } else if (span > 0) {
+            pieces = span + 1;
+        }
+    }
+    const uint32_t most = __reduce_max_sync(0xffffffffu, pieces);
+    T acc;
+    c_set_zero(acc);
+    if (pieces) acc = quad_get<false>(piece_at(slot_pts, u0, 0));
+    for (uint32_t t = 1; t < most; t++) {
+        T v;
+        c_set_zero(v);
+        if (t < pieces) v = quad_get<false>(piece_at(slot_pts, u0, t));
+        acc = quad_add(acc, v);
+    }
+    if (pieces) quad_put(buckets + k, acc);
+}
+
+// A bucket per thread, or (kQuad) per quad.
+template <class C, bool kQuad>
 __global__ void __launch_bounds__(128, C::kRedMinBlocks) msm_fixup_kernel(const uint32_t* __restrict__ row_ptr, uint32_t nbuckets,
                                                         uint32_t seg, uint32_t fixmax,
                                                         const typename C::P* __restrict__ slot_pts,
                                                         typename C::P* __restrict__ buckets,
                                                         uint32_t* __restrict__ long_list, uint32_t lcap,
                                                         uint32_t* __restrict__ long_count, uint32_t hcap) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nbuckets) return;
-    fixup_bucket<C, false>(row_ptr, seg, fixmax, slot_pts, buckets, long_list, lcap, long_count, hcap, k);
-}
-
-// Piece t of a bucket whose first unit is u0: slot 1 of unit u0, slot 0 of the later ones.
-template <class P>
-__device__ __forceinline__ const P* piece_at(const P* slot_pts, uint32_t u0, uint32_t t) {
-    return slot_pts + 2 * (size_t)(u0 + t) + (t == 0 ? 1 : 0);
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (kQuad) {
+        fixup_quad<C>(row_ptr, nbuckets, seg, fixmax, slot_pts, buckets, long_list, lcap, long_count, hcap, t >> 2);
+    } else {
+        if (t < nbuckets)
+            fixup_bucket<C, false>(row_ptr, seg, fixmax, slot_pts, buckets, long_list, lcap, long_count, hcap, t);
+    }
 }
 
 // The chunks of the huge buckets (units item0, item0 + stride, ... of the CTAs: unit
@@ -1548,6 +1691,7 @@ static int pipe_init(MsmPipeT<C>& p, uint32_t c, bool fixed, bool glv, const std
         uint64_t largest = 0;
         for (const MsmInst& mi : jobs) largest = std::max<uint64_t>(largest, (uint64_t)mi.n * (fixed ? p.sh.W : halves));
         p.te = (uint32_t)std::max<uint64_t>(std::max<uint64_t>(8192u, 2ull * p.sh.B), ((largest + 63) / 64 + 1023) & ~1023ull);
+        if (largest <= kOneTileMax) p.te = (uint32_t)std::max<uint64_t>(largest, 1024u);  // one tile a set
         p.set_base_h.assign(p.sh.sets + 1, 0);
         p.set_tile0_h.assign(p.sh.sets + 1, 0);
         uint64_t pos = 0, tiles = 0;
@@ -1618,6 +1762,9 @@ static int set_sort_smem_attr(int device) {
     if (!done[device]) {
         ZK_TRY_CUDA(cudaFuncSetAttribute(msm_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTiledMaxB * 4));
         ZK_TRY_CUDA(cudaFuncSetAttribute(msm_scatter_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kTiledMaxB * 4));
+        ZK_TRY_CUDA(cudaFuncSetAttribute(msm_set_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTiledMaxB * 4));
+        ZK_TRY_CUDA(cudaFuncSetAttribute(msm_set_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kTiledMaxB * 4));
         done[device] = true;
     }
@@ -1703,6 +1850,15 @@ static int enqueue_tiled_sort(Ctx* c, MsmPipeT<C>& p, int scalars_mont) {
         ZK_TRY_CUDA(cudaGetLastError());
     }
     const size_t smem = (size_t)sh.B * 4;
+    if (p.tiles == sh.sets && p.te <= kOneTileMax) {
+        ZK_LAUNCH(c, "msm_set_hist", msm_set_hist_kernel, sh.sets, kTiledThreads, smem, codes, p.set_base, sh.B,
+                  p.row_ptr, p.tile_hist);
+        ZK_TRY_CUDA(cudaGetLastError());
+        ZK_LAUNCH(c, "msm_set_scatter", msm_set_scatter_kernel, sh.sets, kTiledThreads, smem, codes, p.set_base, sh,
+                  p.d_inst, p.tile_hist, p.row_ptr, p.entries);
+        ZK_TRY_CUDA(cudaGetLastError());
+        return ZK_OK;
+    }
     ZK_LAUNCH(c, "msm_hist", msm_hist_kernel, p.tiles, kTiledThreads, smem, codes, p.set_base, p.set_tile0, sh.sets,
               p.te, sh.B, p.tile_hist);
     ZK_TRY_CUDA(cudaGetLastError());
@@ -1772,7 +1928,12 @@ static int pipe_enqueue_reduce(Ctx* c, MsmPipeT<C>& p) {
         // counts and chunk counters to zero (the keys are written before they are read)
         const uint32_t lcap = long_cap(p.units, sh.fixmax);
         ZK_TRY_CUDA(cudaMemsetAsync(p.long_count, 0, (kCountHead + (size_t)hcap) * 4, st));
-        ZK_LAUNCH(c, "msm_fixup", msm_fixup_kernel<C>, (unsigned)((p.nbuckets + 127) / 128), 128, 0, p.row_ptr,
+        // a quad a bucket while its lanes are few: measured (whole MSM, us, thread / quad) 2^8 236 /
+        // 220, 2^12 276 / 262, 2^14 348 / 340, 2^16 (53248 buckets) 520 / 504, 2^20 2942 / 2962;
+        // G2 with its larger points 1000 491 / 455, 2^16 (40960 buckets) 1269 / 1291
+        const bool quad = p.nbuckets < (uint64_t)c->num_sms * (sizeof(P) > 128 ? kSmallBucketsPerSm / 4 : kSmallBucketsPerSm);
+        auto* fixup = quad ? &msm_fixup_kernel<C, true> : &msm_fixup_kernel<C, false>;
+        ZK_LAUNCH(c, "msm_fixup", fixup, (unsigned)((p.nbuckets * (quad ? 4 : 1) + 127) / 128), 128, 0, p.row_ptr,
                   (uint32_t)p.nbuckets, sh.seg, sh.fixmax, p.slot_pts_a, p.buckets, p.long_list, lcap, p.long_count, hcap);
         ZK_TRY_CUDA(cudaGetLastError());
         // the chunk sums of huge buckets go to slot_pts_b (merge-round space, unused in fixup mode)
