@@ -161,23 +161,24 @@ uint32_t msm_auto_window(size_t n) {
     return (uint32_t)c;
 }
 
-// GLV: the same rule over n scalars (2n half-scalars of 128 bits), lowered while the window
-// count stays the same (fewer buckets for the same entries: c = 14 -> 13, 12 stays).
-// Window size of the GLV split (halves of ~127 bits). Measured on GB300 for n = 2^8 .. 2^20
-// (G1, every c from about log2(n) - 6 to log2(n), uniform and witness-like scalars); the
-// table holds the c with the smallest product of the two times relative to their best.
-// A sparse top window (c = 9: 2 of its 9 bits used, c = 14: 2 of 14) puts a large share of
-// all points into a few buckets, and so do repeated small scalars (0 and 1 in witnesses);
-// the long-bucket fixup adds their pieces in trees of serial point additions (0.04 - 0.6
-// ms), which the merge rounds of larger c avoid. Against the earlier rule (log2(n) - 3,
-// lowered while W stays): uniform 2^8 -22%, 2^10 -19%, 2^12 -7%; witness-like 2^11 -10%,
-// 2^17 -27%, 2^18 -31% (uniform +3% / +6% there). From 2^19 on c = 16 stays (uniform
-// 2^19 / 2^20 best at 16, witness-like at 13 / 14).
+// Window size of the GLV split (halves of ~127 bits), n scalars. Measured on GB300 (G1, n = 2^8 ..
+// 3 * 2^20 in half powers of two, every c from about log2(n) - 6 to log2(n), uniform and
+// witness-like scalars): the table holds the c with the smallest product of the two times
+// relative to their best. Windows that leave the top one sparse (c = 9 uses 2 of its 9 bits,
+// c = 14 2 of 14) crowd a few buckets, and so do repeated small scalars. Against one c per
+// ceil(log2 n) (8, 8, 8, 9, 10, 11, 11, 13, 13, 13, 15 for 2^8 .. 2^18, then 16), us uniform /
+// witness-like: 768 216 / 220 -> 212 / 204, 1536 231 / 220 -> 219 / 219, 3072 236 / 231 -> 231 /
+// 222, 196608 961 / 730 -> 925 / 664, 262144 1147 / 840 -> 1156 / 805.
 uint32_t msm_auto_window_glv(size_t n) {
-    uint32_t lg = 0;
-    while ((1ull << lg) < n) lg++;
-    static const uint8_t kMeasured[19] = {0, 0, 0, 0, 0, 0, 0, 0, 8, 8, 8, 9, 10, 11, 11, 13, 13, 13, 15};
-    if (lg >= 8 && lg <= 18) return kMeasured[lg];
+    static const struct {
+        size_t upto;
+        uint32_t c;
+    } kMeasured[] = {{640, 8}, {1280, 9}, {2560, 10}, {20000, 11}, {229376, 13}, {280000, 14}};
+    if (n > 128) {
+        for (const auto& m : kMeasured)
+            if (n <= m.upto) return m.c;
+        return 16;
+    }
     uint32_t c = msm_auto_window(n);
     while (c > 4 && (128 + c - 2) / (c - 1) == (128 + c - 1) / c) c--;
     return c;
@@ -545,11 +546,22 @@ static constexpr uint32_t kTiledMaxB = 1u << 15;  // 128 KB of shared-memory cou
 static constexpr uint32_t kTiledThreads = 1024;
 static constexpr uint32_t kSortBatch = 8;  // codes loaded per thread before they are counted / placed
 
+// Memory that the first kernel of a pipeline clears: n16 16-byte units and n4 words.
+struct MsmZero {
+    uint4* wide;
+    size_t n16;
+    uint32_t* words;
+    size_t n4;
+};
+
 template <class C>
 __global__ void msm_codes_kernel(const MsmInst* __restrict__ insts, const uint32_t* __restrict__ offs, uint32_t j0,
                                  uint32_t N, int scalars_mont, MsmShape sh, const uint32_t* __restrict__ set_base,
-                                 uint32_t* __restrict__ codes) {
-    const uint32_t j = j0 + blockIdx.x * blockDim.x + threadIdx.x;
+                                 uint32_t* __restrict__ codes, MsmZero zero) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, j = j0 + t;
+    // the pipeline's buckets and fixup counts start at zero (no memsets of their own)
+    for (size_t i = t; i < zero.n16; i += (size_t)gridDim.x * blockDim.x) zero.wide[i] = make_uint4(0, 0, 0, 0);
+    for (size_t i = t; i < zero.n4; i += (size_t)gridDim.x * blockDim.x) zero.words[i] = 0;
     if (j >= N) return;
     const uint32_t k = find_inst(offs, sh.inst, j);
     const uint32_t i = j - __ldg(offs + k);
@@ -1309,8 +1321,11 @@ __device__ __forceinline__ void targets_cta(const typename C::P* lines, const Ms
 
 template <class C>
 __global__ void __launch_bounds__(128) msm_targets_kernel(const typename C::P* __restrict__ lines, MsmShape sh,
-                                                          typename C::P* __restrict__ out) {
+                                                          typename C::P* __restrict__ out,
+                                                          const uint32_t* __restrict__ d_total,
+                                                          uint32_t* __restrict__ total) {
     __shared__ typename C::P red[4];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *total = *d_total;
     targets_cta<C, false>(lines, sh, out, red, blockIdx.x);
 }
 
@@ -1634,8 +1649,17 @@ struct MsmPipeT {
     uint32_t te = 0, tiles = 0;
     std::vector<uint32_t> set_base_h, set_tile0_h;  // sets + 1 entries each
     uint32_t *set_base = nullptr, *set_tile0 = nullptr, *tile_hist = nullptr;
-    P* h_tgt = nullptr;  // host copy of the per-set targets (sets * targets)
+    std::vector<char> desc_h;  // the packed descriptors: d_inst .. d_inst + desc_bytes on the device
+    size_t desc_bytes = 0;
+    // page-locked host memory: the per-set targets (sets * targets), which the targets kernel
+    // writes there, then the entry count
+    P* h_tgt = nullptr;
     uint32_t* h_total = nullptr;
+    size_t host_bytes() const { return host_elems() * sizeof(P) + 16; }
+    void set_host(char* at) {
+        h_tgt = reinterpret_cast<P*>(at);
+        h_total = reinterpret_cast<uint32_t*>(at + host_elems() * sizeof(P));
+    }
     size_t host_elems() const { return (size_t)sh.sets * sh.targets; }
 };
 
@@ -1727,6 +1751,11 @@ static size_t pipe_layout(MsmPipeT<C>& p, char* base) {
     const size_t first_out = (p.units + kFirstGroup - 1) / kFirstGroup;
     p.d_inst = reinterpret_cast<MsmInst*>(take(p.inst.size() * sizeof(MsmInst)));
     p.d_offs = reinterpret_cast<uint32_t*>(take(p.offs.size() * 4));
+    if (p.tiled) {
+        p.set_base = reinterpret_cast<uint32_t*>(take(p.set_base_h.size() * 4));
+        p.set_tile0 = reinterpret_cast<uint32_t*>(take(p.set_tile0_h.size() * 4));
+    }
+    p.desc_bytes = off;
     p.digits = reinterpret_cast<uint32_t*>(
         take(std::max<uint64_t>(p.max_entries * 4, p.N * sizeof(fe) * (sh.glv ? 2 : 1))));
     p.row_ptr = reinterpret_cast<uint32_t*>(take((p.nbuckets + 1) * 4));
@@ -1745,11 +1774,7 @@ static size_t pipe_layout(MsmPipeT<C>& p, char* base) {
     p.Eb = sh.g > 1 ? reinterpret_cast<P*>(take((size_t)sh.sets * sh.G * sizeof(P))) : nullptr;
     p.lines = reinterpret_cast<P*>(take((size_t)sh.sets * lines_per_set(sh) * sizeof(P)));
     p.tgt = reinterpret_cast<P*>(take(p.host_elems() * sizeof(P)));
-    if (p.tiled) {
-        p.set_base = reinterpret_cast<uint32_t*>(take(p.set_base_h.size() * 4));
-        p.set_tile0 = reinterpret_cast<uint32_t*>(take(p.set_tile0_h.size() * 4));
-        p.tile_hist = reinterpret_cast<uint32_t*>(take((size_t)p.tiles * sh.B * 4));
-    }
+    if (p.tiled) p.tile_hist = reinterpret_cast<uint32_t*>(take((size_t)p.tiles * sh.B * 4));
     return off;
 }
 
@@ -1771,18 +1796,22 @@ static int set_sort_smem_attr(int device) {
     return ZK_OK;
 }
 
-// The pipeline's descriptors to the device: instances, scalar offsets, sort layout.
+// The pipeline's descriptors to the device: instances, scalar offsets, sort layout, packed as
+// pipe_layout places them (one copy: four small ones took ~10 us of a single MSM's call).
 template <class C>
 static int pipe_upload(Ctx* c, MsmPipeT<C>& p) {
-    cudaStream_t st = c->stream;
-    ZK_TRY_CUDA(cudaMemcpyAsync(p.d_inst, p.inst.data(), p.inst.size() * sizeof(MsmInst), cudaMemcpyHostToDevice, st));
-    ZK_TRY_CUDA(cudaMemcpyAsync(p.d_offs, p.offs.data(), p.offs.size() * 4, cudaMemcpyHostToDevice, st));
+    p.desc_h.resize(p.desc_bytes);
+    char* const base = reinterpret_cast<char*>(p.d_inst);
+    auto put = [&](const void* dev, const void* src, size_t bytes) {
+        std::memcpy(p.desc_h.data() + (static_cast<const char*>(dev) - base), src, bytes);
+    };
+    put(p.d_inst, p.inst.data(), p.inst.size() * sizeof(MsmInst));
+    put(p.d_offs, p.offs.data(), p.offs.size() * 4);
     if (p.tiled) {
-        ZK_TRY_CUDA(cudaMemcpyAsync(p.set_base, p.set_base_h.data(), p.set_base_h.size() * 4, cudaMemcpyHostToDevice,
-                                    st));
-        ZK_TRY_CUDA(cudaMemcpyAsync(p.set_tile0, p.set_tile0_h.data(), p.set_tile0_h.size() * 4,
-                                    cudaMemcpyHostToDevice, st));
+        put(p.set_base, p.set_base_h.data(), p.set_base_h.size() * 4);
+        put(p.set_tile0, p.set_tile0_h.data(), p.set_tile0_h.size() * 4);
     }
+    ZK_TRY_CUDA(cudaMemcpyAsync(base, p.desc_h.data(), p.desc_bytes, cudaMemcpyHostToDevice, c->stream));
     return ZK_OK;
 }
 
@@ -1833,20 +1862,26 @@ static int enqueue_tiled_sort(Ctx* c, MsmPipeT<C>& p, int scalars_mont) {
     int rc = set_sort_smem_attr(c->device);
     if (rc != ZK_OK) return rc;
     uint32_t* codes = p.digits;
+    MsmZero zero{reinterpret_cast<uint4*>(p.buckets), p.nbuckets * sizeof(typename C::P) / 16, p.long_count,
+                 kCountHead + (size_t)huge_cap(p.units)};
+    // CTAs for the scalars, and enough of them to clear with (few scalars, many buckets)
+    const unsigned zero_ctas = (unsigned)std::min<size_t>((zero.n16 + 1023) / 1024, (size_t)c->num_sms * 4);
+    auto ctas = [&](uint32_t n) { return std::max((n + 255) / 256, zero.n16 ? zero_ctas : 0u); };
     if (!c->scalar_chunks.empty() && c->scalar_chunks.back().first == N && p.inst.size() == 1) {
         // scalars still arriving: each chunk's codes wait for its copy only
         uint32_t j0 = 0;
         for (const auto& ch : c->scalar_chunks) {
             ZK_TRY_CUDA(cudaStreamWaitEvent(st, ch.second, 0));
-            ZK_LAUNCH(c, "msm_codes", msm_codes_kernel<C>, (unsigned)((ch.first - j0 + 255) / 256), 256, 0, p.d_inst,
-                      p.d_offs, j0, ch.first, scalars_mont, sh, p.set_base, codes);
+            ZK_LAUNCH(c, "msm_codes", msm_codes_kernel<C>, ctas(ch.first - j0), 256, 0, p.d_inst,
+                      p.d_offs, j0, ch.first, scalars_mont, sh, p.set_base, codes, zero);
             ZK_TRY_CUDA(cudaGetLastError());
+            zero.n16 = zero.n4 = 0;  // cleared by the first chunk
             j0 = ch.first;
         }
     } else {
         if (!c->scalar_chunks.empty()) ZK_TRY_CUDA(cudaStreamWaitEvent(st, c->scalar_chunks.back().second, 0));
-        ZK_LAUNCH(c, "msm_codes", msm_codes_kernel<C>, (unsigned)((p.N + 255) / 256), 256, 0, p.d_inst, p.d_offs, 0u,
-                  N, scalars_mont, sh, p.set_base, codes);
+        ZK_LAUNCH(c, "msm_codes", msm_codes_kernel<C>, ctas(N), 256, 0, p.d_inst, p.d_offs, 0u,
+                  N, scalars_mont, sh, p.set_base, codes, zero);
         ZK_TRY_CUDA(cudaGetLastError());
     }
     const size_t smem = (size_t)sh.B * 4;
@@ -1892,11 +1927,14 @@ static int pipe_enqueue_sort(Ctx* c, MsmPipeT<C>& p, int scalars_mont, bool uplo
         int rc = pipe_upload(c, p);
         if (rc != ZK_OK) return rc;
     }
+    if (p.tiled) return enqueue_tiled_sort<C>(c, p, scalars_mont);  // clears buckets and counts itself
     ZK_TRY_CUDA(cudaMemsetAsync(p.buckets, 0, p.nbuckets * sizeof(P), c->stream));
-    return p.tiled ? enqueue_tiled_sort<C>(c, p, scalars_mont) : enqueue_atomic_sort<C>(c, p, scalars_mont);
+    ZK_TRY_CUDA(cudaMemsetAsync(p.long_count, 0, (kCountHead + (size_t)huge_cap(p.units)) * 4, c->stream));
+    return enqueue_atomic_sort<C>(c, p, scalars_mont);
 }
 
-// The copies of the targets and the entry count to p.h_tgt / p.h_total.
+// The copies of the targets and the entry count to the host (work-queue form; the targets kernel
+// of the other form writes them there).
 template <class C>
 static int pipe_enqueue_copies(Ctx* c, MsmPipeT<C>& p) {
     using P = typename C::P;
@@ -1925,9 +1963,8 @@ static int pipe_enqueue_reduce(Ctx* c, MsmPipeT<C>& p) {
     // fixup pass, longer ones by merge rounds (kFixupDensity).
     if (p.max_entries <= (uint64_t)p.nbuckets * kFixupDensity) {
         const uint32_t hcap = huge_cap(p.units);
-        // counts and chunk counters to zero (the keys are written before they are read)
+        // counts and chunk counters are zero since the sort (the keys are written before they are read)
         const uint32_t lcap = long_cap(p.units, sh.fixmax);
-        ZK_TRY_CUDA(cudaMemsetAsync(p.long_count, 0, (kCountHead + (size_t)hcap) * 4, st));
         // a quad a bucket while its lanes are few: measured (whole MSM, us, thread / quad) 2^8 236 /
         // 220, 2^12 276 / 262, 2^14 348 / 340, 2^16 (53248 buckets) 520 / 504, 2^20 2942 / 2962;
         // G2 with its larger points 1000 491 / 455, 2^16 (40960 buckets) 1269 / 1291
@@ -1976,19 +2013,19 @@ static int pipe_enqueue_reduce(Ctx* c, MsmPipeT<C>& p) {
     ZK_TRY_CUDA(cudaGetLastError());
     uint32_t tw = 1;
     while (tw < 4 && 16 * tw < len) tw *= 2;
-    ZK_LAUNCH(c, "msm_targets", msm_targets_kernel<C>, sh.sets * sh.targets, 32 * tw, 0, p.lines, sh, p.tgt);
+    ZK_LAUNCH(c, "msm_targets", msm_targets_kernel<C>, sh.sets * sh.targets, 32 * tw, 0, p.lines, sh, p.h_tgt, d_total,
+              p.h_total);
     ZK_TRY_CUDA(cudaGetLastError());
     return ZK_OK;
 }
 
-// Enqueue the device part of a pipeline on the context stream, ending with the copies of
-// the targets and the entry count to p.h_tgt / p.h_total. Allocates nothing, so it can be
+// Enqueue the device part of a pipeline on the context stream, ending with the targets and the
+// entry count in p.h_tgt / p.h_total. Allocates nothing, so it can be
 // captured into a CUDA graph (the instance descriptors are uploaded only if `upload`).
 template <class C>
 static int pipe_enqueue(Ctx* c, MsmPipeT<C>& p, int scalars_mont, bool upload) {
     int rc = pipe_enqueue_sort<C>(c, p, scalars_mont, upload);
     if (rc == ZK_OK) rc = pipe_enqueue_reduce<C>(c, p);
-    if (rc == ZK_OK) rc = pipe_enqueue_copies<C>(c, p);
     return rc;
 }
 
@@ -2570,6 +2607,18 @@ static int enqueue_all(Ctx* c, std::vector<MsmPipeT<C>>& pipes, int scalars_mont
     return rc == ZK_OK ? finish() : rc;
 }
 
+// A page-locked block of the context's pool for the span of one call (the device is done with it
+// when the call returns, also after an error: those paths synchronise first).
+struct PinnedBlock {
+    Ctx* c;
+    void* p = nullptr;
+    size_t bytes = 0;
+    explicit PinnedBlock(Ctx* ctx) : c(ctx) {}
+    PinnedBlock(const PinnedBlock&) = delete;
+    int take(size_t n) { return pinned_take(c, n, &p, &bytes); }
+    ~PinnedBlock() { pinned_give(c, p, bytes); }
+};
+
 template <class C>
 static int batch_run(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mont, uint32_t window_bits, uint8_t* out_xy,
                      int32_t* out_is_inf) {
@@ -2579,12 +2628,12 @@ static int batch_run(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mont,
     if (rc != ZK_OK) return rc;
     set_infinity(out_xy, out_is_inf, empty, 2 * sizeof(typename HostOf<C>::T));
     if (pipes.empty()) return ZK_OK;
-    size_t bytes = 0, host_elems = 0;
+    size_t bytes = 0, host_bytes = 0;
     std::vector<size_t> at(pipes.size());
     for (size_t q = 0; q < pipes.size(); q++) {
         at[q] = bytes;
         bytes += (pipe_layout(pipes[q], nullptr) + 255) & ~(size_t)255;
-        host_elems += pipes[q].host_elems();
+        host_bytes += pipes[q].host_bytes();
     }
     // the work-queue form (zk_msm_batch_set_queue): its descriptors after the pipelines
     std::unique_ptr<MsmQueueT<C>> queue;
@@ -2596,16 +2645,15 @@ static int batch_run(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mont,
         bytes += queue->bytes;
         queue->h_status = &queue_status;
     }
+    PinnedBlock host(c);
+    if ((rc = host.take(host_bytes)) != ZK_OK) return rc;
     char* arena = nullptr;
     if ((rc = scratch_alloc(c, bytes, reinterpret_cast<void**>(&arena))) != ZK_OK) return rc;
-    std::vector<typename C::P> host_t(host_elems);
-    std::vector<uint32_t> host_total(pipes.size());
     size_t h = 0;
     for (size_t q = 0; q < pipes.size(); q++) {
         pipe_layout(pipes[q], arena + at[q]);
-        pipes[q].h_tgt = host_t.data() + h;
-        pipes[q].h_total = &host_total[q];
-        h += pipes[q].host_elems();
+        pipes[q].set_host(static_cast<char*>(host.p) + h);
+        h += pipes[q].host_bytes();
     }
     if (queue) {
         for (auto& p : pipes)
@@ -2671,12 +2719,12 @@ static int batch_submit(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mo
         return ZK_OK;
     }
     std::vector<MsmPipeT<C>>& pipes = a->pipes;
-    size_t bytes = 0, host_elems = 0;
+    size_t bytes = 0, host_bytes = 0;
     std::vector<size_t> at(pipes.size());
     for (size_t q = 0; q < pipes.size(); q++) {
         at[q] = bytes;
         bytes += (pipe_layout(pipes[q], nullptr) + 255) & ~(size_t)255;
-        host_elems += pipes[q].host_elems();
+        host_bytes += pipes[q].host_bytes();
     }
     const size_t queue_at = bytes;
     if (c->msm_queue && kQueueForm<C>) {
@@ -2684,25 +2732,20 @@ static int batch_submit(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mo
         if ((rc = queue_plan<C>(c, pipes, *a->queue)) != ZK_OK) return rc;
         bytes += a->queue->bytes;
     }
-    // pinned host targets (then the entry totals and the queue status): the device-to-host
-    // copies stay asynchronous
-    const size_t host_bytes = host_elems * sizeof(typename C::P) + (pipes.size() + 1) * sizeof(uint32_t);
+    // page-locked host targets and entry totals of each pipeline, then the queue status
     a->ctx = c;
-    if ((rc = pinned_take(c, host_bytes, &a->pinned, &a->pinned_bytes)) != ZK_OK) return rc;
+    if ((rc = pinned_take(c, host_bytes + 16, &a->pinned, &a->pinned_bytes)) != ZK_OK) return rc;
     ZK_TRY_CUDA(cudaEventCreateWithFlags(&a->done_ev, cudaEventDisableTiming));
     char* arena = nullptr;
     if ((rc = scratch_alloc(c, bytes, reinterpret_cast<void**>(&arena))) != ZK_OK) return rc;
-    auto* host_t = static_cast<typename C::P*>(a->pinned);
-    auto* totals = reinterpret_cast<uint32_t*>(host_t + host_elems);
     size_t h = 0;
     for (size_t q = 0; q < pipes.size(); q++) {
         pipe_layout(pipes[q], arena + at[q]);
-        pipes[q].h_tgt = host_t + h;
-        pipes[q].h_total = totals + q;
-        h += pipes[q].host_elems();
+        pipes[q].set_host(static_cast<char*>(a->pinned) + h);
+        h += pipes[q].host_bytes();
     }
     if (a->queue) {
-        a->queue->h_status = totals + pipes.size();
+        a->queue->h_status = reinterpret_cast<uint32_t*>(static_cast<char*>(a->pinned) + h);
         *a->queue->h_status = 0;
         for (auto& p : pipes)
             if ((rc = pipe_upload(c, p)) != ZK_OK) break;
@@ -2831,7 +2874,7 @@ int msm_plan_create(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mont, 
     for (size_t q = 0; q < plan->pipes.size(); q++) {
         at[q] = bytes;
         bytes += (pipe_layout(plan->pipes[q], nullptr) + 255) & ~(size_t)255;
-        host_bytes += plan->pipes[q].host_elems() * sizeof(xyzz_t) + 16;
+        host_bytes += plan->pipes[q].host_bytes();
     }
     const size_t queue_at = bytes;
     if (plan->queue) {
@@ -2859,10 +2902,8 @@ int msm_plan_create(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mont, 
         MsmPipeT<CurveG1>& p = plan->pipes[q];
         for (size_t k = 0; k < p.inst.size(); k++) p.inst[k].scalars = plan->slots[p.out_index[k]];
         pipe_layout(p, plan->arena + at[q]);
-        p.h_tgt = reinterpret_cast<xyzz_t*>(hp);
-        hp += p.host_elems() * sizeof(xyzz_t);
-        p.h_total = reinterpret_cast<uint32_t*>(hp);
-        hp += 16;
+        p.set_host(hp);
+        hp += p.host_bytes();
         const int urc = pipe_upload(c, p);
         if (urc != ZK_OK) return fail(urc);
     }
