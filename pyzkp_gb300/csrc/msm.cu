@@ -1608,12 +1608,6 @@ static zkh::XyzzT<typename HostOf<C>::T> to_host(const typename C::P& d) {
     return h;
 }
 
-template <class H>
-static zkh::XyzzT<H> host_dbl_n(zkh::XyzzT<H> p, uint32_t times) {
-    for (uint32_t i = 0; i < times; i++) p = zkh::xyzz_dbl(p);
-    return p;
-}
-
 uint32_t msm_window_for(const Ctx* c, size_t n, bool glv) {
     uint32_t lg = 0;
     while ((1ull << lg) < n) lg++;
@@ -2043,28 +2037,43 @@ class HostPool {
     }
 
     void run(size_t count, const std::function<void(size_t)>& fn) {
-        if (count == 1 || workers_ == 0) {  // no helper: no shared state, no lock
+        // no helper: no shared state, no lock; and a few tasks do not wait for a run that itself still
+        // waits for its data
+        if (count == 1 || workers_ == 0 || (count <= 16 && early())) {
             for (size_t i = 0; i < count; i++) fn(i);
             return;
         }
         run_with(count, fn, [] {});
     }
 
+    // Whether the run in progress was started before its data (see run_with).
+    bool early() const { return early_.load(std::memory_order_acquire); }
+
     // run() in which the calling thread first executes own(): own() may take tasks itself
     // through run_one() (the same ticket, so in the same index order as the workers), e.g.
-    // to consume results in order and compute whichever no worker has taken yet.
+    // to consume results in order and compute whichever no worker has taken yet. early: own()
+    // first waits for the tasks' data and the tasks wait for own() to say so, so that the
+    // workers are awake by then. only_if_free: returns false, having done nothing, if another
+    // run is in progress.
     template <class Own>
-    void run_with(size_t count, const std::function<void(size_t)>& fn, Own&& own, size_t max_helpers = ~size_t(0)) {
+    bool run_with(size_t count, const std::function<void(size_t)>& fn, Own&& own, size_t max_helpers = ~size_t(0),
+                  bool early = false, bool only_if_free = false) {
         if (count > kMaxTasks) {
             for (size_t i = 0; i < count; i++) fn(i);
             own();
-            return;
+            return true;
         }
         if (count == 0) {
             own();
-            return;
+            return true;
         }
-        std::lock_guard<std::mutex> serial(run_mu_);
+        std::unique_lock<std::mutex> serial(run_mu_, std::defer_lock);
+        if (only_if_free) {
+            if (!serial.try_lock()) return false;
+        } else {
+            serial.lock();
+        }
+        early_.store(early, std::memory_order_release);
         gen_ = (gen_ + 1) & 0xffffu;
         fn_ = &fn;
         done_.store(0, std::memory_order_relaxed);
@@ -2090,6 +2099,8 @@ class HostPool {
         while (done_.load(std::memory_order_acquire) < count)
             done_cv_.wait_for(g, std::chrono::milliseconds(1),
                               [&] { return done_.load(std::memory_order_acquire) >= count; });
+        early_.store(false, std::memory_order_release);
+        return true;
     }
 
     // Claim and run the next task of the run in progress; false if none is left.
@@ -2144,6 +2155,7 @@ class HostPool {
     const std::function<void(size_t)>* fn_ = nullptr;
     std::atomic<uint64_t> ticket_{0};
     std::atomic<size_t> done_{0};
+    std::atomic<bool> early_{false};   // the run in progress was started before its data (run_with)
     std::atomic<int64_t> pending_{0};  // wake-ups the woken workers still have to pass on
     static constexpr size_t kFanout = 2;
     uint64_t wake_ = 0;  // under mu_
@@ -2166,7 +2178,7 @@ static zkh::XyzzT<typename HostOf<C>::T> window_sum(const MsmPipeT<C>& p, uint32
     }
     zkh::XyzzT<H> sw = zkh::xyzz_add(h, to_host<C>(T[sh.plain - 1]));
     if (sh.g == 1) return sw;
-    sw = host_dbl_n(sw, log_g);
+    sw = zkh::xyzz_dbl_n(sw, log_g);
     return zkh::xyzz_add(sw, to_host<C>(T[0]));
 }
 
@@ -2178,7 +2190,7 @@ static void horner_out(const MsmPipeT<C>& p, Get&& get, uint8_t* out_xy, int32_t
     using H = typename HostOf<C>::T;
     zkh::XyzzT<H> total = zkh::xyzz_inf<H>();
     for (int w = (int)p.sh.Wr - 1; w >= 0; w--) {
-        total = host_dbl_n(total, p.sh.c);
+        total = zkh::xyzz_dbl_n(total, p.sh.c);
         total = zkh::xyzz_add(total, get((uint32_t)w));
     }
     H x, y;
@@ -2195,21 +2207,26 @@ static constexpr size_t kCombineHelpers = ZK_COMBINE_HELPERS;  // pool workers o
 // Combine every instance of `pipes`: the window sums of all instances in parallel on the
 // host pool, then each instance's Horner (in parallel across instances); a single instance
 // overlaps its Horner with its window sums.
+// CSR entries of a pipeline up to which a single MSM wakes its helpers early (~0.5 ms of device
+// time at 2 M).
+static constexpr uint64_t kEarlyEntries = 1u << 21;
+
+// `wait` (optional) waits for the device to have written the targets; its error is returned. A
+// single instance calls it with the pool's helpers already woken: a wake-up takes 10 - 20 us,
+// as long as two or three window sums.
 template <class C>
-static void combine_all(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, uint8_t* out_xy, int32_t* out_is_inf,
-                        bool record = true) {
+static int combine_all(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, uint8_t* out_xy, int32_t* out_is_inf,
+                       bool record = true, const std::function<int()>& wait = nullptr) {
     using H = typename HostOf<C>::T;
     constexpr size_t kOut = 2 * sizeof(H);  // bytes of one affine result
-    const auto t0 = std::chrono::steady_clock::now();
+    auto t0 = std::chrono::steady_clock::now();
     struct Inst {
         uint32_t q, k;
         size_t first;  // index of its first window sum
     };
     std::vector<Inst> insts;
     std::vector<std::pair<uint32_t, uint32_t>> win;  // (instance, window)
-    uint64_t entries = 0;
     for (uint32_t q = 0; q < pipes.size(); q++) {
-        entries += *pipes[q].h_total;
         for (uint32_t k = 0; k < pipes[q].sh.inst; k++) {
             insts.push_back({q, k, win.size()});
             for (uint32_t w = 0; w < pipes[q].sh.Wr; w++) win.emplace_back((uint32_t)insts.size() - 1, w);
@@ -2225,22 +2242,48 @@ static void combine_all(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, uint8_t* 
         const MsmPipeT<C>& p = pipes[insts[0].q];
         const uint32_t k = insts[0].k, W = (uint32_t)win.size();
         std::unique_ptr<std::atomic<uint32_t>[]> ready(new std::atomic<uint32_t>[W]());
+        std::atomic<int> data{wait ? 0 : 1};  // 0: not there yet, 1: there, 2: it will not come
+        int rc = ZK_OK;
         const std::function<void(size_t)> task = [&](size_t t) {
-            sums[t] = window_sum<C>(p, k, W - 1 - (uint32_t)t);
+            int d;
+            while ((d = data.load(std::memory_order_acquire)) == 0) std::this_thread::yield();
+            if (d == 1) sums[t] = window_sum<C>(p, k, W - 1 - (uint32_t)t);
             ready[t].store(1, std::memory_order_release);
+        };
+        auto wait_data = [&] {
+            if (data.load(std::memory_order_relaxed) != 0) return;
+            rc = wait();
+            t0 = std::chrono::steady_clock::now();
+            data.store(rc == ZK_OK ? 1 : 2, std::memory_order_release);
         };
         const size_t o = p.out_index[k];
         // a few helpers keep ahead of the Horner (a window sum costs about as much as 2-3
         // windows of its doublings)
-        pool.run_with(W, task, [&] {
+        auto own = [&] {
+            wait_data();
+            if (rc != ZK_OK) return;
             horner_out<C>(p, [&](uint32_t w) -> const zkh::XyzzT<H>& {
                 const uint32_t t = W - 1 - w;
                 while (!ready[t].load(std::memory_order_acquire))
                     if (!pool.run_one()) std::this_thread::yield();  // a worker is on it
                 return sums[t];
             }, out_xy + kOut * o, out_is_inf + o);
-        }, kCombineHelpers);
+        };
+        if (!pool.run_with(W, task, own, kCombineHelpers, wait != nullptr, true)) {
+            wait_data();
+            if (rc == ZK_OK && pool.early()) {  // another thread's run still waits for its device: do without the pool
+                for (uint32_t t = 0; t < W; t++) task(t);
+                horner_out<C>(p, [&](uint32_t w) -> const zkh::XyzzT<H>& { return sums[W - 1 - w]; }, out_xy + kOut * o,
+                              out_is_inf + o);
+            } else if (rc == ZK_OK) {
+                pool.run_with(W, task, own, kCombineHelpers);
+            }
+        }
+        if (rc != ZK_OK) return rc;
     } else {
+        if (wait)
+            if (const int rc = wait(); rc != ZK_OK) return rc;
+        t0 = std::chrono::steady_clock::now();
         pool.run(win.size(), [&](size_t t) {
             const Inst& in = insts[win[t].first];
             sums[t] = window_sum<C>(pipes[in.q], in.k, win[t].second);
@@ -2253,7 +2296,9 @@ static void combine_all(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, uint8_t* 
                           out_xy + kOut * o, out_is_inf + o);
         });
     }
-    if (!record) return;  // a worker thread of an asynchronous batch leaves the context's tables alone
+    if (!record) return ZK_OK;  // a worker thread of an asynchronous batch leaves the context's tables alone
+    uint64_t entries = 0;
+    for (const auto& p : pipes) entries += *p.h_total;
     prof_host(c, "msm_host_combine",
               std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
     c->msm_entries = entries;
@@ -2261,6 +2306,7 @@ static void combine_all(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, uint8_t* 
         c->msm_window_bits = pipes.back().sh.c;
         c->msm_windows = pipes.back().sh.W;
     }
+    return ZK_OK;
 }
 
 // Group jobs into pipelines: one per (window bits, fixed-base mode, GLV), split where a
@@ -2666,10 +2712,15 @@ static int batch_run(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mont,
         return rc;
     }
     scratch_free(c, arena);
-    ZK_TRY_CUDA(cudaStreamSynchronize(c->stream));
-    if (queue && (rc = queue_check(queue_status)) != ZK_OK) return rc;
-    combine_all<C>(c, pipes, out_xy, out_is_inf);
-    return ZK_OK;
+    auto wait = [&]() -> int {
+        ZK_TRY_CUDA(cudaStreamSynchronize(c->stream));
+        return queue ? queue_check(queue_status) : ZK_OK;
+    };
+    // helpers woken before the device is done, where that is soon (they wait awake)
+    if (pipes.size() == 1 && pipes[0].max_entries <= kEarlyEntries)
+        return combine_all<C>(c, pipes, out_xy, out_is_inf, true, wait);
+    if ((rc = wait()) != ZK_OK) return rc;
+    return combine_all<C>(c, pipes, out_xy, out_is_inf);
 }
 
 // ---- asynchronous batches: the device part is enqueued and the call returns; a worker

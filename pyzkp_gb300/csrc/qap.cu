@@ -150,10 +150,7 @@ void host_point_mul(const uint8_t* p, const uint8_t k[32], uint8_t* out) {
         std::memcpy(kk.v, k, 32);
         const zkh::Field& R = zkh::fr();
         while (zkh::geq(kk.v, R.p)) zkh::sub4(kk.v, kk.v, R.p);
-        for (int i = 255; i >= 0; i--) {
-            acc = zkh::xyzz_dbl(acc);
-            if ((kk.v[i >> 6] >> (i & 63)) & 1) acc = zkh::xyzz_add(acc, base);
-        }
+        acc = zkh::xyzz_mul(base, kk);  // kk < r < 2^254
     }
     H ox, oy;
     zkh::xyzz_to_affine_canonical(acc, &ox, &oy);
