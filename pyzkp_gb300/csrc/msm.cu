@@ -558,6 +558,7 @@ template <class C>
 __global__ void msm_codes_kernel(const MsmInst* __restrict__ insts, const uint32_t* __restrict__ offs, uint32_t j0,
                                  uint32_t N, int scalars_mont, MsmShape sh, const uint32_t* __restrict__ set_base,
                                  uint32_t* __restrict__ codes, MsmZero zero) {
+    if (!grid_enter()) return;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, j = j0 + t;
     // the pipeline's buckets and fixup counts start at zero (no memsets of their own)
     for (size_t i = t; i < zero.n16; i += (size_t)gridDim.x * blockDim.x) zero.wide[i] = make_uint4(0, 0, 0, 0);
@@ -610,6 +611,7 @@ __global__ void __launch_bounds__(kTiledThreads) msm_hist_kernel(const uint32_t*
                                                                  const uint32_t* __restrict__ set_tile0,
                                                                  uint32_t sets, uint32_t te, uint32_t B,
                                                                  uint32_t* __restrict__ M) {
+    if (!grid_enter()) return;
     extern __shared__ uint32_t hist[];
     const uint32_t t = blockIdx.x;
     const uint32_t s = set_of_tile(set_tile0, sets, t);
@@ -637,6 +639,7 @@ __global__ void __launch_bounds__(kTiledThreads) msm_hist_kernel(const uint32_t*
 // row_ptr[s B + b] = the count of bucket b of set s over the set's tiles.
 __global__ void msm_hist_total_kernel(const uint32_t* __restrict__ M, const uint32_t* __restrict__ set_tile0,
                                       uint32_t sets, uint32_t B, uint32_t* __restrict__ row_ptr) {
+    if (!grid_enter()) return;
     const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= (uint64_t)sets * B) return;
     const uint32_t s = (uint32_t)(x / B), b = (uint32_t)(x % B);
@@ -648,6 +651,7 @@ __global__ void msm_hist_total_kernel(const uint32_t* __restrict__ M, const uint
 // M[t][b] := the first position of tile t's entries of bucket b (row_ptr: scanned).
 __global__ void msm_hist_offsets_kernel(uint32_t* __restrict__ M, const uint32_t* __restrict__ set_tile0,
                                         uint32_t sets, uint32_t B, const uint32_t* __restrict__ row_ptr) {
+    if (!grid_enter()) return;
     const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= (uint64_t)sets * B) return;
     const uint32_t s = (uint32_t)(x / B), b = (uint32_t)(x % B);
@@ -681,6 +685,7 @@ __global__ void __launch_bounds__(kMetaThreads) msm_sort_meta_kernel(uint32_t* _
                                                                      const uint32_t* __restrict__ set_tile0,
                                                                      uint32_t sets, uint32_t B,
                                                                      uint32_t* __restrict__ row_ptr) {
+    if (!grid_enter()) return;
     __shared__ uint32_t part[kMetaThreads];
     const uint32_t nb = sets * B;
     // counts of bucket x over its set's tiles
@@ -738,6 +743,7 @@ __global__ void __launch_bounds__(kTiledThreads) msm_set_hist_kernel(const uint3
                                                                      const uint32_t* __restrict__ set_base, uint32_t B,
                                                                      uint32_t* __restrict__ row_ptr,
                                                                      uint32_t* __restrict__ set_total) {
+    if (!grid_enter()) return;
     extern __shared__ uint32_t hist[];
     __shared__ uint32_t warp_sum[kTiledThreads / 32];
     const uint32_t s = blockIdx.x;
@@ -803,6 +809,7 @@ __global__ void __launch_bounds__(kTiledThreads) msm_set_scatter_kernel(const ui
                                                                         const uint32_t* __restrict__ set_total,
                                                                         uint32_t* __restrict__ row_ptr,
                                                                         uint32_t* __restrict__ entries) {
+    if (!grid_enter()) return;
     extern __shared__ uint32_t cursor[];
     __shared__ uint32_t warp_sum[kTiledThreads / 32];
     const uint32_t s = blockIdx.x;
@@ -844,6 +851,7 @@ __global__ void __launch_bounds__(kTiledThreads) msm_scatter_tiles_kernel(const 
                                                                           const MsmInst* __restrict__ insts,
                                                                           const uint32_t* __restrict__ M,
                                                                           uint32_t* __restrict__ entries) {
+    if (!grid_enter()) return;
     extern __shared__ uint32_t cursor[];
     const uint32_t t = blockIdx.x;
     const uint32_t s = set_of_tile(set_tile0, sh.sets, t);
@@ -967,6 +975,7 @@ __global__ void __launch_bounds__(128, C::kAccMinBlocks) msm_accumulate_kernel(c
                                                              uint32_t* __restrict__ slot_keys,
                                                              typename C::P* __restrict__ slot_pts,
                                                              const uint32_t* __restrict__ inf_flag) {
+    if (!grid_enter()) return;
     const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= units) return;
     // kSkipInf: the points may hold infinity; a flag (when given) says whether they do
@@ -1015,6 +1024,7 @@ __global__ void __launch_bounds__(128, C::kRedMinBlocks) msm_merge_kernel(const 
                                                         uint32_t units, typename C::P* __restrict__ buckets,
                                                         uint32_t* __restrict__ slot_keys,
                                                         typename C::P* __restrict__ slot_pts) {
+    if (!grid_enter()) return;
     const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= units) return;
     merge_unit<C, false>(in_keys, in_pts, in_units, group, *d_total, row_ptr, span, u, buckets, slot_keys, slot_pts);
@@ -1121,6 +1131,7 @@ __global__ void __launch_bounds__(128, C::kRedMinBlocks) msm_fixup_kernel(const 
                                                         typename C::P* __restrict__ buckets,
                                                         uint32_t* __restrict__ long_list, uint32_t lcap,
                                                         uint32_t* __restrict__ long_count, uint32_t hcap) {
+    if (!grid_enter()) return;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (kQuad) {
         fixup_quad<C>(row_ptr, nbuckets, seg, fixmax, slot_pts, buckets, long_list, lcap, long_count, hcap, t >> 2);
@@ -1223,6 +1234,7 @@ __global__ void __launch_bounds__(C::kFixupLongThreads, C::kFixupLongMinBlocks) 
                                                                            uint32_t* __restrict__ long_count,
                                                                            uint32_t hcap,
                                                                            typename C::P* __restrict__ chunk_pts) {
+    if (!grid_enter()) return;
     __shared__ typename C::P red[C::kFixupLongThreads / 32];
     fixup_long_cta<C, false>(row_ptr, seg, slot_pts, buckets, long_list, lcap, long_count, hcap, chunk_pts, red,
                              blockIdx.x, gridDim.x);
@@ -1254,6 +1266,7 @@ template <class C>
 __global__ void __launch_bounds__(128) msm_bucket_blocks_kernel(const typename C::P* __restrict__ buckets,
                                                                 MsmShape sh, typename C::P* __restrict__ Y,
                                                                 typename C::P* __restrict__ E) {
+    if (!grid_enter()) return;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= sh.sets * sh.G) return;
     blocks_thread<C, false>(buckets, sh, Y, E, t);
@@ -1287,6 +1300,7 @@ template <class C>
 __global__ void __launch_bounds__(128) msm_lines_kernel(const typename C::P* __restrict__ Y,
                                                         const typename C::P* __restrict__ E, MsmShape sh,
                                                         typename C::P* __restrict__ lines) {
+    if (!grid_enter()) return;
     __shared__ typename C::P red[4];
     lines_cta<C, false>(Y, E, sh, lines, red, blockIdx.x);
 }
@@ -1324,6 +1338,7 @@ __global__ void __launch_bounds__(128) msm_targets_kernel(const typename C::P* _
                                                           typename C::P* __restrict__ out,
                                                           const uint32_t* __restrict__ d_total,
                                                           uint32_t* __restrict__ total) {
+    if (!grid_enter()) return;
     __shared__ typename C::P red[4];
     if (blockIdx.x == 0 && threadIdx.x == 0) *total = *d_total;
     targets_cta<C, false>(lines, sh, out, red, blockIdx.x);
@@ -1880,34 +1895,34 @@ static int enqueue_tiled_sort(Ctx* c, MsmPipeT<C>& p, int scalars_mont) {
     }
     const size_t smem = (size_t)sh.B * 4;
     if (p.tiles == sh.sets && p.te <= kOneTileMax) {
-        ZK_LAUNCH(c, "msm_set_hist", msm_set_hist_kernel, sh.sets, kTiledThreads, smem, codes, p.set_base, sh.B,
+        ZK_LAUNCH_NEXT(c, "msm_set_hist", msm_set_hist_kernel, sh.sets, kTiledThreads, smem, codes, p.set_base, sh.B,
                   p.row_ptr, p.tile_hist);
         ZK_TRY_CUDA(cudaGetLastError());
-        ZK_LAUNCH(c, "msm_set_scatter", msm_set_scatter_kernel, sh.sets, kTiledThreads, smem, codes, p.set_base, sh,
+        ZK_LAUNCH_NEXT(c, "msm_set_scatter", msm_set_scatter_kernel, sh.sets, kTiledThreads, smem, codes, p.set_base, sh,
                   p.d_inst, p.tile_hist, p.row_ptr, p.entries);
         ZK_TRY_CUDA(cudaGetLastError());
         return ZK_OK;
     }
-    ZK_LAUNCH(c, "msm_hist", msm_hist_kernel, p.tiles, kTiledThreads, smem, codes, p.set_base, p.set_tile0, sh.sets,
+    ZK_LAUNCH_NEXT(c, "msm_hist", msm_hist_kernel, p.tiles, kTiledThreads, smem, codes, p.set_base, p.set_tile0, sh.sets,
               p.te, sh.B, p.tile_hist);
     ZK_TRY_CUDA(cudaGetLastError());
     if (p.nbuckets <= kMetaMaxBuckets && (uint64_t)p.tiles * sh.B <= kMetaMaxCounts) {
-        ZK_LAUNCH(c, "msm_sort_meta", msm_sort_meta_kernel, 1, kMetaThreads, 0, p.tile_hist, p.set_tile0, sh.sets,
+        ZK_LAUNCH_NEXT(c, "msm_sort_meta", msm_sort_meta_kernel, 1, kMetaThreads, 0, p.tile_hist, p.set_tile0, sh.sets,
                   sh.B, p.row_ptr);
         ZK_TRY_CUDA(cudaGetLastError());
     } else {
         const unsigned nb = (unsigned)((p.nbuckets + 255) / 256);
-        ZK_LAUNCH(c, "msm_hist_total", msm_hist_total_kernel, nb, 256, 0, p.tile_hist, p.set_tile0, sh.sets, sh.B,
+        ZK_LAUNCH_NEXT(c, "msm_hist_total", msm_hist_total_kernel, nb, 256, 0, p.tile_hist, p.set_tile0, sh.sets, sh.B,
                   p.row_ptr);
         ZK_TRY_CUDA(cudaGetLastError());
         // row_ptr[0..nbuckets) := exclusive scan; row_ptr[nbuckets] := total
         rc = device_exclusive_scan(c, p.row_ptr, p.nbuckets, p.row_ptr + p.nbuckets, p.scan_tmp);
         if (rc != ZK_OK) return rc;
-        ZK_LAUNCH(c, "msm_hist_offsets", msm_hist_offsets_kernel, nb, 256, 0, p.tile_hist, p.set_tile0, sh.sets,
+        ZK_LAUNCH_NEXT(c, "msm_hist_offsets", msm_hist_offsets_kernel, nb, 256, 0, p.tile_hist, p.set_tile0, sh.sets,
                   sh.B, p.row_ptr);
         ZK_TRY_CUDA(cudaGetLastError());
     }
-    ZK_LAUNCH(c, "msm_scatter_tiles", msm_scatter_tiles_kernel, p.tiles, kTiledThreads, smem, codes, p.set_base,
+    ZK_LAUNCH_NEXT(c, "msm_scatter_tiles", msm_scatter_tiles_kernel, p.tiles, kTiledThreads, smem, codes, p.set_base,
               p.set_tile0, p.te, sh, p.d_inst, p.tile_hist, p.entries);
     ZK_TRY_CUDA(cudaGetLastError());
     return ZK_OK;
@@ -1950,7 +1965,7 @@ static int pipe_enqueue_reduce(Ctx* c, MsmPipeT<C>& p) {
     const uint32_t* d_total = p.row_ptr + p.nbuckets;
     // point sets without infinity skip the per-entry test
     auto* accumulate = p.skip_inf ? msm_accumulate_kernel<C, true> : msm_accumulate_kernel<C, false>;
-    ZK_LAUNCH(c, "msm_accumulate", accumulate, (p.units + 127) / 128, 128, 0, p.entries, d_total, p.row_ptr,
+    ZK_LAUNCH_NEXT(c, "msm_accumulate", accumulate, (p.units + 127) / 128, 128, 0, p.entries, d_total, p.row_ptr,
               p.d_inst, sh, p.units, p.buckets, p.slot_keys_a, p.slot_pts_a, p.skip_inf ? c->inf_flag : nullptr);
     ZK_TRY_CUDA(cudaGetLastError());
     // Partial sums of straddling buckets: short buckets (up to ~3 segments on average) by one
@@ -1964,12 +1979,12 @@ static int pipe_enqueue_reduce(Ctx* c, MsmPipeT<C>& p) {
         // G2 with its larger points 1000 491 / 455, 2^16 (40960 buckets) 1269 / 1291
         const bool quad = p.nbuckets < (uint64_t)c->num_sms * (sizeof(P) > 128 ? kSmallBucketsPerSm / 4 : kSmallBucketsPerSm);
         auto* fixup = quad ? &msm_fixup_kernel<C, true> : &msm_fixup_kernel<C, false>;
-        ZK_LAUNCH(c, "msm_fixup", fixup, (unsigned)((p.nbuckets * (quad ? 4 : 1) + 127) / 128), 128, 0, p.row_ptr,
+        ZK_LAUNCH_NEXT(c, "msm_fixup", fixup, (unsigned)((p.nbuckets * (quad ? 4 : 1) + 127) / 128), 128, 0, p.row_ptr,
                   (uint32_t)p.nbuckets, sh.seg, sh.fixmax, p.slot_pts_a, p.buckets, p.long_list, lcap, p.long_count, hcap);
         ZK_TRY_CUDA(cudaGetLastError());
         // the chunk sums of huge buckets go to slot_pts_b (merge-round space, unused in fixup mode)
         // as many CTAs as fit at once (at least 2 per SM)
-        ZK_LAUNCH(c, "msm_fixup_long", msm_fixup_long_kernel<C>,
+        ZK_LAUNCH_NEXT(c, "msm_fixup_long", msm_fixup_long_kernel<C>,
                   (unsigned)(c->num_sms * std::max(2, C::kFixupLongMinBlocks)), C::kFixupLongThreads, 0,
                   p.row_ptr, sh.seg, p.slot_pts_a, p.buckets, p.long_list, lcap, p.long_count, hcap, p.slot_pts_b);
         ZK_TRY_CUDA(cudaGetLastError());
@@ -1982,7 +1997,7 @@ static int pipe_enqueue_reduce(Ctx* c, MsmPipeT<C>& p) {
         while (in_units > 1) {
             const uint32_t out_units = (in_units + group - 1) / group;
             span *= group;
-            ZK_LAUNCH(c, group == kFirstGroup ? "msm_merge_pairs" : "msm_merge", msm_merge_kernel<C>, (out_units + 127) / 128,
+            ZK_LAUNCH_NEXT(c, group == kFirstGroup ? "msm_merge_pairs" : "msm_merge", msm_merge_kernel<C>, (out_units + 127) / 128,
                       128, 0, ik, ip, in_units, group, d_total, p.row_ptr, span, out_units, p.buckets, ok, op);
             ZK_TRY_CUDA(cudaGetLastError());
             std::swap(ik, ok);
@@ -1995,7 +2010,7 @@ static int pipe_enqueue_reduce(Ctx* c, MsmPipeT<C>& p) {
     // window reduction
     if (sh.g > 1) {
         const uint32_t nb = sh.sets * sh.G;
-        ZK_LAUNCH(c, "msm_bucket_blocks", msm_bucket_blocks_kernel<C>, (nb + 127) / 128, 128, 0, p.buckets, sh, p.Yb,
+        ZK_LAUNCH_NEXT(c, "msm_bucket_blocks", msm_bucket_blocks_kernel<C>, (nb + 127) / 128, 128, 0, p.buckets, sh, p.Yb,
                   p.Eb);
         ZK_TRY_CUDA(cudaGetLastError());
     }
@@ -2003,11 +2018,11 @@ static int pipe_enqueue_reduce(Ctx* c, MsmPipeT<C>& p) {
     const uint32_t nl = sh.sets * lines_per_set(sh), len = 1u << (sh.K - sh.m);
     uint32_t lw = 1;
     while (lw < 4 && nl * lw < (uint32_t)c->num_sms * kLineWarps && 16 * lw < len) lw *= 2;
-    ZK_LAUNCH(c, "msm_lines", msm_lines_kernel<C>, nl, 32 * lw, 0, p.Yb, p.Eb, sh, p.lines);
+    ZK_LAUNCH_NEXT(c, "msm_lines", msm_lines_kernel<C>, nl, 32 * lw, 0, p.Yb, p.Eb, sh, p.lines);
     ZK_TRY_CUDA(cudaGetLastError());
     uint32_t tw = 1;
     while (tw < 4 && 16 * tw < len) tw *= 2;
-    ZK_LAUNCH(c, "msm_targets", msm_targets_kernel<C>, sh.sets * sh.targets, 32 * tw, 0, p.lines, sh, p.h_tgt, d_total,
+    ZK_LAUNCH_NEXT(c, "msm_targets", msm_targets_kernel<C>, sh.sets * sh.targets, 32 * tw, 0, p.lines, sh, p.h_tgt, d_total,
               p.h_total);
     ZK_TRY_CUDA(cudaGetLastError());
     return ZK_OK;

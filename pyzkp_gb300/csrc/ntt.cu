@@ -359,6 +359,7 @@ __device__ __forceinline__ void ntt_pass_body(const NttPassParams& P, uint32_t t
 
 template <bool kWide>
 __global__ void __launch_bounds__(kNttThreads, ZK_NTT_MINB) ntt_pass_kernel(NttPassParams P) {
+    if (!grid_enter()) return;
     extern __shared__ uint4 smem[];
     ntt_pass_body<kWide>(P, blockIdx.x, smem);
 }
@@ -370,6 +371,7 @@ template <bool kWide>
 __global__ void __launch_bounds__(kNttThreads, kWide ? ZK_NTT_MINB : ZK_NTT_BATCH_MINB) ntt_pass_batch_kernel(const NttPassParams* __restrict__ items,
                                                                        const uint32_t* __restrict__ first_tile,
                                                                        uint32_t nitems) {
+    if (!grid_enter()) return;
     extern __shared__ uint4 smem[];
     __shared__ NttPassParams sP;
     __shared__ uint32_t s_tile;
@@ -870,7 +872,7 @@ int ntt_run(Ctx* c, int mode, fe* out, const fe* in, size_t in_len, uint32_t log
     make_passes(plan, out, in, valid, scratch, &launches, wide, canon_io);
     auto* kernel = wide ? &ntt_pass_kernel<true> : &ntt_pass_kernel<false>;
     for (const PassLaunch& L : launches) {
-        ZK_LAUNCH(c, "ntt_pass", kernel, L.blocks, L.threads, L.smem,
+        ZK_LAUNCH_NEXT(c, "ntt_pass", kernel, L.blocks, L.threads, L.smem,
                   L.P);
         ZK_TRY_CUDA(cudaGetLastError());
     }
@@ -1050,7 +1052,7 @@ static int batch_enqueue(Ctx* c, const NttBatch* b) {
     auto* kernel = b->wide ? &ntt_pass_batch_kernel<true> : &ntt_pass_batch_kernel<false>;
     for (size_t L = 0; L < b->items.size(); L++) {
         if (b->blocks[L] == 0) continue;
-        ZK_LAUNCH(c, "ntt_pass_batch", kernel, b->blocks[L], b->threads[L], b->smem[L],
+        ZK_LAUNCH_NEXT(c, "ntt_pass_batch", kernel, b->blocks[L], b->threads[L], b->smem[L],
                   reinterpret_cast<const NttPassParams*>(b->desc + b->items_at[L]),
                   reinterpret_cast<const uint32_t*>(b->desc + b->first_at[L]), (uint32_t)b->items[L].size());
         ZK_TRY_CUDA(cudaGetLastError());
@@ -1471,7 +1473,7 @@ static int ntt_run_noalloc(Ctx* c, int mode, fe* out, const fe* in, size_t in_le
         P.post_hi = (has_post && !post_const) ? tables + off_post_hi : nullptr;
         P.in_len = valid;
         P.last = 1;
-        ZK_LAUNCH(c, "ntt_pass", ntt_pass_kernel<false>, 1, 32, 2 * 16, P);
+        ZK_LAUNCH_NEXT(c, "ntt_pass", ntt_pass_kernel<false>, 1, 32, 2 * 16, P);
         ZK_TRY_CUDA(cudaGetLastError());
         return ZK_OK;
     }
@@ -1499,7 +1501,7 @@ static int ntt_run_noalloc(Ctx* c, int mode, fe* out, const fe* in, size_t in_le
         const uint32_t elems = 1u << (lr + lt);
         const uint32_t threads = elems / 2 < (uint32_t)kNttThreads ? (elems / 2 < 32 ? 32 : elems / 2) : kNttThreads;
         const uint32_t blocks = (uint32_t)(n >> (lr + lt));
-        ZK_LAUNCH(c, "ntt_pass", ntt_pass_kernel<false>, blocks, threads, (size_t)elems * 32, P);
+        ZK_LAUNCH_NEXT(c, "ntt_pass", ntt_pass_kernel<false>, blocks, threads, (size_t)elems * 32, P);
         ZK_TRY_CUDA(cudaGetLastError());
         src = dst;
         log_l += lr;

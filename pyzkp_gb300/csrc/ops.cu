@@ -19,6 +19,7 @@ static unsigned grid_for(size_t n, int threads, int num_sms) {
 
 template <class F, int DIR>
 __global__ void convert_kernel(fe* out, const fe* in, size_t n) {
+    if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         fe v = fe_ldg(in + i);
         fe_store(out + i, DIR ? fe_to_mont<F>(v) : fe_from_mont<F>(v));
@@ -26,16 +27,19 @@ __global__ void convert_kernel(fe* out, const fe* in, size_t n) {
 }
 
 __global__ void fr_mul_kernel(fe* out, const fe* a, const fe* b, size_t n) {
+    if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         fe_store(out + i, fe_mul<FrP>(fe_ldg(a + i), fe_ldg(b + i)));
 }
 
 __global__ void fr_sub_kernel(fe* out, const fe* a, const fe* b, size_t n) {
+    if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         fe_store(out + i, fe_sub<FrP>(fe_ldg(a + i), fe_ldg(b + i)));
 }
 
 __global__ void fr_add_kernel(fe* out, const fe* a, const fe* b, size_t n) {
+    if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         fe_store(out + i, fe_add<FrP>(fe_ldg(a + i), fe_ldg(b + i)));
 }
@@ -68,7 +72,7 @@ template <class F, int DIR>
 int convert(Ctx* c, void* out, const void* in, size_t n) {
     if (n == 0) return ZK_OK;
     ZK_CHECK_ARG(out != nullptr && in != nullptr, "null buffer");
-    ZK_LAUNCH(c, DIR ? "to_mont" : "from_mont", (convert_kernel<F, DIR>), grid_for(n, 256, c->num_sms), 256, 0,
+    ZK_LAUNCH_NEXT(c, DIR ? "to_mont" : "from_mont", (convert_kernel<F, DIR>), grid_for(n, 256, c->num_sms), 256, 0,
               static_cast<fe*>(out), static_cast<const fe*>(in), n);
     ZK_TRY_CUDA(cudaGetLastError());
     return ZK_OK;
@@ -83,13 +87,13 @@ int fr_binary(Ctx* c, int op, void* out, const void* a, const void* b, size_t n)
     if (n == 0) return ZK_OK;
     ZK_CHECK_ARG(out != nullptr && a != nullptr && b != nullptr, "null buffer");
     if (op == 0)
-        ZK_LAUNCH(c, "fr_mul", fr_mul_kernel, grid_for(n, 256, c->num_sms), 256, 0, static_cast<fe*>(out),
+        ZK_LAUNCH_NEXT(c, "fr_mul", fr_mul_kernel, grid_for(n, 256, c->num_sms), 256, 0, static_cast<fe*>(out),
                   static_cast<const fe*>(a), static_cast<const fe*>(b), n);
     else if (op == 1)
-        ZK_LAUNCH(c, "fr_sub", fr_sub_kernel, grid_for(n, 256, c->num_sms), 256, 0, static_cast<fe*>(out),
+        ZK_LAUNCH_NEXT(c, "fr_sub", fr_sub_kernel, grid_for(n, 256, c->num_sms), 256, 0, static_cast<fe*>(out),
                   static_cast<const fe*>(a), static_cast<const fe*>(b), n);
     else
-        ZK_LAUNCH(c, "fr_add", fr_add_kernel, grid_for(n, 256, c->num_sms), 256, 0, static_cast<fe*>(out),
+        ZK_LAUNCH_NEXT(c, "fr_add", fr_add_kernel, grid_for(n, 256, c->num_sms), 256, 0, static_cast<fe*>(out),
                   static_cast<const fe*>(a), static_cast<const fe*>(b), n);
     ZK_TRY_CUDA(cudaGetLastError());
     return ZK_OK;

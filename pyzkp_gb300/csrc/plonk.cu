@@ -44,6 +44,7 @@ __device__ fe fe_pow_fermat_inv(const fe& a) {
 
 // out must not alias in: the backward pass reads in[] again (out holds the prefixes).
 __global__ void fr_batch_inv_kernel(fe* __restrict__ out, const fe* __restrict__ in, size_t n) {
+    if (!grid_enter()) return;
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t i0 = t * kInvChunk;
     if (i0 >= n) return;
@@ -88,6 +89,7 @@ static constexpr uint32_t kQWarpPoints = 32 * kQChunk;
 
 __global__ void plonk_quotient_kernel(QuotientIn in, QuotientK K, size_t m, const fe* __restrict__ pw, uint32_t H,
                                       fe* __restrict__ num, fe* __restrict__ zh) {
+    if (!grid_enter()) return;
     // a warp covers 32 * kQChunk consecutive points, lane l the points base + l + 32 k (each
     // load of the warp reads 32 consecutive elements)
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -166,7 +168,7 @@ int zk_fr_batch_inv(zk_ctx* ctx, void* out, const void* in, size_t n) {
         src = static_cast<const fe*>(copy);
     }
     const size_t chunks = (n + zk::kInvChunk - 1) / zk::kInvChunk;
-    ZK_LAUNCH(c, "fr_batch_inv", zk::fr_batch_inv_kernel, (unsigned)((chunks + 127) / 128), 128, 0,
+    ZK_LAUNCH_NEXT(c, "fr_batch_inv", zk::fr_batch_inv_kernel, (unsigned)((chunks + 127) / 128), 128, 0,
               static_cast<fe*>(out), src, n);
     ZK_TRY_CUDA(cudaGetLastError());
     if (copy) zk::scratch_free(c, copy);
@@ -250,7 +252,7 @@ int zk_plonk_quotient_evals(zk_ctx* ctx, const void* const* inputs, size_t m, ui
     if (rc != ZK_OK) return rc;
     ZK_TRY_CUDA(cudaMemcpyAsync(d_pw, pw.data(), pw.size() * 32, cudaMemcpyHostToDevice, c->stream));
     const size_t chunks = (m + zk::kQChunk - 1) / zk::kQChunk;
-    ZK_LAUNCH(c, "plonk_quotient", zk::plonk_quotient_kernel, (unsigned)((chunks + 127) / 128), 128, 0, in, K, m,
+    ZK_LAUNCH_NEXT(c, "plonk_quotient", zk::plonk_quotient_kernel, (unsigned)((chunks + 127) / 128), 128, 0, in, K, m,
               static_cast<const fe*>(d_pw), H, static_cast<fe*>(num_out), static_cast<fe*>(zh_out));
     ZK_TRY_CUDA(cudaGetLastError());
     zk::scratch_free(c, d_pw);

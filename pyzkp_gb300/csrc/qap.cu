@@ -38,6 +38,7 @@ static fe host_mont_fr(const uint8_t canonical[32]) {
 __global__ void fr_spmv_kernel(uint32_t nrows, const uint32_t* __restrict__ row_ptr,
                                const uint32_t* __restrict__ cols, const fe* __restrict__ coeffs,
                                const fe* __restrict__ x, fe* __restrict__ out) {
+    if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nrows; i += (size_t)gridDim.x * blockDim.x) {
         fe acc = fe_zero();
         for (uint32_t j = row_ptr[i]; j < row_ptr[i + 1]; j++)
@@ -48,6 +49,7 @@ __global__ void fr_spmv_kernel(uint32_t nrows, const uint32_t* __restrict__ row_
 
 __global__ void fr_r1cs_check_kernel(const fe* __restrict__ a, const fe* __restrict__ b, const fe* __restrict__ c,
                                      size_t n, unsigned long long* __restrict__ bad) {
+    if (!grid_enter()) return;
     unsigned long long local = 0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const fe ab = fe_mul<FrP>(fe_ldg(a + i), fe_ldg(b + i));
@@ -62,6 +64,7 @@ __global__ void fr_r1cs_check_kernel(const fe* __restrict__ a, const fe* __restr
 
 __global__ void fr_qap_quotient_kernel(fe* __restrict__ out, const fe* __restrict__ a, const fe* __restrict__ b,
                                        const fe* __restrict__ c, size_t n, fe zinv) {
+    if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const fe ab = fe_mul<FrP>(fe_ldg(a + i), fe_ldg(b + i));
         fe_store(out + i, fe_mul<FrP>(fe_sub<FrP>(ab, fe_ldg(c + i)), zinv));
@@ -70,11 +73,13 @@ __global__ void fr_qap_quotient_kernel(fe* __restrict__ out, const fe* __restric
 
 __global__ void fr_gather_kernel(fe* __restrict__ out, const fe* __restrict__ in, const uint32_t* __restrict__ idx,
                                  size_t n) {
+    if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         fe_store(out + i, fe_ldg(in + idx[i]));
 }
 
 __global__ void fr_scale_kernel(fe* __restrict__ out, const fe* __restrict__ in, size_t n, fe s) {
+    if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         fe_store(out + i, fe_mul<FrP>(fe_ldg(in + i), s));
 }
@@ -121,7 +126,7 @@ static int count_bad(Ctx* c, const fe* a, const fe* b, const fe* cc, size_t n, u
     int rc = scratch_alloc(c, sizeof(unsigned long long), reinterpret_cast<void**>(&d));
     if (rc != ZK_OK) return rc;
     ZK_TRY_CUDA(cudaMemsetAsync(d, 0, sizeof(unsigned long long), c->stream));
-    ZK_LAUNCH(c, "fr_r1cs_check", fr_r1cs_check_kernel, grid_of(n, 256, c->num_sms), 256, 0, a, b, cc, n, d);
+    ZK_LAUNCH_NEXT(c, "fr_r1cs_check", fr_r1cs_check_kernel, grid_of(n, 256, c->num_sms), 256, 0, a, b, cc, n, d);
     ZK_TRY_CUDA(cudaGetLastError());
     unsigned long long h = 0;
     ZK_TRY_CUDA(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
@@ -209,7 +214,7 @@ int zk_fr_spmv(zk_ctx* ctx, uint32_t nrows, const uint32_t* row_ptr_dev, const u
         return ZK_EINVAL;
     }
     zk::Ctx* c = &ctx->impl;
-    ZK_LAUNCH(c, "fr_spmv", zk::fr_spmv_kernel, zk::grid_of(nrows, 256, c->num_sms), 256, 0, nrows, row_ptr_dev,
+    ZK_LAUNCH_NEXT(c, "fr_spmv", zk::fr_spmv_kernel, zk::grid_of(nrows, 256, c->num_sms), 256, 0, nrows, row_ptr_dev,
               cols_dev, static_cast<const fe*>(coeffs_dev), static_cast<const fe*>(x_dev), static_cast<fe*>(out_dev));
     ZK_TRY_CUDA(cudaGetLastError());
     return ZK_OK;
@@ -235,7 +240,7 @@ int zk_fr_r1cs_check_async(zk_ctx* ctx, const void* a, const void* b, const void
     }
     if (n == 0) return ZK_OK;
     zk::Ctx* cc = &ctx->impl;
-    ZK_LAUNCH(cc, "fr_r1cs_check", zk::fr_r1cs_check_kernel, zk::grid_of(n, 256, cc->num_sms), 256, 0,
+    ZK_LAUNCH_NEXT(cc, "fr_r1cs_check", zk::fr_r1cs_check_kernel, zk::grid_of(n, 256, cc->num_sms), 256, 0,
               static_cast<const fe*>(a), static_cast<const fe*>(b), static_cast<const fe*>(c), n,
               static_cast<unsigned long long*>(bad_dev));
     ZK_TRY_CUDA(cudaGetLastError());
@@ -251,7 +256,7 @@ int zk_fr_qap_quotient(zk_ctx* ctx, void* out, const void* a, const void* b, con
         return ZK_EINVAL;
     }
     zk::Ctx* cx = &ctx->impl;
-    ZK_LAUNCH(cx, "fr_qap_quotient", zk::fr_qap_quotient_kernel, zk::grid_of(n, 256, cx->num_sms), 256, 0,
+    ZK_LAUNCH_NEXT(cx, "fr_qap_quotient", zk::fr_qap_quotient_kernel, zk::grid_of(n, 256, cx->num_sms), 256, 0,
               static_cast<fe*>(out), static_cast<const fe*>(a), static_cast<const fe*>(b),
               static_cast<const fe*>(c), n, zk::host_mont_fr(zinv));
     ZK_TRY_CUDA(cudaGetLastError());
@@ -266,7 +271,7 @@ int zk_fr_gather(zk_ctx* ctx, void* out, const void* in, const uint32_t* idx_dev
         return ZK_EINVAL;
     }
     zk::Ctx* c = &ctx->impl;
-    ZK_LAUNCH(c, "fr_gather", zk::fr_gather_kernel, zk::grid_of(n, 256, c->num_sms), 256, 0, static_cast<fe*>(out),
+    ZK_LAUNCH_NEXT(c, "fr_gather", zk::fr_gather_kernel, zk::grid_of(n, 256, c->num_sms), 256, 0, static_cast<fe*>(out),
               static_cast<const fe*>(in), idx_dev, n);
     ZK_TRY_CUDA(cudaGetLastError());
     return ZK_OK;
@@ -280,7 +285,7 @@ int zk_fr_scale(zk_ctx* ctx, void* out, const void* in, const uint8_t s[32], siz
         return ZK_EINVAL;
     }
     zk::Ctx* c = &ctx->impl;
-    ZK_LAUNCH(c, "fr_scale", zk::fr_scale_kernel, zk::grid_of(n, 256, c->num_sms), 256, 0, static_cast<fe*>(out),
+    ZK_LAUNCH_NEXT(c, "fr_scale", zk::fr_scale_kernel, zk::grid_of(n, 256, c->num_sms), 256, 0, static_cast<fe*>(out),
               static_cast<const fe*>(in), n, zk::host_mont_fr(s));
     ZK_TRY_CUDA(cudaGetLastError());
     return ZK_OK;

@@ -23,6 +23,7 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
 
 // In-place exclusive scan of one tile; tile total to sums[blockIdx.x].
 __global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(uint32_t* data, size_t n, uint32_t* sums) {
+    if (!grid_enter()) return;
     __shared__ uint32_t warp_tot[kScanThreads / 32];
     const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanPerThread;
     uint32_t v[kScanPerThread];
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(uint32_t* data
 }
 
 __global__ void scan_add_kernel(uint32_t* data, size_t n, const uint32_t* offs) {
+    if (!grid_enter()) return;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) data[i] += offs[i / kScanTile];
 }
@@ -79,13 +81,13 @@ int device_exclusive_scan(Ctx* c, uint32_t* data, size_t n, uint32_t* total, uin
         int rc = scratch_alloc(c, (tiles + 1) * sizeof(uint32_t), reinterpret_cast<void**>(&sums));
         if (rc != ZK_OK) return rc;
     }
-    ZK_LAUNCH(c, "scan_tiles", scan_tiles_kernel, (unsigned)tiles, kScanThreads, 0, data, n, sums);
+    ZK_LAUNCH_NEXT(c, "scan_tiles", scan_tiles_kernel, (unsigned)tiles, kScanThreads, 0, data, n, sums);
     ZK_TRY_CUDA(cudaGetLastError());
     if (tiles > 1) {
         // sums[tiles] receives the grand total through the recursive scan's total slot
         int rc = device_exclusive_scan(c, sums, tiles, total, scratch ? scratch + tiles + 1 : nullptr);
         if (rc != ZK_OK) return rc;
-        ZK_LAUNCH(c, "scan_add", scan_add_kernel, (unsigned)((n + 255) / 256), 256, 0, data, n, sums);
+        ZK_LAUNCH_NEXT(c, "scan_add", scan_add_kernel, (unsigned)((n + 255) / 256), 256, 0, data, n, sums);
         ZK_TRY_CUDA(cudaGetLastError());
     } else if (total != nullptr) {
         ZK_TRY_CUDA(cudaMemcpyAsync(total, sums, sizeof(uint32_t), cudaMemcpyDeviceToDevice, c->stream));

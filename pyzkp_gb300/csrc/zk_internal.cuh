@@ -195,6 +195,46 @@ __device__ __forceinline__ uint32_t queue_ticket(uint32_t* state, uint32_t nitem
         ::zk::prof_end((ctxp), _tok);                                         \
     } while (0)
 
+// Programmatic dependent launch: a kernel launched with ZK_LAUNCH_NEXT is set up while the
+// kernel before it on the stream drains; grid_enter, the first thing every thread of such a
+// kernel does, waits until that kernel has completed and its writes are visible. Every CTA
+// waits, so completion stays transitive along the stream. (The result of the asm guards the
+// body: no load of it, read-only ones included, can be moved before the wait.) Without the
+// launch attribute it does nothing.
+// Measured on GB300, a few us a launch (us, before -> after): NTT 2^8 8.2 -> 6.8, 2^12 16.4 -> 10.8,
+// 2^16 25 -> 20, 2^18 57 -> 51; MSM 4096 200 -> 182, 2^16 455 -> 429, 2^20 2906 -> 2873, 64 MSMs 29.9 ->
+// 28.0 ms. Releasing the next kernel at the start of each (griddepcontrol.launch_dependents)
+// is worse: its CTAs then fill the SMs that happen to have room, unevenly (NTT 2^18 82 us,
+// 100003 witness-like points 403 -> 573); for grids of up to one CTA per SM alone, 1 - 8% worse.
+__device__ __forceinline__ bool grid_enter() {
+    uint32_t go;
+    asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 1;" : "=r"(go)::"memory");
+    return go != 0;
+}
+
+template <class... P, class... A>
+inline void launch_next(cudaStream_t stream, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// ZK_LAUNCH of a kernel that begins with grid_enter.
+#define ZK_LAUNCH_NEXT(ctxp, name, kernel, grid, block, smem, ...)                          \
+    do {                                                                                    \
+        int _tok = ::zk::prof_begin((ctxp), (name));                                        \
+        ::zk::launch_next((ctxp)->stream, (kernel), (grid), (block), (smem), __VA_ARGS__);  \
+        ::zk::prof_end((ctxp), _tok);                                                       \
+    } while (0)
+
 // Stream-ordered scratch allocation on the context stream (pooled by the driver).
 int scratch_alloc(Ctx* c, size_t bytes, void** p);
 void scratch_free(Ctx* c, void* p);
