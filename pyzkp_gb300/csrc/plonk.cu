@@ -2,9 +2,9 @@
 // PLONK_T_QUOTIENT_EVALS op.
 //
 // BATCH_INV (runtime/kernels/cpu/kernels.py:_batch_inv -> crypto/field/batch.py:8-38):
-// out[i] = in[i]^-1, and 0 where in[i] == 0. Each thread inverts a chunk of kInvChunk
-// elements with Montgomery's trick (prefix products, one Fermat inversion, a backward
-// pass), so an element costs about three multiplications plus 1/kInvChunk of an inversion.
+// out[i] = in[i]^-1, and 0 where in[i] == 0, by Montgomery's trick: each lane takes kInvChunk
+// elements (prefix products, a backward pass), the lanes' products are combined by the warp
+// and inverted once, by every lane alike (binary extended Euclid: no divergence).
 //
 // PLONK_T_QUOTIENT_EVALS (runtime/kernels/cpu/kernels.py:_plonk_t_quotient_evals, used by
 // protocols/plonk/prove.py:395-416): at x_i = shift * omega_m^i, i < m, from the
@@ -15,7 +15,7 @@
 //         - (a + beta s1 + gamma)(b + beta s2 + gamma)(c + beta s3 + gamma) z(omega x)
 //   num_i = gate + alpha perm + alpha^2 (z - 1) L1
 //   zh_i  = shift_n u^i - 1
-// One thread per kQChunk points, 32 apart (a warp covers 32 * kQChunk consecutive points, so
+// One thread per `chunk` points, 32 apart (a warp covers 32 * chunk consecutive points, so
 // its loads are contiguous), the powers of omega_m and u carried from the thread's first
 // point (computed by square-and-multiply) in steps of omega_m^32 and u^32.
 #include <cstring>
@@ -25,38 +25,151 @@
 
 namespace zk {
 
-static constexpr uint32_t kInvChunk = 32;
+// (8 / 16 / 32 elements a lane: 86 / 66 / 78 us at 2^19, 260 / 188 / 185 at 2^21, 40 / 51 / 74 at 2^10)
+static constexpr uint32_t kInvChunk = 16;
+static constexpr uint32_t kInvWarp = 32 * kInvChunk;  // elements of a warp
+// Points a thread takes at most: the starting powers cost it 7 products. Fewer while there are
+// fewer than kQWarps warps per SM (a point is a chain of ~25
+// products). Measured on GB300, 16 points always / so: the quotient step of 2^8 (m = 2^10) 316 -> 126
+// us, 2^12 345 -> 148, 2^17 1576 -> 1498.
 static constexpr uint32_t kQChunk = 16;
+static constexpr uint32_t kQWarps = 32;
 
-template <class F>
-__device__ fe fe_pow_fermat_inv(const fe& a) {
-    // a^(p - 2), left-to-right over the constant exponent
-    fe r = fe_one<F>();
-    for (int limb = 7; limb >= 0; limb--) {
-        const uint32_t e = limb == 0 ? F::P(0) - 2u : F::P(limb);
-        for (int b = 31; b >= 0; b--) {
-            r = fe_sqr<F>(r);
-            if ((e >> b) & 1) r = fe_mul<F>(r, a);
-        }
-    }
+// a >> z and a << z for z < 32 (no bit is lost to the left)
+__device__ __forceinline__ void limbs_shr(fe& a, uint32_t z) {
+#pragma unroll
+    for (int i = 0; i < 7; i++) a.v[i] = __funnelshift_r(a.v[i], a.v[i + 1], z);
+    a.v[7] >>= z;
+}
+__device__ __forceinline__ void limbs_shl(fe& a, uint32_t z) {
+#pragma unroll
+    for (int i = 7; i > 0; i--) a.v[i] = __funnelshift_l(a.v[i - 1], a.v[i], z);
+    a.v[0] <<= z;
+}
+__device__ __forceinline__ fe limbs_add(const fe& a, const fe& b) {
+    fe r;
+    r.v[0] = u_add_cc(a.v[0], b.v[0]);
+#pragma unroll
+    for (int i = 1; i < 7; i++) r.v[i] = u_addc_cc(a.v[i], b.v[i]);
+    r.v[7] = u_addc(a.v[7], b.v[7]);
+    return r;
+}
+__device__ __forceinline__ fe limbs_sub(const fe& a, const fe& b, uint32_t* borrow) {
+    fe r;
+    r.v[0] = u_sub_cc(a.v[0], b.v[0]);
+#pragma unroll
+    for (int i = 1; i < 8; i++) r.v[i] = u_subc_cc(a.v[i], b.v[i]);
+    *borrow = u_subc(0u, 0u);
     return r;
 }
 
-// out must not alias in: the backward pass reads in[] again (out holds the prefixes).
-__global__ void fr_batch_inv_kernel(fe* __restrict__ out, const fe* __restrict__ in, size_t n) {
+// The inverse of a Montgomery form a = x R (a != 0, canonical): x^-1 R. Binary extended Euclid
+// without modular halvings (Kaliski's almost inverse): with u = p, v = a, r = 0, s = 1 the steps
+// keep p = u s + v r and a s = v 2^k (mod p), k counting the halvings of u and v; at u = v = 1
+// s = a^-1 2^k = x^-1 R^-1 2^k, 253 <= k <= 508. Then x^-1 R = s 2^(512 - k), by a product with
+// 2^(512 - k) / R and one with R^2.
+//
+// What bounds it: ~180 steps of a subtraction, an addition and two shifts, chains of 8
+// limbs. a^(p - 2) takes 384 dependent products, ~150 us a thread.
+template <class F>
+__device__ fe fe_inverse_binary(const fe& a) {
+    fe u, v = a, r = fe_zero(), s = fe_zero();
+#pragma unroll
+    for (int i = 0; i < 8; i++) u.v[i] = F::P(i);
+    s.v[0] = 1;
+    uint32_t k = 0;
+    while (!(v.v[0] & 1)) {  // u stays odd until the first subtraction
+        const uint32_t z = v.v[0] ? __ffs(v.v[0]) - 1 : 31;
+        limbs_shr(v, z);
+        k += z;  // r = 0
+    }
+    for (;;) {  // u and v odd
+        uint32_t less;
+        fe d = limbs_sub(u, v, &less);
+        if (fe_is_zero(d)) break;
+        if (!less) {
+            u = d;
+            r = limbs_add(r, s);
+            do {
+                const uint32_t z = u.v[0] ? __ffs(u.v[0]) - 1 : 31;
+                limbs_shr(u, z);
+                limbs_shl(s, z);
+                k += z;
+            } while (!(u.v[0] & 1));
+        } else {
+            v = limbs_sub(v, u, &less);
+            s = limbs_add(s, r);
+            do {
+                const uint32_t z = v.v[0] ? __ffs(v.v[0]) - 1 : 31;
+                limbs_shr(v, z);
+                limbs_shl(r, z);
+                k += z;
+            } while (!(v.v[0] & 1));
+        }
+    }
+    uint32_t j = 512 - k;
+    while (j > 253) {  // 2^j below 2^254
+        s = fe_add<F>(s, s);
+        j--;
+    }
+    fe t = fe_zero(), r2;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) {
+        t.v[i] = i == j / 32 ? 1u << (j % 32) : 0u;
+        r2.v[i] = F::R2(i);
+    }
+    return fe_mul<F>(fe_mul<F>(s, t), r2);
+}
+
+__device__ __forceinline__ fe fe_shfl_up(const fe& a, uint32_t d) {
+    fe r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = __shfl_up_sync(0xffffffffu, a.v[i], d);
+    return r;
+}
+__device__ __forceinline__ fe fe_shfl_down(const fe& a, uint32_t d) {
+    fe r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = __shfl_down_sync(0xffffffffu, a.v[i], d);
+    return r;
+}
+
+// out must not alias in: the backward pass reads in[] again (out holds the prefixes). A lane's
+// elements are 32 apart, so that the warp reads and writes whole lines. Measured at 2^19
+// elements: 229 -> 66 us against a Fermat inversion per 32 consecutive elements (384 dependent
+// products, and each lane's accesses a kilobyte from the next one's).
+__global__ void __launch_bounds__(128) fr_batch_inv_kernel(fe* __restrict__ out, const fe* __restrict__ in, size_t n) {
     if (!grid_enter()) return;
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t i0 = t * kInvChunk;
-    if (i0 >= n) return;
-    const size_t i1 = i0 + kInvChunk < n ? i0 + kInvChunk : n;
+    const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    const size_t i0 = warp * kInvWarp + lane;
+    if (warp * kInvWarp >= n) return;
     fe acc = fe_one<FrP>();
-    for (size_t i = i0; i < i1; i++) {
-        fe_store(out + i, acc);  // product of the non-zero inputs before i
+    for (uint32_t j = 0; j < kInvChunk; j++) {
+        const size_t i = i0 + 32 * j;
+        if (i >= n) break;
+        fe_store(out + i, acc);  // product of the lane's non-zero inputs before i
         const fe x = fe_ldg(in + i);
         if (!fe_is_zero(x)) acc = fe_mul<FrP>(acc, x);
     }
-    fe inv = fe_pow_fermat_inv<FrP>(acc);  // acc != 0: a product of non-zero field elements
-    for (size_t i = i1; i-- > i0;) {
+    __syncwarp();
+    // products of the lanes before (pre) and after (suf) this one
+    fe pre = fe_shfl_up(acc, 1), suf = fe_shfl_down(acc, 1);
+    if (lane == 0) pre = fe_one<FrP>();
+    if (lane == 31) suf = fe_one<FrP>();
+#pragma unroll 1
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+        const fe a = fe_shfl_up(pre, d), b = fe_shfl_down(suf, d);
+        if (lane >= d) pre = fe_mul<FrP>(pre, a);
+        if (lane + d < 32) suf = fe_mul<FrP>(suf, b);
+        __syncwarp();
+    }
+    const fe others = fe_mul<FrP>(pre, suf);
+    fe total = fe_mul<FrP>(others, acc);  // the same value in every lane, and not zero
+    fe inv = fe_mul<FrP>(fe_inverse_binary<FrP>(total), others);
+    for (uint32_t j = kInvChunk; j-- > 0;) {
+        const size_t i = i0 + 32 * j;
+        if (i >= n) continue;
         const fe x = fe_ldg(in + i);
         if (fe_is_zero(x)) {
             fe_store(out + i, fe_zero());
@@ -79,29 +192,28 @@ struct QuotientK {  // Montgomery constants
     fe omega_step, u_step;  // omega_m^32, u^32: a lane's step
 };
 
-// Starting powers of a lane, from tables (Montgomery): with i0 = 512 g + l (warp g, lane l),
-// v^i0 = v^l * v^(512 (g mod 64)) * v^(32768 (g / 64)) for v = omega_m and v = u:
+// Starting powers of a lane, from tables (Montgomery): with i0 = w g + l (warp g of w = 32 chunk
+// points, lane l), v^i0 = v^l * v^(w (g mod 64)) * v^(64 w (g / 64)) for v = omega_m and v = u:
 //   pw[l], pw[32 + l]              omega_m^l, u^l                        (l < 32)
-//   pw[64 + j], pw[128 + j]        omega_m^(512 j), u^(512 j)           (j < 64)
-//   pw[192 + h], pw[192 + H + h]   omega_m^(32768 h), u^(32768 h)       (h < H)
+//   pw[64 + j], pw[128 + j]        omega_m^(w j), u^(w j)           (j < 64)
+//   pw[192 + h], pw[192 + H + h]   omega_m^(64 w h), u^(64 w h)       (h < H)
 // 4 products per thread instead of ~2 log2(i0) by square-and-multiply for each of the two.
-static constexpr uint32_t kQWarpPoints = 32 * kQChunk;
 
-__global__ void plonk_quotient_kernel(QuotientIn in, QuotientK K, size_t m, const fe* __restrict__ pw, uint32_t H,
-                                      fe* __restrict__ num, fe* __restrict__ zh) {
+__global__ void plonk_quotient_kernel(QuotientIn in, QuotientK K, size_t m, uint32_t chunk, const fe* __restrict__ pw,
+                                      uint32_t H, fe* __restrict__ num, fe* __restrict__ zh) {
     if (!grid_enter()) return;
-    // a warp covers 32 * kQChunk consecutive points, lane l the points base + l + 32 k (each
+    // a warp covers 32 * chunk consecutive points, lane l the points base + l + 32 k (each
     // load of the warp reads 32 consecutive elements)
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t lane = t & 31;
-    const size_t i0 = (t - lane) * kQChunk + lane;
+    const size_t i0 = (t - lane) * chunk + lane;
     if (i0 >= m) return;
-    const size_t g = i0 / kQWarpPoints;
+    const size_t g = t >> 5;
     const uint32_t glo = (uint32_t)(g & 63), ghi = (uint32_t)(g >> 6);
     fe x = fe_mul<FrQ>(fe_mul<FrQ>(fe_ldg(pw + lane), fe_ldg(pw + 64 + glo)), fe_ldg(pw + 192 + ghi));
     x = fe_mul<FrQ>(K.shift, x);
     fe un = fe_mul<FrQ>(fe_mul<FrQ>(fe_ldg(pw + 32 + lane), fe_ldg(pw + 128 + glo)), fe_ldg(pw + 192 + H + ghi));
-    for (size_t i = i0, k = 0; k < kQChunk && i < m; k++, i += 32) {
+    for (size_t i = i0, k = 0; k < chunk && i < m; k++, i += 32) {
         const fe a = fe_ldg(in.v[0] + i), b = fe_ldg(in.v[1] + i), c = fe_ldg(in.v[2] + i);
         const fe z = fe_ldg(in.v[3] + i);
         fe gate = fe_add<FrQ>(fe_mul<FrQ>(fe_ldg(in.v[5] + i), a), fe_mul<FrQ>(fe_ldg(in.v[6] + i), b));
@@ -167,8 +279,8 @@ int zk_fr_batch_inv(zk_ctx* ctx, void* out, const void* in, size_t n) {
         ZK_TRY_CUDA(cudaMemcpyAsync(copy, in, n * 32, cudaMemcpyDeviceToDevice, c->stream));
         src = static_cast<const fe*>(copy);
     }
-    const size_t chunks = (n + zk::kInvChunk - 1) / zk::kInvChunk;
-    ZK_LAUNCH_NEXT(c, "fr_batch_inv", zk::fr_batch_inv_kernel, (unsigned)((chunks + 127) / 128), 128, 0,
+    const size_t warps = (n + zk::kInvWarp - 1) / zk::kInvWarp;
+    ZK_LAUNCH_NEXT(c, "fr_batch_inv", zk::fr_batch_inv_kernel, (unsigned)((warps + 3) / 4), 128, 0,
               static_cast<fe*>(out), src, n);
     ZK_TRY_CUDA(cudaGetLastError());
     if (copy) zk::scratch_free(c, copy);
@@ -224,7 +336,9 @@ int zk_plonk_quotient_evals(zk_ctx* ctx, const void* const* inputs, size_t m, ui
     K.u_step = zk::mont_of(zkh::pow_u64(F, zkh::pow_u64(F, zkh::to_mont(F, om), n), 32));
     zk::Ctx* c = &ctx->impl;
     // the starting-power tables of the kernel (see plonk_quotient_kernel)
-    const uint64_t warps = (m + zk::kQWarpPoints - 1) / zk::kQWarpPoints;
+    uint32_t chunk = zk::kQChunk;
+    while (chunk > 1 && m < 32ull * chunk * zk::kQWarps * c->num_sms) chunk /= 2;
+    const uint64_t points = 32ull * chunk, warps = (m + points - 1) / points;
     const uint32_t H = (uint32_t)((warps + 63) / 64);
     std::vector<zkh::F4> pw(192 + 2 * (size_t)H);
     const zkh::F4 om_m = zkh::to_mont(F, om);
@@ -236,10 +350,10 @@ int zk_plonk_quotient_evals(zk_ctx* ctx, const void* const* inputs, size_t m, ui
     };
     const Run runs[6] = {{0, om_m, 32},
                          {32, u_m, 32},
-                         {64, zkh::pow_u64(F, om_m, zk::kQWarpPoints), 64},
-                         {128, zkh::pow_u64(F, u_m, zk::kQWarpPoints), 64},
-                         {192, zkh::pow_u64(F, om_m, 64ull * zk::kQWarpPoints), H},
-                         {192 + (size_t)H, zkh::pow_u64(F, u_m, 64ull * zk::kQWarpPoints), H}};
+                         {64, zkh::pow_u64(F, om_m, points), 64},
+                         {128, zkh::pow_u64(F, u_m, points), 64},
+                         {192, zkh::pow_u64(F, om_m, 64 * points), H},
+                         {192 + (size_t)H, zkh::pow_u64(F, u_m, 64 * points), H}};
     for (const Run& r : runs) {
         zkh::F4 cur = zkh::one(F);
         for (size_t i = 0; i < r.count; i++) {
@@ -251,8 +365,7 @@ int zk_plonk_quotient_evals(zk_ctx* ctx, const void* const* inputs, size_t m, ui
     int rc = zk::scratch_alloc(c, pw.size() * 32, &d_pw);
     if (rc != ZK_OK) return rc;
     ZK_TRY_CUDA(cudaMemcpyAsync(d_pw, pw.data(), pw.size() * 32, cudaMemcpyHostToDevice, c->stream));
-    const size_t chunks = (m + zk::kQChunk - 1) / zk::kQChunk;
-    ZK_LAUNCH_NEXT(c, "plonk_quotient", zk::plonk_quotient_kernel, (unsigned)((chunks + 127) / 128), 128, 0, in, K, m,
+    ZK_LAUNCH_NEXT(c, "plonk_quotient", zk::plonk_quotient_kernel, (unsigned)((warps + 3) / 4), 128, 0, in, K, m, chunk,
               static_cast<const fe*>(d_pw), H, static_cast<fe*>(num_out), static_cast<fe*>(zh_out));
     ZK_TRY_CUDA(cudaGetLastError());
     zk::scratch_free(c, d_pw);
