@@ -1711,7 +1711,10 @@ static int pipe_init(MsmPipeT<C>& p, uint32_t c, bool fixed, bool glv, const std
     while (p.sh.seg > kMinSegment && p.max_entries / p.sh.seg < acc_threads && p.sh.seg / 2 >= density / 2)
         p.sh.seg /= 2;
     const bool small = p.nbuckets < (uint64_t)num_sms * kSmallBucketsPerSm;
-    shape_blocks(p.sh, small ? 1u : kBlockG);
+    // G2 additions take three times as long, so chains of 2 * 8 - 1 cost while blocks are few: 262144
+    // points (81920 buckets) 3.29 ms with 8, 3.18 with 4; 500000 (262144 buckets) 5.04 / 5.10
+    const bool few = sizeof(typename C::P) > 128 && p.nbuckets < (uint64_t)num_sms * 1024;
+    shape_blocks(p.sh, small ? 1u : few ? kBlockG / 2 : kBlockG);
     if (small) p.sh.fixmax = kFixupMaxSmall;
     p.units = (uint32_t)((p.max_entries + p.sh.seg - 1) / p.sh.seg);
     // tiled sort when a set's counters fit shared memory: set s = k Wr + w holds n_k halves
