@@ -592,9 +592,14 @@ static std::vector<ConstPair> wide_table(const std::vector<ConstPair>& t, uint32
     return v;
 }
 
+static constexpr uint32_t kAloneMinLog = 9;
+
 // Radix bits per pass: the tuned split for log_n when one is set (bits summing to log_n,
-// each 1..11), else the fewest passes of at most 11 bits, as equal as possible.
-static void split_passes(uint32_t log_n, NttPlan* plan, const uint8_t* tuned = nullptr) {
+// each 1..11), else the fewest passes of at most 11 bits, as equal as possible. alone: the
+// transform is (part of) a launch that leaves the GPU mostly idle; one of 2^9 .. 2^11 then takes two
+// passes, each over several CTAs, instead of one CTA's chain (measured, us: 2^9 10.6 -> 8.9, 2^10
+// 15.0 -> 9.6, 2^11 32.3 -> 10.1; 2^8 6.8 -> 8.2; three passes for 2^12 and more slower or the same).
+static void split_passes(uint32_t log_n, NttPlan* plan, const uint8_t* tuned = nullptr, bool alone = false) {
     if (log_n == 0) {
         plan->npass = 0;
         return;
@@ -607,17 +612,18 @@ static void split_passes(uint32_t log_n, NttPlan* plan, const uint8_t* tuned = n
     }
     int np = (int)((log_n + kMaxLogR - 1) / kMaxLogR);
     if (np < 1) np = 1;
+    if (alone && log_n >= kAloneMinLog && np == 1) np = 2;
     uint32_t base = log_n / np, extra = log_n % np;
     plan->npass = np;
     for (int p = 0; p < np; p++) plan->pass_log_r[p] = base + ((uint32_t)p < extra ? 1u : 0u);
 }
 
 static int build_plan(Ctx* c, int mode, uint32_t log_n, const zkh::F4& omega_m, const zkh::F4& shift_m,
-                      NttPlan** out) {
+                      bool alone, NttPlan** out) {
     const zkh::Field& F = zkh::fr();
     NttPlan* plan = new NttPlan();
     plan->log_n = log_n;
-    split_passes(log_n, plan, c->tune_ntt_split[log_n]);
+    split_passes(log_n, plan, c->tune_ntt_split[log_n], alone);
     const bool inverse = (mode == ZK_NTT_COEFFS_FROM_EVALS || mode == ZK_NTT_COSET_COEFFS_FROM_EVALS);
     const zkh::F4 w = inverse ? zkh::inv(F, omega_m) : omega_m;
     const uint64_t n = 1ull << log_n;
@@ -691,13 +697,16 @@ static int build_plan(Ctx* c, int mode, uint32_t log_n, const zkh::F4& omega_m, 
     return ZK_OK;
 }
 
-static int get_plan(Ctx* c, int mode, uint32_t log_n, const uint8_t omega[32], const uint8_t shift[32],
+// alone: see split_passes
+static int get_plan(Ctx* c, int mode, uint32_t log_n, const uint8_t omega[32], const uint8_t shift[32], bool alone,
                     NttPlan** out) {
+    alone = alone && log_n >= kAloneMinLog && log_n <= (uint32_t)kMaxLogR;  // the splits differ there only
     std::string key(reinterpret_cast<const char*>(omega), 32);
     key.append(reinterpret_cast<const char*>(shift), 32);
     key.push_back((char)mode);
     key.push_back((char)log_n);
     key.append(reinterpret_cast<const char*>(c->tune_ntt_split[log_n]), 4);
+    key.push_back(alone ? 1 : 0);
     auto it = c->ntt_plans.find(key);
     if (it != c->ntt_plans.end()) {
         *out = it->second;
@@ -716,7 +725,7 @@ static int get_plan(Ctx* c, int mode, uint32_t log_n, const uint8_t omega[32], c
         }
     }
     NttPlan* plan = nullptr;
-    int rc = build_plan(c, mode, log_n, om, sh, &plan);
+    int rc = build_plan(c, mode, log_n, om, sh, alone, &plan);
     if (rc != ZK_OK) return rc;
     c->ntt_plans[key] = plan;
     *out = plan;
@@ -860,7 +869,7 @@ int ntt_run(Ctx* c, int mode, fe* out, const fe* in, size_t in_len, uint32_t log
     NttPlan* plan = nullptr;
     {
         std::lock_guard<std::mutex> g(c->mu);
-        if ((rc = get_plan(c, mode, log_n, omega, shift, &plan)) != ZK_OK) return rc;
+        if ((rc = get_plan(c, mode, log_n, omega, shift, n < kWideElems, &plan)) != ZK_OK) return rc;
     }
     if ((rc = set_smem_attr(c->device)) != ZK_OK) return rc;
     const uint32_t valid = (uint32_t)(in_len < n ? in_len : n);
@@ -897,6 +906,7 @@ struct NttBatch {
     // and the state words (ticket, status, finished items per entry), all inside desc
     bool queue = false;
     bool wide = false;  // the wide form of the pass kernel (never in the queue form)
+    bool alone() const { return !wide && !queue; }  // see split_passes
     std::vector<NttQueueEntry> qentries;
     uint32_t qitems = 0, qsmem = 32, qgrid = 0;
     size_t queue_at = 0, limit_at = 0, state_at = 0;
@@ -906,6 +916,9 @@ struct NttBatch {
 static int batch_prepare(Ctx* c, const NttJob* jobs, size_t count, NttBatch* b) {
     b->jobs.assign(count, {});
     b->scratch_at.assign(count, 0);
+    uint64_t elems = 0;
+    for (size_t j = 0; j < count; j++) elems += 1ull << std::min<uint32_t>(jobs[j].log_n, 28);
+    b->wide = !b->queue && elems >= kWideElems;
     std::vector<NttPlan*> plans(count, nullptr);
     for (size_t j = 0; j < count; j++) {
         const NttJob& J = jobs[j];
@@ -914,13 +927,11 @@ static int batch_prepare(Ctx* c, const NttJob* jobs, size_t count, NttBatch* b) 
         ZK_CHECK_ARG(J.omega != nullptr, "null omega");
         std::lock_guard<std::mutex> g(c->mu);
         static const uint8_t one[32] = {1};
-        if ((rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, &plans[j])) != ZK_OK) return rc;
+        if ((rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, b->alone(), &plans[j])) != ZK_OK)
+            return rc;
         b->scratch_at[j] = b->scratch_elems;
         b->scratch_elems += pass_scratch_elems(plans[j], J.out, J.in);
     }
-    uint64_t elems = 0;
-    for (size_t j = 0; j < count; j++) elems += 1ull << jobs[j].log_n;
-    b->wide = !b->queue && elems >= kWideElems;
     size_t levels = 0;
     for (size_t j = 0; j < count; j++) levels = std::max<size_t>(levels, std::max(plans[j]->npass, 1));
     b->items.assign(levels, {});
@@ -943,7 +954,7 @@ static int batch_layout(const NttJob* jobs, size_t count, NttBatch* b, Ctx* c) {
         {
             std::lock_guard<std::mutex> g(c->mu);
             static const uint8_t one[32] = {1};
-            int rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, &plan);
+            int rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, b->alone(), &plan);
             if (rc != ZK_OK) return rc;
         }
         const uint64_t n = 1ull << J.log_n;

@@ -69,6 +69,23 @@ def _expected(mode, v, n, om):
     return _cache[mode]
 
 
+@pytest.mark.parametrize("log_n", [8, 9, 10, 11, 12])
+def test_small_sizes_match_oracle(ctx, log_n):
+    """2^9 .. 2^11 alone take two passes; in and out of place, every mode."""
+    n = 1 << log_n
+    om = G.omega_for_size(n)
+    v = synth.fr_uniform(log_n, n)
+    for mode in range(4):
+        want = O.ntt_op(mode, v, n, om, 5 if mode >= 2 else 1)
+        d, out = ctx.to_device(v), ctx.alloc(n * 32)
+        ctx.fr_to_mont(d, d, n)
+        ctx.ntt(mode, out, d, n, log_n, om, 5 if mode >= 2 else 1)
+        ctx.ntt(mode, d, d, n, log_n, om, 5 if mode >= 2 else 1)
+        for o in (out, d):
+            ctx.fr_from_mont(o, o, n)
+            assert (o.download().view("<u8").reshape(n, 4) == want).all(), mode
+
+
 @pytest.mark.parametrize("log_n", [18, 19, 20])
 def test_extreme_values(ctx, log_n):
     """All values r - 1 and alternating r - 1, 0: sums and differences at the ends of their range."""
