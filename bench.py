@@ -569,9 +569,9 @@ def run_gpu_ntt_sweep(ctx, args, flush, sizes=(12, 16, 20, 22)) -> dict:
 #   ncu --set full --clock-control none -k regex:<kernel> -s <skip> -c 1 -o <report>
 #       python bench.py --only <msm|ntt> [--log-n 22] --steps 2 --warmup 3 --no-cpu-baseline
 # keyed by (kernel, log2 n); the NTT figure is the mean of the two passes of a 2^22 transform
-# (first 134.3 + 81.8 MB, second, with the twiddle-table gathers, 290.2 + 101.4 MB).
-NCU_TRAFFIC_BYTES = {("msm_accumulate", 20): 1351.736e6 + 110.563e6,
-                     ("ntt_pass", 22): (134.305e6 + 81.835e6 + 290.209e6 + 101.394e6) / 2}
+# (first 134.4 + 89.8 MB, second, with the twiddle-table gathers, 296.9 + 108.9 MB).
+NCU_TRAFFIC_BYTES = {("msm_accumulate", 20): 1341e6 + 102e6,
+                     ("ntt_pass", 22): (134.429e6 + 89.783e6 + 296.936e6 + 108.895e6) / 2}
 
 
 def traffic_of(kernel: str, log_n: int):
@@ -599,8 +599,8 @@ def sort_kernels(table: dict, steps: int, n: int, entries: int, hbm_peak: float)
         t = ms / la
         gbs = nbytes / (t * 1e-3) / 1e9
         out[name] = {"ms": round(t, 4), "bytes": nbytes, "GB_s": round(gbs, 1), "frac": round(gbs / hbm_peak, 4)}
-    names = ("msm_codes", "msm_hist", "msm_hist_total", "msm_hist_offsets", "msm_sort_meta", "msm_scatter_tiles",
-             "msm_digits", "msm_scatter", "scan_tiles", "scan_add")
+    names = ("msm_codes", "msm_hist", "msm_hist_total", "msm_hist_offsets", "msm_sort_meta", "msm_set_hist", "msm_set_scatter",
+             "msm_scatter_tiles", "msm_digits", "msm_scatter", "scan_tiles", "scan_add")
     t = sum(table[k][1] / steps for k in names if k in table and table[k][0])
     if t > 0:
         nbytes = n * 32 + entries * 4
@@ -629,7 +629,9 @@ def imad_model(ctx, achieved_tops: float) -> dict:
     """The denominator checked without the probe: SMs x SM clock x the nominal 64 32-bit
     integer multiply-adds per clock per SM (the CUDA throughput table for compute capability
     10.x). The probe's mad.wide rate counted as 2 IMAD per wide product exceeds it (about 82
-    per clock per SM), so the probe's peak is the stricter denominator and the one used."""
+    per clock per SM: its product does not change over the loop), so the probe's peak is the
+    stricter denominator and the one used. The algorithmic count keeps 10 full products (1360 wide
+    multiply-adds) per entry; the accumulation executes 1160, so it may read above 1 here."""
     sms = ctx.num_sms()
     mhz = None
     try:

@@ -63,9 +63,8 @@ constexpr bool kFq2Schoolbook = true;
 constexpr bool kFq2Schoolbook = false;
 #endif
 // Default: Karatsuba with lazy reduction (fe2_mul_lazy: 3 unreduced 512-bit products, 2
-// reductions; ZK_FQ2_FULL keeps 3 full products). Measured on GB300 (G2 MSM): 2.03 / 2.45 ms
-// at 2^16, 4.55 / 5.27 ms at 2^18, 12.71 / 13.35 ms at 2^20 (accumulation -2%, window
-// reduction and fixup kernels -18 to -28%).
+// reductions; ZK_FQ2_FULL keeps 3 full products). Measured on GB300 with add-carry products
+// (lazy / full, G2 MSM): 2.03 / 2.45 ms at 2^16, 4.55 / 5.27 ms at 2^18, 12.71 / 13.35 ms at 2^20.
 #ifdef ZK_FQ2_FULL
 constexpr bool kFq2Lazy = false;
 #else
@@ -500,15 +499,11 @@ __device__ __forceinline__ T cta_quad_sum(uint32_t terms, Get&& get, XyzzT<T>* r
 #ifndef ZK_ACC_MINB_G2
 #define ZK_ACC_MINB_G2 1
 #endif
-// Threads of the CTA that sums one long bucket's pieces (strided partial sums, then a
-// shared-memory tree of the threads' partials); G2 points (256 B) keep it at 128 so that
-// the tree fits 32 KB of static shared memory. G1 runs 128 threads with four CTAs per SM
-// (a grid of as many): since huge buckets are summed in chunks by many CTAs, the CTA size
-// serves the long buckets of small pipelines, whose few pieces leave most of a wide CTA
-// idle. Measured on GB300 against 256 threads at two CTAs per SM: single MSMs 2^14 / 2^16
-// 0.476 / 0.758 -> 0.466 / 0.713 ms, 64 instances of 2^10..2^14 4.41 -> 4.28 ms; 2^18
-// +0.5%, witness-like 2^20 fixup 0.139 -> 0.158 ms. (Before the chunks, 256 threads had
-// won: one CTA summed the ~1600-segment bucket that witness-like 0/1 values make at 2^20.)
+// Threads of the CTA that sums one long bucket's pieces (quads of lanes sum strided pieces, then a
+// tree of the quads). G1 runs 128 threads with four CTAs per SM (a grid of as many): huge buckets
+// are summed in chunks by many CTAs, so the CTA size serves the long buckets of small pipelines,
+// whose few pieces leave most of a wide CTA idle (with one lane a point, 128 against 256 threads:
+// single MSMs 2^14 / 2^16 0.466 / 0.713 against 0.476 / 0.758 ms).
 #ifndef ZK_FIXUP_LONG_G1
 #define ZK_FIXUP_LONG_G1 128
 #endif

@@ -22,8 +22,8 @@
 //                         even when one bucket holds 5% of all points; a segment finds
 //                         its first bucket by binary search over the row pointers);
 //                         buckets wholly inside a segment are final; a bucket that
-//                         straddles segment boundaries leaves partial sums that one fixup
-//                         thread per bucket adds (short buckets), or tree rounds (pairs,
+//                         straddles segment boundaries leaves partial sums that a fixup thread or quad
+//                         per bucket adds (short buckets; a CTA for long ones), or tree rounds (pairs,
 //                         then groups of 4 units) merge, deciding "straddles" from the row
 //                         pointers.
 //  5. msm_bucket_blocks   per window, blocks of g buckets (large pipelines): sum_b b*B_b =
@@ -76,11 +76,10 @@ static constexpr uint32_t kGroup = ZK_MSM_GROUP;      // units merged per thread
 static constexpr uint32_t kBlockG = ZK_MSM_BLOCKG;
 static constexpr uint32_t kLineWarps = 8;  // lines get a second and fourth warp while below this per SM
 // Straddling buckets over more than kFixupMax + 1 segments go to the long-bucket fixup (a
-// CTA tree per bucket); small pipelines, latency-bound, send them there from kFixupMaxSmall
-// + 2 segments on (a tree of log2(pieces) additions instead of a chain). Measured on GB300
-// (single MSMs, 4 against 8): 2^12 0.390 -> 0.371 ms, 2^16 0.767 -> 0.753 ms, 2^14 the same;
-// then 3 against 4: 2^12 0.348 -> 0.331 ms, 2^10 / 2^14 / 2^16 -0.5..-1.5% (2 is slower: the
-// CTA trees of many 4-piece buckets, 2^16 0.98 ms).
+// CTA per bucket); small pipelines, latency-bound, send them there from kFixupMaxSmall + 2 segments
+// on (a tree of log2(pieces) additions instead of a chain). Measured on GB300 with one lane a
+// point: 3 / 4 / 8 at 2^12 0.331 / 0.348 / 0.365 ms; with quads 3 against 7 moves single MSMs by
+// under 3% either way.
 static constexpr uint32_t kFixupMax = 8;
 #ifndef ZK_FIXUP_MAX_SMALL
 #define ZK_FIXUP_MAX_SMALL 3

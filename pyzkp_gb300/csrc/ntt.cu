@@ -11,8 +11,9 @@
 // where w_N = omega^(n/N). Radix 2 with n/2 threads per pass is the reference's
 // Metal v2 (runtime/metal/runtime.py:336-362); here one CTA runs a whole radix-R
 // column group in shared memory (R up to 2^11) so a 2^22 transform makes two HBM
-// round trips instead of 22. Inside the CTA the R-point DFT is a decimation-in-
-// frequency sequence of radix-2 stages in place in shared memory, read back in
+// round trips instead of 22. Inside the CTA the R-point DFT is decimation in
+// frequency in place in shared memory (narrow form: two stages a step, four elements a
+// thread; wide form: three stages, eight elements a thread in registers), read back in
 // bit-reversed order. Coset scaling (shift^g) is applied while loading the first
 // pass and the inverse scale (n^-1 shift^-i) while storing the last pass.
 //
@@ -32,21 +33,21 @@ namespace zk {
 static constexpr int kNttThreads = 256;
 #ifndef ZK_NTT_MINB
 // resident CTAs per SM the single-transform pass kernel is compiled for: 2 (up to 128
-// registers) against 3 (85: the radix-4 steps then spill ~80 bytes) measured on GB300 with
-// radix-4 steps: 2^20 0.282 / 0.292 ms, 2^22 1.222 / 1.234 ms, 2^12 0.022 / 0.023 ms
+// registers); 3 leave 85, where the radix-4 steps spill ~80 bytes (with add-carry products
+// 2^20 0.282 / 0.292 ms, 2^12 0.022 / 0.023 ms) and radix-8 more
 #define ZK_NTT_MINB 2
 #endif
 #ifndef ZK_NTT_BATCH_MINB
 // ... and the batch and queue kernels: their many small tiles (256-element tiles of 128
-// active threads) want the third CTA per SM (64 coset NTTs of 2^10..2^20: 2.87 ms at 3,
-// 3.00 ms at 2)
+// active threads) want the third CTA per SM in the narrow form (64 coset NTTs of 2^10..2^20 with
+// add-carry products: 2.87 ms at 3, 3.00 ms at 2)
 #define ZK_NTT_BATCH_MINB 3
 #endif
 static constexpr int kMaxLogR = 11;       // 2048 elements * 32 B = 64 KB of shared memory
 static constexpr int kTileLogElems = 11;  // largest tile: R * T = 2048 elements per CTA
 // Default tile: 2^8 elements per CTA, or one radix-R column when R is larger. Measured on
-// GB300 (forward NTT, L2 flushed): 2^12 74 -> 22 us, 2^16 91 -> 34 us, 2^20 333 -> 298 us
-// against 2^11-element tiles; tiles of 2^6..2^8 are within 5% of one another at every size.
+// GB300 with radix-2 stages, 2^11- / 2^8-element tiles: 2^12 74 / 22 us, 2^16 91 / 34 us, 2^20 333 /
+// 298 us; tiles of 2^6..2^8 are within 5% of one another at every size.
 static constexpr int kDefaultTileLog = 8;
 
 // Elements a thread loads before it multiplies the first: 1 / 2 / 4 / 8 at 2^22 (narrow form) 893 / 879

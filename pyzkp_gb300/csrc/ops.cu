@@ -235,7 +235,10 @@ namespace zk {
 // MODE 1: 8 independent mad.lo.u32 accumulators per thread (raw IMAD issue rate);
 // MODE 2: 8 independent mad.hi.u32 accumulators per thread;
 // MODE 3: 8 independent mad.wide.u32 (32x32 -> 64-bit) accumulators per thread, counted
-//         as 2 IMAD each (one full-width product replaces a lo + hi pair).
+//         as 2 IMAD each (one full-width product replaces a lo + hi pair). Its two factors do
+//         not change over the loop, so the compiler may keep their product and the figure (12.9 T
+//         wide/s) is above the pipe's rate: with changing factors a wide multiply-add, with or
+//         without carries, takes 4 cycles of a quarter SM's pipe per warp, 10.07 T/s.
 template <int MODE>
 __global__ void imad_probe_kernel(uint32_t iters, uint32_t seed, uint32_t* sink) {
     uint32_t a[8], x = seed ^ threadIdx.x, y = seed * 2654435761u + blockIdx.x;
