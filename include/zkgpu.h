@@ -276,7 +276,8 @@ int zk_fr_div_xn_minus_1(zk_ctx *ctx, const void *a, size_t len, size_t n, void 
  * PLONK quotient step (protocols/plonk/prove.py:395-420).
  *   zk_fr_batch_inv          BATCH_INV (crypto/field/batch.py:8-38 through
  *                            runtime/kernels/cpu/kernels.py:_batch_inv): out[i] = in[i]^-1,
- *                            0 for a zero input; out may equal in. Asynchronous.
+ *                            0 for a zero input (any multiple of r); out may equal in.
+ *                            Asynchronous.
  *   zk_plonk_quotient_evals  PLONK_T_QUOTIENT_EVALS (runtime/kernels/cpu/kernels.py:
  *                            _plonk_t_quotient_evals): from 15 extended-coset evaluation
  *                            vectors of length m (a, b, c, z, pi, ql, qr, qm, qo, qc, s1, s2,

@@ -88,14 +88,14 @@ __device__ __forceinline__ fe fe_one() {
     return r;
 }
 
-__device__ __forceinline__ fe fe_zero() {
+__host__ __device__ __forceinline__ fe fe_zero() {
     fe r;
 #pragma unroll
     for (int i = 0; i < 8; i++) r.v[i] = 0;
     return r;
 }
 
-__device__ __forceinline__ bool fe_is_zero(const fe& a) {
+__host__ __device__ __forceinline__ bool fe_is_zero(const fe& a) {
     uint32_t x = a.v[0] | a.v[1] | a.v[2] | a.v[3] | a.v[4] | a.v[5] | a.v[6] | a.v[7];
     return x == 0;
 }

@@ -21,6 +21,7 @@
 #include <cstring>
 #include <vector>
 
+#include "inverse.cuh"
 #include "zk_internal.cuh"
 
 namespace zk {
@@ -35,78 +36,14 @@ static constexpr uint32_t kInvWarp = 32 * kInvChunk;  // elements of a warp
 static constexpr uint32_t kQChunk = 16;
 static constexpr uint32_t kQWarps = 32;
 
-// a >> z and a << z for z < 32 (no bit is lost to the left)
-__device__ __forceinline__ void limbs_shr(fe& a, uint32_t z) {
-#pragma unroll
-    for (int i = 0; i < 7; i++) a.v[i] = __funnelshift_r(a.v[i], a.v[i + 1], z);
-    a.v[7] >>= z;
-}
-__device__ __forceinline__ void limbs_shl(fe& a, uint32_t z) {
-#pragma unroll
-    for (int i = 7; i > 0; i--) a.v[i] = __funnelshift_l(a.v[i - 1], a.v[i], z);
-    a.v[0] <<= z;
-}
-__device__ __forceinline__ fe limbs_add(const fe& a, const fe& b) {
-    fe r;
-    r.v[0] = u_add_cc(a.v[0], b.v[0]);
-#pragma unroll
-    for (int i = 1; i < 7; i++) r.v[i] = u_addc_cc(a.v[i], b.v[i]);
-    r.v[7] = u_addc(a.v[7], b.v[7]);
-    return r;
-}
-__device__ __forceinline__ fe limbs_sub(const fe& a, const fe& b, uint32_t* borrow) {
-    fe r;
-    r.v[0] = u_sub_cc(a.v[0], b.v[0]);
-#pragma unroll
-    for (int i = 1; i < 8; i++) r.v[i] = u_subc_cc(a.v[i], b.v[i]);
-    *borrow = u_subc(0u, 0u);
-    return r;
-}
-
-// The inverse of a Montgomery form a = x R (a != 0, canonical): x^-1 R. Binary extended Euclid
-// without modular halvings (Kaliski's almost inverse): with u = p, v = a, r = 0, s = 1 the steps
-// keep p = u s + v r and a s = v 2^k (mod p), k counting the halvings of u and v; at u = v = 1
-// s = a^-1 2^k = x^-1 R^-1 2^k, 253 <= k <= 508. Then x^-1 R = s 2^(512 - k), by a product with
-// 2^(512 - k) / R and one with R^2.
-//
-// What bounds it: ~180 steps of a subtraction, an addition and two shifts, chains of 8
-// limbs. a^(p - 2) takes 384 dependent products, ~150 us a thread.
+// The inverse of a Montgomery form a = x R (canonical): x^-1 R, and 0 for 0. s = a^-1 2^k =
+// x^-1 R^-1 2^k from fe_almost_inverse, then x^-1 R = s 2^(512 - k), by a product with
+// 2^(512 - k) / R and one with R^2. (a^(p - 2) takes 384 dependent products, ~150 us a thread.)
 template <class F>
 __device__ fe fe_inverse_binary(const fe& a) {
-    fe u, v = a, r = fe_zero(), s = fe_zero();
-#pragma unroll
-    for (int i = 0; i < 8; i++) u.v[i] = F::P(i);
-    s.v[0] = 1;
-    uint32_t k = 0;
-    while (!(v.v[0] & 1)) {  // u stays odd until the first subtraction
-        const uint32_t z = v.v[0] ? __ffs(v.v[0]) - 1 : 31;
-        limbs_shr(v, z);
-        k += z;  // r = 0
-    }
-    for (;;) {  // u and v odd
-        uint32_t less;
-        fe d = limbs_sub(u, v, &less);
-        if (fe_is_zero(d)) break;
-        if (!less) {
-            u = d;
-            r = limbs_add(r, s);
-            do {
-                const uint32_t z = u.v[0] ? __ffs(u.v[0]) - 1 : 31;
-                limbs_shr(u, z);
-                limbs_shl(s, z);
-                k += z;
-            } while (!(u.v[0] & 1));
-        } else {
-            v = limbs_sub(v, u, &less);
-            s = limbs_add(s, r);
-            do {
-                const uint32_t z = v.v[0] ? __ffs(v.v[0]) - 1 : 31;
-                limbs_shr(v, z);
-                limbs_shl(r, z);
-                k += z;
-            } while (!(v.v[0] & 1));
-        }
-    }
+    fe s;
+    uint32_t k;
+    if (!fe_almost_inverse<F>(a, &s, &k)) return fe_zero();
     uint32_t j = 512 - k;
     while (j > 253) {  // 2^j below 2^254
         s = fe_add<F>(s, s);
@@ -138,6 +75,10 @@ __device__ __forceinline__ fe fe_shfl_down(const fe& a, uint32_t d) {
 // elements are 32 apart, so that the warp reads and writes whole lines. Measured at 2^19
 // elements: 229 -> 66 us against a Fermat inversion per 32 consecutive elements (384 dependent
 // products, and each lane's accesses a kilobyte from the next one's).
+//
+// An element counts as zero when it is a multiple of r, whatever its bits: when its product with
+// a value that is not zero is (fe_mul takes any 256-bit second factor), so the running products
+// stay non-zero.
 __global__ void __launch_bounds__(128) fr_batch_inv_kernel(fe* __restrict__ out, const fe* __restrict__ in, size_t n) {
     if (!grid_enter()) return;
     const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -149,8 +90,8 @@ __global__ void __launch_bounds__(128) fr_batch_inv_kernel(fe* __restrict__ out,
         const size_t i = i0 + 32 * j;
         if (i >= n) break;
         fe_store(out + i, acc);  // product of the lane's non-zero inputs before i
-        const fe x = fe_ldg(in + i);
-        if (!fe_is_zero(x)) acc = fe_mul<FrP>(acc, x);
+        const fe t = fe_mul<FrP>(acc, fe_ldg(in + i));
+        if (!fe_is_zero(t)) acc = t;
     }
     __syncwarp();
     // products of the lanes before (pre) and after (suf) this one
@@ -170,12 +111,12 @@ __global__ void __launch_bounds__(128) fr_batch_inv_kernel(fe* __restrict__ out,
     for (uint32_t j = kInvChunk; j-- > 0;) {
         const size_t i = i0 + 32 * j;
         if (i >= n) continue;
-        const fe x = fe_ldg(in + i);
-        if (fe_is_zero(x)) {
+        const fe t = fe_mul<FrP>(inv, fe_ldg(in + i));
+        if (fe_is_zero(t)) {
             fe_store(out + i, fe_zero());
         } else {
             fe_store(out + i, fe_mul<FrP>(fe_load(out + i), inv));
-            inv = fe_mul<FrP>(inv, x);
+            inv = t;
         }
     }
 }
