@@ -13,7 +13,10 @@
  * Data layout (identical bytes to the reference's "fr_mont_u64x4" buffers,
  * runtime/metal/buffer.py:7-15 and runtime/kernels/cpu/kernels.py:135-141):
  *   - a field element is 32 bytes, little endian, 8 x uint32 (= 4 x uint64) limbs;
- *     "Montgomery" means the value a * 2^256 mod p, "canonical" the value itself;
+ *     "Montgomery" means the value a * 2^256 mod p, "canonical" the value itself, both
+ *     below p. Nothing checks device buffers for that bound: zk_fr_mul, zk_fr_scale,
+ *     zk_fr_batch_inv, zk_fr_from_mont and the forward coset NTT take any 256 bits as
+ *     their residue, the other calls need values below p;
  *   - an affine G1 point is 64 bytes: x then y (Fq); (0, 0) denotes infinity.
  * Device pointers are CUDA device addresses on the context's device.
  * All functions return ZK_OK (0) or an error code; zk_last_error() describes the

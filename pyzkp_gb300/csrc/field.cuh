@@ -520,7 +520,9 @@ __host__ __device__ __forceinline__ fe row_result(const uint32_t* e, const uint3
 }
 
 // a b 2^-256 mod p, below ab / 2^256 + (1 + 2^-31) p (CIOS rows): below 2p for a, b below 2p. T
-// is largest in the first row with p, below 2^32 (a + N' + p) (1 + 2^-31) < 4p 2^32 < 2^288.
+// is largest in the first row with p, below 2^32 (a + N' + p) (1 + 2^-31), which has to stay below
+// 2^288: for a below 3.35p (r; 3.39p for q). b may be any 256 bits. A value of a caller, which
+// nothing has reduced, is therefore the second factor, or a factor of fe_mul_any.
 template <class F>
 __host__ __device__ __forceinline__ fe mul_rows(const fe& a, const fe& b) {
     uint32_t e[8], o[8];
@@ -709,7 +711,8 @@ __device__ __noinline__ fe fe_mul_call(const fe a, const fe b) {
     return mul_rows<F>(a, b);
 }
 
-// r = a * b * 2^-256 mod p. F::CALL_MUL: one non-inlined copy of the product, called from
+// r = a * b * 2^-256 mod p for a below 3.35p and any b (see mul_rows); in [0, p), or [0, 2p) when
+// lazy, for a, b that are. F::CALL_MUL: one non-inlined copy of the product, called from
 // every site. The curve formulas hold 10-14 products per loop body, so inlining them all
 // overflows the instruction cache; the NTT butterflies hold one to four.
 template <class F>
@@ -834,6 +837,18 @@ __host__ __device__ __forceinline__ fe sos_reduce_2p(const fe& t) {
 #pragma unroll
     for (int j = 0; j < 8; j++) r.v[j] = borrow ? t.v[j] : s.v[j];
     return r;
+}
+
+// The product rows for any 256-bit a and b: a below 2^256 - 2p < 3.3p first.
+template <class F>
+__host__ __device__ __forceinline__ fe mul_rows_any(const fe& a, const fe& b) {
+    return mul_rows<F>(sos_reduce_2p<F>(a), b);
+}
+
+// fe_mul for any 256-bit a and b (vectors of a caller)
+template <class F>
+__device__ __forceinline__ fe fe_mul_any(const fe& a, const fe& b) {
+    return fe_mul<F>(sos_reduce_2p<F>(a), b);
 }
 
 // a^2 * 2^-256 mod p in [0, 2p) for a in [0, 2p)
@@ -995,7 +1010,8 @@ __device__ __forceinline__ fe fe_to_mont(fe a) {
     return fe_mul<F>(a, r2);
 }
 
-// Montgomery -> canonical in [0, p) (also for lazy inputs below 2p: a * 1 * 2^-256 <= p).
+// Montgomery -> canonical in [0, p), for any 256-bit a: the product with 1 is below
+// (1 + 2^-31) p + 1, one subtraction of p from its residue.
 template <class F>
 __device__ __forceinline__ fe fe_from_mont(const fe& a) {
     fe one;

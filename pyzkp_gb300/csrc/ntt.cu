@@ -324,7 +324,7 @@ __device__ __forceinline__ void ntt_pass_body(const NttPassParams& P, uint32_t t
             if (P.log_l != 0) {
                 if (m != 0 && ((c0 + t) & l_mask) != 0) x = fe_mul<FrN>(x, f[q]);
             } else if (P.pre_lo != nullptr && c0 + t + (m << stride_log) < P.in_len) {
-                x = fe_mul<FrN>(x, f[q]);
+                x = fe_mul<FrN>(f[q], x);  // x of the caller: the second factor
             }
             smem_put(s_lo, s_hi, (swz(m) << log_t) + t, x);
         }

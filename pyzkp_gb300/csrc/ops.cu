@@ -29,7 +29,7 @@ __global__ void convert_kernel(fe* out, const fe* in, size_t n) {
 __global__ void fr_mul_kernel(fe* out, const fe* a, const fe* b, size_t n) {
     if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        fe_store(out + i, fe_mul<FrP>(fe_ldg(a + i), fe_ldg(b + i)));
+        fe_store(out + i, fe_mul_any<FrP>(fe_ldg(a + i), fe_ldg(b + i)));
 }
 
 __global__ void fr_sub_kernel(fe* out, const fe* a, const fe* b, size_t n) {

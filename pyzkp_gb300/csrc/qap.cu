@@ -42,7 +42,7 @@ __global__ void fr_spmv_kernel(uint32_t nrows, const uint32_t* __restrict__ row_
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nrows; i += (size_t)gridDim.x * blockDim.x) {
         fe acc = fe_zero();
         for (uint32_t j = row_ptr[i]; j < row_ptr[i + 1]; j++)
-            acc = fe_add<FrP>(acc, fe_mul<FrP>(fe_ldg(coeffs + j), fe_ldg(x + cols[j])));
+            acc = fe_add<FrP>(acc, fe_mul_any<FrP>(fe_ldg(coeffs + j), fe_ldg(x + cols[j])));
         fe_store(out + i, acc);
     }
 }
@@ -52,7 +52,7 @@ __global__ void fr_r1cs_check_kernel(const fe* __restrict__ a, const fe* __restr
     if (!grid_enter()) return;
     unsigned long long local = 0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const fe ab = fe_mul<FrP>(fe_ldg(a + i), fe_ldg(b + i));
+        const fe ab = fe_mul_any<FrP>(fe_ldg(a + i), fe_ldg(b + i));
         const fe cc = fe_ldg(c + i);
         bool eq = true;
 #pragma unroll
@@ -66,8 +66,8 @@ __global__ void fr_qap_quotient_kernel(fe* __restrict__ out, const fe* __restric
                                        const fe* __restrict__ c, size_t n, fe zinv) {
     if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const fe ab = fe_mul<FrP>(fe_ldg(a + i), fe_ldg(b + i));
-        fe_store(out + i, fe_mul<FrP>(fe_sub<FrP>(ab, fe_ldg(c + i)), zinv));
+        const fe ab = fe_mul_any<FrP>(fe_ldg(a + i), fe_ldg(b + i));
+        fe_store(out + i, fe_mul<FrP>(zinv, fe_sub<FrP>(ab, fe_ldg(c + i))));
     }
 }
 
@@ -81,7 +81,7 @@ __global__ void fr_gather_kernel(fe* __restrict__ out, const fe* __restrict__ in
 __global__ void fr_scale_kernel(fe* __restrict__ out, const fe* __restrict__ in, size_t n, fe s) {
     if (!grid_enter()) return;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        fe_store(out + i, fe_mul<FrP>(fe_ldg(in + i), s));
+        fe_store(out + i, fe_mul<FrP>(s, fe_ldg(in + i)));
 }
 
 // out[i] = base^i (Montgomery): chunk t of kPowChunk consecutive powers starts from
