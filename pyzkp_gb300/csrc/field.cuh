@@ -42,11 +42,7 @@ struct FqP {
     // (INV p + 1) / 2^32 (see the products below)
     __host__ __device__ static constexpr uint32_t NP(int i) { return i == 0 ? 0x705c70f2u : i == 1 ? 0xb5b479a3u : i == 2 ? 0x699a472au : i == 3 ? 0xef510c54u : i == 4 ? 0xb6c9df27u : i == 5 ? 0xb27cd0b5u : i == 6 ? 0x10b67b2fu : 0x2b32bd30u; }
     static constexpr bool CALL_MUL = true;
-#ifdef ZK_FQ_STRICT
-    static constexpr bool LAZY = false;
-#else
     static constexpr bool LAZY = true;
-#endif
     __host__ __device__ static constexpr uint32_t ONE(int i) { return i == 0 ? 0xc58f0d9du : i == 1 ? 0xd35d438du : i == 2 ? 0xf5c70b3du : i == 3 ? 0x0a78eb28u : i == 4 ? 0x7879462cu : i == 5 ? 0x666ea36fu : i == 6 ? 0x9a07df2fu : 0x0e0a77c1u; }
     // 4 q^2 as 16 limbs (the offset that keeps a difference of two products below 4q^2 each
     // non-negative)
@@ -62,11 +58,7 @@ struct FqP {
 // Fr with lazy values in [0, 2r): for the NTT pass kernel only, whose last pass reduces
 // every output once more (all other Fr code sees canonical values).
 struct FrLazyP : FrP {
-#ifdef ZK_NTT_STRICT
-    static constexpr bool LAZY = false;
-#else
     static constexpr bool LAZY = true;
-#endif
 };
 
 // Fr with one non-inlined copy of the product, for kernels whose loop bodies hold many
@@ -944,11 +936,6 @@ __device__ __noinline__ fe fe_sqr_sos_call(const fe a) {
 }
 
 template <class F>
-__device__ __noinline__ fe fe_mul_add_sos_call(const fe a, const fe b, const fe c, const fe d) {
-    return fe_mul_add_sos<F>(a, b, c, d);
-}
-
-template <class F>
 __device__ __noinline__ fe fe_mul_sub_sos_call(const fe a, const fe b, const fe c, const fe d) {
     return fe_mul_sub_sos<F>(a, b, c, d);
 }
@@ -971,12 +958,6 @@ template <class F>
 __device__ __forceinline__ fe fe_mul_sub(const fe& a, const fe& b, const fe& c, const fe& d) {
     if constexpr (use_sos<F>()) return fe_mul_sub_sos_call<F>(a, b, c, d);
     else return fe_sub<F>(fe_mul<F>(a, b), fe_mul<F>(c, d));
-}
-
-template <class F>
-__device__ __forceinline__ fe fe_mul_add(const fe& a, const fe& b, const fe& c, const fe& d) {
-    if constexpr (use_sos<F>()) return fe_mul_add_sos_call<F>(a, b, c, d);
-    else return fe_add<F>(fe_mul<F>(a, b), fe_mul<F>(c, d));
 }
 
 // canonical value (any 256-bit input, reduced mod p first) -> Montgomery form

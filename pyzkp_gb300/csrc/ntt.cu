@@ -78,6 +78,7 @@ struct NttPassParams {
 // Butterflies, twiddles and scales run on lazy Fr values in [0, 2r) (FrLazyP); inputs are
 // canonical, intermediate passes store lazy values, the last pass stores canonical ones.
 using FrN = FrLazyP;
+static_assert(FrN::LAZY, "the butterflies take and leave values in [0, 2r)");
 
 __device__ __forceinline__ fe lookup2(const fe* lo, const fe* hi, uint32_t e, uint32_t s_bits) {
     if (s_bits == kNttFullTable) return fe_ldg(lo + e);
