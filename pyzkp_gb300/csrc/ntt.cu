@@ -567,14 +567,25 @@ struct ConstPair {
     zkh::F4 w, ws;
 };
 
-static int upload_pairs(Ctx* c, NttPlan* plan, const std::vector<ConstPair>& v, fe_const** out) {
-    static_assert(sizeof(ConstPair) == sizeof(fe_const), "fe_const layout");
-    std::vector<zkh::F4> flat(2 * v.size());
-    std::memcpy(flat.data(), v.data(), v.size() * sizeof(ConstPair));
-    fe* table = nullptr;
-    const int rc = upload_table(c, plan, flat, &table);
-    *out = reinterpret_cast<fe_const*>(table);
-    return rc;
+// ... from the Montgomery form t of w: w = (t + ws r) / 2^256, a sum that 2^256 divides (t != 0, so
+// the low halves carry one).
+static ConstPair const_pair(const zkh::F4& t) {
+    const uint64_t* r = zkh::fr().p;
+    ConstPair c;
+    c.ws = shoup_quotient(t);
+    uint64_t x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int i = 0; i < 4; i++) {
+        uint64_t carry = 0;
+        for (int j = 0; j < 4; j++) {
+            const unsigned __int128 s = (unsigned __int128)c.ws.v[i] * r[j] + x[i + j] + carry;
+            x[i + j] = (uint64_t)s;
+            carry = (uint64_t)(s >> 64);
+        }
+        x[i + 4] = carry;
+    }
+    const uint64_t one[4] = {1, 0, 0, 0};
+    zkh::add4(c.w.v, x + 4, one);
+    return c;
 }
 
 // The wide form's table of a radix-2^lr pass from t[i] = w_R^i, i < R = 2^lr (see dft_wide).
@@ -592,6 +603,48 @@ static std::vector<ConstPair> wide_table(const std::vector<ConstPair>& t, uint32
             for (size_t j = 0; j < h; j++) v.push_back(t[j * k * step]);
     }
     return v;
+}
+
+// The radix tables of one form, if the plan does not hold them yet: one table per radix (passes of
+// the same radix share it), in one upload. A launch takes one form, so a plan's first use pays for
+// that one alone (first transform with a new shift, us, against both forms at once: 2^8 82 -> 67, 2^16
+// 289 -> 236, 2^20 722 -> 545).
+static int radix_tables(Ctx* c, NttPlan* plan, bool wide) {
+    fe_const** out = wide ? plan->wide_tw : plan->radix_tw;
+    if (plan->npass == 0 || out[0] != nullptr) return ZK_OK;
+    const zkh::Field& F = zkh::fr();
+    std::vector<ConstPair> all;
+    size_t at[4] = {0, 0, 0, 0};
+    for (int p = 0; p < plan->npass; p++) {
+        const uint32_t lr = plan->pass_log_r[p];
+        int same = 0;
+        while (plan->pass_log_r[same] != lr) same++;
+        at[p] = all.size();
+        if (same < p) {
+            at[p] = at[same];
+            continue;
+        }
+        const size_t half = ((size_t)1 << lr) / 2;
+        std::vector<ConstPair> t;
+        for (const zkh::F4& x : powers(zkh::pow_u64(F, plan->root, 1ull << (plan->log_n - lr)), half)) t.push_back(const_pair(x));
+        if (wide) {
+            // w_R^(i + R/2) = -w_R^i, and floor((r - w) 2^256 / r) = 2^256 - 1 - floor(w 2^256 / r)
+            for (size_t i = 0; i < half; i++) {
+                ConstPair m{zkh::neg(F, t[i].w), {}};
+                for (int j = 0; j < 4; j++) m.ws.v[j] = ~t[i].ws.v[j];
+                t.push_back(m);
+            }
+            t = wide_table(t, lr);
+        }
+        all.insert(all.end(), t.begin(), t.end());
+    }
+    static_assert(sizeof(ConstPair) == sizeof(fe_const), "fe_const layout");
+    void* dev = nullptr;
+    ZK_TRY_CUDA(cudaMalloc(&dev, all.size() * sizeof(ConstPair)));
+    plan->allocations.push_back(dev);
+    ZK_TRY_CUDA(cudaMemcpyAsync(dev, all.data(), all.size() * sizeof(ConstPair), cudaMemcpyHostToDevice, c->stream));
+    for (int p = 0; p < plan->npass; p++) out[p] = static_cast<fe_const*>(dev) + at[p];
+    return ZK_OK;
 }
 
 static constexpr uint32_t kAloneMinLog = 9;
@@ -628,6 +681,7 @@ static int build_plan(Ctx* c, int mode, uint32_t log_n, const zkh::F4& omega_m, 
     split_passes(log_n, plan, c->tune_ntt_split[log_n], alone);
     const bool inverse = (mode == ZK_NTT_COEFFS_FROM_EVALS || mode == ZK_NTT_COSET_COEFFS_FROM_EVALS);
     const zkh::F4 w = inverse ? zkh::inv(F, omega_m) : omega_m;
+    plan->root = w;
     const uint64_t n = 1ull << log_n;
     plan->s_bits = (log_n + 1) / 2;
     const uint64_t lo_count = 1ull << plan->s_bits;
@@ -640,16 +694,6 @@ static int build_plan(Ctx* c, int mode, uint32_t log_n, const zkh::F4& omega_m, 
         std::vector<zkh::F4> hi = powers(ws, hi_count);
         if ((rc = upload_table(c, plan, lo, &plan->tw_lo)) != ZK_OK) return rc;
         if ((rc = upload_table(c, plan, hi, &plan->tw_hi)) != ZK_OK) return rc;
-    }
-    for (int p = 0; p < plan->npass; p++) {
-        const uint32_t lr = plan->pass_log_r[p];
-        const zkh::F4 wr = zkh::pow_u64(F, w, n >> lr);
-        std::vector<ConstPair> t;
-        for (const zkh::F4& x : powers(wr, 1ull << lr)) t.push_back({zkh::from_mont(F, x), shoup_quotient(x)});
-        const std::vector<ConstPair> wide = wide_table(t, lr);
-        t.resize(std::max<size_t>(1, t.size() / 2));
-        if ((rc = upload_pairs(c, plan, t, &plan->radix_tw[p])) != ZK_OK) return rc;
-        if ((rc = upload_pairs(c, plan, wide, &plan->wide_tw[p])) != ZK_OK) return rc;
     }
     if (mode == ZK_NTT_COSET_EVALS_FROM_COEFFS) {
         std::vector<zkh::F4> lo = powers(shift_m, lo_count);
@@ -699,9 +743,9 @@ static int build_plan(Ctx* c, int mode, uint32_t log_n, const zkh::F4& omega_m, 
     return ZK_OK;
 }
 
-// alone: see split_passes
+// alone: see split_passes; wide: the form of the pass kernel that the launch takes
 static int get_plan(Ctx* c, int mode, uint32_t log_n, const uint8_t omega[32], const uint8_t shift[32], bool alone,
-                    NttPlan** out) {
+                    bool wide, NttPlan** out) {
     alone = alone && log_n >= kAloneMinLog && log_n <= (uint32_t)kMaxLogR;  // the splits differ there only
     std::string key(reinterpret_cast<const char*>(omega), 32);
     key.append(reinterpret_cast<const char*>(shift), 32);
@@ -712,7 +756,7 @@ static int get_plan(Ctx* c, int mode, uint32_t log_n, const uint8_t omega[32], c
     auto it = c->ntt_plans.find(key);
     if (it != c->ntt_plans.end()) {
         *out = it->second;
-        return ZK_OK;
+        return radix_tables(c, it->second, wide);
     }
     const zkh::Field& F = zkh::fr();
     zkh::F4 om = zkh::to_mont(F, load_canon(omega));
@@ -731,7 +775,7 @@ static int get_plan(Ctx* c, int mode, uint32_t log_n, const uint8_t omega[32], c
     if (rc != ZK_OK) return rc;
     c->ntt_plans[key] = plan;
     *out = plan;
-    return ZK_OK;
+    return radix_tables(c, plan, wide);
 }
 
 // Dynamic shared memory of the pass kernels (set once per device).
@@ -869,9 +913,10 @@ int ntt_run(Ctx* c, int mode, fe* out, const fe* in, size_t in_len, uint32_t log
     if (rc != ZK_OK) return rc;
     const uint64_t n = 1ull << log_n;
     NttPlan* plan = nullptr;
+    const bool wide = n >= kWideElems;
     {
         std::lock_guard<std::mutex> g(c->mu);
-        if ((rc = get_plan(c, mode, log_n, omega, shift, n < kWideElems, &plan)) != ZK_OK) return rc;
+        if ((rc = get_plan(c, mode, log_n, omega, shift, !wide, wide, &plan)) != ZK_OK) return rc;
     }
     if ((rc = set_smem_attr(c->device)) != ZK_OK) return rc;
     const uint32_t valid = (uint32_t)(in_len < n ? in_len : n);
@@ -879,7 +924,6 @@ int ntt_run(Ctx* c, int mode, fe* out, const fe* in, size_t in_len, uint32_t log
     const size_t se = pass_scratch_elems(plan, out, in);
     if (se && (rc = scratch_alloc(c, se * 32, reinterpret_cast<void**>(&scratch))) != ZK_OK) return rc;
     std::vector<PassLaunch> launches;
-    const bool wide = n >= kWideElems;
     make_passes(plan, out, in, valid, scratch, &launches, wide, canon_io);
     auto* kernel = wide ? &ntt_pass_kernel<true> : &ntt_pass_kernel<false>;
     for (const PassLaunch& L : launches) {
@@ -929,7 +973,8 @@ static int batch_prepare(Ctx* c, const NttJob* jobs, size_t count, NttBatch* b) 
         ZK_CHECK_ARG(J.omega != nullptr, "null omega");
         std::lock_guard<std::mutex> g(c->mu);
         static const uint8_t one[32] = {1};
-        if ((rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, b->alone(), &plans[j])) != ZK_OK)
+        if ((rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, b->alone(), b->wide,
+                           &plans[j])) != ZK_OK)
             return rc;
         b->scratch_at[j] = b->scratch_elems;
         b->scratch_elems += pass_scratch_elems(plans[j], J.out, J.in);
@@ -956,7 +1001,7 @@ static int batch_layout(const NttJob* jobs, size_t count, NttBatch* b, Ctx* c) {
         {
             std::lock_guard<std::mutex> g(c->mu);
             static const uint8_t one[32] = {1};
-            int rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, b->alone(), &plan);
+            int rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, b->alone(), b->wide, &plan);
             if (rc != ZK_OK) return rc;
         }
         const uint64_t n = 1ull << J.log_n;

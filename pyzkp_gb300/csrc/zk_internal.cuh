@@ -55,8 +55,11 @@ struct NttPlan {
     uint32_t log_n = 0;
     int npass = 0;
     uint32_t pass_log_r[4] = {0, 0, 0, 0};
-    fe_const* radix_tw[4] = {nullptr, nullptr, nullptr, nullptr};  // omega_R^i, i < R/2, per pass
-    fe_const* wide_tw[4] = {nullptr, nullptr, nullptr, nullptr};   // the wide form's tables, per pass
+    // per pass, each form's built when a launch first takes it: omega_R^i, i < R/2, and the wide
+    // form's tables
+    fe_const* radix_tw[4] = {nullptr, nullptr, nullptr, nullptr};
+    fe_const* wide_tw[4] = {nullptr, nullptr, nullptr, nullptr};
+    zkh::F4 root = {};  // omega (inverse modes: its inverse), Montgomery
     uint32_t s_bits = 0;  // split of two-level tables; kNttFullTable: tw/pre/post_lo are full tables
     fe* tw_lo = nullptr;                                       // omega^i, i < 2^s
     fe* tw_hi = nullptr;                                       // omega^(i 2^s), i < n / 2^s
