@@ -799,6 +799,10 @@ static int set_smem_attr(int device) {
 // many threads). Measured on GB300, narrow / wide (us): 2^16 26.5 / 41.3, 2^17 37.5 / 43.2, 2^18
 // 72.0 / 57.5.
 static constexpr uint64_t kWideElems = 1ull << 18;
+// ... in transforms of at least this size, if these are half of a batch or more: an eighth of a
+// smaller one's tile is less than a warp. Batches of 2^20 elements as 2^6 / 2^7 / 2^8 / 2^9, us, narrow
+// 61 / 70 / 80 / 98, wide 138 / 98 / 64 / 70; 2^18 elements as 2^7 / 2^8 25 / 28, 33 / 23.
+static constexpr uint32_t kWideMinLog = 8;
 // Its tiles: 2^8 .. 2^10 elements are within 2% of one another, 2^11 12% slower at 2^20 (fewer,
 // longer CTAs: an emptier last wave).
 static constexpr int kWideTileLog = 10;
@@ -951,8 +955,8 @@ struct NttBatch {
     // queue form (one persistent launch): entries in queue order, then the wait limit (ns)
     // and the state words (ticket, status, finished items per entry), all inside desc
     bool queue = false;
-    bool wide = false;  // the wide form of the pass kernel (never in the queue form)
-    bool alone() const { return !wide && !queue; }  // see split_passes
+    bool wide = false;   // the wide form of the pass kernel (never in the queue form)
+    bool alone = false;  // see split_passes
     std::vector<NttQueueEntry> qentries;
     uint32_t qitems = 0, qsmem = 32, qgrid = 0;
     size_t queue_at = 0, limit_at = 0, state_at = 0;
@@ -962,9 +966,10 @@ struct NttBatch {
 static int batch_prepare(Ctx* c, const NttJob* jobs, size_t count, NttBatch* b) {
     b->jobs.assign(count, {});
     b->scratch_at.assign(count, 0);
-    uint64_t elems = 0;
-    for (size_t j = 0; j < count; j++) elems += 1ull << std::min<uint32_t>(jobs[j].log_n, 28);
-    b->wide = !b->queue && elems >= kWideElems;
+    uint64_t large = 0, small = 0;  // elements
+    for (size_t j = 0; j < count; j++) (jobs[j].log_n >= kWideMinLog ? large : small) += 1ull << std::min<uint32_t>(jobs[j].log_n, 28);
+    b->wide = !b->queue && large >= kWideElems && large >= small;
+    b->alone = !b->queue && large + small < kWideElems;
     std::vector<NttPlan*> plans(count, nullptr);
     for (size_t j = 0; j < count; j++) {
         const NttJob& J = jobs[j];
@@ -973,7 +978,7 @@ static int batch_prepare(Ctx* c, const NttJob* jobs, size_t count, NttBatch* b) 
         ZK_CHECK_ARG(J.omega != nullptr, "null omega");
         std::lock_guard<std::mutex> g(c->mu);
         static const uint8_t one[32] = {1};
-        if ((rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, b->alone(), b->wide,
+        if ((rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, b->alone, b->wide,
                            &plans[j])) != ZK_OK)
             return rc;
         b->scratch_at[j] = b->scratch_elems;
@@ -1001,7 +1006,7 @@ static int batch_layout(const NttJob* jobs, size_t count, NttBatch* b, Ctx* c) {
         {
             std::lock_guard<std::mutex> g(c->mu);
             static const uint8_t one[32] = {1};
-            int rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, b->alone(), b->wide, &plan);
+            int rc = get_plan(c, J.mode, J.log_n, J.omega, J.shift ? J.shift : one, b->alone, b->wide, &plan);
             if (rc != ZK_OK) return rc;
         }
         const uint64_t n = 1ull << J.log_n;
