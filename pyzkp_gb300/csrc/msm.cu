@@ -41,12 +41,14 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <optional>
 #include <string>
 #include <thread>
 #include <tuple>
 #include <type_traits>
 #include <vector>
 
+#include "host_pool.hpp"
 #include "zk_internal.cuh"
 
 namespace zk {
@@ -2040,145 +2042,6 @@ static int pipe_enqueue(Ctx* c, MsmPipeT<C>& p, int scalars_mont, bool upload) {
     return rc;
 }
 
-// A persistent pool of host threads for the combination step (created on first use,
-// never destroyed: its threads sleep between jobs). run() executes fn(0 .. count-1) on the
-// calling thread and on at most count - 1 woken workers, and returns when every task is
-// done -- not when every worker has woken: a late worker finds no task left and sleeps
-// again. Tasks are claimed from one atomic ticket (generation | count | next index), so a
-// worker can only claim a task of the run in progress; calls are serialised.
-class HostPool {
-   public:
-    static HostPool& get() {
-        static HostPool* pool = new HostPool();
-        return *pool;
-    }
-
-    void run(size_t count, const std::function<void(size_t)>& fn) {
-        // no helper: no shared state, no lock; and a few tasks do not wait for a run that itself still
-        // waits for its data
-        if (count == 1 || workers_ == 0 || (count <= 16 && early())) {
-            for (size_t i = 0; i < count; i++) fn(i);
-            return;
-        }
-        run_with(count, fn, [] {});
-    }
-
-    // Whether the run in progress was started before its data (see run_with).
-    bool early() const { return early_.load(std::memory_order_acquire); }
-
-    // run() in which the calling thread first executes own(): own() may take tasks itself
-    // through run_one() (the same ticket, so in the same index order as the workers), e.g.
-    // to consume results in order and compute whichever no worker has taken yet. early: own()
-    // first waits for the tasks' data and the tasks wait for own() to say so, so that the
-    // workers are awake by then. only_if_free: returns false, having done nothing, if another
-    // run is in progress.
-    template <class Own>
-    bool run_with(size_t count, const std::function<void(size_t)>& fn, Own&& own, size_t max_helpers = ~size_t(0),
-                  bool early = false, bool only_if_free = false) {
-        if (count > kMaxTasks) {
-            for (size_t i = 0; i < count; i++) fn(i);
-            own();
-            return true;
-        }
-        if (count == 0) {
-            own();
-            return true;
-        }
-        std::unique_lock<std::mutex> serial(run_mu_, std::defer_lock);
-        if (only_if_free) {
-            if (!serial.try_lock()) return false;
-        } else {
-            serial.lock();
-        }
-        early_.store(early, std::memory_order_release);
-        gen_ = (gen_ + 1) & 0xffffu;
-        fn_ = &fn;
-        done_.store(0, std::memory_order_relaxed);
-        ticket_.store(gen_ << 48 | (uint64_t)count << 24, std::memory_order_release);
-        const size_t helpers = std::min(std::min(count - 1, workers_), max_helpers);
-        if (helpers > 0) {
-            // the caller wakes up to kFanout workers and each woken worker up to kFanout more
-            // (a wake-up is a system call of a few microseconds: a tree of them instead of a
-            // row on the caller)
-            const size_t first = std::min(helpers, kFanout);
-            pending_.store((int64_t)(helpers - first), std::memory_order_relaxed);
-            {
-                std::lock_guard<std::mutex> g(mu_);
-                wake_++;
-            }
-            for (size_t i = 0; i < first; i++) cv_.notify_one();
-        }
-        own();
-        work();
-        // the tasks still running were claimed by awake workers; the wait re-checks every
-        // millisecond, so even a lost wakeup of the condition variable only costs that much
-        std::unique_lock<std::mutex> g(mu_);
-        while (done_.load(std::memory_order_acquire) < count)
-            done_cv_.wait_for(g, std::chrono::milliseconds(1),
-                              [&] { return done_.load(std::memory_order_acquire) >= count; });
-        early_.store(false, std::memory_order_release);
-        return true;
-    }
-
-    // Claim and run the next task of the run in progress; false if none is left.
-    bool run_one() {
-        for (;;) {
-            uint64_t cur = ticket_.load(std::memory_order_acquire);
-            const uint64_t count = (cur >> 24) & kMaxTasks, i = cur & kMaxTasks;
-            if (i >= count) return false;
-            if (!ticket_.compare_exchange_weak(cur, cur + 1, std::memory_order_acq_rel)) continue;
-            (*fn_)(i);
-            if (done_.fetch_add(1, std::memory_order_acq_rel) + 1 == count) {
-                std::lock_guard<std::mutex> g(mu_);
-                done_cv_.notify_all();
-            }
-            return true;
-        }
-    }
-
-   private:
-    static constexpr size_t kMaxTasks = (1u << 24) - 1;
-
-    HostPool() {
-        const size_t hw = std::max<size_t>(1, std::thread::hardware_concurrency());
-        workers_ = std::min<size_t>(hw, 16) - 1;
-        for (size_t i = 0; i < workers_; i++) std::thread([this] { loop(); }).detach();
-    }
-
-    void loop() {
-        uint64_t seen = 0;
-        for (;;) {
-            {
-                std::unique_lock<std::mutex> g(mu_);
-                cv_.wait(g, [&] { return wake_ != seen; });
-                seen = wake_;
-            }
-            for (size_t i = 0; i < kFanout; i++)
-                if (pending_.fetch_sub(1, std::memory_order_acq_rel) > 0) cv_.notify_one();
-            work();
-        }
-    }
-
-    // Claim and run tasks while the ticket has some left. A successful claim of task i means
-    // the run that published the ticket is still waiting for task i, so fn_ is its function.
-    void work() {
-        while (run_one()) {
-        }
-    }
-
-    size_t workers_ = 0;
-    std::mutex run_mu_, mu_;
-    std::condition_variable cv_, done_cv_;
-    const std::function<void(size_t)>* fn_ = nullptr;
-    std::atomic<uint64_t> ticket_{0};
-    std::atomic<size_t> done_{0};
-    std::atomic<bool> early_{false};   // the run in progress was started before its data (run_with)
-    std::atomic<int64_t> pending_{0};  // wake-ups the woken workers still have to pass on
-    static constexpr size_t kFanout = 2;
-    uint64_t wake_ = 0;  // under mu_
-    uint64_t gen_ = 0;   // under run_mu_
-};
-
 // Host: the sum S_w of window (or set) w of instance k from its targets: S_w = g (T_Y + H) + T_E
 // with T_Y = sum Y, H = sum_k 2^k M_k (Horner) and, for g > 1, T_E = sum E (target 0).
 template <class C>
@@ -2221,19 +2084,20 @@ static void horner_out(const MsmPipeT<C>& p, Get&& get, uint8_t* out_xy, int32_t
 #endif
 static constexpr size_t kCombineHelpers = ZK_COMBINE_HELPERS;  // pool workers of a one-instance combine
 
+// CSR entries of a pipeline up to which a single MSM wakes its helpers early (~0.5 ms of device
+// time at 2 M), and how long these stay awake at most: the stream may hold other work before this
+// call's.
+static constexpr uint64_t kEarlyEntries = 1u << 21;
+static constexpr std::chrono::microseconds kEarlyLimit{4000};
+
 // Combine every instance of `pipes`: the window sums of all instances in parallel on the
 // host pool, then each instance's Horner (in parallel across instances); a single instance
 // overlaps its Horner with its window sums.
-// CSR entries of a pipeline up to which a single MSM wakes its helpers early (~0.5 ms of device
-// time at 2 M).
-static constexpr uint64_t kEarlyEntries = 1u << 21;
-
-// `wait` (optional) waits for the device to have written the targets; its error is returned. A
-// single instance calls it with the pool's helpers already woken: a wake-up takes 10 - 20 us,
-// as long as two or three window sums.
+// `wait` (optional) waits for the device to have written the targets; its error is returned. early:
+// a single instance wakes the pool's helpers before that.
 template <class C>
 static int combine_all(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, uint8_t* out_xy, int32_t* out_is_inf,
-                       bool record = true, const std::function<int()>& wait = nullptr) {
+                       bool record = true, const std::function<int()>& wait = nullptr, bool early = false) {
     using H = typename HostOf<C>::T;
     constexpr size_t kOut = 2 * sizeof(H);  // bytes of one affine result
     auto t0 = std::chrono::steady_clock::now();
@@ -2259,44 +2123,28 @@ static int combine_all(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, uint8_t* o
         const MsmPipeT<C>& p = pipes[insts[0].q];
         const uint32_t k = insts[0].k, W = (uint32_t)win.size();
         std::unique_ptr<std::atomic<uint32_t>[]> ready(new std::atomic<uint32_t>[W]());
-        std::atomic<int> data{wait ? 0 : 1};  // 0: not there yet, 1: there, 2: it will not come
-        int rc = ZK_OK;
         const std::function<void(size_t)> task = [&](size_t t) {
-            int d;
-            while ((d = data.load(std::memory_order_acquire)) == 0) std::this_thread::yield();
-            if (d == 1) sums[t] = window_sum<C>(p, k, W - 1 - (uint32_t)t);
+            sums[t] = window_sum<C>(p, k, W - 1 - (uint32_t)t);
             ready[t].store(1, std::memory_order_release);
-        };
-        auto wait_data = [&] {
-            if (data.load(std::memory_order_relaxed) != 0) return;
-            rc = wait();
-            t0 = std::chrono::steady_clock::now();
-            data.store(rc == ZK_OK ? 1 : 2, std::memory_order_release);
         };
         const size_t o = p.out_index[k];
         // a few helpers keep ahead of the Horner (a window sum costs about as much as 2-3
         // windows of its doublings)
         auto own = [&] {
-            wait_data();
-            if (rc != ZK_OK) return;
             horner_out<C>(p, [&](uint32_t w) -> const zkh::XyzzT<H>& {
                 const uint32_t t = W - 1 - w;
+                // a window that a worker is on comes sooner than this thread would be through another one
                 while (!ready[t].load(std::memory_order_acquire))
-                    if (!pool.run_one()) std::this_thread::yield();  // a worker is on it
+                    if (pool.claimed(t) || !pool.run_one()) std::this_thread::yield();
                 return sums[t];
             }, out_xy + kOut * o, out_is_inf + o);
         };
-        if (!pool.run_with(W, task, own, kCombineHelpers, wait != nullptr, true)) {
-            wait_data();
-            if (rc == ZK_OK && pool.early()) {  // another thread's run still waits for its device: do without the pool
-                for (uint32_t t = 0; t < W; t++) task(t);
-                horner_out<C>(p, [&](uint32_t w) -> const zkh::XyzzT<H>& { return sums[W - 1 - w]; }, out_xy + kOut * o,
-                              out_is_inf + o);
-            } else if (rc == ZK_OK) {
-                pool.run_with(W, task, own, kCombineHelpers);
-            }
-        }
-        if (rc != ZK_OK) return rc;
+        std::optional<HostPool::Expect> awake;
+        if (early) awake.emplace(pool, kCombineHelpers, kEarlyLimit);
+        if (wait)
+            if (const int rc = wait(); rc != ZK_OK) return rc;
+        t0 = std::chrono::steady_clock::now();
+        pool.run_with(W, task, own, kCombineHelpers);
     } else {
         if (wait)
             if (const int rc = wait(); rc != ZK_OK) return rc;
@@ -2733,11 +2581,9 @@ static int batch_run(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mont,
         ZK_TRY_CUDA(cudaStreamSynchronize(c->stream));
         return queue ? queue_check(queue_status) : ZK_OK;
     };
-    // helpers woken before the device is done, where that is soon (they wait awake)
-    if (pipes.size() == 1 && pipes[0].max_entries <= kEarlyEntries)
-        return combine_all<C>(c, pipes, out_xy, out_is_inf, true, wait);
-    if ((rc = wait()) != ZK_OK) return rc;
-    return combine_all<C>(c, pipes, out_xy, out_is_inf);
+    // helpers woken before the device is done, where that is soon
+    const bool early = pipes.size() == 1 && pipes[0].max_entries <= kEarlyEntries;
+    return combine_all<C>(c, pipes, out_xy, out_is_inf, true, wait, early);
 }
 
 // ---- asynchronous batches: the device part is enqueued and the call returns; a worker
