@@ -30,27 +30,19 @@ void scratch_free(Ctx* c, void* p) {
     if (p) cudaFreeAsync(p, c->stream);
 }
 
-int pinned_take(Ctx* c, size_t bytes, void** p, size_t* got) {
-    {
-        std::lock_guard<std::mutex> g(c->pinned_mu);
-        auto it = c->pinned_free.lower_bound(bytes);
-        // reuse a block of up to 4x the size asked for; a larger one stays for larger asks
-        if (it != c->pinned_free.end() && it->first <= 4 * bytes + 4096) {
-            *p = it->second;
-            *got = it->first;
-            c->pinned_free.erase(it);
-            return ZK_OK;
-        }
-    }
-    ZK_TRY_CUDA(cudaMallocHost(p, bytes ? bytes : 16));
-    *got = bytes ? bytes : 16;
+int pinned_take(Ctx* c, size_t bytes, void** p) {
+    cudaError_t e = cudaSuccess;
+    *p = c->pinned.take(bytes, [&](size_t size) {
+        void* block = nullptr;
+        e = cudaMallocHost(&block, size);
+        return e == cudaSuccess ? block : nullptr;
+    });
+    ZK_TRY_CUDA(e);
     return ZK_OK;
 }
 
 void pinned_give(Ctx* c, void* p, size_t bytes) {
-    if (p == nullptr) return;
-    std::lock_guard<std::mutex> g(c->pinned_mu);
-    c->pinned_free.emplace(bytes, p);
+    c->pinned.give(p, bytes, [](void* block) { cudaFreeHost(block); });
 }
 
 static cudaEvent_t take_event(Ctx* c) {
@@ -172,6 +164,10 @@ int zk_ctx_create_prio(int device, int priority, zk_ctx** out) {
         uint64_t threshold = UINT64_MAX;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
     }
+    // the result block of single MSMs, so that a context's first call does not allocate it
+    void* block = nullptr;
+    if (zk::pinned_take(&c->impl, 1, &block) == ZK_OK) zk::pinned_give(&c->impl, block, 1);
+    else cudaGetLastError();  // that call will report it
     *out = c.release();
     return ZK_OK;
 }
@@ -227,7 +223,7 @@ int zk_ctx_destroy(zk_ctx* ctx) {
             if (ev) cudaEventDestroy(ev);
     }
     if (ctx->impl.ntt_queue_err) cudaFree(ctx->impl.ntt_queue_err);
-    for (auto& kv : ctx->impl.pinned_free) cudaFreeHost(kv.second);
+    ctx->impl.pinned.clear([](void* block) { cudaFreeHost(block); });
     cudaStreamDestroy(ctx->impl.stream);
     delete ctx;
     return ZK_OK;

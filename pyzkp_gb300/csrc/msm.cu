@@ -2526,7 +2526,10 @@ struct PinnedBlock {
     size_t bytes = 0;
     explicit PinnedBlock(Ctx* ctx) : c(ctx) {}
     PinnedBlock(const PinnedBlock&) = delete;
-    int take(size_t n) { return pinned_take(c, n, &p, &bytes); }
+    int take(size_t n) {
+        bytes = n;
+        return pinned_take(c, n, &p);
+    }
     ~PinnedBlock() { pinned_give(c, p, bytes); }
 };
 
@@ -2648,7 +2651,8 @@ static int batch_submit(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mo
     }
     // page-locked host targets and entry totals of each pipeline, then the queue status
     a->ctx = c;
-    if ((rc = pinned_take(c, host_bytes + 16, &a->pinned, &a->pinned_bytes)) != ZK_OK) return rc;
+    a->pinned_bytes = host_bytes + 16;
+    if ((rc = pinned_take(c, a->pinned_bytes, &a->pinned)) != ZK_OK) return rc;
     ZK_TRY_CUDA(cudaEventCreateWithFlags(&a->done_ev, cudaEventDisableTiming));
     char* arena = nullptr;
     if ((rc = scratch_alloc(c, bytes, reinterpret_cast<void**>(&arena))) != ZK_OK) return rc;

@@ -12,6 +12,7 @@
 #include "curve.cuh"
 #include "field.cuh"
 #include "host_field.hpp"
+#include "pinned_pool.hpp"
 
 namespace zk {
 
@@ -155,15 +156,12 @@ struct Ctx {
     // tuning tables (zk_tune_*, zk_autotune_*): 0 means the built-in rule
     uint8_t tune_msm_window[32] = {};    // MSM window bits by ceil(log2 n)
     uint8_t tune_ntt_split[29][4] = {};  // NTT radix bits per pass by log2 n
-    // page-locked result buffers of asynchronous MSM batches, kept for reuse: allocating
-    // and freeing page-locked memory per batch can wait for the whole device
-    std::mutex pinned_mu;
-    std::multimap<size_t, void*> pinned_free;  // size -> block
+    PinnedPool pinned;  // page-locked result blocks of MSM calls and batches
 };
 
-// A page-locked block of at least `bytes` from the context's free list (else a new one of
-// exactly `bytes`; *got = its size); pinned_give returns it. Both are thread-safe.
-int pinned_take(Ctx* c, size_t bytes, void** p, size_t* got);
+// A page-locked block of at least `bytes` from the context's pool; pinned_give returns it. Both
+// are thread-safe.
+int pinned_take(Ctx* c, size_t bytes, void** p);
 void pinned_give(Ctx* c, void* p, size_t bytes);
 
 int prof_begin(Ctx* c, const char* name);
