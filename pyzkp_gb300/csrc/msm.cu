@@ -162,22 +162,29 @@ uint32_t msm_auto_window(size_t n) {
     return (uint32_t)c;
 }
 
-// Window size of the GLV split (halves of ~127 bits), n scalars. Measured on GB300 (G1, n = 2^8 ..
-// 3 * 2^20 in half powers of two, every c from about log2(n) - 6 to log2(n), uniform and
-// witness-like scalars): the table holds the c with the smallest product of the two times
-// relative to their best. Windows that leave the top one sparse (c = 9 uses 2 of its 9 bits,
-// c = 14 2 of 14) crowd a few buckets, and so do repeated small scalars. Against one c per
-// ceil(log2 n) (8, 8, 8, 9, 10, 11, 11, 13, 13, 13, 15 for 2^8 .. 2^18, then 16), us uniform /
-// witness-like: 768 216 / 220 -> 212 / 204, 1536 231 / 220 -> 219 / 219, 3072 236 / 231 -> 231 /
-// 222, 196608 961 / 730 -> 925 / 664, 262144 1147 / 840 -> 1156 / 805.
-uint32_t msm_auto_window_glv(size_t n) {
+// Window size of the GLV split (halves of ~127 bits), n scalars. Measured on GB300 for 70 sizes from
+// 150 to 10^6 (G1; 23 of them G2 too), every c near the best, uniform and witness-like scalars: each
+// line lies between the two sizes where the c with the smallest product of the two times (relative to
+// their best) changes. Two are limits of other rules: 16384 points are the most that sort in one
+// tile a set with c = 11, and above 196608 a bucket of c = 13 holds more than kFixupDensity entries.
+// Windows that leave the top one sparse (c = 9 uses 2 of its 9 bits, c = 14 2 of 14) crowd a few
+// buckets, and so do repeated small scalars. Either side of the lines, us uniform / witness-like,
+// chosen c first: 512 c8 135 / 139, c9 145 / 138; 640 c9 146 / 141, c8 151 / 157; 1024 c9 155 / 143, c10
+// 151 / 149; 1280 c10 154 / 152, c9 165 / 157; 2048 c10 156 / 156, c11 162 / 156; 2560 c11 161 / 157, c10 171
+// / 171; 16384 c11 254 / 226, c13 258 / 238; 20000 c13 277 / 247, c11 295 / 296; 196608 c13 864 / 605, c15
+// 921 / 662; 196700 c15 898 / 661, c13 1025 / 753; 258000 c15 1047 / 742, c14 1090 / 736; 262144 c14 1089
+// / 734, c15 1086 / 778; 285000 c14 1183 / 747, c15 1184 / 753; 290000 c15 1184 / 749, c14 1187 / 824, c16
+// 1191 / 932; 310000 c16 1149 / 860, c15 1192 / 839. In a batch every c in use is a pipeline of its
+// own, and its few sizes of c = 15 go with c = 14: 64 MSMs of 2^10 .. 2^20 28.03 ms, 28.23 with 15.
+uint32_t msm_auto_window_glv(size_t n, bool batch) {
     static const struct {
         size_t upto;
         uint32_t c;
-    } kMeasured[] = {{640, 8}, {1280, 9}, {2560, 10}, {20000, 11}, {229376, 13}, {280000, 14}};
+    } kMeasured[] = {{575, 8},     {1100, 9},    {2300, 10},   {16384, 11}, {196608, 13},
+                     {260000, 15}, {287000, 14}, {298000, 15}};
     if (n > 128) {
         for (const auto& m : kMeasured)
-            if (n <= m.upto) return m.c;
+            if (n <= m.upto) return batch && m.c == 15 ? 14u : m.c;
         return 16;
     }
     uint32_t c = msm_auto_window(n);
@@ -1624,11 +1631,11 @@ static zkh::XyzzT<typename HostOf<C>::T> to_host(const typename C::P& d) {
     return h;
 }
 
-uint32_t msm_window_for(const Ctx* c, size_t n, bool glv) {
+uint32_t msm_window_for(const Ctx* c, size_t n, bool glv, bool batch) {
     uint32_t lg = 0;
     while ((1ull << lg) < n) lg++;
     if (lg < sizeof(c->tune_msm_window) && c->tune_msm_window[lg] != 0) return c->tune_msm_window[lg];
-    return glv ? msm_auto_window_glv(n) : msm_auto_window(n);
+    return glv ? msm_auto_window_glv(n, batch) : msm_auto_window(n);
 }
 
 // One pipeline: MSM instances with the same window size and mode, sharing every launch.
@@ -2190,7 +2197,7 @@ static int build_pipes(Ctx* c, const MsmJob* jobs, size_t count, uint32_t window
         }
         const bool fixed = b.shifted != nullptr && (window_bits == 0 || window_bits == b.shifted_c);
         const bool glv = !fixed && b.glv;  // fixed-base rows hold P only (plain 255-bit windows)
-        const uint32_t cb = fixed ? b.shifted_c : (window_bits ? window_bits : msm_window_for(c, b.n, glv));
+        const uint32_t cb = fixed ? b.shifted_c : window_bits ? window_bits : msm_window_for(c, b.n, glv, count > 1);
         groups[std::make_tuple(cb, fixed, glv)].push_back(j);
     }
     for (auto& kv : groups) {

@@ -270,8 +270,8 @@ struct MsmJob {
 };
 struct MsmPlan;
 uint32_t msm_auto_window(size_t n);
-uint32_t msm_auto_window_glv(size_t n);
-uint32_t msm_window_for(const Ctx* c, size_t n, bool glv = false);
+uint32_t msm_auto_window_glv(size_t n, bool batch = false);
+uint32_t msm_window_for(const Ctx* c, size_t n, bool glv = false, bool batch = false);
 int msm_batch_run(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mont, uint32_t window_bits, uint8_t* out_xy,
                   int32_t* out_is_inf);
 // G2: out_xy holds 128 bytes per instance (x.c0, x.c1, y.c0, y.c1); no fixed-base mode
