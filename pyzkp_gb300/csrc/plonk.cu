@@ -17,7 +17,7 @@
 //   zh_i  = shift_n u^i - 1
 // One thread per `chunk` points, 32 apart (a warp covers 32 * chunk consecutive points, so
 // its loads are contiguous), the powers of omega_m and u carried from the thread's first
-// point (computed by square-and-multiply) in steps of omega_m^32 and u^32.
+// point (from tables) in steps of omega_m^32 and u^32.
 #include <cstring>
 #include <vector>
 
@@ -154,14 +154,14 @@ __global__ void plonk_quotient_kernel(QuotientIn in, QuotientK K, size_t m, uint
     fe x = fe_mul<FrQ>(fe_mul<FrQ>(fe_ldg(pw + lane), fe_ldg(pw + 64 + glo)), fe_ldg(pw + 192 + ghi));
     x = fe_mul<FrQ>(K.shift, x);
     fe un = fe_mul<FrQ>(fe_mul<FrQ>(fe_ldg(pw + 32 + lane), fe_ldg(pw + 128 + glo)), fe_ldg(pw + 192 + H + ghi));
-    // vectors of a caller as first factors of products (see fe_mul)
+    // the vectors of a caller that are first factors of products (see fe_mul)
     auto first = [](const fe* v) { return sos_reduce_2p<FrQ>(fe_ldg(v)); };
     for (size_t i = i0, k = 0; k < chunk && i < m; k++, i += 32) {
         const fe a = first(in.v[0] + i), b = first(in.v[1] + i), c = first(in.v[2] + i);
         const fe z = first(in.v[3] + i);
-        fe gate = fe_add<FrQ>(fe_mul<FrQ>(first(in.v[5] + i), a), fe_mul<FrQ>(first(in.v[6] + i), b));
-        gate = fe_add<FrQ>(gate, fe_mul<FrQ>(fe_mul<FrQ>(first(in.v[7] + i), a), b));
-        gate = fe_add<FrQ>(gate, fe_mul<FrQ>(first(in.v[8] + i), c));
+        fe gate = fe_add<FrQ>(fe_mul<FrQ>(a, fe_ldg(in.v[5] + i)), fe_mul<FrQ>(b, fe_ldg(in.v[6] + i)));
+        gate = fe_add<FrQ>(gate, fe_mul<FrQ>(fe_mul<FrQ>(a, fe_ldg(in.v[7] + i)), b));
+        gate = fe_add<FrQ>(gate, fe_mul<FrQ>(c, fe_ldg(in.v[8] + i)));
         gate = fe_add<FrQ>(gate, fe_add<FrQ>(fe_ldg(in.v[9] + i), fe_ldg(in.v[4] + i)));
         const fe t1 = fe_add<FrQ>(fe_add<FrQ>(a, fe_mul<FrQ>(K.beta, x)), K.gamma);
         const fe t2 = fe_add<FrQ>(fe_add<FrQ>(b, fe_mul<FrQ>(K.beta_k1, x)), K.gamma);
