@@ -162,8 +162,8 @@ uint32_t msm_auto_window(size_t n) {
     return (uint32_t)c;
 }
 
-// Window size of the GLV split (halves of ~127 bits), n scalars. Measured on GB300 for 70 sizes from
-// 150 to 10^6 (G1; 23 of them G2 too), every c near the best, uniform and witness-like scalars: each
+// Window size of the GLV split (halves of ~127 bits), n scalars. Measured on GB300 for 71 sizes from
+// 150 to 10^6 (G1; 33 for G2), every c near the best, uniform and witness-like scalars: each
 // line lies between the two sizes where the c with the smallest product of the two times (relative to
 // their best) changes. Two are limits of other rules: 16384 points are the most that sort in one
 // tile a set with c = 11, and above 196608 a bucket of c = 13 holds more than kFixupDensity entries.
@@ -174,18 +174,24 @@ uint32_t msm_auto_window(size_t n) {
 // / 171; 16384 c11 254 / 226, c13 258 / 238; 20000 c13 277 / 247, c11 295 / 296; 196608 c13 864 / 605, c15
 // 921 / 662; 196700 c15 898 / 661, c13 1025 / 753; 258000 c15 1047 / 742, c14 1090 / 736; 262144 c14 1089
 // / 734, c15 1086 / 778; 285000 c14 1183 / 747, c15 1184 / 753; 290000 c15 1184 / 749, c14 1187 / 824, c16
-// 1191 / 932; 310000 c16 1149 / 860, c15 1192 / 839. In a batch every c in use is a pipeline of its
-// own, and its few sizes of c = 15 go with c = 14: 64 MSMs of 2^10 .. 2^20 28.03 ms, 28.23 with 15.
+// 1191 / 932; 310000 c16 1149 / 860, c15 1192 / 839.
+//
+// A batch has lines of its own: there the sum of the work counts and not one chain, and every c in
+// use is a pipeline. Ten MSMs of 6171 .. 72329 points with c = 11 / 13 for the one of 18427: 1.50 / 1.57
+// ms; 64 of 2^10 .. 2^20 28.03 ms, 28.23 with c = 15 as well.
 uint32_t msm_auto_window_glv(size_t n, bool batch) {
-    static const struct {
+    struct Line {
         size_t upto;
         uint32_t c;
-    } kMeasured[] = {{575, 8},     {1100, 9},    {2300, 10},   {16384, 11}, {196608, 13},
-                     {260000, 15}, {287000, 14}, {298000, 15}};
+    };
+    static const Line kOne[] = {{575, 8},     {1100, 9},    {2300, 10},   {16384, 11}, {196608, 13},
+                                {260000, 15}, {287000, 14}, {298000, 15}, {~size_t(0), 16}};
+    static const Line kBatch[] = {{640, 8},     {1280, 9},    {2560, 10},        {20000, 11},
+                                  {229376, 13}, {280000, 14}, {~size_t(0), 16}};
     if (n > 128) {
-        for (const auto& m : kMeasured)
-            if (n <= m.upto) return batch && m.c == 15 ? 14u : m.c;
-        return 16;
+        const Line* l = batch ? kBatch : kOne;
+        while (n > l->upto) l++;
+        return l->c;
     }
     uint32_t c = msm_auto_window(n);
     while (c > 4 && (128 + c - 2) / (c - 1) == (128 + c - 1) / c) c--;
