@@ -1666,7 +1666,9 @@ struct MsmPipeT {
     P *slot_pts_a = nullptr, *slot_pts_b = nullptr;
     uint32_t *long_list = nullptr, *long_count = nullptr;  // fixup mode
     P *buckets = nullptr, *Yb = nullptr, *Eb = nullptr;  // Yb: the buckets themselves when g = 1
-    P *lines = nullptr, *tgt = nullptr;
+    P *lines = nullptr;
+    bool queued = false;  // the later stages run in the work queue: targets in device memory first
+    P* tgt = nullptr;
     // tiled CSR sort (B <= kTiledMaxB): set positions, tiles and per-tile bucket counts
     bool tiled = false;
     uint32_t te = 0, tiles = 0;
@@ -1799,7 +1801,7 @@ static size_t pipe_layout(MsmPipeT<C>& p, char* base) {
     p.Yb = sh.g > 1 ? reinterpret_cast<P*>(take((size_t)sh.sets * sh.G * sizeof(P))) : p.buckets;
     p.Eb = sh.g > 1 ? reinterpret_cast<P*>(take((size_t)sh.sets * sh.G * sizeof(P))) : nullptr;
     p.lines = reinterpret_cast<P*>(take((size_t)sh.sets * lines_per_set(sh) * sizeof(P)));
-    p.tgt = reinterpret_cast<P*>(take(p.host_elems() * sizeof(P)));
+    p.tgt = p.queued ? reinterpret_cast<P*>(take(p.host_elems() * sizeof(P))) : nullptr;
     if (p.tiled) p.tile_hist = reinterpret_cast<uint32_t*>(take((size_t)p.tiles * sh.B * 4));
     return off;
 }
@@ -2190,7 +2192,7 @@ static int combine_all(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, uint8_t* o
 // Group jobs into pipelines: one per (window bits, fixed-base mode, GLV), split where a
 // group would exceed the 31-bit point / 32-bit entry limits.
 template <class C>
-static int build_pipes(Ctx* c, const MsmJob* jobs, size_t count, uint32_t window_bits,
+static int build_pipes(Ctx* c, const MsmJob* jobs, size_t count, uint32_t window_bits, bool queued,
                        std::vector<MsmPipeT<C>>* out, std::vector<size_t>* empty) {
     ZK_CHECK_ARG(window_bits == 0 || (window_bits >= 4 && window_bits <= 20), "window_bits must be 0 or 4..20");
     std::map<std::tuple<uint32_t, bool, bool>, std::vector<size_t>> groups;
@@ -2219,6 +2221,7 @@ static int build_pipes(Ctx* c, const MsmJob* jobs, size_t count, uint32_t window
             if (part.empty()) return ZK_OK;
             out->emplace_back();
             int rc = pipe_init<C>(out->back(), cb, fixed, glv, part, idx, c->num_sms);
+            out->back().queued = queued;
             // the sort kernels' shared-memory limit, set here and not inside a graph capture
             if (rc == ZK_OK && out->back().tiled) rc = set_sort_smem_attr(c->device);
             out->back().skip_inf = part_inf;
@@ -2551,7 +2554,7 @@ static int batch_run(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mont,
                      int32_t* out_is_inf) {
     std::vector<MsmPipeT<C>> pipes;
     std::vector<size_t> empty;
-    int rc = build_pipes<C>(c, jobs, count, window_bits, &pipes, &empty);
+    int rc = build_pipes<C>(c, jobs, count, window_bits, c->msm_queue && kQueueForm<C>, &pipes, &empty);
     if (rc != ZK_OK) return rc;
     set_infinity(out_xy, out_is_inf, empty, 2 * sizeof(typename HostOf<C>::T));
     if (pipes.empty()) return ZK_OK;
@@ -2640,7 +2643,7 @@ static int batch_submit(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mo
                         uint8_t* out_xy, int32_t* out_is_inf, MsmAsync** out) {
     std::unique_ptr<MsmAsyncT<C>> a(new MsmAsyncT<C>());
     std::vector<size_t> empty;
-    int rc = build_pipes<C>(c, jobs, count, window_bits, &a->pipes, &empty);
+    int rc = build_pipes<C>(c, jobs, count, window_bits, c->msm_queue && kQueueForm<C>, &a->pipes, &empty);
     if (rc != ZK_OK) return rc;
     set_infinity(out_xy, out_is_inf, empty, 2 * sizeof(typename HostOf<C>::T));
     if (a->pipes.empty()) {
@@ -2787,7 +2790,7 @@ int msm_plan_create(Ctx* c, const MsmJob* jobs, size_t count, int scalars_mont, 
     std::unique_ptr<MsmPlan> plan(new MsmPlan());
     plan->count = count;
     plan->scalars_mont = scalars_mont;
-    int rc = build_pipes<CurveG1>(c, jobs, count, window_bits, &plan->pipes, &plan->empty);
+    int rc = build_pipes<CurveG1>(c, jobs, count, window_bits, queue, &plan->pipes, &plan->empty);
     if (rc != ZK_OK) return rc;
     if (queue && !plan->pipes.empty()) {
         plan->queue.reset(new MsmQueueT<CurveG1>());
