@@ -230,10 +230,10 @@ def run_gpu(args, ranks: Ranks) -> dict:
     acc_launches, acc_ms = table.get("msm_accumulate", (1, 0.0))
     acc_ms_launch = acc_ms / max(1, acc_launches)
     entries = stats["entries"]
-    # algorithmic work of one accumulate launch: one XYZZ mixed addition (8M + 2S = 10 Fq
-    # multiplications) per CSR entry; a Montgomery multiplication with 8 limbs is 2*8^2 + 8 = 136
-    # 32x32->64 multiply-accumulates, i.e. 272 IMAD (lo + hi) instructions.
-    acc_imad = entries * 10 * 272
+    # work of one accumulate launch: one XYZZ mixed addition per CSR entry, 32x32->64 multiply-adds as
+    # executed (6 products of 128, a product pair with one reduction of 192, two squares of 100),
+    # counted as two IMAD (lo + hi) each
+    acc_imad = entries * ACC_WIDE * 2
     acc_tops = acc_imad / (acc_ms_launch * 1e-3) / 1e12
     # algorithmic bytes: per entry the 4-byte CSR entry + the 64-byte affine base
     acc_bytes = entries * 68
@@ -246,11 +246,10 @@ def run_gpu(args, ranks: Ranks) -> dict:
         "peak": round(imad_tops, 3),
         "unit": "T IMAD/s",
         "frac": round(acc_tops / imad_tops, 4),
-        "peak_source": ("measured in this run (no IMAD figure in MEASURED_PEAKS.json): the fastest rate of "
-                        "32x32->64 multiply-accumulates, as lo+hi pairs (harmonic mean of the mad.lo and mad.hi "
-                        "probes) or as mad.wide, counted as 2 IMAD each like the algorithmic work"),
+        "peak_source": ("SMs x maximum SM clock x 64 32-bit integer multiply-adds per clock (CUDA throughput table, "
+                        "compute capability 10.x); a 32x32->64 one counts as two, as in the work: 4 cycles of a "
+                        "quarter SM's pipe per warp, as ncu's pipe counters show"),
         "imad_probes_T_per_s": imad_probes,
-        "peak_model": imad_model(ctx, acc_tops),
         "launch_ms": round(acc_ms_launch, 4),
         "share_of_step": round(acc_ms / max(1e-9, sum(v[1] for v in table.values())), 4),
         "traffic": traffic_of("msm_accumulate", log_n),
@@ -258,7 +257,7 @@ def run_gpu(args, ranks: Ranks) -> dict:
         "hbm": {"achieved": round(acc_bytes / (acc_ms_launch * 1e-3) / 1e9, 1), "peak": hbm_peak,
                 "unit": "GB/s", "frac": round(acc_bytes / (acc_ms_launch * 1e-3) / 1e9 / hbm_peak, 4),
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks.get("hbm_gbs") else "fallback 6800"},
-        "algorithmic_work": f"{entries} CSR entries x 10 Fq mults x 272 IMAD; {entries} x 68 B",
+        "algorithmic_work": f"{entries} CSR entries x {ACC_WIDE} wide multiply-adds (2 IMAD each); {entries} x 68 B",
         "whole_msm_model": msm_model(n, total_ms / args.steps, imad_tops),
         "sort_kernels": sort_kernels(table, prof_steps, n, entries, hbm_peak),
     }
@@ -433,11 +432,9 @@ def run_gpu_ntt(ctx, args, ranks, log_n, flush, imad_tops, hbm_peak, brief=False
     ctx.prof_reset()
     passes = la // 3
     pass_ms = ms / max(1, la)
-    # per pass: every element read once and written once (64 B); radix-2 work of log2(R) stages,
-    # (n/2) log2(R) butterflies of one Montgomery multiplication (136 wide MACs = 272 IMAD)
-    log_r = log_n / max(1, passes)
+    # per pass: every element read once and written once (64 B); the products as executed
     pass_bytes = 64 * n
-    pass_imad = (n / 2) * log_r * 272
+    pass_imad = n * ntt_imad(log_n, passes) / max(1, passes)
     gbs = pass_bytes / (pass_ms * 1e-3) / 1e9
     tops = pass_imad / (pass_ms * 1e-3) / 1e12
     out["roofline"] = {"kernel": "ntt_pass", "bound": "imad", "achieved": round(tops, 3), "peak": round(imad_tops, 3),
@@ -449,7 +446,9 @@ def run_gpu_ntt(ctx, args, ranks, log_n, flush, imad_tops, hbm_peak, brief=False
                                          "peak": hbm_peak, "unit": "GB/s",
                                          "frac": round(64 * n / (passes * pass_ms * 1e-3) / 1e9 / hbm_peak, 4),
                                          "per": "transform (64 B/element in and out once, over all passes)"},
-                       "algorithmic_work": "per pass 64 B/element; (n/2) log2(R) butterflies x 272 IMAD"}
+                       "algorithmic_work": f"per pass 64 B/element; {ntt_imad(log_n, passes):.0f} IMAD/element over all passes "
+                                           "(radix-8 steps or radix-2 stages of constant products, and the factors "
+                                           "between passes)"}
     if not brief:
         # e2e: canonical host input -> device, to Montgomery, NTT, back to canonical, device -> host
         pin_in = ctx.pinned(n * 32)
@@ -610,6 +609,30 @@ def sort_kernels(table: dict, steps: int, n: int, entries: int, hbm_peak: float)
     return out
 
 
+ACC_WIDE = 6 * 128 + 192 + 2 * 100  # 32x32->64 multiply-adds of one mixed addition, as the accumulation executes it
+
+
+def ntt_imad(log_n: int, passes: int) -> float:
+    """IMAD per element that a lone forward transform executes: products with a known constant
+    (99 wide and 16 low multiply-adds) in its radix-8 steps (5 + 7 per 8 elements, the 7 where
+    offsets are left; a radix-4 rest 1 per 4) or, below 2^18, radix-2 stages (1 per 2 elements);
+    a full product (128 wide, 2 low) per element between passes."""
+    const, full = 99 * 2 + 16, 128 * 2 + 2
+    total = 0.0
+    for p in range(passes):
+        lr = log_n // passes + (1 if p < log_n % passes else 0)
+        if log_n < 18:
+            total += lr / 2 * const
+        else:
+            rest = lr
+            while rest >= 3:
+                total += (12 if rest > 3 else 5) / 8 * const
+                rest -= 3
+            total += const / 4 if rest == 2 else 0
+        total += full if p else 0
+    return total
+
+
 def msm_model(n: int, ms: float, imad_tops: float) -> dict:
     """Implementation-independent work of a whole G1 MSM of n points: with the window c* that
     minimises the model (not the implementation's window), W = ceil(255/c*),
@@ -625,38 +648,22 @@ def msm_model(n: int, ms: float, imad_tops: float) -> dict:
             "frac": round(tops / imad_tops, 4), "ms": round(ms, 4)}
 
 
-def imad_model(ctx, achieved_tops: float) -> dict:
-    """The denominator checked without the probe: SMs x SM clock x the nominal 64 32-bit
-    integer multiply-adds per clock per SM (the CUDA throughput table for compute capability
-    10.x). The probe's mad.wide rate counted as 2 IMAD per wide product exceeds it (about 82
-    per clock per SM: its product does not change over the loop), so the probe's peak is the
-    stricter denominator and the one used. The algorithmic count keeps 10 full products (1360 wide
-    multiply-adds) per entry; the accumulation executes 1160, so it may read above 1 here."""
-    sms = ctx.num_sms()
-    mhz = None
+def imad_peak(ctx):
+    """(probes, peak) of the integer multiply-add pipe in 10^12 IMAD/s (a wide multiply-add = 2
+    IMAD). The peak is the nominal 64 per clock per SM: the probes' single forms (mad.hi, carry
+    chains) stay below it, and mad.wide with factors that do not change reads above."""
+    pr = {"carry_chain": ctx.imad_probe(0), "mad_lo": ctx.imad_probe(1), "mad_hi": ctx.imad_probe(2),
+          "mad_wide_as_2": ctx.imad_probe(3)}
+    mhz = 2070.0
     try:
         import subprocess
 
         out = subprocess.run(["nvidia-smi", "--query-gpu=clocks.max.sm", "--format=csv,noheader,nounits", "-i", "0"],
                              capture_output=True, text=True, timeout=10).stdout.strip().splitlines()
-        mhz = float(out[0]) if out else None
-    except Exception:  # noqa: BLE001 -- no nvidia-smi: the model is left out
-        mhz = None
-    if not mhz:
-        return {"note": "SM clock unavailable"}
-    nominal = sms * mhz * 1e6 * 64 / 1e12
-    return {"sms": sms, "sm_max_mhz": mhz, "imad_per_clock_per_sm": 64, "T_IMAD_s": round(nominal, 2),
-            "frac_of_nominal": round(achieved_tops / nominal, 4)}
-
-
-def imad_peak(ctx):
-    """Probe the integer pipe; return (probes, peak) in 10^12 IMAD/s (a wide MAC = 2 IMAD)."""
-    pr = {"carry_chain": ctx.imad_probe(0), "mad_lo": ctx.imad_probe(1), "mad_hi": ctx.imad_probe(2),
-          "mad_wide_as_2": ctx.imad_probe(3)}
-    pair = 1.0 / (1.0 / pr["mad_lo"] + 1.0 / pr["mad_hi"])  # wide MACs/s as lo + hi
-    wide = pr["mad_wide_as_2"] / 2.0  # wide MACs/s as mad.wide
-    peak = 2.0 * max(pair, wide)
-    return {k: round(v, 3) for k, v in pr.items()}, peak
+        mhz = float(out[0]) if out else mhz
+    except Exception:  # noqa: BLE001 -- no nvidia-smi: the maximum clock of this GPU
+        pass
+    return {k: round(v, 3) for k, v in pr.items()}, ctx.num_sms() * mhz * 1e6 * 64 / 1e12
 
 
 def run_gpu_msm_sweep(ctx, args, flush, sizes=(16, 17, 18, 19, 20, 21, 22)) -> dict:

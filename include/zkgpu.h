@@ -89,8 +89,9 @@ int zk_timer_stop(zk_ctx *ctx, double *ms);
 int zk_msm_last_stats(zk_ctx *ctx, uint64_t *entries, uint32_t *window_bits, uint32_t *windows);
 /* Measured throughput of the 32-bit integer multiply-add pipe, in 10^12 IMAD instructions
  * per second: probe mode 0 = carry chains shaped like a Montgomery row (mad.lo.cc /
- * madc.hi.cc), 1 = independent mad.lo.u32, 2 = independent mad.hi.u32; zk_imad_peak is
- * the largest of the three (the roofline denominator of the IMAD-bound kernels). */
+ * madc.hi.cc), 1 = independent mad.lo.u32, 2 = independent mad.hi.u32, 3 = mad.wide.u32 of
+ * factors that do not change, counted as two (above the rate with changing ones);
+ * zk_imad_peak is the largest of the four. */
 int zk_imad_probe(zk_ctx *ctx, int mode, double *tera_imad_per_s);
 int zk_imad_peak(zk_ctx *ctx, double *tera_imad_per_s);
 
@@ -310,8 +311,9 @@ int zk_host_g2_add(const uint8_t p[128], const uint8_t q[128], uint8_t out[128])
  * ceil(log2 n) is log_n (the reference's fixed rule is max(4, min(16, bitlen(n) - 2)),
  * runtime/kernels/cpu/kernels.py:553-571; this library's default is a measured table per
  * size). NTT: radix bits of each pass for 2^log_n (1..4 passes of 1..11 bits summing
- * to log_n; default: the fewest passes, as equal as possible). zk_tune_get_* report the
- * effective choice. zk_autotune_msm / zk_autotune_ntt time the built-in choice and the
+ * to log_n; default: the fewest passes, as equal as possible, and two for 2^9 .. 2^11 in
+ * launches of fewer than 2^18 elements). zk_tune_get_* report the effective choice (of a
+ * single MSM; of a transform in a larger launch). zk_autotune_msm / zk_autotune_ntt time the built-in choice and the
  * candidates on the device and keep a candidate only if it beats the built-in choice by
  * more than 3% (else the entry stays 0; best_ms: the kept choice's time); zk_autotune_save / _load write and read the
  * tables as JSON ({"msm_window": {"20": 17}, "ntt_split": {"20": [10, 10]}}). Tuning

@@ -55,9 +55,9 @@ __device__ __forceinline__ fq2 c_dbl(const fq2& a) { return {c_dbl(a.c0), c_dbl(
 __device__ __forceinline__ fq2 c_neg(const fq2& a) { return {c_neg(a.c0), c_neg(a.c1)}; }
 // (a0 + a1 u)(b0 + b1 u) = (a0 b0 - a1 b1) + (a0 b1 + a1 b0) u, Karatsuba with lazy reduction: the u
 // coefficient is (a0 + a1)(b0 + b1) - a0 b0 - a1 b1, 3 unreduced 512-bit products and 2 reductions.
-// Measured with add-carry products: G2 MSM lazy / 3 full products 2.03 / 2.45 ms at 2^16, 12.71 / 13.35
-// ms at 2^20; accumulation at 2^20 with a0 b0 - a1 b1, a0 b1 + a1 b0 (4 products, 2 reductions) / 3 full
-// products 12.1 / 10.5 ms.
+// Measured, G2 MSM, lazy / 3 full products: 2^16 1.13 / 1.27 ms (accumulation 0.64 / 0.77), 2^18 3.16 /
+// 3.46, 500000 points 5.02 / 5.52; a0 b0 - a1 b1, a0 b1 + a1 b0 (4 products, 2 reductions) was 15% slower
+// than 3 full products in the accumulation when it was measured, with add-carry chains.
 __device__ __forceinline__ fq2 c_mul(const fq2& a, const fq2& b) {
     const fe_pair r = fe2_mul_lazy_call<FqP>(a.c0, a.c1, b.c0, b.c1);
     return {r.c0, r.c1};
@@ -90,15 +90,12 @@ __device__ __forceinline__ c_pair<fq2> c_mul2(const fq2& a, const fq2& b, const 
 }
 
 // Pairs with squares, {a^2, b^2} and {a^2, c d}: over Fq a square has its own product form
-// (field.cuh) when the separated forms are on; over Fq2 a square takes 2 Fq products
-// instead of 3. c_mul_sub(a, b, c, d) = a b - c d, one reduction over Fq.
+// (field.cuh); over Fq2 a square takes 2 Fq products instead of 3. c_mul_sub(a, b, c, d) = a b - c d, one reduction over Fq.
 __device__ __forceinline__ c_pair<fe> c_sqr2(const fe& a, const fe& b) {
-    if constexpr (use_sos<FqP>()) return {c_sqr(a), c_sqr(b)};
-    else return c_mul2(a, a, b, b);
+    return {c_sqr(a), c_sqr(b)};
 }
 __device__ __forceinline__ c_pair<fe> c_sqr_mul(const fe& a, const fe& c, const fe& d) {
-    if constexpr (use_sos<FqP>()) return {c_sqr(a), c_mul(c, d)};
-    else return c_mul2(a, a, c, d);
+    return {c_sqr(a), c_mul(c, d)};
 }
 __device__ __forceinline__ fq2 c_mul_sub(const fq2& a, const fq2& b, const fq2& c, const fq2& d) {
     return c_sub(c_mul(a, b), c_mul(c, d));
@@ -475,19 +472,20 @@ __device__ __forceinline__ T cta_quad_sum(uint32_t terms, Get&& get, XyzzT<T>* r
 #ifndef ZK_ACC_MINB
 #define ZK_ACC_MINB 4
 #endif
+// G2: 1 takes the registers it wants (2 CTAs per SM), 3 spill: 2^16 1.13 -> 1.25 ms, 2^18 3.16 -> 3.53.
 #ifndef ZK_ACC_MINB_G2
 #define ZK_ACC_MINB_G2 1
 #endif
 // Threads of the CTA that sums one long bucket's pieces (quads of lanes sum strided pieces, then a
 // tree of the quads). G1 runs 128 threads with four CTAs per SM (a grid of as many): huge buckets
 // are summed in chunks by many CTAs, so the CTA size serves the long buckets of small pipelines,
-// whose few pieces leave most of a wide CTA idle (with one lane a point, 128 against 256 threads:
-// single MSMs 2^14 / 2^16 0.466 / 0.713 against 0.476 / 0.758 ms).
+// whose few pieces leave most of a wide CTA idle (128 threads against 256 at two CTAs per SM: within
+// 1% up to 2^18, 64 instances of 2^10 .. 2^20 27.95 / 28.0 ms, witness-like 2^19 1.16 / 1.12).
 #ifndef ZK_FIXUP_LONG_G1
 #define ZK_FIXUP_LONG_G1 128
 #endif
 // Minimum resident 128-thread CTAs per SM asked of the G1 merge and fixup kernels (G2 keeps
-// 1: its points need the registers).
+// 1: its points need the registers). 1 / 4: 2^20 2.89 / 2.89 ms, 64 instances 27.95 / 27.83.
 #ifndef ZK_RED_MINB
 #define ZK_RED_MINB 1
 #endif

@@ -953,7 +953,7 @@ __device__ __forceinline__ fe fe_sqr(const fe& a) {
     else return fe_mul<F>(a, a);
 }
 
-// a b - c d, and a b + c d (inputs in the field's representation)
+// a b - c d (inputs in the field's representation)
 template <class F>
 __device__ __forceinline__ fe fe_mul_sub(const fe& a, const fe& b, const fe& c, const fe& d) {
     if constexpr (use_sos<F>()) return fe_mul_sub_sos_call<F>(a, b, c, d);

@@ -64,9 +64,13 @@ static constexpr uint32_t kNone = 0xffffffffu;
 #define ZK_MSM_BLOCKG 8
 #endif
 #ifndef ZK_MSM_GROUP
-#define ZK_MSM_GROUP 4  // measured at 2^20 / 2^22: merge 0.73 / 1.36 ms with 16, 0.48 / 1.02 ms with 4
+#define ZK_MSM_GROUP 4  // whole MSM of 2^21 / 2^22 points: 5.53 / 10.45 ms with 4, 5.65 / 10.51 with 8
 #endif
-static constexpr uint32_t kSegment = ZK_MSM_SEGMENT;  // entries per thread in the first accumulation round
+// Entries per thread in the first accumulation round. With 24 / 32 / 48 / 64 (the shorter ones of small
+// pipelines are halves of it), ms: 2^14 witness-like 0.264 / 0.232 / 0.265 / 0.232, 2^18 witness-like 0.730
+// / 0.748 / 0.871 / 0.744, 2^20 2.91 / 2.89 / 2.87 / 2.89, 2^22 10.51 / 10.45 / 10.36 / 10.33, 64 instances of
+// 2^10 .. 2^20 28.2 / 27.95 / 27.7 / 27.6.
+static constexpr uint32_t kSegment = ZK_MSM_SEGMENT;
 static constexpr uint32_t kMinSegment = 4;            // ... at least, in small pipelines
 static constexpr uint32_t kFirstGroup = 2;            // units merged per thread in the first merge round
 static constexpr uint32_t kGroup = ZK_MSM_GROUP;      // units merged per thread in later rounds
@@ -938,7 +942,7 @@ __device__ __forceinline__ uint32_t bucket_of(const uint32_t* __restrict__ row_p
 // Unit u: the CSR entries [u seg, (u + 1) seg) (M = total entries), bucket by bucket.
 //
 // What bounds the accumulation: the wide multiply-adds of the mixed addition, 1160 a G1 entry
-// (7 products, a product pair with one reduction, two squares) = 1.93 ms at 2^20 (16.8 M entries).
+// (6 products, a product pair with one reduction, two squares) = 1.93 ms at 2^20 (16.8 M entries).
 // Measured there: 2.18 ms with the formula's products inlined in this one loop (2.37 ms
 // through the called product), the entry read one ahead 2.17 ms; prefetching its point too
 // measured the same, 3 or 5 CTAs per SM instead of 4: 2.26 / 2.17 ms. G2 2^16: 0.685 -> 0.672 ms.
@@ -1050,8 +1054,8 @@ __global__ void __launch_bounds__(128, C::kRedMinBlocks) msm_merge_kernel(const 
 // began before the segment). One thread per bucket adds up to sh.fixmax + 1 pieces; longer
 // buckets are listed for msm_fixup_long_kernel (a CTA each).
 #ifndef ZK_FIXUP_DENSITY
-// measured on GB300: 2^20 plain (32 entries per bucket) fixup 0.32 vs rounds 0.48 ms; 2^20 GLV
-// (64) fixup 0.27 vs rounds 0.48 ms; 2^22 GLV (256) rounds 1.0 vs fixup 6.8 ms
+// Whole MSM with 48 / 96 / 200: 2^17 (64 entries per bucket) 849 / 675 / 675 us, 2^20 (64) 3.08 / 2.89 / 2.89
+// ms, 2^21 (128) 5.53 / 5.53 / 5.44; with one lane a point the fixup at 2^22 (256) took 6.8 ms, rounds 1.0.
 #define ZK_FIXUP_DENSITY 96
 #endif
 static constexpr uint64_t kFixupDensity = ZK_FIXUP_DENSITY;  // CSR entries per bucket up to which the fixup is used
@@ -1362,9 +1366,9 @@ __global__ void __launch_bounds__(128) msm_targets_kernel(const typename C::P* _
 // All pipelines of a batch, after their sorts, in ONE launch: the queue lists (pipeline,
 // stage) entries, each owning one item per CTA-sized piece of the stage -- 128 accumulation
 // units (entry ranges of one instance's window sets), 128 merge units, 128 buckets of the
-// fixup, a share of the long-bucket list, 128 level-1 / level-2 blocks, one (set, target,
-// part) or one (set, target) merge. Entries go stage by stage (largest pipelines first within
-// a stage); an item waits until its pipeline's previous stage has published all its items.
+// fixup, a share of the long-bucket list, 128 blocks, one line or one target of a set. Entries go
+// stage by stage (largest pipelines first within a stage); an item waits until its pipeline's
+// previous stage has published all its items.
 // The same ticket discipline as the NTT queue keeps it deadlock-free for any number of
 // resident CTAs (the earliest unfinished item never waits), and every wait is bounded.
 enum : uint32_t { kQAcc = 0, kQMerge, kQFix, kQFixLong, kQBlk, kQLines, kQTgt };

@@ -32,15 +32,14 @@ namespace zk {
 
 static constexpr int kNttThreads = 256;
 #ifndef ZK_NTT_MINB
-// resident CTAs per SM the single-transform pass kernel is compiled for: 2 (up to 128
-// registers); 3 leave 85, where the radix-4 steps spill ~80 bytes (with add-carry products
-// 2^20 0.282 / 0.292 ms, 2^12 0.022 / 0.023 ms) and radix-8 more
+// resident CTAs per SM the pass kernel is compiled for: 2 (up to 128 registers); 3 leave 85, where
+// the steps spill: wide form 2^18 51 -> 71 us, 2^20 181 -> 257, 2^22 718 -> 831; narrow 2^12 .. 2^17 the
+// same within 2%
 #define ZK_NTT_MINB 2
 #endif
 #ifndef ZK_NTT_BATCH_MINB
-// ... and the batch and queue kernels: their many small tiles (256-element tiles of 128
-// active threads) want the third CTA per SM in the narrow form (64 coset NTTs of 2^10..2^20 with
-// add-carry products: 2.87 ms at 3, 3.00 ms at 2)
+// ... and the narrow batch kernel and the queue kernel: their many small tiles (256-element tiles
+// of 128 active threads) want the third CTA per SM (64 coset NTTs of 2^10 .. 2^14 95.5 us at 3, 97.3 at 2)
 #define ZK_NTT_BATCH_MINB 3
 #endif
 static constexpr int kMaxLogR = 11;       // 2048 elements * 32 B = 64 KB of shared memory

@@ -58,7 +58,8 @@ static void get_split(const Ctx* c, uint32_t log_n, uint32_t* npass, uint32_t bi
         *npass = np;
         return;
     }
-    // the built-in split (fewest passes of <= 11 bits, as equal as possible)
+    // the built-in split (fewest passes of <= 11 bits, as equal as possible; small launches of 2^9 .. 2^11
+    // elements take two, see split_passes)
     if (log_n == 0) {
         *npass = 0;
         return;
