@@ -36,19 +36,22 @@ class HostPool {
 
     // run() in which the calling thread first executes own(): own() may take tasks itself
     // through run_one() (the same ticket, so in the same index order as the workers), e.g.
-    // to consume results in order and compute whichever no worker has taken yet.
+    // to consume results in order and compute whichever no worker has taken yet. Returns true;
+    // if_free: returns false with nothing done when another run is in progress (for a few tasks:
+    // by the time that one is over, the calling thread would be through with them).
     template <class Own>
-    void run_with(size_t count, const std::function<void(size_t)>& fn, Own&& own, size_t max_helpers = ~size_t(0)) {
-        if (count > kMaxTasks) {
+    bool run_with(size_t count, const std::function<void(size_t)>& fn, Own&& own, size_t max_helpers = ~size_t(0),
+                  bool if_free = false) {
+        if (count == 0 || count > kMaxTasks) {
             for (size_t i = 0; i < count; i++) fn(i);
             own();
-            return;
+            return true;
         }
-        if (count == 0) {
-            own();
-            return;
+        std::unique_lock<std::mutex> serial(run_mu_, std::try_to_lock);
+        if (!serial.owns_lock()) {
+            if (if_free) return false;
+            serial.lock();
         }
-        std::lock_guard<std::mutex> serial(run_mu_);
         gen_ = (gen_ + 1) & 0xffffu;
         fn_ = &fn;
         done_.store(0, std::memory_order_relaxed);
@@ -78,6 +81,7 @@ class HostPool {
         while (done_.load(std::memory_order_acquire) < count)
             done_cv_.wait_for(g, std::chrono::milliseconds(1),
                               [&] { return done_.load(std::memory_order_acquire) >= count; });
+        return true;
     }
 
     // Wakes up to `helpers` workers ahead of a run that this thread is about to start: they wait awake
@@ -86,20 +90,26 @@ class HostPool {
     class Expect {
        public:
         Expect(HostPool& pool, size_t helpers, std::chrono::microseconds limit) : pool_(pool) {
+            // one at a time: with several callers about, the workers that one of them woke serve all
+            size_t none = 0;
+            if (helpers == 0 || !pool_.expected_.compare_exchange_strong(none, helpers, std::memory_order_acq_rel)) return;
+            mine_ = true;
             pool_.until_.store((Clock::now() + limit).time_since_epoch().count(), std::memory_order_release);
-            pool_.expecting_.fetch_add(1, std::memory_order_acq_rel);
             {
                 std::lock_guard<std::mutex> g(pool_.mu_);
                 pool_.wake_++;
             }
             for (size_t i = 0; i < std::min(helpers, pool_.workers_); i++) pool_.cv_.notify_one();
         }
-        ~Expect() { pool_.expecting_.fetch_sub(1, std::memory_order_acq_rel); }
+        ~Expect() {
+            if (mine_) pool_.expected_.store(0, std::memory_order_release);
+        }
         Expect(const Expect&) = delete;
         Expect& operator=(const Expect&) = delete;
 
        private:
         HostPool& pool_;
+        bool mine_ = false;
     };
 
     // Workers that wait awake.
@@ -145,10 +155,11 @@ class HostPool {
                 if (pending_.fetch_sub(1, std::memory_order_acq_rel) > 0) cv_.notify_one();
             work();
             // the run that an Expect announces: its wake-up takes 10 - 20 us, as long as two or three window sums
-            awake_.fetch_add(1, std::memory_order_acq_rel);
-            while (expecting_.load(std::memory_order_acquire) != 0 &&
-                   Clock::now().time_since_epoch().count() < until_.load(std::memory_order_acquire))
-                if (!run_one()) std::this_thread::yield();
+            // (twice as many may stay: some of those asked for may still be on their way to sleep)
+            if (awake_.fetch_add(1, std::memory_order_acq_rel) < 2 * expected_.load(std::memory_order_acquire))
+                while (expected_.load(std::memory_order_acquire) != 0 &&
+                       Clock::now().time_since_epoch().count() < until_.load(std::memory_order_acquire))
+                    if (!run_one()) std::this_thread::yield();
             awake_.fetch_sub(1, std::memory_order_acq_rel);
         }
     }
@@ -172,9 +183,9 @@ class HostPool {
     std::atomic<int64_t> pending_{0};  // wake-ups the woken workers still have to pass on
     alignas(128) std::atomic<uint64_t> ticket_{0};
     alignas(128) std::atomic<size_t> done_{0};
-    alignas(128) std::atomic<uint32_t> expecting_{0};  // Expects alive
-    std::atomic<Clock::rep> until_{0};                 // when workers that wait for one go to sleep
-    alignas(128) std::atomic<size_t> awake_{0};        // workers that do
+    alignas(128) std::atomic<size_t> expected_{0};  // workers that the Expect alive asked for
+    std::atomic<Clock::rep> until_{0};              // when they go to sleep all the same
+    alignas(128) std::atomic<size_t> awake_{0};     // workers that wait awake
 };
 
 }  // namespace zk

@@ -2152,9 +2152,9 @@ static int combine_all(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, uint8_t* o
         auto own = [&] {
             horner_out<C>(p, [&](uint32_t w) -> const zkh::XyzzT<H>& {
                 const uint32_t t = W - 1 - w;
-                // a window that a worker is on comes sooner than this thread would be through another one
+                // a window that an awake worker is on comes sooner than this thread would be through another
                 while (!ready[t].load(std::memory_order_acquire))
-                    if (pool.claimed(t) || !pool.run_one()) std::this_thread::yield();
+                    if ((early && pool.claimed(t)) || !pool.run_one()) std::this_thread::yield();
                 return sums[t];
             }, out_xy + kOut * o, out_is_inf + o);
         };
@@ -2163,7 +2163,10 @@ static int combine_all(Ctx* c, const std::vector<MsmPipeT<C>>& pipes, uint8_t* o
         if (wait)
             if (const int rc = wait(); rc != ZK_OK) return rc;
         t0 = std::chrono::steady_clock::now();
-        pool.run_with(W, task, own, kCombineHelpers);
+        if (!pool.run_with(W, task, own, kCombineHelpers, true)) {  // another caller has the pool
+            for (uint32_t t = 0; t < W; t++) task(t);
+            own();
+        }
     } else {
         if (wait)
             if (const int rc = wait(); rc != ZK_OK) return rc;

@@ -76,6 +76,22 @@ int main() {
         b.join();
         check("tasks beside another run", mine.once());
     }
+    {  // a busy pool is not waited for, and one Expect at a time wakes workers
+        Tasks outer(4), inner(3);
+        bool refused = false, owned = false;
+        pool.run_with(4, outer.fn(), [&] {
+            std::thread([&] { refused = !pool.run_with(3, inner.fn(), [&] { owned = true; }, 4, true); }).join();
+        });
+        check("a busy pool was not refused", refused && !owned && inner.ran[0] + inner.ran[1] + inner.ran[2] == 0);
+        check("tasks of the outer run", outer.once());
+        check("a free pool was refused", pool.run_with(3, inner.fn(), [&] { owned = true; }, 4, true) && owned && inner.once());
+        zk::HostPool::Expect a(pool, 1, us(5000000));
+        check("no worker woke", workers == 0 || settles([&] { return pool.awake() > 0; }));
+        zk::HostPool::Expect b(pool, 4, us(5000000));
+        std::this_thread::sleep_for(us(2000));
+        check("a second Expect woke workers", pool.awake() <= 2);
+    }
+    check("workers stay awake", settles([&] { return pool.awake() == 0; }));
     // mixed runs from several threads
     std::vector<std::thread> ts;
     for (int k = 0; k < 6; k++)
@@ -85,7 +101,7 @@ int main() {
                 if (k % 2) {
                     zk::HostPool::Expect e(pool, 4, us(i % 3 * 50));
                     std::this_thread::sleep_for(us(i % 5 * 20));
-                    pool.run_with(t.n, t.fn(), [] {}, 4);
+                    if (i % 2 || !pool.run_with(t.n, t.fn(), [] {}, 4, true)) pool.run_with(t.n, t.fn(), [] {}, 4);
                 } else {
                     pool.run(t.n, t.fn());
                 }
