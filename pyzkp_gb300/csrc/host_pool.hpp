@@ -95,11 +95,17 @@ class HostPool {
             if (helpers == 0 || !pool_.expected_.compare_exchange_strong(none, helpers, std::memory_order_acq_rel)) return;
             mine_ = true;
             pool_.until_.store((Clock::now() + limit).time_since_epoch().count(), std::memory_order_release);
+            helpers = std::min(helpers, pool_.workers_);
+            const size_t first = std::min(helpers, kFanout);
+            const int64_t rest = (int64_t)(helpers - first);  // passed on, beside what a run has left to pass on
+            int64_t p = pool_.pending_.load(std::memory_order_relaxed);
+            while (p < rest && !pool_.pending_.compare_exchange_weak(p, rest, std::memory_order_acq_rel)) {
+            }
             {
                 std::lock_guard<std::mutex> g(pool_.mu_);
                 pool_.wake_++;
             }
-            for (size_t i = 0; i < std::min(helpers, pool_.workers_); i++) pool_.cv_.notify_one();
+            for (size_t i = 0; i < first; i++) pool_.cv_.notify_one();
         }
         ~Expect() {
             if (mine_) pool_.expected_.store(0, std::memory_order_release);
