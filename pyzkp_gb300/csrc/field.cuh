@@ -831,16 +831,24 @@ __host__ __device__ __forceinline__ fe sos_reduce_2p(const fe& t) {
     return r;
 }
 
-// The product rows for any 256-bit a and b: a below 2^256 - 2p < 3.3p first.
+// A vector element of a caller as the first factor of a product: below 2p as it is (its top limb
+// tells, and in earnest no thread of a warp goes on), else less 2p, below 2^256 - 2p < 3.3p.
+template <class F>
+__host__ __device__ __forceinline__ fe fe_first_factor(const fe& a) {
+    if (a.v[7] < p2_limb<F>(7)) return a;
+    return sos_reduce_2p<F>(a);
+}
+
+// The product rows for any 256-bit a and b.
 template <class F>
 __host__ __device__ __forceinline__ fe mul_rows_any(const fe& a, const fe& b) {
-    return mul_rows<F>(sos_reduce_2p<F>(a), b);
+    return mul_rows<F>(fe_first_factor<F>(a), b);
 }
 
 // fe_mul for any 256-bit a and b (vectors of a caller)
 template <class F>
 __device__ __forceinline__ fe fe_mul_any(const fe& a, const fe& b) {
-    return fe_mul<F>(sos_reduce_2p<F>(a), b);
+    return fe_mul<F>(fe_first_factor<F>(a), b);
 }
 
 // a^2 * 2^-256 mod p in [0, 2p) for a in [0, 2p)

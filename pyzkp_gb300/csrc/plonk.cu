@@ -155,7 +155,7 @@ __global__ void plonk_quotient_kernel(QuotientIn in, QuotientK K, size_t m, uint
     x = fe_mul<FrQ>(K.shift, x);
     fe un = fe_mul<FrQ>(fe_mul<FrQ>(fe_ldg(pw + 32 + lane), fe_ldg(pw + 128 + glo)), fe_ldg(pw + 192 + H + ghi));
     // the vectors of a caller that are first factors of products (see fe_mul)
-    auto first = [](const fe* v) { return sos_reduce_2p<FrQ>(fe_ldg(v)); };
+    auto first = [](const fe* v) { return fe_first_factor<FrQ>(fe_ldg(v)); };
     for (size_t i = i0, k = 0; k < chunk && i < m; k++, i += 32) {
         const fe a = first(in.v[0] + i), b = first(in.v[1] + i), c = first(in.v[2] + i);
         const fe z = first(in.v[3] + i);
